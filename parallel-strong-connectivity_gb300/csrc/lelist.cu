@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "engines.cuh"
+#include "levels.cuh"
 #include "scan.cuh"
 
 namespace psc {
@@ -213,10 +214,32 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
   uint64_t nf = 1, nf_edges = 0;
   bool pull = false;
   uint32_t level = 0;
+  const bool cluster = !(g->m >> 40) && levels_ready<BfsClaim>(g->device);
   while (nf > 0) {
+    const bool want_pull = (nf + nf_edges) >= threshold;
+    // narrow push levels run back to back on one cluster (levels.cuh)
+    if (cluster && !want_pull && !pull && nf <= kLvMaxFront && nf_edges <= kLvMaxEdges) {
+      PSC_TRY(zero_counters(g));
+      {
+        ProfScope ps(g, F_LE);
+        PSC_TRY(launch_levels(LvArgs{g->off, g->E, qa, nf, qb, threshold, level, g->ctr},
+                              BfsClaim{dist}, g->stream));
+      }
+      PSC_TRY(read_counters(g));
+      const Counters& c = g->hctr[0];
+      if (c.aux0) {  // else the first level was too wide: a round of the whole grid
+        level += (uint32_t)c.aux0;
+        if (level > n + 1) return PSC_ERR_ITER_LIMIT;
+        if (g->profiling) g->prof[F_LE].bytes += 24.0 * c.expanded + 8.0 * c.edges;
+        std::swap(qa, qb);
+        swap_bufs(g, B_QA, B_QB);
+        nf = c.next;
+        nf_edges = c.next_edges;
+        continue;
+      }
+    }
     level++;
     if (level > n + 1) return PSC_ERR_ITER_LIMIT;
-    const bool want_pull = (nf + nf_edges) >= threshold;
     if (want_pull && !pull) {
       PSC_CUDA(cudaMemsetAsync(fa, 0, nwords * 4, g->stream));
       k_bfs_q2b<<<grid_for(g, nf, 256), 256, 0, g->stream>>>(qa, nf, fa);

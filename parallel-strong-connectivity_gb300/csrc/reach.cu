@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "engines.cuh"
+#include "levels.cuh"
 
 namespace psc {
 
@@ -1616,10 +1617,26 @@ extern "C" int psc_reach_noalloc(const uint64_t* d_off, const uint32_t* d_E,
   uint64_t nf = 1, nf_edges = 0;
   bool pull = false;
   uint32_t r = 0;
+  const bool cluster = levels_ready<ReachClaim>(dev);
   while (nf > 0) {
+    const bool want_pull = (nf + nf_edges) >= threshold;
+    // narrow push rounds run back to back on one cluster (levels.cuh)
+    if (cluster && !want_pull && !pull && nf <= kLvMaxFront && nf_edges <= kLvMaxEdges) {
+      PSC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), s));
+      PSC_TRY(launch_levels(LvArgs{A_off, A_E, qa, nf, qb, threshold, r, ctr}, ReachClaim{vis}, s));
+      PSC_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+      PSC_CUDA(cudaStreamSynchronize(s));
+      if (hc.aux0) {  // else the first round was too wide: one of the whole grid
+        r += (uint32_t)hc.aux0;
+        if (r > n + 2) return PSC_ERR_ITER_LIMIT;
+        std::swap(qa, qb);
+        nf = hc.next;
+        nf_edges = hc.next_edges;
+        continue;
+      }
+    }
     r++;
     if (r > n + 2) return PSC_ERR_ITER_LIMIT;
-    const bool want_pull = (nf + nf_edges) >= threshold;
     if (want_pull && !pull) {
       PSC_CUDA(cudaMemsetAsync(fa, 0, nwords * 4, s));
       k_queue_to_bitmap<<<na_grid(nd.num_sms, nf, 256), 256, 0, s>>>(qa, nf, fa);
