@@ -474,6 +474,8 @@ static int scc_batch_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t
     const auto sched = batch_schedule(cbase, G, p->beta);
     size_t words = 0;
     for (const auto& ws : sched) words += 3 * ws.size() + 1;
+    const size_t head_at = words;  // per round: first word, windows (k_ms_batches)
+    words += 2 * sched.size();
     uint64_t* sched_d;
     PSC_TRY(ensure_t(g, B_SCHED, words + 1, &sched_d));
     std::vector<uint64_t> hs(words);
@@ -495,6 +497,8 @@ static int scc_batch_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t
           acc += ws[a].len;
         }
         wpre[c] = acc;
+        hs[head_at + 2 * j] = o;
+        hs[head_at + 2 * j + 1] = c;
         o += 3 * c + 1;
       }
     }
@@ -503,7 +507,30 @@ static int scc_batch_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t
     PSC_TRY(ensure_t(g, B_FRONT, np + 1, &front));
     PSC_TRY(ensure_t(g, B_FLAB, np + 1, &flab));
     uint64_t in_ne = 1, out_ne = 1;
+    const bool resident = ms_run_ready(g);
     for (size_t j = 0; j < sched.size(); j++) {
+      if (resident) {
+        // rounds back to back in one launch, up to one that it leaves to the
+        // steps below
+        MsRun run;
+        run.centres = centres;
+        run.sched = sched_d;
+        run.heads = sched_d + head_at;
+        run.rounds = sched.size();
+        run.round = j;
+        run.lo = A.lo;
+        run.fb = A.fb;
+        run.front = front;
+        run.win = flab;
+        run.vgc_max = kBatchVgcMax;
+        run.ne[0] = out_ne;
+        run.ne[1] = in_ne;
+        PSC_TRY(ms_run(g, labels, p, &run, hs[at[j] + 3 * sched[j].size()]));
+        out_ne = run.ne[0];
+        in_ne = run.ne[1];
+        if (run.done) break;
+        j = run.round;
+      }
       const uint32_t c = (uint32_t)sched[j].size();
       const uint32_t* wg = (const uint32_t*)(sched_d + at[j]);
       const uint64_t* wstart = sched_d + at[j] + c;

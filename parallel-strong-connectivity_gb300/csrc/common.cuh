@@ -75,7 +75,8 @@ struct Counters {
   unsigned long long pad[2];
 };
 // sets 0-1: search sides; 2-3: staging; 4-19: the rounds of a chained VGC
-// sequence (reach.cu), two sides per round
+// sequence (reach.cu), two sides per round, or the sub-rounds and the state of
+// the resident multi-search (multisearch.cu)
 constexpr int kCounterSets = 20;
 
 // ---------------------------------------------------------------------------
@@ -185,6 +186,9 @@ enum Buf : int {
   B_FLAB,         // u32 labels of a batch's pivots
   B_SCHED,        // window schedule of a batch's prefix-doubling rounds
   B_SCANBITS,     // u32[n/32] selection bits of scan_emit_flags
+  B_TF2,          // second set of label tables (k_ms_batches)
+  B_TB2,
+  B_BLOCKS,       // u32 per block of a resident grid
   B_DEAD,         // u32[2][n/32 + 1] vertices with no in-edge, then no out-edge
   B_COUNT
 };
@@ -258,6 +262,40 @@ inline unsigned grid_for(psc_graph_s* g, uint64_t items, unsigned block, unsigne
 // ---------------------------------------------------------------------------
 // Device helpers
 // ---------------------------------------------------------------------------
+// Barrier of a grid whose blocks are all resident (cooperative launch):
+// *arrive counts arrivals, *target what it has to reach (one per thread,
+// starting at 0).  The wait is bounded: past kGridSpin polls, or once another
+// block has given up, *failed is set and false is returned to every thread of
+// the block, which then leaves the kernel.
+constexpr uint32_t kGridSpin = 1u << 23;
+
+__device__ __forceinline__ bool grid_barrier(uint32_t* arrive, uint32_t* failed,
+                                             uint32_t& target) {
+  __shared__ uint32_t s_ok;
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    uint32_t seen, bad = 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrive) : "memory");
+    uint32_t spin = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
+      if ((int32_t)(seen - target) >= 0) break;
+      if ((++spin & 1023u) == 0) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(bad) : "l"(failed) : "memory");
+        if (bad || spin >= kGridSpin) {
+          atomicExch(failed, 1u);
+          bad = 1;
+          break;
+        }
+      }
+    }
+    s_ok = !bad;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 // Rejects a CSR whose offsets do not run from 0 to m without decreasing or

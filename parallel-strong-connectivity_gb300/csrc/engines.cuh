@@ -18,9 +18,6 @@ int batch_attach(psc_graph_s* g, const uint64_t* vbase, uint32_t num_graphs, boo
 int call_begin(psc_graph_s* g);
 int call_end(psc_graph_s* g);
 
-// g->max_deg (largest out- / in-degree), computed once per handle.
-int ensure_max_degrees(psc_graph_s* g);
-
 // Builds in_off/in_E from off/E on the device (in-lists sorted by source).
 int build_transpose(psc_graph_s* g);
 // Replaces off/E by their symmetrisation on the device (both directions,
@@ -56,20 +53,34 @@ struct MsResult {
   uint64_t cap = 0;  // table capacity (power of two)
   uint64_t ne = 0;   // entries
 };
-// Asynchronous start of a batch (MsAsync given): the pivot count is read on
-// the device at *nf_dev (n_front is only its upper bound), so the seeds and
-// the first sub-round are launched without waiting for the compaction that
-// wrote front.  On return n_front holds the pivot count.  (The partition
-// cannot start early: later sub-rounds test subproblems on the labels it
-// writes.)
-struct MsAsync {
-  const unsigned long long* nf_dev = nullptr;
-  uint64_t n_front = 0;
-};
 int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t label_offset,
             const uint64_t* labels, const psc_params_t* p, const uint64_t prev_ne[2],
-            MsResult out[2], const uint32_t* front_labels = nullptr, uint64_t vgc_max = 0,
-            MsAsync* async = nullptr);
+            MsResult out[2], const uint32_t* front_labels = nullptr, uint64_t vgc_max = 0);
+
+// Prefix-doubling batches back to back in one resident launch (k_ms_batches):
+// from the state in *run on, until all centres are done (run->done) or a batch
+// needs more table than the launch has, which is then left to ms_pair
+// untouched (its labels are written only by its partition).
+struct MsRun {
+  const uint32_t* centres = nullptr;
+  uint64_t n_remaining = 0;  // plain: centres in all
+  uint64_t cur = 0, step = 1;
+  uint64_t label_offset = 0;
+  // batch of graphs: the windows of every round (see scc_batch_phases)
+  const uint64_t* sched = nullptr;
+  const uint64_t* heads = nullptr;  // per round: first word in sched, windows
+  uint64_t rounds = 0, round = 0;
+  uint64_t *lo = nullptr, *fb = nullptr;
+  uint32_t *front = nullptr, *win = nullptr;
+  uint64_t vgc_max = 0;
+  uint64_t ne[2] = {1, 1};  // table sizes of the last batch
+  bool done = false;
+};
+// False when the device cannot hold the launch (the caller then runs every
+// batch through ms_pair).
+bool ms_run_ready(psc_graph_s* g);
+// window: candidates of the first batch.
+int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, uint64_t window);
 
 // Partition of one batch (src/scc.hpp:437-464): (v, l) in both tables left by
 // ms_pair -> labels[v] = max(l | TOP), else max(l).

@@ -29,6 +29,7 @@
 // restart of the whole search (scc.hpp:263-272) with the same fixed point.
 #include <algorithm>
 #include <cstdio>
+#include <mutex>
 
 #include "common.cuh"
 #include "engines.cuh"
@@ -54,9 +55,6 @@ struct MsSide {
   uint32_t* hflag;
   Counters* ctr;
   uint32_t vgc_budget;  // new pairs one VGC local search may insert
-  // when set, the frontier size is read here instead of nin (the first
-  // sub-round of a batch started without waiting for its pivot count)
-  const unsigned long long* nin_dev;
 };
 
 constexpr int kMsHeavyK = 4;  // heavy pairs: edges in flight per lane
@@ -87,8 +85,7 @@ struct MsSrc {
 __global__ void k_ms_seed(const uint32_t* __restrict__ front, uint64_t nf, uint64_t label_offset,
                           const uint32_t* __restrict__ front_labels, unsigned long long* T0,
                           uint64_t mask0, uint64_t* F0, unsigned long long* T1, uint64_t mask1,
-                          uint64_t* F1, const unsigned long long* nf_dev) {
-  if (nf_dev) nf = *nf_dev;
+                          uint64_t* F1) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nf;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t lab = front_labels ? front_labels[i] : (uint32_t)(label_offset + i);
@@ -148,7 +145,7 @@ template <int K, bool DIRECT, bool PF, class Emit>
 __device__ __forceinline__ void ms_expand_claim(WarpExpandSmem& sm, MsSrc& src, uint64_t beg,
                                                 uint32_t deg, const uint64_t* __restrict__ off,
                                                 const uint32_t* __restrict__ E,
-                                                const uint64_t* __restrict__ labels,
+                                                const uint64_t* labels,
                                                 unsigned long long* T, uint64_t mask,
                                                 uint32_t& probes, Emit&& emit) {
   const unsigned lane = lane_id();
@@ -189,7 +186,7 @@ __device__ __forceinline__ void ms_expand_claim(WarpExpandSmem& sm, MsSrc& src, 
       key[k] = kEmpty;
       vb[k] = ve[k] = 0;
       if (w[k] != 0xFFFFFFFFu) {
-        const uint64_t lw = __ldg(&labels[w[k]]);
+        const uint64_t lw = ld_cg(&labels[w[k]]);
         if (PF) {
           vb[k] = __ldg(&off[w[k]]);
           ve[k] = __ldg(&off[w[k] + 1]);
@@ -279,19 +276,13 @@ __device__ __forceinline__ void flush_ms_counters(Counters* c0, Counters* c1,
   }
 }
 
-// Expansion sub-round for up to two sides: 32 pairs per warp step.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, (768 / BLOCK) > 0 ? (768 / BLOCK) : 1)
-    k_ms_expand(MsSide s0, MsSide s1, const uint64_t* __restrict__ labels) {
-  if (s0.nin_dev) s0.nin = *s0.nin_dev;
-  if (s1.nin_dev) s1.nin = *s1.nin_dev;
-  __shared__ WarpExpandSmem sm[BLOCK / 32];
-  __shared__ MsSrc ssrc[BLOCK / 32];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+// Expansion sub-round for up to two sides: 32 pairs per warp step (warp gw of
+// nw, with its own sm and src).
+__device__ __forceinline__ void ms_expand_round(const MsSide& s0, const MsSide& s1,
+                                                const uint64_t* labels, WarpExpandSmem& sm,
+                                                MsSrc& src, uint64_t gw, uint64_t nw) {
+  const unsigned lane = lane_id();
   const uint64_t c0 = (s0.nin + 31) / 32, c1 = (s1.nin + 31) / 32;
-  MsSrc& src = ssrc[wid];
   unsigned long long sc0 = 0, sc1 = 0, rq0 = 0, rq1 = 0, ex0 = 0, ex1 = 0, in0 = 0, in1 = 0;
   uint32_t pr0 = 0, pr1 = 0;
   for (uint64_t c = gw; c < c0 + c1; c += nw) {
@@ -301,11 +292,11 @@ __global__ void __launch_bounds__(BLOCK, (768 / BLOCK) > 0 ? (768 / BLOCK) : 1)
     uint64_t beg = 0, key = 0, sub = 0;
     uint32_t deg = 0;
     if (i < S.nin) {
-      key = S.Fin[i];
+      key = ld_cg(&S.Fin[i]);
       const uint32_t u = (uint32_t)(key >> 32);
       beg = S.off[u];
       uint64_t d = S.off[u + 1] - beg;
-      sub = labels[u];
+      sub = ld_cg(&labels[u]);
       (sd ? ex1 : ex0)++;
       if (d > kHeavyDeg) {
         ms_heavy_push(S, key, d);
@@ -320,7 +311,7 @@ __global__ void __launch_bounds__(BLOCK, (768 / BLOCK) > 0 ? (768 / BLOCK) : 1)
     __syncwarp();
     uint32_t probes = 0;
     ms_expand_claim<kMsExpandK, false, false>(
-        sm[wid], src, beg, deg, S.off, S.E, labels, S.T, S.mask, probes,
+        sm, src, beg, deg, S.off, S.E, labels, S.T, S.mask, probes,
         [&](uint32_t tm, const uint64_t* keys) {
           (sd ? in1 : in0) += __popc(tm);
           warp_append_batch<kMsExpandK>(tm, keys, S.Fout, &S.ctr->next);
@@ -338,6 +329,16 @@ __global__ void __launch_bounds__(BLOCK, (768 / BLOCK) > 0 ? (768 / BLOCK) : 1)
   flush_ms_counters(s0.ctr, s1.ctr, sc0, sc1, rq0, rq1, pr0, pr1, ex0, ex1, in0, in1);
 }
 
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, (768 / BLOCK) > 0 ? (768 / BLOCK) : 1)
+    k_ms_expand(MsSide s0, MsSide s1, const uint64_t* labels) {
+  __shared__ WarpExpandSmem sm[BLOCK / 32];
+  __shared__ MsSrc ssrc[BLOCK / 32];
+  const unsigned wid = threadIdx.x >> 5;
+  ms_expand_round(s0, s1, labels, sm[wid], ssrc[wid],
+                  (uint64_t)blockIdx.x * (BLOCK / 32) + wid, (uint64_t)gridDim.x * (BLOCK / 32));
+}
+
 struct MsQEnt {
   uint64_t beg;
   uint32_t v;
@@ -352,7 +353,7 @@ template <int K, bool ADJ = true>
 __device__ __forceinline__ uint32_t ms_vgc_claim(const uint32_t* w, uint64_t* vb, uint64_t* ve,
                                                  uint64_t sub, uint32_t lab,
                                                  const uint64_t* __restrict__ off,
-                                                 const uint64_t* __restrict__ labels,
+                                                 const uint64_t* labels,
                                                  unsigned long long* T, uint64_t mask,
                                                  uint32_t& probes, bool& failed) {
   uint64_t key[K], old[K], h[K];
@@ -361,7 +362,7 @@ __device__ __forceinline__ uint32_t ms_vgc_claim(const uint32_t* w, uint64_t* vb
     key[k] = kEmpty;
     vb[k] = ve[k] = 0;
     if (w[k] != 0xFFFFFFFFu) {
-      const uint64_t lw = __ldg(&labels[w[k]]);
+      const uint64_t lw = ld_cg(&labels[w[k]]);
       if (ADJ) {
         vb[k] = __ldg(&off[w[k]]);
         ve[k] = __ldg(&off[w[k] + 1]);
@@ -438,29 +439,25 @@ __device__ __forceinline__ void ms_vgc_place(uint32_t tm, const uint32_t* w, con
 // frontier.  Queued vertices with more than tq out-edges and the queue's
 // remainder spill too.  A queued vertex whose expansion hit a failed insert is
 // re-queued as a pair.
-template <int BLOCK, int QCAP>
-__global__ void __launch_bounds__(BLOCK)
-    k_ms_vgc(MsSide s0, MsSide s1, const uint64_t* __restrict__ labels, uint32_t tau) {
-  if (s0.nin_dev) s0.nin = *s0.nin_dev;
-  if (s1.nin_dev) s1.nin = *s1.nin_dev;
-  __shared__ WarpExpandSmem sm[BLOCK / 32];
-  __shared__ MsQEnt sq[BLOCK / 32][QCAP];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+// (warp gw of nw, with its own sm and queue Q; kMsK edges in flight per lane)
+template <int kMsK, int QCAP>
+__device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,
+                                             const uint64_t* labels, uint32_t tau,
+                                             WarpExpandSmem& sm, MsQEnt* Q, uint64_t gw,
+                                             uint64_t nw) {
+  const unsigned lane = lane_id();
   const uint32_t tq = tau < (uint32_t)QCAP ? tau : (uint32_t)QCAP;
-  MsQEnt* Q = sq[wid];
   unsigned long long sc0 = 0, sc1 = 0, rq0 = 0, rq1 = 0, ex0 = 0, ex1 = 0, in0 = 0, in1 = 0;
   uint32_t pr0 = 0, pr1 = 0;
-  if (lane == 0) sm[wid].fail = 0;
+  if (lane == 0) sm.fail = 0;
   __syncwarp();
   for (uint64_t i = gw; i < s0.nin + s1.nin; i += nw) {
     const int sd = i < s0.nin ? 0 : 1;
     const MsSide S = sd ? s1 : s0;
-    const uint64_t key = S.Fin[sd ? i - s0.nin : i];
+    const uint64_t key = ld_cg(&S.Fin[sd ? i - s0.nin : i]);
     const uint32_t u = (uint32_t)(key >> 32);
     const uint32_t lab = (uint32_t)key;
-    const uint64_t sub = labels[u];
+    const uint64_t sub = ld_cg(&labels[u]);
     const uint64_t ub = S.off[u], ue = S.off[u + 1];
     const uint64_t du = ue - ub;
     auto emit = [&](bool take, uint32_t w) {
@@ -534,8 +531,8 @@ __global__ void __launch_bounds__(BLOCK)
         if ((int)lane >= o) incl += t;
       }
       const uint32_t total = __shfl_sync(kFull, incl, 31);
-      sm[wid].excl[lane] = incl - deg;
-      sm[wid].beg[lane] = beg;
+      sm.excl[lane] = incl - deg;
+      sm.beg[lane] = beg;
       __syncwarp();
       for (uint32_t base = 0; base < total; base += 32 * kMsK) {
         uint32_t w[kMsK];
@@ -550,13 +547,13 @@ __global__ void __launch_bounds__(BLOCK)
             int lo = 0, hi = 31;
             while (lo < hi) {
               int mid = (lo + hi + 1) >> 1;
-              if (sm[wid].excl[mid] <= gi)
+              if (sm.excl[mid] <= gi)
                 lo = mid;
               else
                 hi = mid - 1;
             }
             sl[k] = lo;
-            w[k] = __ldg(&S.E[sm[wid].beg[lo] + (gi - sm[wid].excl[lo])]);
+            w[k] = __ldg(&S.E[sm.beg[lo] + (gi - sm.excl[lo])]);
           }
         }
         bool fk = false;
@@ -566,16 +563,16 @@ __global__ void __launch_bounds__(BLOCK)
         if (fk) {
 #pragma unroll
           for (int k = 0; k < kMsK; k++)
-            if (w[k] != 0xFFFFFFFFu) atomicOr(&sm[wid].fail, 1u << sl[k]);
+            if (w[k] != 0xFFFFFFFFu) atomicOr(&sm.fail, 1u << sl[k]);
         }
         (sd ? in1 : in0) += __popc(tm);
         ins += __reduce_add_sync(kFull, (unsigned)__popc(tm));
         ms_vgc_place<kMsK>(tm, w, vb, ve, lab, Q, tail, tq, S.Fout, &S.ctr->next);
       }
       __syncwarp();
-      failed = (sm[wid].fail >> lane) & 1u;
+      failed = (sm.fail >> lane) & 1u;
       __syncwarp();
-      if (lane == 0) sm[wid].fail = 0;
+      if (lane == 0) sm.fail = 0;
       __syncwarp();
       (sd ? pr1 : pr0) += probes;
       probes = 0;
@@ -599,30 +596,38 @@ __global__ void __launch_bounds__(BLOCK)
   flush_ms_counters(s0.ctr, s1.ctr, sc0, sc1, rq0, rq1, pr0, pr1, ex0, ex1, in0, in1);
 }
 
+template <int BLOCK, int QCAP>
+__global__ void __launch_bounds__(BLOCK)
+    k_ms_vgc(MsSide s0, MsSide s1, const uint64_t* labels, uint32_t tau) {
+  __shared__ WarpExpandSmem sm[BLOCK / 32];
+  __shared__ MsQEnt sq[BLOCK / 32][QCAP];
+  const unsigned wid = threadIdx.x >> 5;
+  ms_vgc_round<kMsK, QCAP>(s0, s1, labels, tau, sm[wid], sq[wid],
+                           (uint64_t)blockIdx.x * (BLOCK / 32) + wid,
+                           (uint64_t)gridDim.x * (BLOCK / 32));
+}
+
 // Heavy pairs of both sides: the chunks of a side's heavy list are cut into
 // one contiguous range per warp; a warp finds the pair of its first chunk
 // once, then offers kMsHeavyChunk edges per step (a heavy pair has more than
 // 64 chunks, so the next pair is at most one step away).  A step with a
 // failed insert re-queues its pair once (kRequeued), whichever warp failed
 // first.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK)
-    k_ms_heavy(MsSide s0, MsSide s1, const uint64_t* __restrict__ labels) {
+__device__ __forceinline__ void ms_heavy_round(const MsSide& s0, const MsSide& s1,
+                                               const uint64_t* labels, uint64_t gw, uint64_t nw) {
   constexpr int K = kMsHeavyK;
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+  const unsigned lane = lane_id();
 #pragma unroll 1
   for (int sd = 0; sd < 2; sd++) {
     const MsSide S = sd ? s1 : s0;
     if (!S.ctr) continue;
-    const unsigned long long packed = S.ctr->heavy;
+    const unsigned long long packed = __ldcg(&S.ctr->heavy);
     const uint64_t nh = packed >> kPackShift, total = packed & kPackMask;
     const uint64_t per = (total + nw - 1) / nw;
     const uint64_t c_beg = gw * per, c_end = c_beg + per < total ? c_beg + per : total;
     if (nh == 0 || c_beg >= c_end) continue;
     // first chunks: hflag below the kRequeued bit (fixed while other warps set that bit)
-    auto first_chunk = [&](uint64_t i) -> uint64_t { return S.hflag[i] & ~kRequeued; };
+    auto first_chunk = [&](uint64_t i) -> uint64_t { return ld_cg(&S.hflag[i]) & ~kRequeued; };
     uint64_t h = 0, hi = nh - 1;  // last pair whose first chunk is <= c_beg
     while (h < hi) {
       const uint64_t mid = (h + hi + 1) >> 1;
@@ -631,17 +636,17 @@ __global__ void __launch_bounds__(BLOCK)
       else
         hi = mid - 1;
     }
-    uint64_t key = S.Fheavy[h], cs = first_chunk(h), cn = h + 1 < nh ? first_chunk(h + 1) : total;
-    uint64_t sub = labels[key >> 32], beg = S.off[key >> 32], end = S.off[(key >> 32) + 1];
+    uint64_t key = ld_cg(&S.Fheavy[h]), cs = first_chunk(h), cn = h + 1 < nh ? first_chunk(h + 1) : total;
+    uint64_t sub = ld_cg(&labels[key >> 32]), beg = S.off[key >> 32], end = S.off[(key >> 32) + 1];
     unsigned long long scanned = 0, requeued = 0, ins = 0;
     uint32_t probes = 0;
     for (uint64_t c = c_beg; c < c_end; c++) {
       if (c >= cn) {
         h++;
-        key = S.Fheavy[h];
+        key = ld_cg(&S.Fheavy[h]);
         cs = cn;
         cn = h + 1 < nh ? first_chunk(h + 1) : total;
-        sub = labels[key >> 32];
+        sub = ld_cg(&labels[key >> 32]);
         beg = S.off[key >> 32];
         end = S.off[(key >> 32) + 1];
       }
@@ -663,7 +668,7 @@ __global__ void __launch_bounds__(BLOCK)
 #pragma unroll
       for (int k = 0; k < K; k++) {
         nk[k] = 0;
-        if (w[k] != 0xFFFFFFFFu && __ldg(&labels[w[k]]) == sub) {
+        if (w[k] != 0xFFFFFFFFu && ld_cg(&labels[w[k]]) == sub) {
           nk[k] = ((uint64_t)w[k] << 32) | lab;
           const int r = table_insert(S.T, S.mask, nk[k], kProbeLimit, &probes);
           if (r == 1) tm |= 1u << k;
@@ -694,6 +699,436 @@ __global__ void __launch_bounds__(BLOCK)
         atomicAdd(&S.ctr->aux1, requeued);
       }
     }
+  }
+}
+
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK)
+    k_ms_heavy(MsSide s0, MsSide s1, const uint64_t* labels) {
+  ms_heavy_round(s0, s1, labels, (uint64_t)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
+                 (uint64_t)gridDim.x * (BLOCK / 32));
+}
+
+// ---------------------------------------------------------------------------
+// Resident batches.  A prefix-doubling batch is small for most of a solve (1,
+// 2, 3, 5, 8, ... pivots) and a chain of dependent steps: select the live
+// centres of its window, seed the tables, sub-rounds until no pair is new,
+// partition.  Launched step by step that costs about 8 launches and 2 waits, 60
+// to 85 us per batch whatever it holds; here one cooperative launch of a block
+// per SM runs batch after batch with a grid barrier (about 1.5 us) between
+// steps, and every block takes the same decisions from the same counters.
+// Two table sets alternate, so that the next batch's tables are cleared while
+// this batch is partitioned.  A batch that outgrows the tables (load above 1/2,
+// a failed insert, or a first capacity above cap_max) ends the launch before its
+// partition: nothing it wrote is visible, and the host runs it with growing
+// tables.
+// 12 warps a block, 2 edges in flight per lane: 16 warps (spills) and 4 edges were
+// 5 to 7 % slower on kNN and grid.  Multi-search phase, before -> now: R-MAT 2^16
+// (8 batches) 0.38 -> 0.12 ms, kNN 10^7 (26) 2.23 -> 1.20, 4096^2 grid (29) 3.52 ->
+// 1.71, R-MAT 2^26 (24) 1.58 -> 0.56, 256-graph batch (19) 2.91 -> 1.53.
+// ---------------------------------------------------------------------------
+constexpr int kMbThreads = 384;
+constexpr int kMbWarps = kMbThreads / 32;
+constexpr int kMbK = 2;  // VGC edges in flight per lane
+constexpr int kMbCtr = 4;    // counter sets 4-9: three sub-rounds in rotation, two sides
+constexpr int kMbState = 16; // counter sets 16-17
+
+enum MbWhy : uint32_t { MB_RUNNING = 0, MB_DONE = 1, MB_HOST = 2 };
+
+struct MbState {
+  uint32_t arrive, failed, why, pad;
+  unsigned long long cur, step, label_offset, round, ne[2];
+  unsigned long long batches, subrounds;
+  unsigned long long edges, probes, expanded, pairs, heavy, heavy_edges, heavy_probes;
+  unsigned long long slots;
+};
+static_assert(sizeof(MbState) <= 2 * sizeof(Counters) && kMbState + 2 <= kCounterSets,
+              "the state fits its counter sets");
+
+struct MbShared {
+  MsQEnt q[kMbWarps][kMsVgcQueue];
+  WarpExpandSmem sm[kMbWarps];
+  MsSrc src[kMbWarps];
+  uint32_t wcnt[kMbWarps + 1];
+  uint32_t before, total;
+};
+
+struct MbArgs {
+  const uint64_t *off, *in_off;
+  const uint32_t *E, *in_E;
+  uint64_t* labels;
+  MsRun run;
+  double beta;
+  uint32_t tau;
+  int local;
+  uint64_t vgc_limit, cap_max;
+  unsigned long long* T[2][2];  // [set][side]
+  uint64_t* F[2][2];            // [side][buffer]
+  uint64_t* Fh[2];
+  uint32_t* hf[2];
+  uint32_t* counts;  // per block
+  Counters* ctr;
+  MbState* st;
+};
+
+// Slots of a batch's tables: at least 4 per candidate, 4 times the last
+// batch's entries (batches grow by beta), and room for VGC local searches.
+__host__ __device__ inline uint64_t mb_cap(uint64_t window, uint64_t ne0, uint64_t ne1,
+                                           uint64_t vgc_limit, uint32_t tau) {
+  const uint64_t ne = ne0 > ne1 ? ne0 : ne1;
+  const uint64_t vgc = window <= vgc_limit ? window * (tau < 64 ? tau : 64) : 0;
+  uint64_t want = 4 * window > 4 * ne ? 4 * window : 4 * ne;
+  const uint64_t room = 2 * (window + vgc);
+  // (the VGC room is a wish: local searches stop at their share of the table)
+  if (room > want) want = room < (1ull << 20) ? room : (want > (1ull << 20) ? want : (1ull << 20));
+  uint64_t c = 1ull << 13;
+  while (c < want) c <<= 1;
+  return c;
+}
+
+__device__ __forceinline__ void mb_seed(unsigned long long* T0, unsigned long long* T1,
+                                        uint64_t mask, uint64_t* F0, uint64_t* F1, uint64_t r,
+                                        uint32_t v, uint32_t label) {
+  const uint64_t key = ((uint64_t)v << 32) | label;
+  uint32_t pr = 0;
+  table_insert(T0, mask, key, 0xFFFFFFFFu, &pr);  // at most a quarter full
+  table_insert(T1, mask, key, 0xFFFFFFFFu, &pr);
+  F0[r] = key;
+  F1[r] = key;
+}
+
+// GRAPHS: a batch of graphs (windows of many graphs per round).
+template <bool GRAPHS>
+__global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
+  extern __shared__ __align__(16) unsigned char mb_raw[];
+  MbShared& sh = *reinterpret_cast<MbShared*>(mb_raw);
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5, tid = threadIdx.x;
+  const uint64_t gw = (uint64_t)blockIdx.x * kMbWarps + wid, nw = (uint64_t)gridDim.x * kMbWarps;
+  const uint64_t gt = (uint64_t)blockIdx.x * kMbThreads + tid, nt = (uint64_t)gridDim.x * kMbThreads;
+  const bool lead = blockIdx.x == 0 && tid == 0;
+  uint32_t target = 0;
+  auto barrier = [&]() { return grid_barrier(&a.st->arrive, &a.st->failed, target); };
+  if (lane == 0) sh.sm[wid].fail = 0;
+  __syncwarp();
+
+  uint64_t cur = a.run.cur, step = a.run.step, label_offset = a.run.label_offset;
+  uint64_t round = a.run.round, ne0 = a.run.ne[0], ne1 = a.run.ne[1];
+  uint64_t batches = 0, subs = 0, slots = 0;
+  unsigned long long t_edges = 0, t_probes = 0, t_exp = 0, t_pairs = 0, t_heavy = 0, t_he = 0,
+                     t_hp = 0;  // lead thread
+  int set = 0;
+  uint64_t clean = 0;  // slots of this set known to be empty
+  uint32_t why = MB_RUNNING;
+
+  // the next window: plain centres [cur, cur + W), or round's windows
+  const uint64_t *wstart = nullptr, *wpre = nullptr;
+  const uint32_t* wg = nullptr;
+  uint32_t nwin = 0;
+  auto window_size = [&]() -> uint64_t {
+    if (GRAPHS) {
+      if (round >= a.run.rounds) return 0;
+      nwin = (uint32_t)__ldg(&a.run.heads[2 * round + 1]);
+      const uint64_t* w = a.run.sched + __ldg(&a.run.heads[2 * round]);
+      wg = (const uint32_t*)w;
+      wstart = w + nwin;
+      wpre = w + 2 * (uint64_t)nwin;
+      return __ldg(&wpre[nwin]);
+    }
+    const uint64_t left = a.run.n_remaining - cur;
+    return step < left ? step : left;
+  };
+  auto win_of = [&](uint64_t j) -> uint32_t { return last_le(wpre, nwin, j); };
+  auto centre = [&](uint64_t j, uint32_t w) -> uint32_t {
+    return GRAPHS ? __ldg(&a.run.centres[wstart[w] + (j - wpre[w])])
+                  : __ldg(&a.run.centres[cur + j]);
+  };
+  auto advance = [&](uint64_t W) {
+    if (GRAPHS) {
+      round++;
+    } else {
+      cur += W;
+      step = (uint64_t)ceil((double)step * a.beta);
+      if (step > a.run.n_remaining) step = a.run.n_remaining;
+      if (step == 0) step = 1;
+    }
+  };
+
+  for (;;) {
+    const uint64_t W = window_size();
+    if (W == 0) {
+      why = MB_DONE;
+      break;
+    }
+    const uint64_t cap = mb_cap(W, ne0, ne1, a.vgc_limit, a.tau);
+    if (cap > a.cap_max) {
+      why = MB_HOST;
+      break;
+    }
+    const uint64_t mask = cap - 1;
+    unsigned long long* T0 = set ? a.T[1][0] : a.T[0][0];
+    unsigned long long* T1 = set ? a.T[1][1] : a.T[0][1];
+    uint64_t* F0 = a.F[0][0];
+    uint64_t* F1 = a.F[1][0];
+    if (cap > clean) {
+      for (uint64_t i = clean + gt; i < cap; i += nt) {
+        T0[i] = kEmpty;
+        T1[i] = kEmpty;
+      }
+      clean = cap;
+      if (!barrier()) return;
+    }
+    // --- select the live centres in order, and seed both sides with them
+    uint64_t nf = 0;
+    if (!GRAPHS && W <= (uint64_t)kMbThreads) {
+      // every block selects the whole window; rank r is seeded by block r % grid
+      uint32_t v = 0;
+      bool sel = false;
+      if (tid < W) {
+        v = centre(tid, 0);
+        sel = !(ld_cg(&a.labels[v]) & kTopBit);
+      }
+      const unsigned m = __ballot_sync(kFull, sel);
+      if (lane == 0) sh.wcnt[wid] = __popc(m);
+      __syncthreads();
+      uint32_t r = __popc(m & ((1u << lane) - 1u)), tot = 0;
+      for (int w = 0; w < kMbWarps; w++) {
+        const uint32_t c = sh.wcnt[w];
+        if (w < (int)wid) r += c;
+        tot += c;
+      }
+      nf = tot;
+      if (sel && r % gridDim.x == blockIdx.x)
+        mb_seed(T0, T1, mask, F0, F1, r, v, (uint32_t)(label_offset + r));
+      __syncthreads();
+    } else {
+      const uint64_t per = (W + gridDim.x - 1) / gridDim.x;
+      const uint64_t j0 = per * blockIdx.x < W ? per * blockIdx.x : W;
+      const uint64_t j1 = j0 + per < W ? j0 + per : W;
+      uint32_t c = 0;
+      for (uint64_t j = j0 + tid; j < j1; j += kMbThreads) {
+        const uint32_t w = GRAPHS ? win_of(j) : 0;
+        c += !(ld_cg(&a.labels[centre(j, w)]) & kTopBit);
+      }
+      if (tid == 0) sh.before = sh.total = 0;
+      __syncthreads();
+      c = __reduce_add_sync(kFull, c);
+      if (lane == 0 && c) atomicAdd(&sh.total, c);
+      __syncthreads();
+      if (tid == 0) {
+        a.counts[blockIdx.x] = sh.total;
+        sh.total = 0;
+      }
+      if (!barrier()) return;
+      for (uint32_t b = tid; b < gridDim.x; b += kMbThreads) {
+        const uint32_t x = ld_cg(&a.counts[b]);
+        if (x) {
+          atomicAdd(&sh.total, x);
+          if (b < blockIdx.x) atomicAdd(&sh.before, x);
+        }
+      }
+      __syncthreads();
+      nf = sh.total;
+      uint64_t base = sh.before;
+      for (uint64_t t0 = j0; t0 < j1; t0 += kMbThreads) {
+        const uint64_t j = t0 + tid;
+        uint32_t v = 0, w = 0;
+        bool sel = false;
+        if (j < j1) {
+          w = GRAPHS ? win_of(j) : 0;
+          v = centre(j, w);
+          sel = !(ld_cg(&a.labels[v]) & kTopBit);
+        }
+        const unsigned m = __ballot_sync(kFull, sel);
+        if (lane == 0) sh.wcnt[wid] = __popc(m);
+        __syncthreads();
+        uint64_t r = base + __popc(m & ((1u << lane) - 1u));
+        uint32_t tot = 0;
+        for (int x = 0; x < kMbWarps; x++) {
+          const uint32_t cx = sh.wcnt[x];
+          if (x < (int)wid) r += cx;
+          tot += cx;
+        }
+        if (GRAPHS) {
+          // pivot r belongs to window w; a window's first item knows its base
+          if (j < j1 && j == wpre[w]) a.run.fb[w] = r;
+          if (sel) {
+            a.run.front[r] = v;
+            a.run.win[r] = w;
+          }
+        } else if (sel) {
+          mb_seed(T0, T1, mask, F0, F1, r, v, (uint32_t)(label_offset + r));
+        }
+        base += tot;
+        __syncthreads();
+      }
+      if (GRAPHS && nf) {
+        if (lead) a.run.fb[nwin] = nf;
+        if (!barrier()) return;
+        for (uint64_t r = gt; r < nf; r += nt) {
+          const uint32_t w = ld_cg(&a.run.win[r]);
+          const uint64_t lab = ld_cg(&a.run.lo[__ldg(&wg[w])]) + (r - ld_cg(&a.run.fb[w]));
+          mb_seed(T0, T1, mask, F0, F1, r, ld_cg(&a.run.front[r]), (uint32_t)lab);
+        }
+      }
+    }
+    if (nf == 0) {
+      advance(W);
+      // counts[] is rewritten by the next window only after another barrier
+      if (!barrier()) return;
+      continue;
+    }
+    if (!barrier()) return;
+
+    // --- sub-rounds
+    uint64_t n0 = nf, n1 = nf, e0 = nf, e1 = nf;
+    int buf = 0;
+    bool give_up = false;
+    while (n0 | n1) {
+      Counters* c0 = a.ctr + kMbCtr + 2 * (subs % 3);
+      Counters* c1 = c0 + 1;
+      unsigned long long* z = (unsigned long long*)(a.ctr + kMbCtr + 2 * ((subs + 1) % 3));
+      if (blockIdx.x == 0 && tid < 2 * sizeof(Counters) / 8) z[tid] = 0;  // last read a barrier ago
+      subs++;
+      auto side = [&](int k) {
+        MsSide s;
+        s.off = k ? a.in_off : a.off;
+        s.E = k ? a.in_E : a.E;
+        s.Fin = buf ? a.F[k][1] : a.F[k][0];
+        s.Fout = buf ? a.F[k][0] : a.F[k][1];
+        s.nin = k ? n1 : n0;
+        s.T = k ? T1 : T0;
+        s.mask = mask;
+        s.Fheavy = a.Fh[k];
+        s.hflag = a.hf[k];
+        s.ctr = k ? c1 : c0;
+        const uint64_t ne = k ? e1 : e0;
+        const uint64_t room = cap / 2 > ne ? cap / 2 - ne : 0;
+        const uint64_t share = room / (s.nin ? s.nin : 1);
+        s.vgc_budget = (uint32_t)(share < 0xFFFFFFFFull ? share : 0xFFFFFFFFull);
+        return s;
+      };
+      MsSide s0 = side(0), s1 = side(1);
+      const bool v0 = a.local && n0 <= a.vgc_limit, v1 = a.local && n1 <= a.vgc_limit;
+      if ((v0 && n0) || (v1 && n1)) {
+        MsSide x0 = s0, x1 = s1;
+        if (!v0) x0.nin = 0;
+        if (!v1) x1.nin = 0;
+        ms_vgc_round<kMbK, kMsVgcQueue>(x0, x1, a.labels, a.tau, sh.sm[wid], sh.q[wid], gw, nw);
+      }
+      if (!v0 || !v1) {
+        MsSide x0 = s0, x1 = s1;
+        if (v0) x0.nin = 0;
+        if (v1) x1.nin = 0;
+        ms_expand_round(x0, x1, a.labels, sh.sm[wid], sh.src[wid], gw, nw);
+        if (lane == 0) sh.sm[wid].fail = 0;
+      }
+      if (!barrier()) return;
+      if (__ldcg(&c0->heavy) | __ldcg(&c1->heavy)) {
+        ms_heavy_round(s0, s1, a.labels, gw, nw);
+        if (!barrier()) return;
+      }
+      if (lead) {
+        t_edges += __ldcg(&c0->edges) + __ldcg(&c1->edges);
+        t_probes += __ldcg(&c0->probes) + __ldcg(&c1->probes);
+        t_exp += __ldcg(&c0->expanded) + __ldcg(&c1->expanded);
+        t_pairs += n0 + n1;
+        t_heavy += (__ldcg(&c0->heavy) >> kPackShift) + (__ldcg(&c1->heavy) >> kPackShift);
+        t_he += __ldcg(&c0->heavy_edges) + __ldcg(&c1->heavy_edges);
+        t_hp += __ldcg(&c0->heavy_probes) + __ldcg(&c1->heavy_probes);
+      }
+      n0 = __ldcg(&c0->next);
+      n1 = __ldcg(&c1->next);
+      e0 += __ldcg(&c0->inserted);
+      e1 += __ldcg(&c1->inserted);
+      buf ^= 1;
+      if ((__ldcg(&c0->fail) | __ldcg(&c1->fail)) || 2 * e0 > cap || 2 * e1 > cap) {
+        give_up = true;
+        break;
+      }
+    }
+    if (give_up) {
+      why = MB_HOST;
+      break;
+    }
+    // --- partition (scc.hpp:437-464), and clear the other set for the next batch
+    batches++;
+    slots += 2 * cap;
+    const uint64_t this_w = W;
+    if (GRAPHS) {
+      for (uint32_t w = gt; w < nwin; w += nt)
+        a.run.lo[__ldg(&wg[w])] =
+            ld_cg(&a.run.lo[__ldg(&wg[w])]) + ld_cg(&a.run.fb[w + 1]) - ld_cg(&a.run.fb[w]);
+    } else {
+      label_offset += nf;
+    }
+    const bool small0 = e0 <= e1;  // the side with fewer entries probes the other
+    const ulonglong2* Ps = (const ulonglong2*)(small0 ? T0 : T1);
+    const ulonglong2* Pl = (const ulonglong2*)(small0 ? T1 : T0);
+    const unsigned long long* Tl = small0 ? T1 : T0;
+    for (uint64_t i = gt; i < cap; i += nt) {  // cap/2 pairs of slots of each table
+      const bool small = i < cap / 2;
+      const ulonglong2 e2 = __ldcg(small ? &Ps[i] : &Pl[i - cap / 2]);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uint64_t e = h ? e2.y : e2.x;
+        if (e == kEmpty) continue;
+        const uint32_t v = (uint32_t)(e >> 32);
+        const uint64_t l = e & kValMask;
+        bool both = false;
+        if (small) {
+          uint64_t s = hash64(e) & mask;
+          for (uint64_t x = 0; x <= mask; x++) {
+            const uint64_t o = __ldcg(&Tl[s]);
+            both = o == e;
+            if (both || o == kEmpty) break;
+            s = (s + 1) & mask;
+          }
+        }
+        const uint64_t val = both ? (l | kTopBit) : l;
+        if (ld_cg(&a.labels[v]) < val)
+          atomicMax((unsigned long long*)&a.labels[v], (unsigned long long)val);
+      }
+    }
+    ne0 = e0;
+    ne1 = e1;
+    advance(this_w);
+    set ^= 1;
+    clean = 0;
+    const uint64_t next_w = window_size();
+    if (next_w) {
+      const uint64_t next_cap = mb_cap(next_w, ne0, ne1, a.vgc_limit, a.tau);
+      if (next_cap <= a.cap_max) {
+        unsigned long long* N0 = set ? a.T[1][0] : a.T[0][0];
+        unsigned long long* N1 = set ? a.T[1][1] : a.T[0][1];
+        const ulonglong2 none = make_ulonglong2(kEmpty, kEmpty);
+        for (uint64_t i = gt; i < next_cap / 2; i += nt) {
+          ((ulonglong2*)N0)[i] = none;
+          ((ulonglong2*)N1)[i] = none;
+        }
+        clean = next_cap;
+      }
+    }
+    if (!barrier()) return;
+  }
+  if (lead) {
+    MbState& s = *a.st;
+    s.cur = cur;
+    s.step = step;
+    s.label_offset = label_offset;
+    s.round = round;
+    s.ne[0] = ne0;
+    s.ne[1] = ne1;
+    s.batches = batches;
+    s.subrounds = subs;
+    s.edges = t_edges;
+    s.probes = t_probes;
+    s.expanded = t_exp;
+    s.pairs = t_pairs;
+    s.heavy = t_heavy;
+    s.heavy_edges = t_he;
+    s.heavy_probes = t_hp;
+    s.slots = slots;
+    s.why = why;
   }
 }
 
@@ -745,7 +1180,6 @@ MsSide ms_args(psc_graph_s* g, const MsState& s) {
   r.Fheavy = (uint64_t*)g->bufs[s.h_slot].p;
   r.hflag = (uint32_t*)g->bufs[s.f_slot].p;
   r.ctr = g->ctr + s.cset;
-  r.nin_dev = nullptr;
   // VGC local searches share the room left below half load, so one
   // sub-round cannot fill the table
   const uint64_t room = s.cap / 2 > s.ne ? s.cap / 2 - s.ne : 0;
@@ -758,7 +1192,7 @@ MsSide ms_args(psc_graph_s* g, const MsState& s) {
 
 int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t label_offset,
             const uint64_t* labels, const psc_params_t* p, const uint64_t prev_ne[2],
-            MsResult out[2], const uint32_t* front_labels, uint64_t vgc_max, MsAsync* async) {
+            MsResult out[2], const uint32_t* front_labels, uint64_t vgc_max) {
   // heavy-list fields: < 2^24 pairs (m / kHeavyDeg), first chunks < 2^31
   if (g->m >> 36) return PSC_ERR_TOO_LARGE;
   const uint32_t tau = p->tau ? p->tau : 512;
@@ -788,15 +1222,7 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
         front, n_front, label_offset, front_labels, (unsigned long long*)g->bufs[st[0].t_slot].p,
         st[0].cap - 1, (uint64_t*)g->bufs[st[0].a_slot].p,
         (unsigned long long*)g->bufs[st[1].t_slot].p, st[1].cap - 1,
-        (uint64_t*)g->bufs[st[1].a_slot].p, async ? async->nf_dev : nullptr);
-  }
-  // asynchronous start: the first sub-round runs on the device's pivot count
-  // and the heavy walk follows it whenever some vertex could be heavy
-  bool first_async = async && async->nf_dev;
-  bool heavy_possible = false;
-  if (first_async) {
-    PSC_TRY(ensure_max_degrees(g));
-    heavy_possible = g->max_deg[0] > kHeavyDeg || g->max_deg[1] > kHeavyDeg;
+        (uint64_t*)g->bufs[st[1].a_slot].p);
   }
   for (;;) {
     bool any = false;
@@ -825,9 +1251,6 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
     }
     if (!any) break;
     PSC_TRY(zero_counters(g));
-    if (first_async)  // the pivot count comes back with the counters (staging set 3)
-      PSC_CUDA(cudaMemcpyAsync(&g->ctr[3].aux0, async->nf_dev, sizeof(unsigned long long),
-                               cudaMemcpyDeviceToDevice, g->stream));
     MsSide vg[2] = {}, ex[2] = {}, hv[2] = {};
     int nv = 0, ne = 0, nh = 0;
     uint64_t v_items = 0, e_items = 0;
@@ -835,7 +1258,6 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
     for (int k = 0; k < 2; k++) {
       if (st[k].nf == 0) continue;
       MsSide a = ms_args(g, st[k]);
-      if (first_async) a.nin_dev = async->nf_dev;
       is_vgc[k] = local && st[k].nf <= vgc_limit;
       if (is_vgc[k]) {
         vg[nv++] = a;
@@ -875,30 +1297,10 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
       }
     }
     PSC_CUDA(cudaGetLastError());
-    if (first_async && heavy_possible) {  // returns at once when no pair was listed
-      ProfScope ps(g, F_HEAVY);
-      k_ms_heavy<kMsBlock><<<g->num_sms * 4, kMsBlock, 0, g->stream>>>(hv[0], hv[1], labels);
-    }
     PSC_TRY(read_counters(g));
-    if (first_async) {
-      // the pivot count replaces its upper bound
-      const uint64_t nf0 = g->hctr[3].aux0;
-      async->n_front = nf0;
-      for (auto& s : st) {
-        s.ne = s.ne - s.nf + nf0;
-        s.nf = nf0;
-      }
-      if (g->profiling && heavy_possible)
-        for (int k = 0; k < 2; k++) {
-          const Counters& c = g->hctr[st[k].cset];
-          g->prof[F_HEAVY].bytes +=
-              28.0 * (c.heavy >> kPackShift) + 12.0 * c.heavy_edges + 8.0 * c.heavy_probes;
-        }
-    }
     // Heavy pairs are rare: the grid-wide walk is launched only for a round
     // that queued some, then the counters are read again.
-    if (!first_async &&
-        ((st[0].nf && g->hctr[st[0].cset].heavy) || (st[1].nf && g->hctr[st[1].cset].heavy))) {
+    if ((st[0].nf && g->hctr[st[0].cset].heavy) || (st[1].nf && g->hctr[st[1].cset].heavy)) {
       {
         ProfScope ps(g, F_HEAVY);
         k_ms_heavy<kMsBlock><<<g->num_sms * 4, kMsBlock, 0, g->stream>>>(hv[0], hv[1], labels);
@@ -944,13 +1346,104 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
       std::swap(g->bufs[s.a_slot], g->bufs[s.b_slot]);
       s.nf = c.next;
     }
-    first_async = false;
   }
-  if (async && !async->nf_dev) async->n_front = n_front;
   for (int k = 0; k < 2; k++) {
     out[k].cap = st[k].cap;
     out[k].ne = st[k].ne;
   }
+  return PSC_OK;
+}
+
+bool ms_run_ready(psc_graph_s* g) {
+  constexpr int kMaxDev = 64;
+  static std::mutex mu;
+  static int state[kMaxDev] = {};
+  if (g->device < 0 || g->device >= kMaxDev) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  int& st = state[g->device];
+  if (st == 0) {
+    st = -1;
+    int coop = 0, b0 = 0, b1 = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device) == cudaSuccess && coop &&
+        cudaFuncSetAttribute(k_ms_batches<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(MbShared)) == cudaSuccess &&
+        cudaFuncSetAttribute(k_ms_batches<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(MbShared)) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_ms_batches<false>, kMbThreads,
+                                                      sizeof(MbShared)) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_ms_batches<true>, kMbThreads,
+                                                      sizeof(MbShared)) == cudaSuccess &&
+        b0 > 0 && b1 > 0)
+      st = 1;
+    cudaGetLastError();
+  }
+  return st == 1;
+}
+
+// 2^20 slots hold every batch of the R-MAT 2^26, kNN 10^7 and 4096^2 grid
+// solves; a smaller graph's tables are smaller.
+static uint64_t mb_cap_max(const psc_graph_s* g) {
+  return std::min<uint64_t>(1ull << 20, std::max<uint64_t>(1ull << 13, pow2_at_least(16 * g->n)));
+}
+
+int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, uint64_t window) {
+  if (g->m >> 36) return PSC_ERR_TOO_LARGE;  // heavy-list fields, as in ms_pair
+  MbArgs a = {};
+  a.off = g->off;
+  a.in_off = g->in_off;
+  a.E = g->E;
+  a.in_E = g->in_E;
+  a.labels = labels;
+  a.run = *run;
+  a.beta = p->beta;
+  a.tau = p->tau ? p->tau : 512;
+  a.local = p->local_scc != 0;
+  a.vgc_limit = run->vgc_max ? run->vgc_max : (uint64_t)g->num_sms * 32;
+  a.cap_max = mb_cap_max(g);
+  // a first batch that cannot fit goes to ms_pair without a launch
+  if (mb_cap(window, run->ne[0], run->ne[1], a.vgc_limit, a.tau) > a.cap_max) return PSC_OK;
+  static const int kT[2][2] = {{B_TF, B_TB}, {B_TF2, B_TB2}}, kF[2][2] = {{B_PA, B_PB}, {B_PA2, B_PB2}};
+  for (int s = 0; s < 2; s++)
+    for (int k = 0; k < 2; k++) {
+      PSC_TRY(ensure_t(g, kT[s][k], a.cap_max, &a.T[s][k]));
+      PSC_TRY(ensure_t(g, kF[s][k], a.cap_max, &a.F[s][k]));
+    }
+  PSC_TRY(ensure_t(g, B_PH, a.cap_max, &a.Fh[0]));
+  PSC_TRY(ensure_t(g, B_PH2, a.cap_max, &a.Fh[1]));
+  PSC_TRY(ensure_t(g, B_AUX1, a.cap_max, &a.hf[0]));
+  PSC_TRY(ensure_t(g, B_HF2, a.cap_max, &a.hf[1]));
+  PSC_TRY(ensure_t(g, B_BLOCKS, (size_t)g->num_sms, &a.counts));
+  a.ctr = g->ctr;
+  a.st = (MbState*)(g->ctr + kMbState);
+  PSC_TRY(zero_counters(g));
+  {
+    ProfScope ps(g, F_MS_VGC);
+    void* args[] = {&a};
+    PSC_CUDA(cudaLaunchCooperativeKernel(
+        run->sched ? (const void*)k_ms_batches<true> : (const void*)k_ms_batches<false>,
+        dim3((unsigned)g->num_sms), dim3(kMbThreads), args, sizeof(MbShared), g->stream));
+  }
+  PSC_TRY(read_counters(g));
+  const MbState& s = *(const MbState*)(g->hctr + kMbState);
+  if (s.failed || s.why == MB_RUNNING) return PSC_ERR_ITER_LIMIT;
+  run->cur = s.cur;
+  run->step = s.step;
+  run->label_offset = s.label_offset;
+  run->round = s.round;
+  run->ne[0] = s.ne[0];
+  run->ne[1] = s.ne[1];
+  run->done = s.why == MB_DONE;
+  g->stats.batches += s.batches;
+  g->stats.subrounds += 2 * s.subrounds;
+  if (g->profiling) {
+    // as for the separate kernels (see ms_pair and scc_partition)
+    g->prof[F_MS_VGC].bytes += 8.0 * s.pairs + 16.0 * s.expanded + 12.0 * s.edges + 8.0 * s.probes;
+    g->prof[F_HEAVY].bytes += 28.0 * s.heavy + 12.0 * s.heavy_edges + 8.0 * s.heavy_probes;
+    g->prof[F_PARTITION].bytes += 8.0 * s.slots;
+  }
+  if (trace_on())
+    std::fprintf(stderr, "ms resident: %llu batches, %llu sub-rounds, pairs %llu edges %llu %s\n",
+                 s.batches, s.subrounds, s.pairs, s.edges, run->done ? "done" : "to the host");
   return PSC_OK;
 }
 

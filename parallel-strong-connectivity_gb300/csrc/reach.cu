@@ -1143,8 +1143,6 @@ Side make_side(bool backward, uint32_t* vis, int second) {
 
 }  // namespace
 
-int ensure_max_degrees(psc_graph_s* g) { return max_degrees_once(g); }
-
 // Runs the searches of `ns` sides (1 or 2) to completion.  Side k starts from
 // srcs[k], or, when d_srcs is given, every side starts from the n_dsrc device
 // sources d_srcs.

@@ -185,14 +185,6 @@ int scc_partition(psc_graph_s* g, const MsResult res[2], uint64_t* labels) {
   return PSC_OK;
 }
 
-// Batches whose candidate pivots fit the multi-search's VGC range (one pair
-// per resident warp, num_sms * 32) start asynchronously (see the batch loop
-// below): their upper bound chooses the same VGC sub-round as the pivot count
-// would, and sizes their tables modestly.  Larger ones wait for the count.
-#ifndef PSC_ASYNC_BATCHES
-#define PSC_ASYNC_BATCHES 1
-#endif
-
 static int scc_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t* p) {
   const uint64_t n = g->n;
   const unsigned tb = 256;
@@ -246,35 +238,41 @@ static int scc_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t* p) {
     const uint64_t n_remaining = nc;
     uint64_t step_size = 1, cur_offset = 0, finished = 0;
     uint64_t in_ne = 1, out_ne = 1;
+    const bool resident = ms_run_ready(g);
     while (finished != n_remaining) {
+      if (resident) {
+        // batches back to back in one launch, up to one that it leaves to the
+        // steps below
+        MsRun run;
+        run.centres = centers;
+        run.n_remaining = n_remaining;
+        run.cur = cur_offset;
+        run.step = step_size;
+        run.label_offset = label_offset;
+        run.ne[0] = out_ne;
+        run.ne[1] = in_ne;
+        PSC_TRY(ms_run(g, labels, p, &run, std::min(step_size, n_remaining - cur_offset)));
+        cur_offset = finished = run.cur;
+        step_size = run.step;
+        label_offset = run.label_offset;
+        out_ne = run.ne[0];
+        in_ne = run.ne[1];
+        if (run.done) break;
+      }
       const uint64_t end = std::min(cur_offset + step_size, n_remaining);
       const uint64_t vs_size = end - cur_offset;
       finished += vs_size;
       step_size = (uint64_t)std::ceil((double)step_size * p->beta);
       if (step_size > n_remaining) step_size = n_remaining;
       if (step_size == 0) step_size = 1;
-      // Small batches start without waiting for their pivot count: the
-      // compaction's total is read on the device by the seeds and the first
-      // sub-round, so the batch waits on the host once per sub-round only.
-      const bool async = PSC_ASYNC_BATCHES && p->local_scc && vs_size <= (uint64_t)g->num_sms * 32;
       uint64_t nf = 0;
-      const unsigned long long* nf_dev = nullptr;
       PSC_TRY(scan_emit_flags(g, vs_size, NotDoneAt{centers, labels, cur_offset},
-                              CopyAt{centers, front, cur_offset}, async ? nullptr : &nf,
-                              F_COMPACT, 12.0, 4.0, async ? &nf_dev : nullptr));
+                              CopyAt{centers, front, cur_offset}, &nf, F_COMPACT, 12.0, 4.0));
       cur_offset = end;
-      if (!async && nf == 0) continue;
+      if (nf == 0) continue;
       MsResult res[2];
       const uint64_t prev[2] = {out_ne, in_ne};
-      if (async) {
-        MsAsync as;
-        as.nf_dev = nf_dev;
-        PSC_TRY(ms_pair(g, front, vs_size, label_offset, labels, p, prev, res, nullptr, 0, &as));
-        nf = as.n_front;
-        if (nf == 0) continue;
-      } else {
-        PSC_TRY(ms_pair(g, front, nf, label_offset, labels, p, prev, res));
-      }
+      PSC_TRY(ms_pair(g, front, nf, label_offset, labels, p, prev, res));
       g->stats.batches++;
       label_offset += nf;
       PSC_TRY(scc_partition(g, res, labels));
