@@ -74,9 +74,9 @@ struct Counters {
   unsigned long long waves;        // local-search waves of VGC rounds (trace)
   unsigned long long pad[2];
 };
-// sets 0-1: search sides; 2-3: staging; 4-19: the rounds of a chained VGC
-// sequence (reach.cu), two sides per round, or the sub-rounds and the state of
-// the resident multi-search (multisearch.cu)
+// sets 0-1: search sides; 2-3: staging; 4-9: the searches without rounds
+// (reach.cu); 4-17: the sub-rounds and the state of the resident multi-search
+// (multisearch.cu)
 constexpr int kCounterSets = 20;
 
 // ---------------------------------------------------------------------------
@@ -112,10 +112,12 @@ struct psc_graph_s {
   uint32_t* in_E = nullptr;
   int num_sms = 0;
   int vgc_blocks = 0;     // resident blocks per SM of the reach VGC kernel
+  int async_blocks[2] = {0, 0};  // same for its form without rounds (plain, with records)
   int ms_vgc_blocks = 0;  // same for the multi-search VGC kernel
   int ldd_vgc_blocks = 0; // same for the LDD VGC kernel
   int le_heavy_blocks = 0; // same for the LE-list heavy-pair kernel
   bool deg_known = false;    // max_deg holds the largest out- / in-degree
+  bool rec_known[2] = {false, false};  // B_REC_F / B_REC_B hold the adjacency records
   bool dead_known = false;   // B_DEAD holds the unreachable-vertex bitmaps
   uint64_t dead_count[2] = {0, 0};  // vertices with no in-edge / no out-edge
   // per LDD round of the last psc_ldd / psc_cc call: first candidate index,
@@ -189,6 +191,8 @@ enum Buf : int {
   B_TF2,          // second set of label tables (k_ms_batches)
   B_TB2,
   B_BLOCKS,       // u32 per block of a resident grid
+  B_REC_F,        // adjacency records (reach.cu) of the out-lists, of the in-lists
+  B_REC_B,
   B_DEAD,         // u32[2][n/32 + 1] vertices with no in-edge, then no out-edge
   B_COUNT
 };

@@ -11,7 +11,8 @@
 //   VGC:  (local search, reach.hpp:114-171) one frontier vertex per warp runs
 //         a local BFS in a shared-memory queue of up to tau vertices before
 //         spilling the rest to the next frontier — used while the frontier is
-//         small, where rounds, not bandwidth, bound the search;
+//         small, where rounds, not bandwidth, bound the search.  Steady or
+//         low-degree searches leave the rounds altogether (k_reach_async);
 //   pull: the frontier is a bitmap; each warp owns 32 consecutive unvisited
 //         vertices and scans their in-edges until a frontier bit is found,
 //         then writes the visited / next-frontier words with one store
@@ -53,6 +54,17 @@ constexpr int kPushK = 4;       // push: edges in flight per lane
 constexpr int kHeavyK = 4;      // heavy vertices: edges in flight per lane
 constexpr uint64_t kHeavyChunk = 32 * kHeavyK;  // edges of one heavy-list work unit
 
+// A vertex's range with its first kRecEdges targets, in one 32-byte sector.  A
+// local search on a graph of low degree loads the record of a candidate
+// alongside its claim, so a hop is one trip to memory instead of two
+// (range, then targets).  Built once per handle and direction.
+constexpr int kRecEdges = 6;
+struct __align__(32) VRec {
+  uint64_t hdr;  // beg << 24 | deg
+  uint32_t e[kRecEdges];
+};
+static_assert(sizeof(VRec) == 32, "one sector");
+
 // One search side as the kernels see it.
 struct ReachSide {
   const uint64_t* off;  // adjacency of the search direction
@@ -63,9 +75,7 @@ struct ReachSide {
   uint32_t* qout;       // next frontier (queue)
   uint64_t* heavy;      // heavy list: vertex << 32 | first chunk (see heavy_push)
   Counters* ctr;
-  // chained VGC rounds: when set, the frontier size is read here (the
-  // previous round's ctr->next) instead of nin
-  const unsigned long long* nin_dev;
+  const VRec* rec;      // adjacency records, for k_reach_async (or null)
 };
 
 // Lists a vertex with more than kHeavyDeg out-edges for k_reach_heavy.  Its
@@ -341,12 +351,6 @@ __global__ void __launch_bounds__(BLOCK)
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
   const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
   const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
-  if (s0.nin_dev) s0.nin = *s0.nin_dev;
-  if (s1.nin_dev) s1.nin = *s1.nin_dev;
-  if (chunk == 0) {  // chained round: chunk size from the device frontier sizes
-    const uint64_t per = (s0.nin + s1.nin + nw - 1) / nw;
-    chunk = (uint32_t)(per < 1 ? 1 : per > 32 ? 32 : per);
-  }
   const uint32_t tq = tau < (uint32_t)QCAP ? tau : (uint32_t)QCAP;
   // A round lasts as long as its longest local search.  Searches that stay
   // narrow (a few vertices per wave) stop after max_waves waves and spill
@@ -464,6 +468,542 @@ __global__ void __launch_bounds__(BLOCK)
     if (wv1) atomicAdd(&s1.ctr->waves, wv1);
   }
   flush_side_counters(s0.ctr, s1.ctr, scanned0, scanned1, nedges0, nedges1, exp0, exp1);
+}
+
+// ---------------------------------------------------------------------------
+// Local searches without rounds.  In rounds of VGC searches every vertex that
+// a search spills waits for the round's longest search: on kNN 10^7 a round
+// lasted 150 us with a tenth of the warps at work.  Here one launch of the
+// resident grid runs the whole sparse part of a search: a warp's local search
+// goes on until its queue is empty, gives what it holds beyond kAsyncKeep vertices
+// away whenever warps are idle, and an idle warp waits for a vertex, not for a
+// round.
+//
+// Idle warps hold tickets (consecutive indexes drawn from ctl->head) and poll the
+// slot of their ticket; givers reserve slots from ctl->tail and write vertex ids
+// into them, so a slot has one writer and one reader and needs no lock.  A
+// vertex enters the slots at most once (it is claimed once, and a ticket's
+// vertices are expanded before anything is given away).  ctl->fin counts the
+// vertices taken from the slots whose searches have ended; when it equals
+// ctl->tail nothing is queued and nobody works, and whoever sees that marks the
+// side done.  No warp waits for a block that may not be running: all work is
+// held by running warps or lies in the slots.  Every wait is bounded, and any
+// condition that this launch should not handle sets a stop bit: warps then
+// put their queues into the slots and leave, and the host goes on from
+// what was not taken (k_async_collect).  Stop bits: a vertex with more than
+// kHeavyDeg out-edges, a backlog that full-width rounds expand faster, the end
+// of the prepared slots, a wait that reached its bound.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kTaken = 0xFFFFFFFEu;  // a slot whose vertex was taken (ids are smaller)
+constexpr uint32_t kAsyncDone = 1, kAsyncHeavy = 2, kAsyncWide = 4, kAsyncFull = 8, kAsyncYield = 16;
+constexpr uint32_t kAsyncStop = kAsyncHeavy | kAsyncWide | kAsyncFull | kAsyncYield;
+constexpr uint32_t kAsyncKeep = 16;
+constexpr uint32_t kAsyncSpin = 1u << 16;  // polls of one wait: some 50 ms
+// Vertices put into the slots a second time when a launch stops: at most 32 per
+// resident warp.
+constexpr uint64_t kAsyncSlack = 1u << 18;
+
+// Two lines: the flags are polled by idle warps, and every access to one line
+// takes its turn in the L2 (with the flags beside head and tail, and polled four
+// times as often, a wave took 3,400 cycles instead of 2,050).
+struct __align__(128) AsyncCtl {
+  uint32_t head, tail, pad0[30];
+  uint32_t fin, flags, pad1[30];
+};
+static_assert(sizeof(AsyncCtl) == 2 * sizeof(Counters), "two counter sets hold it");
+
+__global__ void k_async_init(AsyncCtl* c0, uint32_t nf0, AsyncCtl* c1, uint32_t nf1) {
+  // (the counter sets are zero)
+  c0->tail = nf0;
+  c0->flags = nf0 ? 0u : kAsyncDone;
+  c1->tail = nf1;
+  c1->flags = nf1 ? 0u : kAsyncDone;
+}
+
+__device__ __forceinline__ uint2 ld_head_tail(const AsyncCtl* c) {
+  uint2 x;
+  asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];"
+               : "=r"(x.x), "=r"(x.y)
+               : "l"(&c->head)
+               : "memory");
+  return x;
+}
+__device__ __forceinline__ uint32_t ld_flags(const AsyncCtl* c) {
+  return *(const volatile uint32_t*)&c->flags;
+}
+
+// One warp's part in the hand-over of vertices on one side.
+struct AsyncLink {
+  AsyncCtl* C;
+  AsyncCtl *c0, *c1;  // both sides: a stop is for both
+  volatile uint32_t* slot;
+  uint32_t slots, nw;  // prepared slots; warps of the grid
+
+  __device__ void stop(uint32_t why) const {
+    atomicOr(&c0->flags, why);
+    atomicOr(&c1->flags, why);
+  }
+
+  // The warp's search has ended (`items` vertices taken for it): accounts for
+  // them, then waits for vertices.  Returns the mask of lanes that got one (v),
+  // or 0 with *fl = the flags that ended the wait.  tk: the lane's ticket.
+  __device__ __forceinline__ unsigned wait(uint32_t items, bool quit, uint32_t& tk, uint32_t& v,
+                                           uint32_t* flags) const {
+    const unsigned lane = lane_id();
+    if (items && lane == 0) {
+      const uint32_t f = atomicAdd(&C->fin, items) + items;
+      __threadfence();
+      if (f == *(volatile uint32_t*)&C->tail) atomicOr(&C->flags, kAsyncDone);
+    }
+    const bool none = !__any_sync(kFull, tk != kNone);
+    uint32_t first = 0, take = 0, fl = 0;
+    if (lane == 0) {
+      const uint2 c = ld_head_tail(C);
+      fl = quit ? kAsyncHeavy : ld_flags(C);
+      if (!fl && none) {
+        // one ticket, or a warp's share of the backlog
+        const int32_t backlog = (int32_t)(c.y - c.x);
+        take = backlog > (int32_t)nw ? min(32u, (uint32_t)backlog / nw) : 1u;
+        first = atomicAdd(&C->head, take);
+      }
+    }
+    fl = __shfl_sync(kFull, fl, 0);
+    first = __shfl_sync(kFull, first, 0);
+    take = __shfl_sync(kFull, take, 0);
+    if (lane < take) tk = first + lane;
+    v = kNone;
+    unsigned got = 0;
+    for (uint32_t spin = 1; !fl; spin++) {
+      if (tk != kNone && tk < slots) v = slot[tk];
+      got = __ballot_sync(kFull, v != kNone);
+      if (got) break;
+      if ((spin & 15u) == 0) {
+        if (lane == 0) {
+          fl = ld_flags(C);
+          if (!fl && spin >= kAsyncSpin) {
+            stop(kAsyncYield);
+            fl = kAsyncYield;
+          }
+        }
+        fl = __shfl_sync(kFull, fl, 0);
+      } else {
+        __nanosleep(spin < 64 ? 100 : 400);
+      }
+    }
+    if (v != kNone) {
+      slot[tk] = kTaken;
+      tk = kNone;
+    }
+    *flags = fl;
+    return got;
+  }
+
+  // Reserves n slots (lane 0's atomic); the result is the same in all lanes.
+  __device__ __forceinline__ uint32_t reserve(uint32_t n) const {
+    uint32_t pos = 0;
+    if (lane_id() == 0) {
+      pos = atomicAdd(&C->tail, n);
+      if (pos + n > slots) stop(kAsyncFull);
+    }
+    return __shfl_sync(kFull, pos, 0);
+  }
+
+  // How many of the `held` queued vertices to give to idle warps, from a look
+  // at head and tail.
+  __device__ __forceinline__ uint32_t share(const uint2& ht, uint32_t held,
+                                            uint32_t backlog_max) const {
+    const int32_t hungry = (int32_t)(ht.x - ht.y);
+    if (hungry < 0 && (uint32_t)-hungry > backlog_max && lane_id() == 0) stop(kAsyncWide);
+    return hungry > 0 && held > kAsyncKeep ? min(held - kAsyncKeep, (uint32_t)hungry) : 0u;
+  }
+
+  // Puts the last n of the ring's vertices (places [t - n, t)) into the slots.
+  __device__ __forceinline__ void put(const uint32_t* V, uint32_t mask, uint32_t& t,
+                                      uint32_t n) const {
+    const uint32_t pos = reserve(n);
+    t -= n;
+    for (uint32_t i = lane_id(); i < n; i += 32) slot[pos + i] = V[(t + i) & mask];
+    __syncwarp();
+  }
+};
+
+// Of every wave: `look` reads head and tail when there may be something to give
+// away, `check` the stop bits now and then.  Both are used only under the same
+// (warp-uniform) conditions, so that nothing waits for them before the end.
+constexpr uint32_t kAsyncLook = kAsyncKeep - 4;
+
+__device__ __forceinline__ uint64_t async_hdr(uint64_t beg, uint64_t end) {
+  const uint64_t d = end - beg;
+  return (beg << 24) | (d < 0xFFFFFFull ? d : 0xFFFFFFull);
+}
+
+// Any degrees: balanced expansion over up to 32 queued vertices per wave, K
+// edges per lane in flight.  S.qout holds the slots; the first `slots` of them
+// are prepared (kNone or the starting frontier).
+template <int BLOCK, int QCAP, int K>
+__global__ void __launch_bounds__(BLOCK)
+    k_reach_async(ReachSide s0, ReachSide s1, AsyncCtl* c0, AsyncCtl* c1, uint32_t slots,
+                  uint32_t backlog_max) {
+  static_assert((QCAP & (QCAP - 1)) == 0, "ring queue");
+  __shared__ WarpExpandSmem ssm[BLOCK / 32];
+  __shared__ uint64_t shdr[BLOCK / 32][QCAP];  // async_hdr of a queued vertex
+  __shared__ uint32_t sv[BLOCK / 32][QCAP];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t gw = blockIdx.x * (BLOCK / 32) + wid;
+  WarpExpandSmem& sm = ssm[wid];
+  uint64_t* H = shdr[wid];
+  uint32_t* V = sv[wid];
+  unsigned long long edges[2] = {0, 0}, expanded[2] = {0, 0};
+  bool leave = false;
+  for (int turn = 0; turn < 2 && !leave; turn++) {
+    const int sd = (int)((gw + turn) & 1);
+    const uint64_t* __restrict__ off = sd ? s1.off : s0.off;
+    const uint32_t* __restrict__ E = sd ? s1.E : s0.E;
+    uint32_t* vis = sd ? s1.vis : s0.vis;
+    const AsyncLink L{sd ? c1 : c0, c0, c1, sd ? s1.qout : s0.qout, slots,
+                      (uint32_t)(gridDim.x * (BLOCK / 32))};
+    uint32_t tk = kNone;               // this lane's ticket
+    uint32_t h = 0, t = 0, items = 0;  // ring queue [h, t); vertices taken for this search
+    unsigned long long ed = 0, ex = 0;
+    bool quit = false;  // this warp met a heavy vertex
+    uint32_t nwave = 0;
+    for (;;) {
+      if (h == t) {
+        uint32_t v, fl;
+        const unsigned got = L.wait(items, quit, tk, v, &fl);
+        if (!got) {
+          leave = (fl & kAsyncStop) != 0;  // stopped: all sides; done: the other side is next
+          break;
+        }
+        if (v != kNone) {
+          const uint32_t at = __popc(got & ((1u << lane) - 1u));
+          V[at] = v;
+          H[at] = async_hdr(__ldg(&off[v]), __ldg(&off[v + 1]));
+        }
+        items = __popc(got);
+        h = 0;
+        t = items;
+        __syncwarp();
+      }
+      const uint32_t wave = min(32u, t - h);
+      const bool look = t - h > kAsyncLook, check = (++nwave & 7u) == 0;
+      uint2 ht;
+      uint32_t flags;
+      if (look) ht = ld_head_tail(L.C);
+      if (check) flags = ld_flags(L.C);
+      uint64_t beg = 0;
+      uint32_t deg = 0, x = 0;
+      if (lane < wave) {
+        const uint64_t r = H[(h + lane) & (QCAP - 1)];
+        x = V[(h + lane) & (QCAP - 1)];
+        beg = r >> 24;
+        deg = (uint32_t)(r & 0xFFFFFFull);
+      }
+      h += wave;
+      ex += lane < wave;
+      const bool big = deg > kHeavyDeg;
+      if (__any_sync(kFull, big)) {  // not for this launch: back to the slots
+        quit = true;  // (so a warp puts back at most 32, see kAsyncSlack)
+        if (big) {
+          L.slot[atomicAdd(&L.C->tail, 1u)] = x;
+          deg = 0;
+          L.stop(kAsyncHeavy);
+        }
+      }
+      ed += deg;
+      uint32_t incl = deg;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if ((int)lane >= o) incl += y;
+      }
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      __syncwarp();
+      sm.excl[lane] = incl - deg;
+      sm.beg[lane] = beg;
+      __syncwarp();
+      for (uint32_t base = 0; base < total; base += 32 * K) {
+        uint32_t w[K], old[K], tm = 0;
+        uint64_t r[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          w[k] = kNone;
+          if (base + k * 32 < total) {
+            const uint32_t gi = base + k * 32 + lane;
+            if (gi < total) {
+              const int src = find_src(sm, gi);
+              w[k] = __ldg(&E[sm.beg[src] + (gi - sm.excl[src])]);
+            }
+          }
+        }
+        // the claims, with the candidates' ranges loaded alongside
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          old[k] = ~0u;
+          r[k] = 0;
+          if (base + k * 32 < total && w[k] != kNone) {
+            old[k] = atomicOr(&vis[w[k] >> 5], 1u << (w[k] & 31));
+            r[k] = async_hdr(__ldg(&off[w[k]]), __ldg(&off[w[k] + 1]));
+          }
+        }
+        // a vertex without out-edges is done once it is claimed
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          if (!((old[k] >> (w[k] & 31)) & 1u) && (r[k] & 0xFFFFFFull)) tm |= 1u << k;
+        const uint32_t cnt = __popc(tm);
+        uint32_t inc = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(kFull, inc, o);
+          if ((int)lane >= o) inc += y;
+        }
+        const uint32_t tot = __shfl_sync(kFull, inc, 31);
+        if (tot == 0) continue;
+        const uint32_t room = QCAP - (t - h);
+        const uint32_t nloc = tot < room ? tot : room;
+        uint32_t spill = 0;
+        if (tot > nloc) spill = L.reserve(tot - nloc);
+        uint32_t at = inc - cnt;
+#pragma unroll
+        for (int k = 0; k < K; k++)
+          if (tm & (1u << k)) {
+            if (at < nloc) {
+              H[(t + at) & (QCAP - 1)] = r[k];
+              V[(t + at) & (QCAP - 1)] = w[k];
+            } else {
+              L.slot[spill + (at - nloc)] = w[k];
+            }
+            at++;
+          }
+        t += nloc;
+        __syncwarp();
+      }
+      if (look) {
+        const uint32_t give = L.share(ht, t - h, backlog_max);
+        if (give) L.put(V, QCAP - 1, t, give);
+      }
+      if ((quit || (check && (flags & kAsyncStop))) && t != h) L.put(V, QCAP - 1, t, t - h);
+    }
+    edges[sd] = ed;
+    expanded[sd] = ex;
+  }
+  flush_side_counters(s0.ctr, s1.ctr, edges[0], edges[1], 0, 0, expanded[0], expanded[1]);
+}
+
+__device__ __forceinline__ void ld_rec(const VRec* p, uint4& a, uint4& b) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+      : "l"(p));
+}
+
+// Low degrees, with records: the queue holds the records themselves, so a
+// wave's targets are in shared memory and its only trip is the claim (a record
+// comes with it, one 256-bit load).  What is left is the warp's own work, which
+// took more than the trip (2,100 of 3,500 cycles a wave on the grid) when the
+// edges were spread over the lanes by a scan and a search: here eight lanes
+// belong to an entry, lane j to its target j, four entries per step and up to
+// kLowWave per wave, and new vertices are placed by ballots.  A vertex with more
+// than kRecEdges targets comes back to the front of the queue with its next
+// ones, which its lanes load during the wave (at most kLowWave such entries,
+// which are never given away: kAsyncKeep stay).
+// Reach of the first pivot (both sides): kNN 10^7 (depth about 3,700) in rounds
+// 10.1 ms, k_reach_async 8.6, this 4.5; 4096^2 grid 8.2, 7.8, 4.2.  Waves of 8 / 12 /
+// 16 entries: 4.6 / 4.5 / 4.9 ms on kNN; kAsyncKeep 12 / 16 / 20: 4.5 / 4.5 / 4.7;
+// 1 / 2 / 3 / 5 blocks per SM: 5.9 / 5.0 / 4.9 / 5.0 (waves of 16), so three.
+constexpr int kLowWave = 12;
+static_assert(kLowWave <= (int)kAsyncKeep, "entries that came back are kept");
+
+template <int BLOCK, int QCAP>
+__global__ void __launch_bounds__(BLOCK)
+    k_reach_async_low(ReachSide s0, ReachSide s1, AsyncCtl* c0, AsyncCtl* c1, uint32_t slots,
+                      uint32_t backlog_max) {
+  static_assert((QCAP & (QCAP - 1)) == 0 && QCAP >= 64, "ring queue");
+  constexpr int K = kLowWave / 4;
+  __shared__ uint4 srec[BLOCK / 32][QCAP][2];
+  __shared__ uint32_t sv[BLOCK / 32][QCAP];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  const unsigned grp = lane >> 3, j = lane & 7, lt = (1u << lane) - 1u;
+  const uint32_t gw = blockIdx.x * (BLOCK / 32) + wid;
+  uint4(*R)[2] = srec[wid];
+  uint32_t* V = sv[wid];
+  unsigned long long edges[2] = {0, 0}, expanded[2] = {0, 0};
+  bool leave = false;
+  for (int turn = 0; turn < 2 && !leave; turn++) {
+    const int sd = (int)((gw + turn) & 1);
+    const VRec* __restrict__ rec = sd ? s1.rec : s0.rec;
+    const uint32_t* __restrict__ E = sd ? s1.E : s0.E;
+    uint32_t* vis = sd ? s1.vis : s0.vis;
+    const AsyncLink L{sd ? c1 : c0, c0, c1, sd ? s1.qout : s0.qout, slots,
+                      (uint32_t)(gridDim.x * (BLOCK / 32))};
+    uint32_t tk = kNone;               // this lane's ticket
+    uint32_t h = 0, t = 0, items = 0;  // ring queue [h, t); vertices taken for this search
+    uint32_t ed = 0;
+    unsigned long long ex = 0;
+    uint32_t nwave = 0;
+    for (;;) {
+      if (h == t) {
+        edges[sd] += ed;
+        ed = 0;
+        uint32_t v, fl;
+        const unsigned got = L.wait(items, false, tk, v, &fl);
+        if (!got) {
+          leave = (fl & kAsyncStop) != 0;  // stopped: all sides; done: the other side is next
+          break;
+        }
+        if (v != kNone) {
+          const uint32_t at = (h + __popc(got & lt)) & (QCAP - 1);
+          V[at] = v;
+          ld_rec(rec + v, R[at][0], R[at][1]);
+        }
+        items = __popc(got);
+        t = h + items;
+        ex += lane == 0 ? items : 0;
+        __syncwarp();
+      }
+      const uint32_t n = min((uint32_t)kLowWave, t - h);
+      const bool look = t - h > kAsyncLook, check = (++nwave & 7u) == 0;
+      uint2 ht;
+      uint32_t flags;
+      if (look) ht = ld_head_tail(L.C);
+      if (check) flags = ld_flags(L.C);
+      // target j of entry 4 k + grp, and the one kRecEdges further on
+      uint32_t w[K], old[K], nx[K], lo[K], more = 0;
+      uint4 ra[K], rb[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t* word = (const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0];
+        lo[k] = word[0];
+        w[k] = word[2 + (j < (unsigned)kRecEdges ? j : 0)];
+      }
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t deg = 4 * k + grp < n ? lo[k] & 0xFFFFFFu : 0u;
+        if (j >= (unsigned)kRecEdges || j >= deg) w[k] = kNone;
+        more |= (deg > (uint32_t)kRecEdges ? 1u : 0u) << k;
+      }
+      const bool any_more = __any_sync(kFull, more);
+      if (any_more) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const uint64_t beg =
+              ((uint64_t)((const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0])[1] << 8) | (lo[k] >> 24);
+          nx[k] = kNone;
+          if (((more >> k) & 1u) && j < (unsigned)kRecEdges && kRecEdges + j < (lo[k] & 0xFFFFFFu))
+            nx[k] = __ldg(&E[beg + kRecEdges + j]);
+        }
+      }
+      // the claims, with the candidates' records
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        old[k] = ~0u;
+        ra[k].x = 0;
+        if (w[k] != kNone) {
+          old[k] = atomicOr(&vis[w[k] >> 5], 1u << (w[k] & 31));
+          ld_rec(rec + w[k], ra[k], rb[k]);
+          ed++;
+        }
+      }
+      // place the claimed ones (a vertex without out-edges is done)
+      unsigned m[K];
+      uint32_t tot = 0;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        m[k] = __ballot_sync(kFull, !((old[k] >> (w[k] & 31)) & 1u) && (ra[k].x & 0xFFFFFFu));
+        tot += __popc(m[k]);
+      }
+      const uint32_t room = QCAP - (t - h);
+      const uint32_t nloc = min(tot, room);
+      uint32_t at = t;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t q = at + __popc(m[k] & lt);
+        if (((m[k] >> lane) & 1u) && q - t < nloc) {
+          R[q & (QCAP - 1)][0] = ra[k];
+          R[q & (QCAP - 1)][1] = rb[k];
+          V[q & (QCAP - 1)] = w[k];
+        }
+        at += __popc(m[k]);
+      }
+      if (tot > nloc) {  // a full queue: the rest goes to the slots
+        const uint32_t spill = L.reserve(tot - nloc);
+        at = t;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const uint32_t q = at + __popc(m[k] & lt) - t;
+          if (((m[k] >> lane) & 1u) && q >= nloc) L.slot[spill + (q - nloc)] = w[k];
+          at += __popc(m[k]);
+        }
+      }
+      t += nloc;
+      if (lane == 0) ex += nloc;
+      // entries with targets left return to the front, in the places just read
+      const uint32_t h0 = h;
+      h += n;
+      if (any_more) {
+#pragma unroll
+        for (int k = K - 1; k >= 0; k--) {
+          const unsigned back = __ballot_sync(kFull, j == 0 && ((more >> k) & 1u));
+          if (back) {
+            // the group's own entry moves from place 4 k + grp to place (h - 1 - later ones)
+            const bool mv = (more >> k) & 1u;
+            const uint32_t from = (h0 + 4 * k + grp) & (QCAP - 1);
+            const uint32_t to = (h - 1 - __popc(back >> (8 * grp + 1))) & (QCAP - 1);
+            uint32_t lo = 0, hi = 0, x = 0;
+            if (mv && j == 0) {
+              const uint2 hd = *(const uint2*)&R[from][0];
+              lo = hd.x;
+              hi = hd.y;
+              x = V[from];
+            }
+            __syncwarp();
+            if (mv) {
+              uint32_t* word = (uint32_t*)&R[to][0];
+              if (j < (unsigned)kRecEdges) word[2 + j] = nx[k];
+              if (j == 0) {
+                const uint64_t r = ((((uint64_t)hi << 32) | lo) + ((uint64_t)kRecEdges << 24)) - kRecEdges;
+                word[0] = (uint32_t)r;
+                word[1] = (uint32_t)(r >> 32);
+                V[to] = x;
+              }
+            }
+            __syncwarp();
+            h -= __popc(back);
+          }
+        }
+      }
+      __syncwarp();
+      if (look) {
+        const uint32_t give = L.share(ht, t - h, backlog_max);
+        if (give) L.put(V, QCAP - 1, t, give);
+      }
+      if (check && (flags & kAsyncStop) && t != h) L.put(V, QCAP - 1, t, t - h);
+    }
+    edges[sd] += ed;
+    expanded[sd] = ex;
+  }
+  flush_side_counters(s0.ctr, s1.ctr, edges[0], edges[1], 0, 0, expanded[0], expanded[1]);
+}
+
+// What a stopped launch left in the slots becomes the frontier (ctr->next,
+// ctr->next_edges): vertices not taken, and all those behind the prepared slots.
+__global__ void k_async_collect(const uint32_t* __restrict__ slot, const AsyncCtl* C, uint32_t slots,
+                                const uint64_t* __restrict__ off, uint32_t* q, Counters* ctr) {
+  if (C->fin == C->tail) return;
+  const uint64_t total = C->tail;
+  unsigned long long e = 0;
+  for (uint64_t base = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; base < total;
+       base += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = base + lane_id();
+    const uint32_t v = i < total ? slot[i] : kNone;
+    const bool left = v < kTaken;
+    const unsigned long long pos = warp_append(&ctr->next, left);
+    if (left) {
+      q[pos] = v;
+      e += off[v + 1] - off[v];
+    }
+  }
+  e = warp_sum(e);
+  if (lane_id() == 0 && e) atomicAdd(&ctr->next_edges, e);
 }
 
 // Heavy vertices of both sides: the chunks of a side's heavy list are cut
@@ -995,6 +1535,31 @@ static int vgc_occupancy(psc_graph_s* g) {
   return PSC_OK;
 }
 
+// The search without rounds: with records on graphs of low degree (queue of
+// kAsyncRecQueue entries), else in the narrow or wide form of the VGC kernel.
+constexpr int kAsyncRecQueue = 128;
+constexpr int kAsyncRecBlocks = 3;  // per SM (see k_reach_async_low)
+template <class F>
+static auto with_async_kernel(const psc_graph_s* g, bool rec, F f) {
+  if (rec) return f(k_reach_async_low<kVgcBlock, kAsyncRecQueue>);
+  if (vgc_narrow(g)) return f(k_reach_async<kVgcBlock, kVgcQueue, kVgcKNarrow>);
+  return f(k_reach_async<kVgcBlock, kVgcQueue, kVgcKWide>);
+}
+
+static int launch_async(psc_graph_s* g, bool rec, const ReachSide& a, const ReachSide& b,
+                        AsyncCtl* ca, AsyncCtl* cb, uint32_t slots, uint32_t backlog) {
+  int& per_sm = g->async_blocks[rec ? 1 : 0];
+  return with_async_kernel(g, rec, [&](auto kernel) -> int {
+    if (!per_sm) {
+      PSC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kVgcBlock, 0));
+      if (rec) per_sm = std::min(per_sm, kAsyncRecBlocks);
+      if (per_sm < 1) per_sm = 1;
+    }
+    kernel<<<(unsigned)(g->num_sms * per_sm), kVgcBlock, 0, g->stream>>>(a, b, ca, cb, slots, backlog);
+    return PSC_OK;
+  });
+}
+
 // spec: speculative range loads (vgc_claim), for rounds whose frontier gives
 // each resident warp at most kVgcSpecChunk vertices (latency-bound rounds)
 #ifndef PSC_VGC_SPEC_CHUNK
@@ -1039,8 +1604,8 @@ __global__ void k_max_degrees(const uint64_t* __restrict__ off, const uint64_t* 
   }
 }
 
-// Once per handle (the graph does not change): max_deg for the heavy-vertex
-// check of chained rounds.
+// Once per handle (the graph does not change): max_deg, for the choice of the
+// search without rounds.
 int max_degrees_once(psc_graph_s* g) {
   if (g->deg_known) return PSC_OK;
   unsigned long long* d = &g->ctr[2].aux0;  // aux0, aux1 of the staging set
@@ -1051,6 +1616,41 @@ int max_degrees_once(psc_graph_s* g) {
   g->max_deg[0] = g->hctr[2].aux0;
   g->max_deg[1] = g->hctr[2].aux1;
   g->deg_known = true;
+  return PSC_OK;
+}
+
+// Adjacency records of one direction (see VRec).
+__global__ void k_build_records(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
+                                uint64_t n, VRec* rec) {
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+       v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t b = off[v], r = async_hdr(b, off[v + 1]), d = r & 0xFFFFFFull;
+    uint32_t e[kRecEdges];
+#pragma unroll
+    for (int j = 0; j < kRecEdges; j++) e[j] = (uint64_t)j < d ? __ldg(&E[b + j]) : kNone;
+    uint4* o = (uint4*)(rec + v);
+    o[0] = make_uint4((uint32_t)r, (uint32_t)(r >> 32), e[0], e[1]);
+    o[1] = make_uint4(e[2], e[3], e[4], e[5]);
+  }
+}
+
+// Once per handle and direction (the graph does not change); a symmetric graph
+// has one set.  *out is null when there is no memory for them.
+static int records_once(psc_graph_s* g, bool backward, const VRec** out) {
+  const int d = backward && !g->symmetric ? 1 : 0;
+  VRec* r = nullptr;
+  *out = nullptr;
+  const int st = ensure_t(g, d ? B_REC_B : B_REC_F, g->n, &r);
+  if (st == PSC_ERR_OOM) return PSC_OK;
+  PSC_TRY(st);
+  if (!g->rec_known[d]) {
+    ProfScope ps(g, F_REACH_VGC);
+    k_build_records<<<grid_for(g, g->n, 256), 256, 0, g->stream>>>(d ? g->in_off : g->off,
+                                                                   d ? g->in_E : g->E, g->n, r);
+    PSC_CUDA(cudaGetLastError());
+    g->rec_known[d] = true;
+  }
+  *out = r;
   return PSC_OK;
 }
 
@@ -1105,12 +1705,13 @@ struct Side {
   uint64_t live = UINT64_MAX;
 };
 
-// Chained VGC rounds (see reach_sides): rounds per chain, and the counter set
-// of side k in round j of a chain.
-constexpr int kVgcChain = 8;
-static_assert(kVgcChain % 2 == 0, "a chain leaves the frontier in the side's first queue");
-constexpr int chain_set(int j, int k) { return 4 + 2 * j + k; }
-static_assert(chain_set(kVgcChain - 1, 1) < kCounterSets, "chain counter sets");
+// Counter sets of k_reach_async: the control words of side k, and its counters.
+constexpr int async_ctl_set(int k) { return 4 + 2 * k; }
+constexpr int async_ctr_set(int k) { return 8 + k; }
+// Slots prepared for one launch (64 MB to clear per side at most), and the
+// largest out-degree of a graph that starts without rounds.
+constexpr uint64_t kAsyncSlots = 1ull << 24;
+constexpr uint64_t kAsyncLowDeg = 64;
 
 enum Mode { M_NONE, M_VGC, M_PUSH, M_PULL };
 
@@ -1124,7 +1725,7 @@ ReachSide side_args(psc_graph_s* g, const Side& s) {
   r.qout = (uint32_t*)g->bufs[s.slot_qb].p;
   r.heavy = (uint64_t*)g->bufs[s.slot_heavy].p;
   r.ctr = g->ctr + s.cset;
-  r.nin_dev = nullptr;
+  r.rec = nullptr;
   return r;
 }
 
@@ -1157,11 +1758,12 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   const uint64_t vgc_limit = vgc_max ? vgc_max : (uint64_t)g->num_sms * 64;
   if (pull_div == 0) pull_div = 20;
   const uint64_t threshold = g->m / pull_div;
+  const uint64_t slack = !local ? 0 : g->m > kHeavyDeg ? kAsyncSlack : std::min(n, kAsyncSlack);
   for (int k = 0; k < ns; k++) {
     Side& s = sides[k];
     void* p;
-    PSC_TRY(ensure(g, s.slot_qa, (n + 1) * 4, &p));
-    PSC_TRY(ensure(g, s.slot_qb, (n + 1) * 4, &p));
+    PSC_TRY(ensure(g, s.slot_qa, (n + 1 + slack) * 4, &p));
+    PSC_TRY(ensure(g, s.slot_qb, (n + 1 + slack) * 4, &p));
     PSC_TRY(ensure(g, s.slot_fa, (nwords + 1) * 4, &p));
     PSC_TRY(ensure(g, s.slot_fb, (nwords + 1) * 4, &p));
     PSC_TRY(ensure(g, s.slot_heavy, (n + 1) * 8, &p));
@@ -1181,95 +1783,89 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
     s.rounds = 0;
   }
   const bool tr = trace_on();
+  bool async = local;
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
-    // Chained VGC rounds: while every active side has a steady frontier well
-    // inside VGC range (at least two rounds done, grown at most 1.5x in the
-    // last one, far from the pull threshold), kVgcChain rounds are launched
-    // back to back, each reading its frontier size from the previous round's
-    // counters on the device, and the counters are read back once for the
-    // whole chain instead of once per round.  Every round is a VGC round as
-    // the switch would have chosen it; a round of a side that ran dry does
-    // nothing.
-    if (local) {
+    // The sparse part of a search in one launch (k_reach_async): from the
+    // start on graphs of low degree (their frontiers grow slowly), else once
+    // every active side's frontier is steady, well inside VGC range (at least
+    // two rounds done, grown at most 1.5x in the last one, far from the pull
+    // threshold).  What a stopped launch left goes on in rounds.
+    if (async) {
       int act[2], na = 0;
-      bool steady = true;
+      bool steady = true, sparse = true;
       for (int k = 0; k < ns; k++) {
         const Side& s = sides[k];
         if (s.nf == 0) continue;
         act[na++] = k;
-        steady = steady && !s.pull && s.rounds >= 2 && s.nf <= vgc_limit &&
-                 2 * s.nf <= 3 * s.prev_nf && 3 * (s.nf + s.nf_edges) < threshold;
+        sparse = sparse && !s.pull && s.nf <= vgc_limit && s.nf <= kAsyncSlots / 4;
+        steady = steady && s.rounds >= 2 && 2 * s.nf <= 3 * s.prev_nf &&
+                 3 * (s.nf + s.nf_edges) < threshold;
       }
-      if (na > 0 && steady) {
+      bool go = na > 0 && sparse;
+      if (go && !steady) {
         PSC_TRY(max_degrees_once(g));
-        bool heavy_possible = false;  // some active direction has a vertex above kHeavyDeg
-        for (int a = 0; a < na; a++)
-          heavy_possible |= g->max_deg[sides[act[a]].backward ? 1 : 0] > kHeavyDeg;
-        PSC_TRY(vgc_occupancy(g));
-        const unsigned blocks = (unsigned)((uint64_t)g->num_sms * g->vgc_blocks);
-        // speculative range loads while the frontier gives each warp at
-        // most kVgcSpecChunk vertices (steady frontiers stay near their
-        // start size)
-        uint64_t chain_nf = 0;
-        for (int a = 0; a < na; a++) chain_nf += sides[act[a]].nf;
-        const bool spec = chain_nf <= (uint64_t)blocks * (kVgcBlock / 32) * kVgcSpecChunk;
+        go = g->max_deg[0] <= kAsyncLowDeg && g->max_deg[1] <= kAsyncLowDeg;
+      }
+      if (go) {
+        const uint32_t slots = (uint32_t)std::min<uint64_t>(n, kAsyncSlots);
+        // queued vertices whose edges reach the pull threshold, or more than a
+        // few rounds' worth of local searches: full-width rounds are faster
+        uint64_t backlog = std::max<uint64_t>(threshold * n / std::max<uint64_t>(g->m, 1), 1);
+        const bool low = g->deg_known && g->max_deg[0] <= kAsyncLowDeg && g->max_deg[1] <= kAsyncLowDeg;
+        if (low) backlog = n;
+        if (!vgc_max) backlog = std::min<uint64_t>(backlog, 4 * vgc_limit);
         PSC_TRY(zero_counters(g));
-        for (int j = 0; j < kVgcChain; j++) {
-          ReachSide vg[2] = {};
-          for (int a = 0; a < na; a++) {
-            const Side& s = sides[act[a]];
-            ReachSide r = side_args(g, s);
-            uint32_t* qa = (uint32_t*)g->bufs[s.slot_qa].p;
-            uint32_t* qb = (uint32_t*)g->bufs[s.slot_qb].p;
-            r.qin = (j & 1) ? qb : qa;
-            r.qout = (j & 1) ? qa : qb;
-            r.ctr = g->ctr + chain_set(j, a);
-            r.nin_dev = j ? &g->ctr[chain_set(j - 1, a)].next : nullptr;
-            vg[a] = r;
-          }
-          {
-            ProfScope ps(g, F_REACH_VGC);
-            launch_vgc(g, blocks, vg[0], vg[1], tau, 0u, spec);
-          }
-          if (heavy_possible) {
-            // heavy vertices queued by this round (the kernel returns at once
-            // when there are none)
-            ProfScope ps(g, F_HEAVY);
-            k_reach_heavy<kReachBlock><<<g->num_sms * 4, kReachBlock, 0, g->stream>>>(vg[0], vg[1]);
-          }
+        ReachSide sd[2] = {};
+        // (a batch of graphs goes without: a server admits batches by what a
+        // solve without records holds)
+        bool rec = low && !(g->m >> 40) && g->num_graphs == 0;
+        AsyncCtl* ctl[2];
+        uint32_t nf[2] = {0, 0};
+        for (int a = 0; a < 2; a++) {
+          ctl[a] = (AsyncCtl*)(g->ctr + async_ctl_set(a));
+          if (a >= na) continue;
+          const Side& s = sides[act[a]];
+          sd[a] = side_args(g, s);
+          sd[a].ctr = g->ctr + async_ctr_set(a);
+          if (rec) PSC_TRY(records_once(g, s.backward, &sd[a].rec));
+          rec = rec && sd[a].rec;
+          nf[a] = (uint32_t)s.nf;
+          PSC_CUDA(cudaMemsetAsync(sd[a].qout, 0xFF, (size_t)slots * 4, g->stream));
+          PSC_CUDA(cudaMemcpyAsync(sd[a].qout, sd[a].qin, s.nf * 4, cudaMemcpyDeviceToDevice,
+                                   g->stream));
         }
+        if (na == 1) {  // the second side is done from the start
+          sd[1] = sd[0];
+          sd[1].ctr = g->ctr + async_ctr_set(1);
+        }
+        k_async_init<<<1, 1, 0, g->stream>>>(ctl[0], nf[0], ctl[1], nf[1]);
+        {
+          ProfScope ps(g, F_REACH_VGC);
+          PSC_TRY(launch_async(g, rec, sd[0], sd[1], ctl[0], ctl[1], slots,
+                               (uint32_t)std::min<uint64_t>(backlog, 0x7FFFFFFFu)));
+        }
+        for (int a = 0; a < na; a++)
+          k_async_collect<<<g->num_sms * 2, 256, 0, g->stream>>>(
+              sd[a].qout, ctl[a], slots, sd[a].off, (uint32_t*)sd[a].qin, sd[a].ctr);
         PSC_CUDA(cudaGetLastError());
         PSC_TRY(read_counters(g));
-        float t_ms = 0;
-        if (tr) {
-          cudaEvent_t e = take_event(g);
-          PSC_CUDA(cudaEventRecord(e, g->stream));
-          PSC_CUDA(cudaEventSynchronize(e));
-          cudaEventElapsedTime(&t_ms, g->t0, e);
-          give_event(g, e);
-        }
         for (int a = 0; a < na; a++) {
           Side& s = sides[act[a]];
-          uint64_t nin = s.nf;
-          for (int j = 0; j < kVgcChain && nin; j++) {
-            const Counters& c = g->hctr[chain_set(j, a)];
-            s.rounds++;
-            if (g->profiling) {
-              g->prof[F_REACH_VGC].bytes += 16.0 * c.expanded + 5.0 * c.edges + 5.0 * c.next;
-              g->prof[F_HEAVY].bytes += 24.0 * (c.heavy >> kPackShift) + 5.0 * c.heavy_edges;
-            }
-            if (tr)
-              std::fprintf(stderr, "reach side %d round %u mode vgc-chain nf %llu next %llu edges %llu "
-                           "expanded %llu waves %llu t %.3f ms\n",
-                           act[a], s.rounds, (unsigned long long)nin, c.next, c.edges, c.expanded,
-                           c.waves, t_ms);
-            s.prev_nf = nin;
-            nin = c.next;
-          }
-          const Counters& last = g->hctr[chain_set(kVgcChain - 1, a)];
-          s.nf = last.next;  // zero when the side ran dry inside the chain
-          s.nf_edges = last.next_edges;
+          const AsyncCtl& c = *(const AsyncCtl*)(g->hctr + async_ctl_set(a));
+          const Counters& k = g->hctr[async_ctr_set(a)];
+          if (g->profiling)
+            g->prof[F_REACH_VGC].bytes += 16.0 * k.expanded + 5.0 * k.edges + 5.0 * k.expanded;
+          if (tr)
+            std::fprintf(stderr, "reach side %d async nf %u left %llu edges %llu expanded %llu "
+                         "given %u flags %u\n", act[a], nf[a], k.next, k.edges, k.expanded,
+                         c.tail, c.flags);
+          if (!(c.flags & kAsyncStop) && k.next) return PSC_ERR_ITER_LIMIT;  // cannot be
+          if (c.flags & (kAsyncHeavy | kAsyncWide)) async = false;
+          s.rounds++;
+          s.prev_nf = s.nf;
+          s.nf = k.next;
+          s.nf_edges = k.next_edges;
         }
         continue;
       }
