@@ -452,6 +452,32 @@ __device__ __forceinline__ void warp_expand(WarpExpandSmem& sm, uint64_t beg, ui
   __syncwarp();
 }
 
+// A vertex's range with its first kRecEdges targets, in one 32-byte sector.  A
+// local search on a graph of low degree loads the record of a candidate
+// alongside its claim, so a hop is one trip to memory instead of two
+// (range, then targets).  Built once per handle and direction.
+constexpr int kRecEdges = 6;
+struct __align__(32) VRec {
+  uint64_t hdr;  // beg << 24 | deg
+  uint32_t e[kRecEdges];
+};
+static_assert(sizeof(VRec) == 32, "one sector");
+
+// Largest degree of a graph that uses records: nearly all of its vertices have
+// few edges beyond the record.
+constexpr uint64_t kRecMaxDeg = 64;
+
+__device__ __forceinline__ uint64_t adj_hdr(uint64_t beg, uint64_t end) {
+  const uint64_t d = end - beg;
+  return (beg << 24) | (d < 0xFFFFFFull ? d : 0xFFFFFFull);
+}
+
+__device__ __forceinline__ void ld_rec(const VRec* p, uint4& a, uint4& b) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+      : "l"(p));
+}
+
 // Insert key into a linear-probing table of 2^k slots.
 // Returns 1 if inserted, 0 if already present, -1 after `limit` probes.
 __device__ __forceinline__ int table_insert(unsigned long long* T, uint64_t mask, uint64_t key,

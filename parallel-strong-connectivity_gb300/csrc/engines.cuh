@@ -18,6 +18,11 @@ int batch_attach(psc_graph_s* g, const uint64_t* vbase, uint32_t num_graphs, boo
 int call_begin(psc_graph_s* g);
 int call_end(psc_graph_s* g);
 
+// The adjacency records of one direction, built once per handle; *out is null for
+// a graph with a vertex above kRecMaxDeg, for a batch of graphs (a server admits
+// batches by what a solve without records holds), or without memory for them.
+int records_if_low(psc_graph_s* g, bool backward, const VRec** out);
+
 // Builds in_off/in_E from off/E on the device (in-lists sorted by source).
 int build_transpose(psc_graph_s* g);
 // Replaces off/E by their symmetrisation on the device (both directions,

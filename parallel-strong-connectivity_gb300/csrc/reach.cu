@@ -54,17 +54,6 @@ constexpr int kPushK = 4;       // push: edges in flight per lane
 constexpr int kHeavyK = 4;      // heavy vertices: edges in flight per lane
 constexpr uint64_t kHeavyChunk = 32 * kHeavyK;  // edges of one heavy-list work unit
 
-// A vertex's range with its first kRecEdges targets, in one 32-byte sector.  A
-// local search on a graph of low degree loads the record of a candidate
-// alongside its claim, so a hop is one trip to memory instead of two
-// (range, then targets).  Built once per handle and direction.
-constexpr int kRecEdges = 6;
-struct __align__(32) VRec {
-  uint64_t hdr;  // beg << 24 | deg
-  uint32_t e[kRecEdges];
-};
-static_assert(sizeof(VRec) == 32, "one sector");
-
 // One search side as the kernels see it.
 struct ReachSide {
   const uint64_t* off;  // adjacency of the search direction
@@ -632,11 +621,6 @@ struct AsyncLink {
 // (warp-uniform) conditions, so that nothing waits for them before the end.
 constexpr uint32_t kAsyncLook = kAsyncKeep - 4;
 
-__device__ __forceinline__ uint64_t async_hdr(uint64_t beg, uint64_t end) {
-  const uint64_t d = end - beg;
-  return (beg << 24) | (d < 0xFFFFFFull ? d : 0xFFFFFFull);
-}
-
 // Any degrees: balanced expansion over up to 32 queued vertices per wave, K
 // edges per lane in flight.  S.qout holds the slots; the first `slots` of them
 // are prepared (kNone or the starting frontier).
@@ -646,7 +630,7 @@ __global__ void __launch_bounds__(BLOCK)
                   uint32_t backlog_max) {
   static_assert((QCAP & (QCAP - 1)) == 0, "ring queue");
   __shared__ WarpExpandSmem ssm[BLOCK / 32];
-  __shared__ uint64_t shdr[BLOCK / 32][QCAP];  // async_hdr of a queued vertex
+  __shared__ uint64_t shdr[BLOCK / 32][QCAP];  // adj_hdr of a queued vertex
   __shared__ uint32_t sv[BLOCK / 32][QCAP];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
   const uint32_t gw = blockIdx.x * (BLOCK / 32) + wid;
@@ -678,7 +662,7 @@ __global__ void __launch_bounds__(BLOCK)
         if (v != kNone) {
           const uint32_t at = __popc(got & ((1u << lane) - 1u));
           V[at] = v;
-          H[at] = async_hdr(__ldg(&off[v]), __ldg(&off[v + 1]));
+          H[at] = adj_hdr(__ldg(&off[v]), __ldg(&off[v + 1]));
         }
         items = __popc(got);
         h = 0;
@@ -743,7 +727,7 @@ __global__ void __launch_bounds__(BLOCK)
           r[k] = 0;
           if (base + k * 32 < total && w[k] != kNone) {
             old[k] = atomicOr(&vis[w[k] >> 5], 1u << (w[k] & 31));
-            r[k] = async_hdr(__ldg(&off[w[k]]), __ldg(&off[w[k] + 1]));
+            r[k] = adj_hdr(__ldg(&off[w[k]]), __ldg(&off[w[k] + 1]));
           }
         }
         // a vertex without out-edges is done once it is claimed
@@ -788,12 +772,6 @@ __global__ void __launch_bounds__(BLOCK)
     expanded[sd] = ex;
   }
   flush_side_counters(s0.ctr, s1.ctr, edges[0], edges[1], 0, 0, expanded[0], expanded[1]);
-}
-
-__device__ __forceinline__ void ld_rec(const VRec* p, uint4& a, uint4& b) {
-  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
-      : "l"(p));
 }
 
 // Low degrees, with records: the queue holds the records themselves, so a
@@ -1606,7 +1584,7 @@ __global__ void k_max_degrees(const uint64_t* __restrict__ off, const uint64_t* 
 
 // Once per handle (the graph does not change): max_deg, for the choice of the
 // search without rounds.
-int max_degrees_once(psc_graph_s* g) {
+static int max_degrees_once(psc_graph_s* g) {
   if (g->deg_known) return PSC_OK;
   unsigned long long* d = &g->ctr[2].aux0;  // aux0, aux1 of the staging set
   PSC_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), g->stream));
@@ -1624,7 +1602,7 @@ __global__ void k_build_records(const uint64_t* __restrict__ off, const uint32_t
                                 uint64_t n, VRec* rec) {
   for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t b = off[v], r = async_hdr(b, off[v + 1]), d = r & 0xFFFFFFull;
+    const uint64_t b = off[v], r = adj_hdr(b, off[v + 1]), d = r & 0xFFFFFFull;
     uint32_t e[kRecEdges];
 #pragma unroll
     for (int j = 0; j < kRecEdges; j++) e[j] = (uint64_t)j < d ? __ldg(&E[b + j]) : kNone;
@@ -1636,7 +1614,7 @@ __global__ void k_build_records(const uint64_t* __restrict__ off, const uint32_t
 
 // Once per handle and direction (the graph does not change); a symmetric graph
 // has one set.  *out is null when there is no memory for them.
-static int records_once(psc_graph_s* g, bool backward, const VRec** out) {
+int records_once_impl(psc_graph_s* g, bool backward, const VRec** out) {
   const int d = backward && !g->symmetric ? 1 : 0;
   VRec* r = nullptr;
   *out = nullptr;
@@ -1708,10 +1686,8 @@ struct Side {
 // Counter sets of k_reach_async: the control words of side k, and its counters.
 constexpr int async_ctl_set(int k) { return 4 + 2 * k; }
 constexpr int async_ctr_set(int k) { return 8 + k; }
-// Slots prepared for one launch (64 MB to clear per side at most), and the
-// largest out-degree of a graph that starts without rounds.
+// Slots prepared for one launch (64 MB to clear per side at most).
 constexpr uint64_t kAsyncSlots = 1ull << 24;
-constexpr uint64_t kAsyncLowDeg = 64;
 
 enum Mode { M_NONE, M_VGC, M_PUSH, M_PULL };
 
@@ -1743,6 +1719,14 @@ Side make_side(bool backward, uint32_t* vis, int second) {
 }
 
 }  // namespace
+
+int records_if_low(psc_graph_s* g, bool backward, const VRec** out) {
+  *out = nullptr;
+  if (g->num_graphs || (g->m >> 40)) return PSC_OK;
+  PSC_TRY(max_degrees_once(g));
+  if (g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg) return PSC_OK;
+  return records_once_impl(g, backward, out);
+}
 
 // Runs the searches of `ns` sides (1 or 2) to completion.  Side k starts from
 // srcs[k], or, when d_srcs is given, every side starts from the n_dsrc device
@@ -1805,21 +1789,19 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       bool go = na > 0 && sparse;
       if (go && !steady) {
         PSC_TRY(max_degrees_once(g));
-        go = g->max_deg[0] <= kAsyncLowDeg && g->max_deg[1] <= kAsyncLowDeg;
+        go = g->max_deg[0] <= kRecMaxDeg && g->max_deg[1] <= kRecMaxDeg;
       }
       if (go) {
         const uint32_t slots = (uint32_t)std::min<uint64_t>(n, kAsyncSlots);
         // queued vertices whose edges reach the pull threshold, or more than a
         // few rounds' worth of local searches: full-width rounds are faster
         uint64_t backlog = std::max<uint64_t>(threshold * n / std::max<uint64_t>(g->m, 1), 1);
-        const bool low = g->deg_known && g->max_deg[0] <= kAsyncLowDeg && g->max_deg[1] <= kAsyncLowDeg;
+        const bool low = g->deg_known && g->max_deg[0] <= kRecMaxDeg && g->max_deg[1] <= kRecMaxDeg;
         if (low) backlog = n;
         if (!vgc_max) backlog = std::min<uint64_t>(backlog, 4 * vgc_limit);
         PSC_TRY(zero_counters(g));
         ReachSide sd[2] = {};
-        // (a batch of graphs goes without: a server admits batches by what a
-        // solve without records holds)
-        bool rec = low && !(g->m >> 40) && g->num_graphs == 0;
+        bool rec = low;
         AsyncCtl* ctl[2];
         uint32_t nf[2] = {0, 0};
         for (int a = 0; a < 2; a++) {
@@ -1828,7 +1810,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
           const Side& s = sides[act[a]];
           sd[a] = side_args(g, s);
           sd[a].ctr = g->ctr + async_ctr_set(a);
-          if (rec) PSC_TRY(records_once(g, s.backward, &sd[a].rec));
+          if (rec) PSC_TRY(records_if_low(g, s.backward, &sd[a].rec));
           rec = rec && sd[a].rec;
           nf[a] = (uint32_t)s.nf;
           PSC_CUDA(cudaMemsetAsync(sd[a].qout, 0xFF, (size_t)slots * 4, g->stream));
