@@ -21,11 +21,13 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
 #include "engines.cuh"
 #include "levels.cuh"
+#include "pull.cuh"
 #include "scan.cuh"
 
 namespace psc {
@@ -37,6 +39,10 @@ constexpr int kLeKLight = 8;  // the same for the warp expansion of light pairs
 // ---------------------------------------------------------------------------
 // BFS
 // ---------------------------------------------------------------------------
+// Vertices with more out-edges go to k_bfs_heavy: a warp expands 32 vertices, so
+// the others are at most 64 steps.
+constexpr uint64_t kBfsHeavy = 256;
+constexpr uint64_t kBfsChunk = 32 * kLeK;
 __global__ void k_fill_u32(uint32_t* a, uint64_t n, uint32_t v) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
@@ -52,7 +58,7 @@ template <int BLOCK, int K>
 __global__ void __launch_bounds__(BLOCK)
     k_bfs_push(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
                const uint32_t* __restrict__ qin, uint64_t nin, uint32_t* dist, uint32_t level,
-               uint32_t* qout, Counters* ctr) {
+               uint32_t* qout, uint64_t* heavy, uint64_t hthr, Counters* ctr) {
   __shared__ WarpExpandSmem sm[BLOCK / 32];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
   const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
@@ -65,10 +71,16 @@ __global__ void __launch_bounds__(BLOCK)
       const uint32_t u = qin[i];
       beg = off[u];
       rem = off[u + 1] - beg;
+      if (rem > hthr) {
+        const unsigned long long old =
+            atomicAdd(&ctr->heavy, (1ull << kPackShift) + (rem + kBfsChunk - 1) / kBfsChunk);
+        heavy[old >> kPackShift] = ((uint64_t)u << 32) | (old & kPackMask);
+        rem = 0;
+      }
     }
     scanned += rem;
-    while (__any_sync(kFull, rem > 0)) {
-      const uint32_t deg = (uint32_t)(rem < (1ull << 26) ? rem : (1ull << 26));
+    {
+      const uint32_t deg = (uint32_t)rem;
       uint32_t incl = deg;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -109,8 +121,6 @@ __global__ void __launch_bounds__(BLOCK)
           if (tm & (1u << k)) next_edges += off[v[k] + 1] - off[v[k]];
       }
       __syncwarp();
-      beg += deg;
-      rem -= deg;
     }
   }
   scanned = warp_sum(scanned);
@@ -121,6 +131,77 @@ __global__ void __launch_bounds__(BLOCK)
   }
 }
 
+// The listed vertices of a push level: their chunks are cut into one contiguous
+// range per warp of the grid (as k_reach_heavy does), instead of leaving a hub to
+// one warp.  Symmetrised R-MAT 2^20: the two push levels of a search took 5.3
+// ms, hubs of up to 10^5 edges on one warp each.
+template <int BLOCK, int K>
+__global__ void __launch_bounds__(BLOCK)
+    k_bfs_heavy(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
+                const uint64_t* __restrict__ heavy, uint32_t* dist, uint32_t level, uint32_t* qout,
+                Counters* ctr) {
+  static_assert(kBfsChunk == 32 * K, "a chunk is one step");
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
+  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+  const unsigned long long packed = ctr->heavy;
+  const uint64_t nh = packed >> kPackShift, total = packed & kPackMask;
+  const uint64_t per = (total + nw - 1) / nw;
+  const uint64_t c_beg = gw * per, c_end = c_beg + per < total ? c_beg + per : total;
+  if (nh == 0 || c_beg >= c_end) return;
+  uint64_t h = 0, hi = nh - 1;  // last entry whose first chunk is <= c_beg
+  while (h < hi) {
+    const uint64_t mid = (h + hi + 1) >> 1;
+    if ((uint32_t)__ldg(&heavy[mid]) <= c_beg)
+      h = mid;
+    else
+      hi = mid - 1;
+  }
+  uint64_t ent = __ldg(&heavy[h]);
+  uint64_t cs = (uint32_t)ent, cn = h + 1 < nh ? (uint32_t)__ldg(&heavy[h + 1]) : total;
+  uint64_t beg = off[ent >> 32], end = off[(ent >> 32) + 1];
+  unsigned long long scanned = 0, next_edges = 0;
+  for (uint64_t c = c_beg; c < c_end; c++) {
+    if (c >= cn) {
+      h++;
+      ent = __ldg(&heavy[h]);
+      cs = cn;
+      cn = h + 1 < nh ? (uint32_t)__ldg(&heavy[h + 1]) : total;
+      beg = off[ent >> 32];
+      end = off[(ent >> 32) + 1];
+    }
+    const uint64_t e0 = beg + (c - cs) * kBfsChunk;
+    uint32_t v[K], tm = 0, pre = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint64_t e = e0 + k * 32 + lane;
+      v[k] = kNone;
+      if (e < end) {
+        scanned++;
+        v[k] = __ldg(&E[e]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (v[k] != kNone && __ldcg(&dist[v[k]]) == kNone) pre |= 1u << k;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if ((pre & (1u << k)) && atomicCAS(&dist[v[k]], kNone, level) == kNone) tm |= 1u << k;
+    warp_append_batch<K>(tm, v, qout, &ctr->next);
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (tm & (1u << k)) next_edges += off[v[k] + 1] - off[v[k]];
+  }
+  scanned = warp_sum(scanned);
+  next_edges = warp_sum(next_edges);
+  if (lane == 0) {
+    if (scanned) atomicAdd(&ctr->edges, scanned);
+    if (next_edges) atomicAdd(&ctr->next_edges, next_edges);
+  }
+}
+
+// Pull level: every unreached vertex scans its in-edges for a frontier bit, kPullP
+// in flight, its first kPullSolo alone and the rest with the whole warp.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
     k_bfs_pull(const uint64_t* __restrict__ B_off, const uint32_t* __restrict__ B_E,
@@ -134,21 +215,18 @@ __global__ void __launch_bounds__(BLOCK)
   for (uint64_t w = gw; w < nwords; w += nw) {
     const uint64_t v = w * 32 + lane;
     bool found = false;
+    uint64_t j = 0, e = 0;
     if (v < n && dist[v] == kNone) {
-      const uint64_t b = B_off[v], e = B_off[v + 1];
-      uint64_t j = b;
-      for (; j < e; j++) {
-        const uint32_t x = __ldg(&B_E[j]);
-        if ((__ldg(&fb_in[x >> 5]) >> (x & 31)) & 1u) {
-          found = true;
-          break;
-        }
-      }
-      scanned += (found ? j + 1 : j) - b;
-      if (found) {
-        dist[v] = level;
-        next_edges += A_off[v + 1] - A_off[v];
-      }
+      const uint64_t b = B_off[v];
+      e = B_off[v + 1];
+      j = b;
+      found = pull_scan(B_E, fb_in, j, e < b + kPullSolo ? e : b + kPullSolo);
+      scanned += j - b;
+    }
+    pull_long(B_E, fb_in, __ballot_sync(kFull, !found && j < e), j, e, found, scanned);
+    if (found) {
+      dist[v] = level;
+      next_edges += A_off[v + 1] - A_off[v];
     }
     const uint32_t mask = __ballot_sync(kFull, found);
     if (lane == 0) {
@@ -204,6 +282,11 @@ __global__ void k_bfs_b2q(const uint32_t* __restrict__ fb, uint64_t nwords, uint
 int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) {
   const uint64_t n = g->n, nwords = (n + 31) / 32;
   uint32_t *qa, *qb, *fa, *fb;
+  // heavy-list fields: at most m / hthr <= 2^23 entries (24 bits); their chunks
+  // stay below 2^32 for any graph that fits the device
+  uint64_t* heavy;
+  const uint64_t hthr = std::max<uint64_t>(kBfsHeavy, g->m >> 23);
+  PSC_TRY(ensure_t(g, B_HEAVY, g->m / hthr + 1, &heavy));
   PSC_TRY(ensure_t(g, B_QA, n + 1, &qa));
   PSC_TRY(ensure_t(g, B_QB, n + 1, &qb));
   PSC_TRY(ensure_t(g, B_FB_A, nwords + 1, &fa));
@@ -253,7 +336,9 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
     if (!pull) {
       ProfScope ps(g, F_LE);
       k_bfs_push<kLeBlock, kLeK><<<grid_for(g, nf, kLeBlock), kLeBlock, 0, g->stream>>>(
-          g->off, g->E, qa, nf, dist, level, qb, g->ctr);
+          g->off, g->E, qa, nf, dist, level, qb, heavy, hthr, g->ctr);
+      k_bfs_heavy<kLeBlock, kLeK><<<g->num_sms * 4, kLeBlock, 0, g->stream>>>(
+          g->off, g->E, heavy, dist, level, qb, g->ctr);
       std::swap(qa, qb);
       swap_bufs(g, B_QA, B_QB);
     } else {
@@ -325,10 +410,34 @@ __global__ void k_le_seed(const uint32_t* __restrict__ centers, uint64_t start, 
 // one 64-bit atomic on ctr->heavy = count << kLeHeavyShift | edge offset, so
 // list order and edge offsets agree: Hs is increasing and entry h owns the
 // virtual edges [Hs[h], Hs[h + 1]).
-constexpr uint64_t kLeHeavy = 256;
+constexpr uint64_t kLeHeavy = 128;
 constexpr int kLeHeavyShift = 40;
 constexpr uint32_t kLeProbes = 256;  // probe limit of a sized-by-estimate level
 constexpr uint64_t kLeHeavyMask = (1ull << kLeHeavyShift) - 1;
+
+// table_insert that also tells the slot of a new key.
+__device__ __forceinline__ int le_insert(unsigned long long* T, uint64_t mask, uint64_t key,
+                                         uint32_t limit, uint32_t* probes, uint32_t& slot) {
+  uint64_t h = hash64(key) & mask;
+  for (uint32_t i = 0; i < limit; i++) {
+    uint64_t cur = __ldcg(&T[h]);
+    if (cur == kEmpty) {
+      cur = atomicCAS(&T[h], (unsigned long long)kEmpty, (unsigned long long)key);
+      if (cur == kEmpty) {
+        *probes += i + 1;
+        slot = (uint32_t)h;
+        return 1;
+      }
+    }
+    if (cur == key) {
+      *probes += i + 1;
+      return 0;
+    }
+    h = (h + 1) & mask;
+  }
+  *probes += limit;
+  return -1;
+}
 
 // Offers the warp's K candidate pairs key[k] = (p, w[k]) (kEmpty: none):
 // new pairs go to the next frontier and become list entries (w, p, level),
@@ -337,22 +446,25 @@ constexpr uint64_t kLeHeavyMask = (1ull << kLeHeavyShift) - 1;
 // Once a lane of the warp has failed, the warp stops probing and counts its
 // further offers as failures (the rerun makes them all again).  Called by all
 // 32 lanes.
+// Ls (optional) receives each new pair's table slot.
 template <int K>
 __device__ __forceinline__ void le_offer(const uint64_t* __restrict__ off, const uint32_t (&w)[K],
                                          const uint64_t (&key)[K], uint32_t level,
                                          unsigned long long* T, uint64_t mask, uint32_t limit,
                                          uint64_t* Fout, uint32_t* next_dist, uint64_t* Lk,
-                                         uint32_t* Ld, Counters* ctr, uint32_t& probes,
-                                         uint32_t& fails, unsigned long long& next_edges) {
+                                         uint32_t* Ld, uint32_t* Ls, Counters* ctr,
+                                         uint32_t& probes, uint32_t& fails,
+                                         unsigned long long& next_edges) {
   const unsigned lane = lane_id();
   uint32_t tm = 0;
+  uint32_t slot[K];
   const bool full = __any_sync(kFull, fails != 0);
 #pragma unroll
   for (int k = 0; k < K; k++)
     if (key[k] != kEmpty && full) {
       fails++;
     } else if (key[k] != kEmpty) {
-      const int r = table_insert(T, mask, key[k], limit, &probes);
+      const int r = le_insert(T, mask, key[k], limit, &probes, slot[k]);
       if (r == 1) {
         tm |= 1u << k;
         atomicMin(&next_dist[w[k]], level);
@@ -381,49 +493,64 @@ __device__ __forceinline__ void le_offer(const uint64_t* __restrict__ off, const
     if (tm & (1u << k)) {
       Fout[fb++] = key[k];
       Lk[lb] = ((uint64_t)w[k] << 32) | (key[k] >> 32);
+      if (Ls) Ls[lb] = slot[k];
       Ld[lb++] = level;
       next_edges += off[w[k] + 1] - off[w[k]];
     }
 }
 
 // One level of a batch: frontier pairs (p, u); every edge (u, w) with
-// level < dist[w] offers (p, w).  A warp expands 32 pairs together; pairs
-// with more than hthr edges are listed for k_le_heavy.
-template <int BLOCK, int K>
-__global__ void __launch_bounds__(BLOCK)
-    k_le_expand(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
-                const uint32_t* __restrict__ dist, const uint64_t* __restrict__ Fin, uint64_t nf,
-                uint32_t level, unsigned long long* T, uint64_t mask, uint32_t limit,
-                uint64_t* Fout, uint32_t* next_dist, uint64_t* Lk, uint32_t* Ld, uint64_t hthr,
-                uint64_t* Hk, uint64_t* Hs, Counters* ctr) {
-  __shared__ WarpExpandSmem sm[BLOCK / 32];
-  __shared__ uint32_t s_p[BLOCK];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+// level < dist[w] offers (p, w).  A warp (gw of nw, with its own sm and sp)
+// expands up to `chunk` pairs together: 32 of a large frontier, fewer when that
+// leaves warps without work (with 32 always, a frontier of a few thousand pairs
+// kept a few warps for 38 us of serial steps); pairs with more than hthr edges are
+// listed for k_le_heavy.
+struct LeLevel {
+  const uint64_t* off;
+  const uint32_t* E;
+  const uint32_t* dist;  // distances of the earlier batches
+  const uint64_t* Fin;
+  uint64_t nf;
+  uint32_t level, limit;
+  unsigned long long* T;
+  uint64_t mask;
+  uint64_t* Fout;
+  uint32_t* next_dist;
+  uint64_t* Lk;
+  uint32_t *Ld, *Ls;
+  uint64_t hthr;
+  uint64_t *Hk, *Hs;
+  Counters* ctr;
+};
+
+template <int K>
+__device__ __forceinline__ void le_expand_round(const LeLevel& a, uint32_t chunk,
+                                                WarpExpandSmem& sm, uint32_t* sp, uint64_t gw,
+                                                uint64_t nw) {
+  const unsigned lane = lane_id();
   unsigned long long scanned = 0, next_edges = 0;
   uint32_t probes = 0, fails = 0;
-  for (uint64_t base = gw * 32; base < nf; base += nw * 32) {
+  for (uint64_t base = gw * chunk; base < a.nf; base += nw * chunk) {
     const uint64_t i = base + lane;
     uint64_t beg = 0, rem = 0;
     uint32_t p = 0;
-    if (i < nf) {
-      const uint64_t key = Fin[i];
+    if (lane < chunk && i < a.nf) {
+      const uint64_t key = ld_cg(&a.Fin[i]);
       const uint32_t u = (uint32_t)key;
       p = (uint32_t)(key >> 32);
-      beg = off[u];
-      rem = off[u + 1] - beg;
-      if (rem > hthr) {
+      beg = a.off[u];
+      rem = a.off[u + 1] - beg;
+      if (rem > a.hthr) {
         const unsigned long long old =
-            atomicAdd(&ctr->heavy, (1ull << kLeHeavyShift) + (unsigned long long)rem);
+            atomicAdd(&a.ctr->heavy, (1ull << kLeHeavyShift) + (unsigned long long)rem);
         const uint64_t h = old >> kLeHeavyShift;
-        Hk[h] = key;
-        Hs[h] = old & kLeHeavyMask;
+        a.Hk[h] = key;
+        a.Hs[h] = old & kLeHeavyMask;
         rem = 0;
       }
     }
     scanned += rem;
-    s_p[wid * 32 + lane] = p;
+    sp[lane] = p;
     while (__any_sync(kFull, rem > 0)) {
       const uint32_t deg = (uint32_t)(rem < (1ull << 26) ? rem : (1ull << 26));
       uint32_t incl = deg;
@@ -433,38 +560,40 @@ __global__ void __launch_bounds__(BLOCK)
         if ((int)lane >= o) incl += t;
       }
       const uint32_t total = __shfl_sync(kFull, incl, 31);
-      sm[wid].excl[lane] = incl - deg;
-      sm[wid].beg[lane] = beg;
+      sm.excl[lane] = incl - deg;
+      sm.beg[lane] = beg;
       __syncwarp();
       for (uint32_t b = 0; b < total; b += 32 * K) {
         uint32_t w[K], src[K];
         uint64_t key[K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          const uint32_t gi = b + k * 32 + lane;
           w[k] = kNone;
           src[k] = 0;
-          if (gi < total) {
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (sm[wid].excl[mid] <= gi)
-                lo = mid;
-              else
-                hi = mid - 1;
+          if (b + k * 32 < total) {
+            const uint32_t gi = b + k * 32 + lane;
+            if (gi < total) {
+              int lo = 0, hi = 31;
+              while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (sm.excl[mid] <= gi)
+                  lo = mid;
+                else
+                  hi = mid - 1;
+              }
+              src[k] = lo;
+              w[k] = __ldg(&a.E[sm.beg[lo] + (gi - sm.excl[lo])]);
             }
-            src[k] = lo;
-            w[k] = __ldg(&E[sm[wid].beg[lo] + (gi - sm[wid].excl[lo])]);
           }
         }
 #pragma unroll
         for (int k = 0; k < K; k++) {
           key[k] = kEmpty;
-          if (w[k] != kNone && level < __ldg(&dist[w[k]]))
-            key[k] = ((uint64_t)s_p[wid * 32 + src[k]] << 32) | w[k];
+          if (w[k] != kNone && a.level < ld_cg(&a.dist[w[k]]))
+            key[k] = ((uint64_t)sp[src[k]] << 32) | w[k];
         }
-        le_offer<K>(off, w, key, level, T, mask, limit, Fout, next_dist, Lk, Ld, ctr, probes,
-                    fails, next_edges);
+        le_offer<K>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld,
+                    a.Ls, a.ctr, probes, fails, next_edges);
       }
       __syncwarp();
       beg += deg;
@@ -476,11 +605,26 @@ __global__ void __launch_bounds__(BLOCK)
   const unsigned long long pr = warp_sum((unsigned long long)probes);
   const unsigned long long nfail = warp_sum((unsigned long long)fails);
   if (lane == 0) {
-    if (scanned) atomicAdd(&ctr->edges, scanned);
-    if (next_edges) atomicAdd(&ctr->next_edges, next_edges);
-    if (pr) atomicAdd(&ctr->probes, pr);
-    if (nfail) atomicAdd(&ctr->fail, nfail);
+    if (scanned) atomicAdd(&a.ctr->edges, scanned);
+    if (next_edges) atomicAdd(&a.ctr->next_edges, next_edges);
+    if (pr) atomicAdd(&a.ctr->probes, pr);
+    if (nfail) atomicAdd(&a.ctr->fail, nfail);
   }
+}
+
+__device__ __forceinline__ uint32_t le_chunk(uint64_t nf, uint64_t nw) {
+  const uint64_t per = (nf + nw - 1) / nw;
+  return (uint32_t)(per < 1 ? 1 : per > 32 ? 32 : per);
+}
+
+template <int BLOCK, int K>
+__global__ void __launch_bounds__(BLOCK) k_le_expand(LeLevel a) {
+  __shared__ WarpExpandSmem sm[BLOCK / 32];
+  __shared__ uint32_t s_p[BLOCK];
+  const unsigned wid = threadIdx.x >> 5;
+  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+  le_expand_round<K>(a, le_chunk(a.nf, nw), sm[wid], s_p + wid * 32,
+                     (uint64_t)blockIdx.x * (BLOCK / 32) + wid, nw);
 }
 
 // The heavy pairs of a level: their edge lists, concatenated, are cut into
@@ -488,20 +632,14 @@ __global__ void __launch_bounds__(BLOCK)
 // the start of its slice once, then walks 32 * K edges per step with the
 // entry's data held warp-uniform; an entry has more than 32 * K edges, so a
 // step spans at most two entries.
-template <int BLOCK, int K>
-__global__ void __launch_bounds__(BLOCK)
-    k_le_heavy(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
-               const uint32_t* __restrict__ dist, const uint64_t* __restrict__ Hk,
-               const uint64_t* __restrict__ Hs, uint32_t level, unsigned long long* T,
-               uint64_t mask, uint32_t limit, uint64_t* Fout, uint32_t* next_dist, uint64_t* Lk,
-               uint32_t* Ld, Counters* ctr) {
+// (warp gw of nw)
+template <int K>
+__device__ __forceinline__ void le_heavy_round(const LeLevel& a, uint64_t gw, uint64_t nw) {
   constexpr uint64_t kStep = 32 * K;
-  const unsigned long long packed = ctr->heavy;
+  const unsigned long long packed = __ldcg(&a.ctr->heavy);
   const uint64_t nh = packed >> kLeHeavyShift, total = packed & kLeHeavyMask;
   if (nh == 0) return;
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+  const unsigned lane = lane_id();
   const uint64_t slice = ((total + nw - 1) / nw + kStep - 1) / kStep * kStep;
   const uint64_t x_beg = gw * slice;
   if (x_beg >= total) return;
@@ -509,23 +647,23 @@ __global__ void __launch_bounds__(BLOCK)
   uint64_t h = 0, hi = nh - 1;  // last entry with Hs <= x_beg
   while (h < hi) {
     const uint64_t mid = (h + hi + 1) >> 1;
-    if (__ldg(&Hs[mid]) <= x_beg)
+    if (ld_cg(&a.Hs[mid]) <= x_beg)
       h = mid;
     else
       hi = mid - 1;
   }
   // entry h: virtual edges [hs, hn), pair key pk, edge list from eb
-  uint64_t hs = __ldg(&Hs[h]), hn = h + 1 < nh ? __ldg(&Hs[h + 1]) : total;
-  uint64_t pk = __ldg(&Hk[h]), eb = off[(uint32_t)pk];
+  uint64_t hs = ld_cg(&a.Hs[h]), hn = h + 1 < nh ? ld_cg(&a.Hs[h + 1]) : total;
+  uint64_t pk = ld_cg(&a.Hk[h]), eb = a.off[(uint32_t)pk];
   unsigned long long scanned = 0, next_edges = 0;
   uint32_t probes = 0, fails = 0;
   for (uint64_t x0 = x_beg; x0 < x_end; x0 += kStep) {
     const bool nxt = x0 + kStep >= hn && h + 1 < nh;
     uint64_t pk2 = 0, eb2 = 0, hn2 = 0;
     if (nxt) {
-      pk2 = __ldg(&Hk[h + 1]);
-      eb2 = off[(uint32_t)pk2];
-      hn2 = h + 2 < nh ? __ldg(&Hs[h + 2]) : total;
+      pk2 = ld_cg(&a.Hk[h + 1]);
+      eb2 = a.off[(uint32_t)pk2];
+      hn2 = h + 2 < nh ? ld_cg(&a.Hs[h + 2]) : total;
     }
     uint32_t w[K];
     uint64_t key[K];
@@ -536,16 +674,16 @@ __global__ void __launch_bounds__(BLOCK)
       key[k] = kEmpty;
       if (x < x_end) {
         const bool second = x >= hn;
-        const uint32_t v = __ldg(&E[second ? eb2 + (x - hn) : eb + (x - hs)]);
+        const uint32_t v = __ldg(&a.E[second ? eb2 + (x - hn) : eb + (x - hs)]);
         scanned++;
-        if (level < __ldg(&dist[v])) {
+        if (a.level < ld_cg(&a.dist[v])) {
           w[k] = v;
           key[k] = ((second ? pk2 : pk) & 0xFFFFFFFF00000000ull) | v;
         }
       }
     }
-    le_offer<K>(off, w, key, level, T, mask, limit, Fout, next_dist, Lk, Ld, ctr, probes, fails,
-                next_edges);
+    le_offer<K>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld, a.Ls,
+                a.ctr, probes, fails, next_edges);
     if (nxt) {
       h++;
       hs = hn;
@@ -559,10 +697,185 @@ __global__ void __launch_bounds__(BLOCK)
   const unsigned long long pr = warp_sum((unsigned long long)probes);
   const unsigned long long nfail = warp_sum((unsigned long long)fails);
   if (lane == 0) {
-    if (scanned) atomicAdd(&ctr->edges, scanned);
-    if (next_edges) atomicAdd(&ctr->next_edges, next_edges);
-    if (pr) atomicAdd(&ctr->probes, pr);
-    if (nfail) atomicAdd(&ctr->fail, nfail);
+    if (scanned) atomicAdd(&a.ctr->edges, scanned);
+    if (next_edges) atomicAdd(&a.ctr->next_edges, next_edges);
+    if (pr) atomicAdd(&a.ctr->probes, pr);
+    if (nfail) atomicAdd(&a.ctr->fail, nfail);
+  }
+}
+
+template <int BLOCK, int K>
+__global__ void __launch_bounds__(BLOCK) k_le_heavy(LeLevel a) {
+  le_heavy_round<K>(a, (uint64_t)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
+                    (uint64_t)gridDim.x * (BLOCK / 32));
+}
+
+// ---------------------------------------------------------------------------
+// Resident batches.  A batch is a handful of levels, most of them narrow (R-MAT
+// 2^20: 31 batches of 131 levels, half of them under 3,000 edges; kNN and grids:
+// hundreds of levels a batch), and a level launched from the host cost 25 to 35 us
+// before any work, a batch another 60 (table clear, seeds, three scan launches,
+// a copy of all distances).  k_le_batches runs batches back to back on a resident
+// grid with a grid barrier between the steps.  The table has one size (a pair's
+// slot is kept beside its list entry, so a batch clears only what it used, and
+// only the distances of its entries move); a batch that outgrows it is undone
+// and left to the host's growing tables.
+// Device time of lists, before -> now (k_bfs_heavy included): symmetrised R-MAT
+// 2^20 14.8 -> 4.3 ms, R-MAT 150,000 8.3 -> 1.9, kNN 30,000 (719 levels) 32.0 ->
+// 6.1, grid 150 x 200 (1,038) 39.9 -> 8.3, R-MAT 6x10^6 33.3 -> 25.1.  16 warps and 4
+// edges per lane: 12 and 8 gave 4.8 / 2.1 / 6.0 / 8.3 / 30.2, 24 and 4 4.4 / 2.3 / 6.8
+// / 9.4 / 24.5.
+// ---------------------------------------------------------------------------
+constexpr int kLbThreads = 512;
+constexpr int kLbK = 4;  // light pairs: edges in flight per lane
+constexpr int kLbWarps = kLbThreads / 32;
+constexpr int kLbCtr = 4;     // counter sets 4-6: three levels in rotation
+constexpr int kLbState = 10;  // counter sets 10-11
+
+enum LbWhy : uint32_t { LB_RUNNING = 0, LB_DONE = 1, LB_HOST = 2, LB_LIST = 3 };
+
+struct LbState {
+  uint32_t arrive, failed, why, pad;
+  unsigned long long finished, step, L, batches, levels, ne;
+  unsigned long long edges, probes, pairs, added;
+};
+static_assert(sizeof(LbState) <= 2 * sizeof(Counters) && kLbState + 2 <= kCounterSets,
+              "the state fits its counter sets");
+
+struct LbShared {
+  WarpExpandSmem sm[kLbWarps];
+  uint32_t sp[kLbWarps][32];
+};
+
+struct LbArgs {
+  LeLevel lv;       // off, E, dist, T, mask, next_dist, hthr, Hk, Hs
+  uint64_t* F[2];
+  const uint32_t* centers;
+  uint64_t n, finished, step, L, lcap;
+  uint64_t *Lk;
+  uint32_t *Ld, *Ls;
+  uint32_t* dist;
+  double beta;
+  Counters* ctr;
+  LbState* st;
+};
+
+__global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
+  __shared__ LbShared sh;
+  const unsigned wid = threadIdx.x >> 5, tid = threadIdx.x;
+  const uint64_t gw = (uint64_t)blockIdx.x * kLbWarps + wid, nw = (uint64_t)gridDim.x * kLbWarps;
+  const uint64_t gt = (uint64_t)blockIdx.x * kLbThreads + tid, nt = (uint64_t)gridDim.x * kLbThreads;
+  const bool lead = blockIdx.x == 0 && tid == 0;
+  const uint64_t cap = a.lv.mask + 1;
+  uint32_t target = 0;
+  auto barrier = [&]() { return grid_barrier(&a.st->arrive, &a.st->failed, target); };
+  uint64_t finished = a.finished, step = a.step, L = a.L, batches = 0, levels = 0, last_ne = 0;
+  unsigned long long t_edges = 0, t_probes = 0, t_pairs = 0, t_added = 0;  // lead thread
+  uint32_t why = LB_RUNNING;
+  for (;;) {
+    if (finished >= a.n) {
+      why = LB_DONE;
+      break;
+    }
+    uint64_t st2 = (uint64_t)ceil((double)step * a.beta);
+    if (st2 < 1) st2 = 1;
+    const uint64_t end = finished + st2 < a.n ? finished + st2 : a.n;
+    const uint64_t start = finished, nf0 = end - start;
+    if (4 * nf0 > cap) {
+      why = LB_HOST;
+      break;
+    }
+    if (L + cap > a.lcap) {  // a batch adds at most cap entries
+      why = LB_LIST;
+      break;
+    }
+    // --- seeds (k_le_seed)
+    for (uint64_t j = gt; j < nf0; j += nt) {
+      const uint64_t i = start + j;
+      const uint32_t c = __ldg(&a.centers[i]);
+      const uint64_t key = (i << 32) | c;
+      uint32_t pr = 0, slot = 0;
+      le_insert(a.lv.T, a.lv.mask, key, 0xFFFFFFFFu, &pr, slot);
+      a.F[0][j] = key;
+      a.lv.next_dist[c] = 0;
+      a.Lk[L + j] = ((uint64_t)c << 32) | i;
+      a.Ld[L + j] = 0;
+      a.Ls[L + j] = slot;
+    }
+    if (!barrier()) return;
+    uint64_t nf = nf0, ne = nf0;
+    uint32_t level = 0, buf = 0;
+    bool undo = false;
+    while (nf) {
+      Counters* c = a.ctr + kLbCtr + levels % 3;
+      if (blockIdx.x == 0 && tid < sizeof(Counters) / 8)  // last read a barrier ago
+        ((unsigned long long*)(a.ctr + kLbCtr + (levels + 1) % 3))[tid] = 0;
+      levels++;
+      level++;
+      LeLevel v = a.lv;
+      v.Fin = buf ? a.F[1] : a.F[0];
+      v.Fout = buf ? a.F[0] : a.F[1];
+      v.nf = nf;
+      v.level = level;
+      v.limit = kLeProbes;
+      v.Lk = a.Lk + L + ne;
+      v.Ld = a.Ld + L + ne;
+      v.Ls = a.Ls + L + ne;
+      v.ctr = c;
+      le_expand_round<kLbK>(v, le_chunk(nf, nw), sh.sm[wid], sh.sp[wid], gw, nw);
+      if (!barrier()) return;
+      if (__ldcg(&c->heavy)) {
+        le_heavy_round<kLeK>(v, gw, nw);
+        if (!barrier()) return;
+      }
+      if (lead) {
+        t_edges += __ldcg(&c->edges);
+        t_probes += __ldcg(&c->probes);
+        t_pairs += nf;
+        t_added += __ldcg(&c->next);
+      }
+      nf = __ldcg(&c->next);
+      ne += nf;
+      buf ^= 1;
+      if (__ldcg(&c->fail) || 2 * ne > cap || (__ldcg(&c->next_edges) >> kLeHeavyShift)) {
+        undo = true;
+        break;
+      }
+    }
+    // --- the batch's entries leave the table; their distances take effect, or
+    // are taken back
+    for (uint64_t i = L + gt; i < L + ne; i += nt) {
+      const uint32_t w = (uint32_t)(ld_cg(&a.Lk[i]) >> 32);
+      a.lv.T[ld_cg(&a.Ls[i])] = kEmpty;
+      if (undo)
+        a.lv.next_dist[w] = ld_cg(&a.dist[w]);
+      else
+        a.dist[w] = ld_cg(&a.lv.next_dist[w]);
+    }
+    if (undo) {
+      why = LB_HOST;
+      break;
+    }
+    if (!barrier()) return;
+    batches++;
+    L += ne;
+    last_ne = ne;
+    finished = end;
+    step = st2;
+  }
+  if (lead) {
+    LbState& s = *a.st;
+    s.finished = finished;
+    s.step = step;
+    s.L = L;
+    s.batches = batches;
+    s.levels = levels;
+    s.ne = last_ne;
+    s.edges = t_edges;
+    s.probes = t_probes;
+    s.pairs = t_pairs;
+    s.added = t_added;
+    s.why = why;
   }
 }
 
@@ -797,6 +1110,95 @@ static int le_list_reserve(psc_graph_s* g, uint64_t need, uint64_t len, uint64_t
   return PSC_OK;
 }
 
+static bool le_batches_ready(psc_graph_s* g) {
+  constexpr int kMaxDev = 64;
+  static std::mutex mu;
+  static int state[kMaxDev] = {};
+  if (g->device < 0 || g->device >= kMaxDev) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  int& st = state[g->device];
+  if (st == 0) {
+    int coop = 0, b = 0;
+    st = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device) == cudaSuccess &&
+                 coop &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_le_batches, kLbThreads, 0) ==
+                     cudaSuccess &&
+                 b > 0
+             ? 1
+             : -1;
+    cudaGetLastError();
+  }
+  return st == 1;
+}
+
+// Batches from *finished on in resident launches, until all are done (*done) or
+// the next one has to go through the host's loop.
+static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint32_t* dist,
+                      uint32_t* next_dist, uint64_t* lcap, uint64_t* L, uint64_t* finished,
+                      uint64_t* step, uint64_t* prev_ne, bool* done) {
+  const uint64_t n = g->n;
+  // room for the pairs of the first batches (a pair for most vertices) at a
+  // quarter load.  Heavy-list fields: a level's pairs are at most cap / 2 = 2^23,
+  // over fewer than 2^40 edges (checked before the level).
+  const uint64_t cap = std::min<uint64_t>(1ull << 24, p2(std::max<uint64_t>(8192, 4 * n)));
+  const uint64_t hthr = kLeHeavy;
+  for (;;) {
+    LbArgs a = {};
+    PSC_TRY(ensure_t(g, B_TF, cap, &a.lv.T));
+    PSC_TRY(ensure_t(g, B_PA, cap, &a.F[0]));
+    PSC_TRY(ensure_t(g, B_PB, cap, &a.F[1]));
+    PSC_TRY(ensure_t(g, B_PA2, cap, &a.lv.Hk));
+    PSC_TRY(ensure_t(g, B_PB2, cap, &a.lv.Hs));
+    PSC_TRY(le_list_reserve(g, *L + 2 * cap, *L, lcap));
+    // (an earlier call may have left longer buffers)
+    *lcap = std::max(*lcap, std::min<uint64_t>((g->bufs[B_PH].bytes - 16) / 8,
+                                               (g->bufs[B_AUX3].bytes - 16) / 4));
+    PSC_TRY(ensure_t(g, B_TB, (*lcap + 1) / 2, &a.Ls));
+    PSC_CUDA(cudaMemsetAsync(a.lv.T, 0xFF, cap * 8, g->stream));
+    PSC_TRY(zero_counters(g));
+    a.lv.off = g->off;
+    a.lv.E = g->E;
+    a.lv.dist = dist;
+    a.lv.mask = cap - 1;
+    a.lv.next_dist = next_dist;
+    a.lv.hthr = hthr;
+    a.centers = centers;
+    a.n = n;
+    a.finished = *finished;
+    a.step = *step;
+    a.L = *L;
+    a.lcap = *lcap;
+    a.Lk = (uint64_t*)g->bufs[B_PH].p;
+    a.Ld = (uint32_t*)g->bufs[B_AUX3].p;
+    a.dist = dist;
+    a.beta = beta;
+    a.ctr = g->ctr;
+    a.st = (LbState*)(g->ctr + kLbState);
+    {
+      ProfScope ps(g, F_LE);
+      void* args[] = {&a};
+      PSC_CUDA(cudaLaunchCooperativeKernel((const void*)k_le_batches, dim3((unsigned)g->num_sms),
+                                           dim3(kLbThreads), args, 0, g->stream));
+    }
+    PSC_TRY(read_counters(g));
+    const LbState& s = *(const LbState*)(g->hctr + kLbState);
+    if (s.failed || s.why == LB_RUNNING) return PSC_ERR_ITER_LIMIT;
+    if (g->profiling)
+      g->prof[F_LE].bytes += 24.0 * s.pairs + 8.0 * s.edges + 8.0 * s.probes + 16.0 * s.added;
+    if (trace_on())
+      std::fprintf(stderr, "le resident: batches %llu levels %llu edges %llu list %llu why %u\n",
+                   s.batches, s.levels, s.edges, s.L, s.why);
+    g->stats.batches += s.batches;
+    g->stats.subrounds += s.levels;
+    *finished = s.finished;
+    *step = s.step;
+    *L = s.L;
+    if (s.ne) *prev_ne = (uint64_t)std::ceil((double)s.ne * beta);
+    if (s.why == LB_DONE) *done = true;
+    if (s.why != LB_LIST) return PSC_OK;
+  }
+}
+
 // LE-list of the graph for priorities centers (device u32[n]); the result
 // (triples) stays in slot B_AUX0; *len = its entry count.
 int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* len_out) {
@@ -829,7 +1231,15 @@ int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* l
   uint64_t prev_ne = n >> 1;
   // inserts per scanned edge at each level of the previous batch
   std::vector<double> ratio, ratio_next;
+  const bool resident = le_batches_ready(g);
   while (finished < n) {
+    if (resident) {
+      bool done = false;
+      PSC_TRY(le_batches(g, centers, beta, dist, next_dist, &lcap, &L, &finished, &step, &prev_ne,
+                         &done));
+      if (done) break;
+      ratio.clear();
+    }
     step = (uint64_t)std::ceil((double)step * beta);
     if (step < 1) step = 1;
     const uint64_t end = std::min<uint64_t>(finished + step, n);
@@ -914,16 +1324,15 @@ int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* l
           uint64_t* Lk = (uint64_t*)g->bufs[B_PH].p + L;
           uint32_t* Ld = (uint32_t*)g->bufs[B_AUX3].p + L;
           const uint32_t limit = exact ? 0xFFFFFFFFu : kLeProbes;
-          k_le_expand<kLeBlock, kLeKLight><<<grid_for(g, nf, kLeBlock), kLeBlock, 0, g->stream>>>(
-              g->off, g->E, dist, FA, nf, level, T, cap - 1, limit, FB, next_dist, Lk, Ld,
-              any_heavy ? hthr : ~0ull, Hk, Hs, g->ctr);
+          const LeLevel lv{g->off, g->E, dist, FA, nf, level, limit, T, cap - 1, FB, next_dist,
+                           Lk, Ld, nullptr, any_heavy ? hthr : ~0ull, Hk, Hs, g->ctr};
+          k_le_expand<kLeBlock, kLeKLight>
+              <<<grid_for(g, nf * 32, kLeBlock), kLeBlock, 0, g->stream>>>(lv);
           if (any_heavy) {
             const uint64_t hblocks = (bound + kLeBlock * kLeK - 1) / (kLeBlock * kLeK);
             const unsigned hgrid = (unsigned)std::min<uint64_t>(
                 hblocks, (uint64_t)g->num_sms * g->le_heavy_blocks);
-            k_le_heavy<kLeBlock, kLeK><<<hgrid, kLeBlock, 0, g->stream>>>(
-                g->off, g->E, dist, Hk, Hs, level, T, cap - 1, limit, FB, next_dist, Lk, Ld,
-                g->ctr);
+            k_le_heavy<kLeBlock, kLeK><<<hgrid, kLeBlock, 0, g->stream>>>(lv);
           }
         }
         PSC_CUDA(cudaGetLastError());

@@ -37,6 +37,7 @@
 #include "common.cuh"
 #include "engines.cuh"
 #include "levels.cuh"
+#include "pull.cuh"
 
 namespace psc {
 
@@ -1057,8 +1058,6 @@ __global__ void __launch_bounds__(BLOCK) k_reach_heavy(ReachSide s0, ReachSide s
 // vertex, kPullP edges in flight, alone for its first kPullSolo in-edges; the
 // longer in-lists left over are then scanned by the whole warp, one vertex at
 // a time, 32 * kPullP edges per step, until a hit.
-constexpr int kPullP = 4;
-constexpr uint32_t kPullSolo = 64;
 #ifndef PSC_PULL_W
 #define PSC_PULL_W 4
 #endif
@@ -1067,62 +1066,6 @@ constexpr int kPullW = PSC_PULL_W;  // bitmap words per warp step
 #define PSC_PULL_STAGED 1
 #endif
 constexpr bool kPullStaged = PSC_PULL_STAGED != 0;  // tiles staged by bulk copies
-
-__device__ __forceinline__ bool fb_test(const uint32_t* __restrict__ fb, uint32_t x) {
-  return (__ldg(&fb[x >> 5]) >> (x & 31)) & 1u;
-}
-
-// Solo scan of one unvisited vertex's in-list [j, lim): kPullP in-edges at a
-// time until a frontier in-neighbour is found.
-__device__ __forceinline__ bool pull_scan(const uint32_t* __restrict__ B_E,
-                                          const uint32_t* __restrict__ fb_in, uint64_t& j,
-                                          uint64_t lim) {
-  bool found = false;
-  while (j < lim && !found) {
-    uint32_t x[kPullP];
-#pragma unroll
-    for (int k = 0; k < kPullP; k++) x[k] = j + k < lim ? __ldg(&B_E[j + k]) : 0xFFFFFFFFu;
-    bool hit[kPullP];
-#pragma unroll
-    for (int k = 0; k < kPullP; k++) hit[k] = x[k] != 0xFFFFFFFFu && fb_test(fb_in, x[k]);
-    uint64_t step = lim - j < (uint64_t)kPullP ? lim - j : (uint64_t)kPullP;
-#pragma unroll
-    for (int k = kPullP - 1; k >= 0; k--)
-      if (hit[k]) {
-        found = true;
-        step = k + 1;
-      }
-    j += step;
-  }
-  return found;
-}
-
-// The whole warp scans the in-lists left over from the solo phase, one
-// vertex at a time, 32 * kPullP in-edges per step, until a hit.
-__device__ __forceinline__ void pull_long(const uint32_t* __restrict__ B_E,
-                                          const uint32_t* __restrict__ fb_in, uint32_t longm,
-                                          uint64_t j, uint64_t e, bool& found,
-                                          unsigned long long& scanned) {
-  const unsigned lane = lane_id();
-  while (longm) {
-    const int l = __ffs(longm) - 1;
-    longm &= longm - 1;
-    const uint64_t lb = __shfl_sync(kFull, j, l), le = __shfl_sync(kFull, e, l);
-    bool f = false;
-    uint64_t jj = lb;
-    for (; jj < le && !f; jj += 32 * kPullP) {
-      bool hit = false;
-#pragma unroll
-      for (int k = 0; k < kPullP; k++) {
-        const uint64_t q = jj + k * 32 + lane;
-        if (q < le) hit |= fb_test(fb_in, __ldg(&B_E[q]));
-      }
-      f = __any_sync(kFull, hit);
-    }
-    if (lane == 0) scanned += (jj < le ? jj : le) - lb;
-    if (lane == (unsigned)l) found = f;
-  }
-}
 
 // One warp step of a pull round over W adjacent bitmap words (32 W vertices)
 // starting at word w: lane's vertex of word k is unvisited when t[k], with
