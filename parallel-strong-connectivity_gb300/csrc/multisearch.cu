@@ -718,10 +718,10 @@ __global__ void __launch_bounds__(BLOCK)
 // per SM runs batch after batch with a grid barrier (about 1.5 us) between
 // steps, and every block takes the same decisions from the same counters.
 // Two table sets alternate, so that the next batch's tables are cleared while
-// this batch is partitioned.  A batch that outgrows the tables (load above 1/2,
-// a failed insert, or a first capacity above cap_max) ends the launch before its
-// partition: nothing it wrote is visible, and the host runs it with growing
-// tables.
+// this batch is partitioned.  A batch that outgrows its tables (load above 1/2 or
+// a failed insert) ends the launch between two sub-rounds; the host grows tables
+// and frontiers and the next launch goes on from there.  A window too large for
+// the tables from the start goes to the host's full-width kernels (ms_pair).
 // 12 warps a block, 2 edges in flight per lane: 16 warps (spills) and 4 edges were
 // 5 to 7 % slower on kNN and grid.  Multi-search phase, before -> now: R-MAT 2^16
 // (8 batches) 0.38 -> 0.12 ms, kNN 10^7 (26) 2.23 -> 1.20, 4096^2 grid (29) 3.52 ->
@@ -733,7 +733,7 @@ constexpr int kMbK = 2;  // VGC edges in flight per lane
 constexpr int kMbCtr = 4;    // counter sets 4-9: three sub-rounds in rotation, two sides
 constexpr int kMbState = 16; // counter sets 16-17
 
-enum MbWhy : uint32_t { MB_RUNNING = 0, MB_DONE = 1, MB_HOST = 2 };
+enum MbWhy : uint32_t { MB_RUNNING = 0, MB_DONE = 1, MB_HOST = 2, MB_GROW = 3 };
 
 struct MbState {
   uint32_t arrive, failed, why, pad;
@@ -741,6 +741,9 @@ struct MbState {
   unsigned long long batches, subrounds;
   unsigned long long edges, probes, expanded, pairs, heavy, heavy_edges, heavy_probes;
   unsigned long long slots;
+  // a batch interrupted between two sub-rounds (MB_GROW)
+  unsigned long long cap, nf, n0, n1, e0, e1;
+  uint32_t set, buf;
 };
 static_assert(sizeof(MbState) <= 2 * sizeof(Counters) && kMbState + 2 <= kCounterSets,
               "the state fits its counter sets");
@@ -767,17 +770,22 @@ struct MbArgs {
   uint64_t* Fh[2];
   uint32_t* hf[2];
   uint32_t* counts;  // per block
+  // an interrupted batch to go on with (cap 0: none)
+  uint64_t cap, nf, n0, n1, e0, e1;
+  uint32_t set, buf;
   Counters* ctr;
   MbState* st;
 };
 
 // Slots of a batch's tables: at least 4 per candidate, 4 times the last
-// batch's entries (batches grow by beta), and room for VGC local searches.
+// batch's entries (batches grow by beta; twice, where that is a lot to clear and
+// to scan), and room for VGC local searches.
 __host__ __device__ inline uint64_t mb_cap(uint64_t window, uint64_t ne0, uint64_t ne1,
                                            uint64_t vgc_limit, uint32_t tau) {
   const uint64_t ne = ne0 > ne1 ? ne0 : ne1;
   const uint64_t vgc = window <= vgc_limit ? window * (tau < 64 ? tau : 64) : 0;
-  uint64_t want = 4 * window > 4 * ne ? 4 * window : 4 * ne;
+  const uint64_t last = ne <= (1ull << 18) ? 4 * ne : 2 * ne;
+  uint64_t want = 4 * window > last ? 4 * window : last;
   const uint64_t room = 2 * (window + vgc);
   // (the VGC room is a wish: local searches stop at their share of the table)
   if (room > want) want = room < (1ull << 20) ? room : (want > (1ull << 20) ? want : (1ull << 20));
@@ -816,8 +824,11 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
   uint64_t batches = 0, subs = 0, slots = 0;
   unsigned long long t_edges = 0, t_probes = 0, t_exp = 0, t_pairs = 0, t_heavy = 0, t_he = 0,
                      t_hp = 0;  // lead thread
-  int set = 0;
+  int set = (int)a.set;
   uint64_t clean = 0;  // slots of this set known to be empty
+  uint64_t nf = 0, n0 = 0, n1 = 0, e0 = 0, e1 = 0, cap = 0;
+  int buf = 0;
+  bool resume = a.cap != 0;
   uint32_t why = MB_RUNNING;
 
   // the next window: plain centres [cur, cur + W), or round's windows
@@ -859,8 +870,9 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
       why = MB_DONE;
       break;
     }
-    const uint64_t cap = mb_cap(W, ne0, ne1, a.vgc_limit, a.tau);
+    cap = resume ? a.cap : mb_cap(W, ne0, ne1, a.vgc_limit, a.tau);
     if (cap > a.cap_max) {
+      nf = W;
       why = MB_HOST;
       break;
     }
@@ -869,7 +881,7 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
     unsigned long long* T1 = set ? a.T[1][1] : a.T[0][1];
     uint64_t* F0 = a.F[0][0];
     uint64_t* F1 = a.F[1][0];
-    if (cap > clean) {
+    if (!resume && cap > clean) {
       for (uint64_t i = clean + gt; i < cap; i += nt) {
         T0[i] = kEmpty;
         T1[i] = kEmpty;
@@ -878,8 +890,10 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
       if (!barrier()) return;
     }
     // --- select the live centres in order, and seed both sides with them
-    uint64_t nf = 0;
-    if (!GRAPHS && W <= (uint64_t)kMbThreads) {
+    nf = 0;
+    if (resume) {
+      nf = a.nf;
+    } else if (!GRAPHS && W <= (uint64_t)kMbThreads) {
       // every block selects the whole window; rank r is seeded by block r % grid
       uint32_t v = 0;
       bool sel = false;
@@ -977,11 +991,20 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
       if (!barrier()) return;
       continue;
     }
-    if (!barrier()) return;
+    if (resume) {
+      n0 = a.n0;
+      n1 = a.n1;
+      e0 = a.e0;
+      e1 = a.e1;
+      buf = (int)a.buf;
+      resume = false;
+    } else {
+      if (!barrier()) return;
+      n0 = n1 = e0 = e1 = nf;
+      buf = 0;
+    }
 
     // --- sub-rounds
-    uint64_t n0 = nf, n1 = nf, e0 = nf, e1 = nf;
-    int buf = 0;
     bool give_up = false;
     while (n0 | n1) {
       Counters* c0 = a.ctr + kMbCtr + 2 * (subs % 3);
@@ -1041,13 +1064,14 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
       e0 += __ldcg(&c0->inserted);
       e1 += __ldcg(&c1->inserted);
       buf ^= 1;
-      if ((__ldcg(&c0->fail) | __ldcg(&c1->fail)) || 2 * e0 > cap || 2 * e1 > cap) {
+      if ((n0 | n1) &&
+          ((__ldcg(&c0->fail) | __ldcg(&c1->fail)) || 2 * e0 > cap || 2 * e1 > cap)) {
         give_up = true;
         break;
       }
     }
     if (give_up) {
-      why = MB_HOST;
+      why = MB_GROW;
       break;
     }
     // --- partition (scc.hpp:437-464), and clear the other set for the next batch
@@ -1128,6 +1152,14 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
     s.heavy_edges = t_he;
     s.heavy_probes = t_hp;
     s.slots = slots;
+    s.cap = cap;
+    s.nf = nf;
+    s.n0 = n0;
+    s.n1 = n1;
+    s.e0 = e0;
+    s.e1 = e1;
+    s.set = (uint32_t)set;
+    s.buf = (uint32_t)buf;
     s.why = why;
   }
 }
@@ -1139,12 +1171,13 @@ static uint64_t pow2_at_least(uint64_t x) {
 }
 
 // Rehash the table in slot tslot into a new table of capacity cap2.
-static int ms_grow(psc_graph_s* g, int tslot, uint64_t cap, uint64_t cap2) {
+// (in a buffer of at least `room` slots).
+static int ms_grow(psc_graph_s* g, int tslot, uint64_t cap, uint64_t cap2, uint64_t room = 0) {
   cudaEvent_t ea = take_event(g), eb = take_event(g);
   PSC_CUDA(cudaEventRecord(ea, g->stream));
   unsigned long long *T, *T2;
   T = (unsigned long long*)g->bufs[tslot].p;
-  PSC_TRY(ensure_t(g, B_TS, cap2, &T2));
+  PSC_TRY(ensure_t(g, B_TS, std::max(cap2, room), &T2));
   PSC_CUDA(cudaMemsetAsync(T2, 0xFF, cap2 * 8, g->stream));
   {
     ProfScope ps(g, F_TABLE);
@@ -1380,8 +1413,12 @@ bool ms_run_ready(psc_graph_s* g) {
   return st == 1;
 }
 
-// 2^20 slots hold every batch of the R-MAT 2^26, kNN 10^7 and 4096^2 grid
-// solves; a smaller graph's tables are smaller.
+// Largest window of the resident launch (a batch's tables have four slots per
+// candidate at least).
+constexpr uint64_t kMbWindow = 1 << 18;
+
+// Tables to begin with: 2^20 slots hold every batch of the R-MAT 2^26, kNN 10^7
+// and 4096^2 grid solves; a smaller graph's tables are smaller.
 static uint64_t mb_cap_max(const psc_graph_s* g) {
   return std::min<uint64_t>(1ull << 20, std::max<uint64_t>(1ull << 13, pow2_at_least(16 * g->n)));
 }
@@ -1394,56 +1431,86 @@ int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, 
   a.E = g->E;
   a.in_E = g->in_E;
   a.labels = labels;
-  a.run = *run;
   a.beta = p->beta;
   a.tau = p->tau ? p->tau : 512;
   a.local = p->local_scc != 0;
   a.vgc_limit = run->vgc_max ? run->vgc_max : (uint64_t)g->num_sms * 32;
   a.cap_max = mb_cap_max(g);
-  // a first batch that cannot fit goes to ms_pair without a launch
-  if (mb_cap(window, run->ne[0], run->ne[1], a.vgc_limit, a.tau) > a.cap_max) return PSC_OK;
+  // windows of more than kMbWindow candidates are full-width work: ms_pair; others
+  // get the tables that they need
+  if (window > kMbWindow) return PSC_OK;
+  a.cap_max = std::max(a.cap_max, mb_cap(window, run->ne[0], run->ne[1], a.vgc_limit, a.tau));
   static const int kT[2][2] = {{B_TF, B_TB}, {B_TF2, B_TB2}}, kF[2][2] = {{B_PA, B_PB}, {B_PA2, B_PB2}};
-  for (int s = 0; s < 2; s++)
-    for (int k = 0; k < 2; k++) {
-      PSC_TRY(ensure_t(g, kT[s][k], a.cap_max, &a.T[s][k]));
-      PSC_TRY(ensure_t(g, kF[s][k], a.cap_max, &a.F[s][k]));
-    }
-  PSC_TRY(ensure_t(g, B_PH, a.cap_max, &a.Fh[0]));
-  PSC_TRY(ensure_t(g, B_PH2, a.cap_max, &a.Fh[1]));
-  PSC_TRY(ensure_t(g, B_AUX1, a.cap_max, &a.hf[0]));
-  PSC_TRY(ensure_t(g, B_HF2, a.cap_max, &a.hf[1]));
   PSC_TRY(ensure_t(g, B_BLOCKS, (size_t)g->num_sms, &a.counts));
   a.ctr = g->ctr;
   a.st = (MbState*)(g->ctr + kMbState);
-  PSC_TRY(zero_counters(g));
-  {
-    ProfScope ps(g, F_MS_VGC);
-    void* args[] = {&a};
-    PSC_CUDA(cudaLaunchCooperativeKernel(
-        run->sched ? (const void*)k_ms_batches<true> : (const void*)k_ms_batches<false>,
-        dim3((unsigned)g->num_sms), dim3(kMbThreads), args, sizeof(MbShared), g->stream));
-  }
-  PSC_TRY(read_counters(g));
   const MbState& s = *(const MbState*)(g->hctr + kMbState);
-  if (s.failed || s.why == MB_RUNNING) return PSC_ERR_ITER_LIMIT;
-  run->cur = s.cur;
-  run->step = s.step;
-  run->label_offset = s.label_offset;
-  run->round = s.round;
-  run->ne[0] = s.ne[0];
-  run->ne[1] = s.ne[1];
-  run->done = s.why == MB_DONE;
-  g->stats.batches += s.batches;
-  g->stats.subrounds += 2 * s.subrounds;
-  if (g->profiling) {
-    // as for the separate kernels (see ms_pair and scc_partition)
-    g->prof[F_MS_VGC].bytes += 8.0 * s.pairs + 16.0 * s.expanded + 12.0 * s.edges + 8.0 * s.probes;
-    g->prof[F_HEAVY].bytes += 28.0 * s.heavy + 12.0 * s.heavy_edges + 8.0 * s.heavy_probes;
-    g->prof[F_PARTITION].bytes += 8.0 * s.slots;
+  for (;;) {
+    a.run = *run;
+    for (int x = 0; x < 2; x++)
+      for (int k = 0; k < 2; k++) {
+        PSC_TRY(ensure_t(g, kT[x][k], a.cap_max, &a.T[x][k]));
+        PSC_TRY(ensure_t(g, kF[x][k], a.cap_max, &a.F[x][k]));
+      }
+    PSC_TRY(ensure_t(g, B_PH, a.cap_max, &a.Fh[0]));
+    PSC_TRY(ensure_t(g, B_PH2, a.cap_max, &a.Fh[1]));
+    PSC_TRY(ensure_t(g, B_AUX1, a.cap_max, &a.hf[0]));
+    PSC_TRY(ensure_t(g, B_HF2, a.cap_max, &a.hf[1]));
+    PSC_TRY(zero_counters(g));
+    {
+      ProfScope ps(g, F_MS_VGC);
+      void* args[] = {&a};
+      PSC_CUDA(cudaLaunchCooperativeKernel(
+          run->sched ? (const void*)k_ms_batches<true> : (const void*)k_ms_batches<false>,
+          dim3((unsigned)g->num_sms), dim3(kMbThreads), args, sizeof(MbShared), g->stream));
+    }
+    PSC_TRY(read_counters(g));
+    if (s.failed || s.why == MB_RUNNING) return PSC_ERR_ITER_LIMIT;
+    run->cur = s.cur;
+    run->step = s.step;
+    run->label_offset = s.label_offset;
+    run->round = s.round;
+    run->ne[0] = s.ne[0];
+    run->ne[1] = s.ne[1];
+    g->stats.batches += s.batches;
+    g->stats.subrounds += 2 * s.subrounds;
+    if (g->profiling) {
+      // as for the separate kernels (see ms_pair and scc_partition)
+      g->prof[F_MS_VGC].bytes += 8.0 * s.pairs + 16.0 * s.expanded + 12.0 * s.edges + 8.0 * s.probes;
+      g->prof[F_HEAVY].bytes += 28.0 * s.heavy + 12.0 * s.heavy_edges + 8.0 * s.heavy_probes;
+      g->prof[F_PARTITION].bytes += 8.0 * s.slots;
+    }
+    if (trace_on())
+      std::fprintf(stderr, "ms resident: %llu batches, %llu sub-rounds, pairs %llu edges %llu why %u\n",
+                   s.batches, s.subrounds, s.pairs, s.edges, s.why);
+    a.cap = 0;
+    a.set = 0;
+    if (s.why == MB_HOST && s.nf <= kMbWindow) {  // a larger table is all it needs
+      a.cap_max = s.cap;
+      continue;
+    }
+    if (s.why != MB_GROW) break;
+    // grow both tables of the batch at hand to a quarter load (the other set and
+    // what a sub-round writes anew need not keep their contents)
+    const uint64_t cap2 = pow2_at_least(std::max<uint64_t>(4 * std::max(s.e0, s.e1), 2 * s.cap));
+    if (cap2 > (1ull << 40)) return PSC_ERR_TABLE_FULL;
+    a.cap = cap2;
+    a.nf = s.nf;
+    a.n0 = s.n0;
+    a.n1 = s.n1;
+    a.e0 = s.e0;
+    a.e1 = s.e1;
+    a.set = s.set;
+    a.buf = s.buf;
+    a.cap_max = std::max(a.cap_max, cap2);
+    const uint64_t keep[2] = {a.n0, a.n1}, old_cap = s.cap;
+    for (int k = 0; k < 2; k++) {
+      PSC_TRY(ms_grow(g, kT[a.set][k], old_cap, cap2, a.cap_max));
+      void* q;
+      PSC_TRY(ensure_keep(g, kF[k][a.buf], a.cap_max * 8 + 16, keep[k] * 8, &q));
+    }
   }
-  if (trace_on())
-    std::fprintf(stderr, "ms resident: %llu batches, %llu sub-rounds, pairs %llu edges %llu %s\n",
-                 s.batches, s.subrounds, s.pairs, s.edges, run->done ? "done" : "to the host");
+  run->done = s.why == MB_DONE;
   return PSC_OK;
 }
 
