@@ -7,43 +7,42 @@
 
 namespace psc {
 
-struct CntValue {
-  const uint32_t* cnt;
-  __device__ uint32_t operator()(uint64_t i) const { return cnt[i]; }
-};
-
-struct OffEmit {
-  uint64_t* in_off;
-  uint32_t* cursor_reset;
-  __device__ void operator()(uint64_t i, uint64_t excl, uint32_t) const {
-    in_off[i] = excl;
-    cursor_reset[i] = 0;
-  }
-};
-
 // ---------------------------------------------------------------------------
 // Radix transpose: the (target, source) pairs of all edges, generated in CSR
 // order (sorted by source), sorted by target with a stable LSD radix sort of
 // kRsBits-bit digits.  Stability keeps every in-list ordered by source, as
-// the reference's sort-based transpose leaves it.  Each pass: a per-tile
-// digit histogram in shared memory, one scan over (digit, tile), and a stable
-// scatter in which every warp ranks its sub-tile with __match_any_sync.  No
-// global atomics, so hub targets cost nothing extra.
+// the reference's sort-based transpose leaves it.
+//
+// What bounds it is the traffic of the passes (16 bytes per pair and pass), as
+// long as nothing else is read: the histograms of all digits come from one read of
+// the keys, and a pass finds the places of its tiles' digit runs while it runs,
+// by looking back over the tiles before it (decoupled look-back: a tile publishes
+// its digit counts, later their prefix sums), so there is no histogram pass and no
+// scan per digit.  Tiles are numbered by a ticket, so the tiles that one waits for
+// are running or done; every wait is bounded.
+// R-MAT 2^22, 6.6e7 edges, 3 passes: histogram 0.37, scan 0.03 and scatter 0.60 ms
+// per pass -> one read of 0.08 ms and 0.53 per pass; sources 0.35 -> 0.15, offsets
+// 0.28 -> 0.08.
 // ---------------------------------------------------------------------------
 constexpr int kRsBits = 8;
 constexpr int kRsBins = 1 << kRsBits;
 constexpr int kRsBlock = 256;
-constexpr int kRsTile = 4096;  // pairs per block and pass (16 per thread)
+constexpr int kRsTile = 3072;  // pairs per block and pass (12 per thread)
+constexpr int kRsMaxPasses = 4;
+constexpr int kRsLook = 4;
+constexpr uint32_t kRsSpin = 1u << 22;  // polls of one wait
+// Status word of a (tile, digit): nothing yet, the tile's count, or the count of
+// all tiles up to it.
+constexpr uint64_t kRsCount = 1ull << 62, kRsPrefix = 2ull << 62, kRsValue = kRsCount - 1;
 
-// src[e] = the vertex whose adjacency holds edge e.  A warp takes 32 * 32
-// consecutive edges; the sources of its first and last edge bound a small
-// vertex range (one vertex for a hub), which every lane's binary search then
-// covers; stores are coalesced.
-constexpr int kSrcRun = 32 * 32;
-
-__device__ __forceinline__ uint64_t edge_owner(const uint64_t* __restrict__ off, uint64_t lo,
-                                               uint64_t hi, uint64_t e) {
-  while (lo < hi) {  // largest u in [lo, hi] with off[u] <= e
+// src[e] = the vertex whose adjacency holds edge e.  A block takes kRsTile
+// consecutive edges: each vertex whose list begins inside the tile marks its first
+// edge, and a running maximum over the marks gives every edge its owner (instead
+// of a binary search per edge).
+__device__ __forceinline__ uint64_t edge_owner(const uint64_t* __restrict__ off, uint64_t n,
+                                               uint64_t e) {
+  uint64_t lo = 0, hi = n - 1;
+  while (lo < hi) {  // largest u with off[u] <= e
     const uint64_t mid = (lo + hi + 1) >> 1;
     if (__ldg(&off[mid]) <= e)
       lo = mid;
@@ -53,230 +52,414 @@ __device__ __forceinline__ uint64_t edge_owner(const uint64_t* __restrict__ off,
   return lo;
 }
 
-__global__ void k_edge_sources(const uint64_t* __restrict__ off, uint64_t n, uint64_t m,
-                               uint32_t* src) {
-  const unsigned lane = lane_id();
-  const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const uint64_t runs = (m + kSrcRun - 1) / kSrcRun;
-  for (uint64_t r = gw; r < runs; r += nw) {
-    const uint64_t e0 = r * kSrcRun;
-    const uint64_t e1 = e0 + kSrcRun < m ? e0 + kSrcRun : m;
-    uint64_t b = 0;
-    if (lane == 0) b = edge_owner(off, 0, n - 1, e0);
-    if (lane == 1) b = edge_owner(off, 0, n - 1, e1 - 1);
-    const uint64_t lo = __shfl_sync(kFull, b, 0), hi = __shfl_sync(kFull, b, 1);
-    for (uint64_t e = e0 + lane; e < e1; e += 32) src[e] = (uint32_t)edge_owner(off, lo, hi, e);
+// owner[2 t], owner[2 t + 1]: the owners of the first and the last edge of tile t
+// (searched for all tiles at once: inside the tile's block the 20-odd dependent
+// steps were most of its time).
+__global__ void k_tile_owners(const uint64_t* __restrict__ off, uint64_t n, uint64_t m,
+                              uint32_t* owner) {
+  const uint64_t ends = 2 * ((m + kRsTile - 1) / kRsTile);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ends;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t e0 = (i >> 1) * kRsTile;
+    const uint64_t e1 = e0 + kRsTile < m ? e0 + kRsTile : m;
+    owner[i] = (uint32_t)edge_owner(off, n, (i & 1) ? e1 - 1 : e0);
   }
 }
 
-// Per-tile digit histograms.  Every thread holds kRsPer keys of its warp's
-// sub-tile in registers (loaded first, so their latencies overlap); equal
-// digits of a warp add to the shared histogram once.
-constexpr int kRsPer = kRsTile / kRsBlock;  // 16 keys per thread
-
 __global__ void __launch_bounds__(kRsBlock)
-    k_rs_hist(const uint32_t* __restrict__ keys, uint64_t m, int shift, uint64_t ntiles,
-              uint32_t* hist) {
-  __shared__ uint32_t cnt[kRsBins];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1;
+    k_edge_sources(const uint64_t* __restrict__ off, const uint32_t* __restrict__ owner,
+                   uint64_t m, uint32_t* src) {
+  constexpr int NW = kRsBlock / 32, PER = kRsTile / NW;
+  __shared__ uint32_t mark[kRsTile];
+  __shared__ uint32_t wmax[NW];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5, tid = threadIdx.x;
+  const uint64_t ntiles = (m + kRsTile - 1) / kRsTile;
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    for (int b = threadIdx.x; b < kRsBins; b += kRsBlock) cnt[b] = 0;
+    const uint64_t e0 = tile * kRsTile;
+    const uint64_t e1 = e0 + kRsTile < m ? e0 + kRsTile : m;
+    const uint64_t v0 = __ldg(&owner[2 * tile]), v1 = __ldg(&owner[2 * tile + 1]);
+    for (int i = tid; i < kRsTile; i += kRsBlock) mark[i] = 0;
     __syncthreads();
-    const uint64_t base = tile * kRsTile + (uint64_t)wid * (kRsTile / (kRsBlock / 32));
-    uint32_t d[kRsPer];
-#pragma unroll
-    for (int c = 0; c < kRsPer; c++) {
-      const uint64_t i = base + c * 32 + lane;
-      d[c] = i < m ? (__ldg(&keys[i]) >> shift) & (kRsBins - 1) : kRsBins;
-    }
-#pragma unroll
-    for (int c = 0; c < kRsPer; c++) {
-      const unsigned peers = __match_any_sync(kFull, d[c]);
-      if (d[c] < (uint32_t)kRsBins && (peers & lt) == 0) atomicAdd(&cnt[d[c]], (uint32_t)__popc(peers));
-    }
+    for (uint64_t v = v0 + 1 + tid; v <= v1; v += kRsBlock)
+      atomicMax(&mark[__ldg(&off[v]) - e0], (uint32_t)(v - v0));
     __syncthreads();
-    for (int b = threadIdx.x; b < kRsBins; b += kRsBlock) hist[(uint64_t)b * ntiles + tile] = cnt[b];
+    uint32_t run = 0;  // maximum so far of the warp's part
+    for (int c = 0; c < PER / 32; c++) {
+      uint32_t x = mark[wid * PER + c * 32 + lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if ((int)lane >= o && y > x) x = y;
+      }
+      x = x > run ? x : run;
+      mark[wid * PER + c * 32 + lane] = x;
+      run = __shfl_sync(kFull, x, 31);
+    }
+    if (lane == 0) wmax[wid] = run;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < (int)wid; w++) before = wmax[w] > before ? wmax[w] : before;
+    for (int c = 0; c < PER / 32; c++) {
+      const uint64_t i = wid * PER + c * 32 + lane;
+      const uint32_t x = mark[i];
+      if (e0 + i < e1) src[e0 + i] = (uint32_t)v0 + (x > before ? x : before);
+    }
     __syncthreads();
   }
 }
 
-// Stable scatter of one pass.  Each warp owns kRsTile / 8 consecutive pairs
-// of the tile (chunks of 32 in order, lanes in order), held in registers.
-// The tile is first sorted by digit in shared memory (warp counts, a block
-// scan over digits, ranked placement), then written out so that consecutive
-// threads write consecutive positions of one digit's run: coalesced stores
-// instead of one sector per pair.
+// Counts of every digit of every pass in one read of the keys (per-warp
+// histograms in shared memory).
+template <int PASSES>
 __global__ void __launch_bounds__(kRsBlock)
-    k_rs_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t m,
-                 int shift, uint64_t ntiles, const uint64_t* __restrict__ offs, uint32_t* kout,
-                 uint32_t* vout) {
+    k_rs_count(const uint32_t* __restrict__ keys, uint64_t m, unsigned long long* hist) {
+  __shared__ uint32_t h[kRsBlock / 32][PASSES][kRsBins];
+  const unsigned wid = threadIdx.x >> 5;
+  uint32_t* all = &h[0][0][0];
+  for (int i = threadIdx.x; i < kRsBlock / 32 * PASSES * kRsBins; i += kRsBlock) all[i] = 0;
+  __syncthreads();
+  const uint64_t stride = (uint64_t)gridDim.x * kRsBlock;
+  const uint64_t t = (uint64_t)blockIdx.x * kRsBlock + threadIdx.x;
+  auto add = [&](uint32_t k) {
+#pragma unroll
+    for (int p = 0; p < PASSES; p++) atomicAdd(&h[wid][p][(k >> (p * kRsBits)) & (kRsBins - 1)], 1u);
+  };
+  const uint64_t nq = m / 4;
+  const uint4* k4 = reinterpret_cast<const uint4*>(keys);  // (pool memory: 16-byte aligned)
+  for (uint64_t q = t; q < nq; q += stride) {
+    const uint4 x = __ldg(&k4[q]);
+    add(x.x);
+    add(x.y);
+    add(x.z);
+    add(x.w);
+  }
+  for (uint64_t i = nq * 4 + t; i < m; i += stride) add(keys[i]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < PASSES * kRsBins; i += kRsBlock) {
+    unsigned long long c = 0;
+    for (int w = 0; w < kRsBlock / 32; w++) c += h[w][i / kRsBins][i % kRsBins];
+    if (c) atomicAdd(&hist[i], c);
+  }
+}
+
+// Digit starts of a pass: the exclusive sums of its counts, in place.
+__global__ void __launch_bounds__(kRsBins) k_rs_starts(unsigned long long* hist) {
+  __shared__ uint64_t sm[33];
+  unsigned long long* h = hist + (uint64_t)blockIdx.x * kRsBins;
+  uint64_t all;
+  const uint64_t start = block_excl_scan<kRsBins>(h[threadIdx.x], sm, &all);
+  h[threadIdx.x] = start;
+}
+
+// One stable pass.  Each warp owns kRsTile / 8 consecutive pairs of the tile
+// (chunks of 32 in order, lanes in order), held in registers.  The tile is sorted
+// by digit in shared memory (warp counts, a block scan over digits, ranked
+// placement), then written out so that consecutive threads write consecutive
+// positions of one digit's run: coalesced stores instead of one sector per pair.
+constexpr int kRsPer = kRsTile / kRsBlock;  // keys per thread
+
+// (Pairs as 64-bit words between passes were measured and dropped: 0.61 ms a pass
+// instead of 0.53, the ranked placement then meets twice the bank conflicts.)
+__global__ void __launch_bounds__(kRsBlock)
+    k_rs_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t m,
+              int shift, const unsigned long long* __restrict__ starts, uint32_t* ticket,
+              unsigned long long* status, uint32_t* kout, uint32_t* vout,
+              unsigned long long* failed) {
   constexpr int NW = kRsBlock / 32;
   constexpr int PER_WARP = kRsTile / NW;
   static_assert(kRsBins == kRsBlock, "one digit per thread in the digit scan");
   __shared__ uint32_t skey[kRsTile];
   __shared__ uint32_t sval[kRsTile];
   __shared__ uint32_t wcnt[NW][kRsBins];
-  __shared__ uint32_t lstart[kRsBins];
   __shared__ uint64_t gbase[kRsBins];
   __shared__ uint64_t scan_sm[33];
+  __shared__ uint32_t s_tile, s_bad;
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5, tid = threadIdx.x;
   const unsigned lt = (1u << lane) - 1;
-  for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint64_t tbase = tile * kRsTile;
-    const uint64_t base = tbase + (uint64_t)wid * PER_WARP;
-    const uint32_t tcount = (uint32_t)(m - tbase < (uint64_t)kRsTile ? m - tbase : kRsTile);
-    uint32_t key[kRsPer], val[kRsPer], d[kRsPer];
+  if (tid == 0) {
+    s_tile = atomicAdd(ticket, 1u);
+    s_bad = 0;
+  }
+  for (int b = lane; b < kRsBins; b += 32) wcnt[wid][b] = 0;
+  __syncthreads();
+  const uint64_t tile = s_tile;
+  const uint64_t tbase = tile * kRsTile;
+  const uint64_t base = tbase + (uint64_t)wid * PER_WARP;
+  const uint32_t tcount = (uint32_t)(m - tbase < (uint64_t)kRsTile ? m - tbase : kRsTile);
+  uint32_t key[kRsPer], val[kRsPer];
 #pragma unroll
-    for (int c = 0; c < kRsPer; c++) {
-      const uint64_t i = base + c * 32 + lane;
-      key[c] = 0;
-      val[c] = 0;
-      d[c] = kRsBins;
-      if (i < m) {
-        key[c] = __ldg(&kin[i]);
-        val[c] = __ldg(&vin[i]);
-        d[c] = (key[c] >> shift) & (kRsBins - 1);
-      }
+  for (int c = 0; c < kRsPer; c++) {
+    const uint64_t i = base + c * 32 + lane;
+    key[c] = i < m ? __ldg(&kin[i]) : 0u;
+  }
+#pragma unroll
+  for (int c = 0; c < kRsPer; c++) {
+    const uint64_t i = base + c * 32 + lane;
+    val[c] = i < m ? __ldg(&vin[i]) : 0u;
+  }
+  // lanes of a chunk with the same digit, found by one ballot per digit bit
+  unsigned peers[kRsPer];
+#pragma unroll
+  for (int c = 0; c < kRsPer; c++) {
+    const bool in = base + c * 32 + lane < m;
+    unsigned p = __ballot_sync(kFull, in);
+    const uint32_t d = key[c] >> shift;
+#pragma unroll
+    for (int b = 0; b < kRsBits; b++) {
+      const bool bit = (d >> b) & 1u;
+      const unsigned v = __ballot_sync(kFull, bit);
+      p &= bit ? v : ~v;
     }
-    for (int b = lane; b < kRsBins; b += 32) wcnt[wid][b] = 0;
+    peers[c] = in ? p : 0u;
+    if (in && (p & lt) == 0) wcnt[wid][d & (kRsBins - 1)] += __popc(p);
     __syncwarp();
-    unsigned peers[kRsPer];
+  }
+  __syncthreads();
+  // digit tid: the tile's count is published, then its start in the sorted tile
+  // and each warp's base inside it
+  uint32_t total = 0;
 #pragma unroll
-    for (int c = 0; c < kRsPer; c++) {
-      peers[c] = __match_any_sync(kFull, d[c]);
-      if (d[c] < (uint32_t)kRsBins && (peers[c] & lt) == 0) wcnt[wid][d[c]] += __popc(peers[c]);
-      __syncwarp();
+  for (int w = 0; w < NW; w++) total += wcnt[w][tid];
+  volatile unsigned long long* row = status + tile * kRsBins + tid;
+  *row = (tile ? kRsCount : kRsPrefix) | total;
+  uint64_t all = 0;
+  const uint32_t start = (uint32_t)block_excl_scan<kRsBlock>(total, scan_sm, &all);
+  uint32_t run = start;
+#pragma unroll
+  for (int w = 0; w < NW; w++) {
+    const uint32_t c = wcnt[w][tid];
+    wcnt[w][tid] = run;
+    run += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < kRsPer; c++) {
+    const uint32_t d = (key[c] >> shift) & (kRsBins - 1);
+    uint32_t lp = 0;
+    if (peers[c]) lp = wcnt[wid][d] + __popc(peers[c] & lt);
+    __syncwarp();
+    if (peers[c]) {
+      skey[lp] = key[c];
+      sval[lp] = val[c];
+      if ((peers[c] & lt) == 0) wcnt[wid][d] += __popc(peers[c]);
     }
-    __syncthreads();
-    // digit tid: its start in the sorted tile, each warp's base inside it, and
-    // the global start of its run for this tile
-    {
-      uint32_t total = 0;
+    __syncwarp();
+  }
+  // look back, kRsLook tiles' words at a time (8 / 16 / 32 at a time: 1 / 2 / 8 %
+  // slower; the pass is bound by instructions, not by this wait)
+  uint64_t before = 0;
+  bool open = tile > 0;
+  for (uint64_t t = tile; open;) {
+    unsigned long long x[kRsLook];
 #pragma unroll
-      for (int w = 0; w < NW; w++) total += wcnt[w][tid];
-      uint64_t all = 0;
-      const uint32_t start = (uint32_t)block_excl_scan<kRsBlock>(total, scan_sm, &all);
-      lstart[tid] = start;
-      gbase[tid] = offs[(uint64_t)tid * ntiles + tile];
-      uint32_t run = start;
+    for (int k = 0; k < kRsLook; k++)
+      x[k] = t > (uint64_t)k ? *(volatile unsigned long long*)(status + (t - 1 - k) * kRsBins + tid)
+                             : kRsPrefix;
 #pragma unroll
-      for (int w = 0; w < NW; w++) {
-        const uint32_t c = wcnt[w][tid];
-        wcnt[w][tid] = run;
-        run += c;
+    for (int k = 0; k < kRsLook; k++) {
+      if (!open) break;
+      uint32_t spin = 0;
+      while (!(x[k] >> 62)) {
+        if (++spin > kRsSpin) {
+          s_bad = 1;
+          open = false;
+          break;
+        }
+        x[k] = *(volatile unsigned long long*)(status + (t - 1 - k) * kRsBins + tid);
       }
+      before += x[k] & kRsValue;
+      if (x[k] >> 63) open = false;
     }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < kRsPer; c++) {
-      uint32_t lp = 0;
-      if (d[c] < (uint32_t)kRsBins) lp = wcnt[wid][d[c]] + __popc(peers[c] & lt);
-      __syncwarp();
-      if (d[c] < (uint32_t)kRsBins) {
-        skey[lp] = key[c];
-        sval[lp] = val[c];
-        if ((peers[c] & lt) == 0) wcnt[wid][d[c]] += __popc(peers[c]);
-      }
-      __syncwarp();
-    }
-    __syncthreads();
-    for (uint32_t j = tid; j < tcount; j += kRsBlock) {
-      const uint32_t k = skey[j];
-      const uint32_t dj = (k >> shift) & (kRsBins - 1);
-      const uint64_t pos = gbase[dj] + (j - lstart[dj]);
-      kout[pos] = k;
-      vout[pos] = sval[j];
-    }
-    __syncthreads();
+    t -= t < (uint64_t)kRsLook ? t : (uint64_t)kRsLook;
+    if (t == 0) open = false;
+  }
+  if (tile) *row = kRsPrefix | (before + total);
+  gbase[tid] = starts[tid] + before - start;
+  __syncthreads();
+  if (s_bad) {
+    if (tid == 0) *failed = 1;
+    return;
+  }
+  for (uint32_t j = tid; j < tcount; j += kRsBlock) {
+    const uint32_t k = skey[j];
+    const uint64_t pos = gbase[(k >> shift) & (kRsBins - 1)] + j;
+    kout[pos] = k;
+    vout[pos] = sval[j];
   }
 }
 
-struct HistValue {
-  const uint32_t* hist;
-  __device__ uint32_t operator()(uint64_t i) const { return hist[i]; }
+// off[v] = first place of the sorted array t[0 .. m) with t >= v, for v in [0, n]:
+// the places between two neighbours t[i - 1] < t[i] belong to v in (t[i - 1], t[i]].
+// Gaps of more than kGapLong ids are listed (end of the range, value, start) and
+// filled by the whole grid afterwards.
+constexpr uint32_t kGapLong = 64;
+
+struct GapEnt {
+  uint64_t first, last, value;  // off[first .. last] = value
 };
 
-struct HistEmit {
-  uint64_t* offs;
-  __device__ void operator()(uint64_t i, uint64_t excl, uint32_t) const { offs[i] = excl; }
-};
-
-// In-degrees from the sorted targets: run starts record their position,
-// run ends turn it into the run length.
-__global__ void k_run_starts(const uint32_t* __restrict__ t, uint64_t m, uint64_t* rs) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    if (i == 0 || t[i - 1] != t[i]) rs[t[i]] = i;
+__global__ void k_bounds(const uint32_t* __restrict__ t, uint64_t m, uint64_t n, uint64_t* off,
+                         GapEnt* gaps, unsigned long long* ngaps) {
+  // ids after the one before place i, up to the one at place i
+  auto place = [&](uint64_t i, uint64_t a, uint64_t b) {
+    if (b + 1 > a + kGapLong) {
+      gaps[atomicAdd(ngaps, 1ull)] = GapEnt{a, b, i};
+    } else {
+      for (uint64_t v = a; v <= b; v++) off[v] = i;
+    }
+  };
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t nq = m / 4;
+  const uint4* t4 = reinterpret_cast<const uint4*>(t);  // (pool memory: 16-byte aligned)
+  for (uint64_t q = g; q < nq; q += stride) {
+    const uint4 x = __ldg(&t4[q]);
+    const uint64_t a = q ? (uint64_t)__ldg(&t[4 * q - 1]) + 1 : 0;
+    place(4 * q, a, x.x);
+    place(4 * q + 1, (uint64_t)x.x + 1, x.y);
+    place(4 * q + 2, (uint64_t)x.y + 1, x.z);
+    place(4 * q + 3, (uint64_t)x.z + 1, x.w);
+  }
+  for (uint64_t i = nq * 4 + g; i <= m; i += stride)
+    place(i, i ? (uint64_t)t[i - 1] + 1 : 0, i < m ? t[i] : n);
 }
 
-__global__ void k_run_lengths(const uint32_t* __restrict__ t, uint64_t m,
-                              const uint64_t* __restrict__ rs, uint32_t* cnt) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (uint64_t)gridDim.x * blockDim.x)
-    if (i == m - 1 || t[i + 1] != t[i]) cnt[t[i]] = (uint32_t)(i + 1 - rs[t[i]]);
+__global__ void k_fill_gaps(const GapEnt* __restrict__ gaps, const unsigned long long* __restrict__ ngaps,
+                            uint64_t* off) {
+  const uint64_t ng = *ngaps;
+  const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // short lists of long gaps: every gap over the grid; else a warp per gap
+  if (ng < 64) {
+    for (uint64_t g = 0; g < ng; g++) {
+      const GapEnt e = gaps[g];
+      for (uint64_t v = e.first + gt; v <= e.last; v += nt) off[v] = e.value;
+    }
+  } else {
+    for (uint64_t g = gt >> 5; g < ng; g += nt >> 5) {
+      const GapEnt e = gaps[g];
+      for (uint64_t v = e.first + (gt & 31); v <= e.last; v += 32) off[v] = e.value;
+    }
+  }
+}
+
+static int fill_bounds(psc_graph_s* g, const uint32_t* t, uint64_t m, uint64_t* off) {
+  const uint64_t n = g->n;
+  GapEnt* gaps;
+  PSC_TRY(ensure_t(g, B_SCAN3, n / kGapLong + 2, &gaps));
+  unsigned long long* ngaps = &g->ctr[3].aux0;  // staging set
+  PSC_CUDA(cudaMemsetAsync(ngaps, 0, 8, g->stream));
+  {
+    ProfScope ps(g, F_TRANSPOSE);
+    ps.bytes = 4.0 * m + 8.0 * n;
+    k_bounds<<<grid_for(g, m + 1, 256), 256, 0, g->stream>>>(t, m, n, off, gaps, ngaps);
+    k_fill_gaps<<<g->num_sms * 4, 256, 0, g->stream>>>(gaps, ngaps, off);
+  }
+  PSC_CUDA(cudaGetLastError());
+  return PSC_OK;
+}
+
+static int digit_passes(uint64_t n) {
+  int bits = 1;
+  while (bits < 32 && ((uint64_t)1 << bits) < n) bits++;
+  return (bits + kRsBits - 1) / kRsBits;
+}
+
+// Scratch of a sort: digit counts of every pass, tickets and status words.
+struct RsScratch {
+  unsigned long long *hist, *status, *failed;
+  uint32_t* ticket;
+};
+
+static int rs_scratch(psc_graph_s* g, uint64_t cnt, RsScratch* r) {
+  const uint64_t ntiles = (cnt + kRsTile - 1) / kRsTile;
+  PSC_TRY(ensure_t(g, B_AUX3, ntiles * kRsBins, &r->status));
+  PSC_TRY(ensure_t(g, B_SCAN2, kRsMaxPasses * kRsBins + 2, &r->hist));
+  r->ticket = (uint32_t*)(r->hist + kRsMaxPasses * kRsBins);
+  r->failed = &g->ctr[3].aux1;  // staging set, read by rs_check
+  PSC_CUDA(cudaMemsetAsync(r->failed, 0, 8, g->stream));
+  return PSC_OK;
+}
+
+// The owners use the status words' room (a sort clears those before each pass).
+static void launch_edge_sources(psc_graph_s* g, const RsScratch& r, uint32_t* src) {
+  const uint64_t ntiles = (g->m + kRsTile - 1) / kRsTile;
+  uint32_t* owner = (uint32_t*)r.status;
+  k_tile_owners<<<grid_for(g, 2 * ntiles, 128), 128, 0, g->stream>>>(g->off, g->n, g->m, owner);
+  k_edge_sources<<<(unsigned)std::min<uint64_t>(ntiles, g->num_sms * 8), kRsBlock, 0, g->stream>>>(
+      g->off, owner, g->m, src);
+}
+
+// The digit counts of all passes over keys.
+static int rs_count(psc_graph_s* g, const uint32_t* keys, uint64_t cnt, int passes,
+                    const RsScratch& r) {
+  PSC_CUDA(cudaMemsetAsync(r.hist, 0, kRsMaxPasses * kRsBins * 8, g->stream));
+  ProfScope ps(g, F_TRANSPOSE);
+  ps.bytes = 4.0 * cnt;
+  const unsigned grid = (unsigned)std::min<uint64_t>((cnt + kRsTile - 1) / kRsTile, g->num_sms * 6);
+  switch (passes) {
+    case 1: k_rs_count<1><<<grid, kRsBlock, 0, g->stream>>>(keys, cnt, r.hist); break;
+    case 2: k_rs_count<2><<<grid, kRsBlock, 0, g->stream>>>(keys, cnt, r.hist); break;
+    case 3: k_rs_count<3><<<grid, kRsBlock, 0, g->stream>>>(keys, cnt, r.hist); break;
+    default: k_rs_count<4><<<grid, kRsBlock, 0, g->stream>>>(keys, cnt, r.hist); break;
+  }
+  k_rs_starts<<<passes, kRsBins, 0, g->stream>>>(r.hist);
+  PSC_CUDA(cudaGetLastError());
+  return PSC_OK;
+}
+
+// All passes over cnt pairs: from (kin, vin), by way of pair[0] and pair[1] (cnt
+// keys, then cnt values, each), into (kout, vout).
+static int rs_sort(psc_graph_s* g, uint64_t cnt, int passes, const uint32_t* kin,
+                   const uint32_t* vin, uint64_t* pair[2], const RsScratch& r, uint32_t* kout,
+                   uint32_t* vout) {
+  const uint64_t ntiles = (cnt + kRsTile - 1) / kRsTile;
+  PSC_TRY(rs_count(g, kin, cnt, passes, r));
+  for (int p = 0; p < passes; p++) {
+    PSC_CUDA(cudaMemsetAsync(r.status, 0, ntiles * kRsBins * 8, g->stream));
+    PSC_CUDA(cudaMemsetAsync(r.ticket, 0, 4, g->stream));
+    ProfScope ps(g, F_TRANSPOSE);
+    ps.bytes = 16.0 * cnt;
+    const bool first = p == 0, last = p + 1 == passes;
+    const uint32_t* ki = first ? kin : (const uint32_t*)pair[(p + 1) & 1];
+    uint32_t* ko = last ? kout : (uint32_t*)pair[p & 1];
+    k_rs_pass<<<(unsigned)ntiles, kRsBlock, 0, g->stream>>>(
+        ki, first ? vin : ki + cnt, cnt, p * kRsBits, r.hist + (uint64_t)p * kRsBins, r.ticket,
+        r.status, ko, last ? vout : ko + cnt, r.failed);
+    PSC_CUDA(cudaGetLastError());
+  }
+  return PSC_OK;
+}
+
+// Waits for the sorts queued so far; an error if one gave up a wait.
+static int rs_check(psc_graph_s* g) {
+  PSC_TRY(read_counters(g));
+  return g->hctr[3].aux1 ? PSC_ERR_ITER_LIMIT : PSC_OK;
 }
 
 int build_transpose(psc_graph_s* g) {
   const uint64_t n = g->n, m = g->m;
-  uint32_t* cnt;
-  PSC_TRY(ensure_t(g, B_TMP32, n + 1, &cnt));
-  PSC_CUDA(cudaMemsetAsync(cnt, 0, (n + 1) * 4, g->stream));
-  if (m > 0) {
-    int bits = 1;
-    while (bits < 32 && ((uint64_t)1 << bits) < n) bits++;
-    const int passes = (bits + kRsBits - 1) / kRsBits;
-    const uint64_t ntiles = (m + kRsTile - 1) / kRsTile;
-    uint32_t *x, *ka, *kb, *hist;
-    uint64_t* offs;
-    PSC_TRY(ensure_t(g, B_AUX0, m, &x));
-    PSC_TRY(ensure_t(g, B_AUX1, m, &ka));
-    PSC_TRY(ensure_t(g, B_AUX2, m, &kb));
-    PSC_TRY(ensure_t(g, B_AUX3, (uint64_t)kRsBins * ntiles, &hist));
-    PSC_TRY(ensure_t(g, B_SCAN2, (uint64_t)kRsBins * ntiles + 1, &offs));
-    // value buffers alternate so that the last pass writes in_E
-    uint32_t* vb[2] = {passes % 2 ? x : g->in_E, passes % 2 ? g->in_E : x};
-    uint32_t* kbuf[2] = {ka, kb};
-    {
-      ProfScope ps(g, F_TRANSPOSE);
-      ps.bytes = 16.0 * n + 4.0 * m;
-      k_edge_sources<<<grid_for(g, (m + kSrcRun - 1) / kSrcRun * 32, 256), 256, 0, g->stream>>>(
-          g->off, n, m, vb[0]);
-    }
-    const uint32_t* kin = g->E;
-    const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)g->num_sms * 8);
-    for (int p = 0; p < passes; p++) {
-      const int shift = p * kRsBits;
-      {
-        ProfScope ps(g, F_TRANSPOSE);
-        ps.bytes = 4.0 * m;
-        k_rs_hist<<<grid, kRsBlock, 0, g->stream>>>(kin, m, shift, ntiles, hist);
-      }
-      PSC_TRY(scan_emit(g, (uint64_t)kRsBins * ntiles, HistValue{hist}, HistEmit{offs}, nullptr,
-                        F_TRANSPOSE));
-      {
-        ProfScope ps(g, F_TRANSPOSE);
-        ps.bytes = 16.0 * m;
-        k_rs_scatter<<<grid, kRsBlock, 0, g->stream>>>(kin, vb[p & 1], m, shift, ntiles, offs,
-                                                       kbuf[p & 1], vb[(p + 1) & 1]);
-      }
-      kin = kbuf[p & 1];
-    }
-    uint64_t* rs;
-    PSC_TRY(ensure_t(g, B_SCAN3, n + 1, &rs));
-    {
-      ProfScope ps(g, F_TRANSPOSE);
-      ps.bytes = 8.0 * m;
-      k_run_starts<<<grid_for(g, m, 256), 256, 0, g->stream>>>(kin, m, rs);
-      k_run_lengths<<<grid_for(g, m, 256), 256, 0, g->stream>>>(kin, m, rs, cnt);
-    }
+  if (m == 0) {
+    PSC_CUDA(cudaMemsetAsync(g->in_off, 0, (n + 1) * 8, g->stream));
+    return PSC_OK;
   }
-  uint64_t total = 0;
-  PSC_TRY(scan_emit(g, n, CntValue{cnt}, OffEmit{g->in_off, cnt}, &total, F_TRANSPOSE));
-  PSC_CUDA(cudaMemcpyAsync(g->in_off + n, &g->m, 8, cudaMemcpyHostToDevice, g->stream));
-  PSC_CUDA(cudaGetLastError());
-  return PSC_OK;
+  const int passes = digit_passes(n);
+  uint32_t *src, *key;
+  uint64_t* pair[2];
+  PSC_TRY(ensure_t(g, B_AUX0, m, &src));
+  PSC_TRY(ensure_t(g, B_QA, m, &key));
+  PSC_TRY(ensure_t(g, B_AUX1, m, &pair[0]));
+  PSC_TRY(ensure_t(g, B_AUX2, m, &pair[1]));
+  RsScratch r;
+  PSC_TRY(rs_scratch(g, m, &r));
+  {
+    ProfScope ps(g, F_TRANSPOSE);
+    ps.bytes = 16.0 * n + 4.0 * m;
+    launch_edge_sources(g, r, src);
+  }
+  PSC_TRY(rs_sort(g, m, passes, g->E, src, pair, r, key, g->in_E));
+  PSC_TRY(fill_bounds(g, key, m, g->in_off));
+  return rs_check(g);
 }
 
 
@@ -286,8 +469,7 @@ int build_transpose(psc_graph_s* g) {
 // dropped.  The 2m pairs (a, b) -- a's list holds b -- are sorted by b and
 // then stably by a with the radix passes above (an LSD sort of the key
 // (a, b)); one compaction keeps the first pair of every run of equal pairs
-// when a != b, writing the targets; out-degrees come from the run lengths of
-// the kept sources.
+// when a != b, writing the targets; the offsets come from the kept sources.
 // ---------------------------------------------------------------------------
 __global__ void k_sym_pairs(const uint32_t* __restrict__ E, const uint32_t* __restrict__ src,
                             uint64_t m, uint32_t* key, uint32_t* val) {
@@ -324,36 +506,6 @@ struct SymEmit {
   }
 };
 
-// Stable LSD radix sort of cnt (key, val) pairs by the low `bits` bits of
-// key, from (k[0], v[0]) through (k[1], v[1]) and back; *at receives the
-// index of the pair of buffers holding the result.
-static int radix_pairs(psc_graph_s* g, uint64_t cnt, int bits, uint32_t* k[2], uint32_t* v[2],
-                       uint32_t* hist, uint64_t* offs, int* at) {
-  const int passes = (bits + kRsBits - 1) / kRsBits;
-  const uint64_t ntiles = (cnt + kRsTile - 1) / kRsTile;
-  const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)g->num_sms * 8);
-  int cur = 0;
-  for (int p = 0; p < passes; p++) {
-    const int shift = p * kRsBits;
-    {
-      ProfScope ps(g, F_TRANSPOSE);
-      ps.bytes = 4.0 * cnt;
-      k_rs_hist<<<grid, kRsBlock, 0, g->stream>>>(k[cur], cnt, shift, ntiles, hist);
-    }
-    PSC_TRY(scan_emit(g, (uint64_t)kRsBins * ntiles, HistValue{hist}, HistEmit{offs}, nullptr,
-                      F_TRANSPOSE));
-    {
-      ProfScope ps(g, F_TRANSPOSE);
-      ps.bytes = 16.0 * cnt;
-      k_rs_scatter<<<grid, kRsBlock, 0, g->stream>>>(k[cur], v[cur], cnt, shift, ntiles, offs,
-                                                     k[cur ^ 1], v[cur ^ 1]);
-    }
-    cur ^= 1;
-  }
-  *at = cur;
-  return PSC_OK;
-}
-
 static void release(psc_graph_s* g, int b) {
   DevBuf& d = g->bufs[b];
   if (d.p) cudaFreeAsync(d.p, g->stream);
@@ -366,58 +518,45 @@ int build_symmetric(psc_graph_s* g) {
   uint64_t* off_s = nullptr;
   uint32_t* E_s = nullptr;
   uint64_t ms = 0;
-  uint32_t* cnt;
-  PSC_TRY(ensure_t(g, B_TMP32, n + 1, &cnt));
-  PSC_CUDA(cudaMemsetAsync(cnt, 0, (n + 1) * 4, g->stream));
   if (m > 0) {
     const uint64_t c = 2 * m;
-    int bits = 1;
-    while (bits < 32 && ((uint64_t)1 << bits) < n) bits++;
-    const uint64_t ntiles = (c + kRsTile - 1) / kRsTile;
-    uint32_t *k[2], *v[2], *hist, *asel;
-    uint64_t* offs;
-    PSC_TRY(ensure_t(g, B_AUX0, c, &k[0]));
-    PSC_TRY(ensure_t(g, B_AUX1, c, &v[0]));
-    PSC_TRY(ensure_t(g, B_AUX2, c, &k[1]));
-    PSC_TRY(ensure_t(g, B_QA, c, &v[1]));
-    PSC_TRY(ensure_t(g, B_AUX3, (uint64_t)kRsBins * ntiles, &hist));
-    PSC_TRY(ensure_t(g, B_SCAN2, (uint64_t)kRsBins * ntiles + 1, &offs));
+    const int passes = digit_passes(n);
+    uint32_t *k, *v;  // the pairs, between and after the sorts
+    uint64_t* pair[2];
+    PSC_TRY(ensure_t(g, B_AUX0, c, &k));
+    PSC_TRY(ensure_t(g, B_QA, c, &v));
+    PSC_TRY(ensure_t(g, B_AUX1, c, &pair[0]));
+    PSC_TRY(ensure_t(g, B_AUX2, c, &pair[1]));
+    RsScratch r;
+    PSC_TRY(rs_scratch(g, c, &r));
+    uint32_t* src = (uint32_t*)pair[0];
     {
       ProfScope ps(g, F_TRANSPOSE);
       ps.bytes = 16.0 * n + 4.0 * m;
-      k_edge_sources<<<grid_for(g, (m + kSrcRun - 1) / kSrcRun * 32, 256), 256, 0, g->stream>>>(
-          g->off, n, m, v[1]);
+      launch_edge_sources(g, r, src);
     }
     {
       ProfScope ps(g, F_TRANSPOSE);
       ps.bytes = 8.0 * m + 16.0 * m;
-      k_sym_pairs<<<grid_for(g, m, 256), 256, 0, g->stream>>>(g->E, v[1], m, k[0], v[0]);
+      k_sym_pairs<<<grid_for(g, m, 256), 256, 0, g->stream>>>(g->E, src, m, k, v);
     }
-    int at = 0;
-    PSC_TRY(radix_pairs(g, c, bits, k, v, hist, offs, &at));  // by target
-    // second pass set: the sources become the keys
-    uint32_t* k2[2] = {v[at], k[at ^ 1]};
-    uint32_t* v2[2] = {k[at], v[at ^ 1]};
-    PSC_TRY(radix_pairs(g, c, bits, k2, v2, hist, offs, &at));  // stably by source
-    const uint32_t* A = k2[at];
-    const uint32_t* B = v2[at];
+    // by target, then stably by source (a single pass cannot end where it begins)
+    uint32_t* k1 = passes == 1 ? (uint32_t*)pair[0] : k;
+    uint32_t* v1 = passes == 1 ? (uint32_t*)pair[1] : v;
+    PSC_TRY(rs_sort(g, c, passes, k, v, pair, r, k1, v1));
+    PSC_TRY(rs_sort(g, c, passes, v1, k1, pair, r, v, k));
+    PSC_TRY(rs_check(g));
+    const uint32_t *A = v, *B = k;  // sources, targets
     release(g, B_AUX3);
     release(g, B_SCAN2);
-    // the kept pairs: targets and sources into the free pair of buffers
-    asel = v2[at ^ 1];
-    uint32_t* bsel = k2[at ^ 1];
+    // the kept pairs: sources and targets
+    uint32_t *asel = (uint32_t*)pair[0], *bsel = (uint32_t*)pair[1];
     PSC_TRY(scan_emit_flags(g, c, SymKeep{A, B}, SymEmit{A, B, asel, bsel}, &ms, F_TRANSPOSE,
                             8.0, 8.0));
     PSC_CUDA(cudaMallocAsync((void**)&E_s, (ms ? ms : 1) * 4, g->stream));
     if (ms) PSC_CUDA(cudaMemcpyAsync(E_s, bsel, ms * 4, cudaMemcpyDeviceToDevice, g->stream));
-    if (ms) {
-      uint64_t* rs;
-      PSC_TRY(ensure_t(g, B_SCAN3, n + 1, &rs));
-      ProfScope ps(g, F_TRANSPOSE);
-      ps.bytes = 8.0 * ms;
-      k_run_starts<<<grid_for(g, ms, 256), 256, 0, g->stream>>>(asel, ms, rs);
-      k_run_lengths<<<grid_for(g, ms, 256), 256, 0, g->stream>>>(asel, ms, rs, cnt);
-    }
+    PSC_CUDA(cudaMallocAsync((void**)&off_s, (n + 1) * 8, g->stream));
+    PSC_TRY(fill_bounds(g, asel, ms, off_s));
     release(g, B_AUX0);
     release(g, B_AUX1);
     release(g, B_AUX2);
@@ -425,13 +564,10 @@ int build_symmetric(psc_graph_s* g) {
     release(g, B_SCAN3);
   } else {
     PSC_CUDA(cudaMallocAsync((void**)&E_s, 4, g->stream));
+    PSC_CUDA(cudaMallocAsync((void**)&off_s, (n + 1) * 8, g->stream));
+    PSC_CUDA(cudaMemsetAsync(off_s, 0, (n + 1) * 8, g->stream));
   }
-  PSC_CUDA(cudaMallocAsync((void**)&off_s, (n + 1) * 8, g->stream));
-  uint64_t total = 0;
-  PSC_TRY(scan_emit(g, n, CntValue{cnt}, OffEmit{off_s, cnt}, &total, F_TRANSPOSE));
-  PSC_CUDA(cudaMemcpyAsync(off_s + n, &ms, 8, cudaMemcpyHostToDevice, g->stream));
-  PSC_CUDA(cudaStreamSynchronize(g->stream));  // ms lives on this stack frame
-  release(g, B_TMP32);
+  PSC_CUDA(cudaStreamSynchronize(g->stream));
   if (g->in_off && g->in_off != g->off) cudaFreeAsync(g->in_off, g->stream);
   if (g->in_E && g->in_E != g->E) cudaFreeAsync(g->in_E, g->stream);
   cudaFreeAsync(g->off, g->stream);
