@@ -188,6 +188,8 @@ enum Buf : int {
   B_FLAB,         // u32 labels of a batch's pivots
   B_SCHED,        // window schedule of a batch's prefix-doubling rounds
   B_SCANBITS,     // u32[n/32] selection bits of scan_emit_flags
+  B_FB_C,         // third frontier bitmaps (k_reach_rounds)
+  B_FB_C2,
   B_TF2,          // second set of label tables (k_ms_batches)
   B_TB2,
   B_BLOCKS,       // u32 per block of a resident grid

@@ -1392,6 +1392,262 @@ __global__ void k_pull_out_edges(const uint32_t* __restrict__ fb, const uint64_t
   if (lane == 0) ctr->next_edges = hits ? nf * (sum / hits) : 0;
 }
 
+// ---------------------------------------------------------------------------
+// Resident rounds, for graphs of up to kRrMaxEdges edges.  A round is 5 to 40 us of
+// work, and launched from the host about 30 more (a
+// memset, one to three kernels, a read-back, a wait, twice that for heavy
+// vertices).  k_reach_rounds runs push and pull rounds of both sides back to
+// back on a resident grid, one grid barrier per round (two when heavy vertices
+// were listed).  Every round leaves its frontier as a queue and as a bitmap, so a
+// change between push and pull needs no conversion: three bitmaps rotate (read,
+// written, cleared).  The switch is the host loop's, with exact out-edge counts.
+// First-pivot phase, host rounds -> this: R-MAT 2^12 0.26 -> 0.12 ms, 2^16 0.34 ->
+// 0.17, 2^18 0.46 -> 0.20, 2^20 (1.6e7 edges) 0.47 -> 0.32, 2^21 (3.2e7) 0.56 ->
+// 0.43, 64-graph batch 0.90 -> 0.67; 3x10^6 vertices with 1.2e7 edges 0.73 -> 0.71.
+// ---------------------------------------------------------------------------
+constexpr int kRrThreads = 512;
+constexpr int kRrWarps = kRrThreads / 32;
+constexpr uint64_t kRrHeavy = 256;        // out-edges of a vertex left to the grid
+constexpr uint64_t kRrMaxEdges = 1 << 25;  // larger graphs: full-width rounds
+constexpr int kRrCtr = 4;                 // counter sets 4-9: three rounds, two sides
+constexpr int kRrState = 10;
+
+struct RrState {
+  uint32_t arrive, failed, rounds[2];
+  unsigned long long nf[2], nf_edges[2], prev_nf[2];
+  unsigned long long edges[2], expanded[2], unvisited[2];
+  uint32_t done, odd;  // the frontiers lie in q[odd]
+};
+static_assert(sizeof(RrState) <= 2 * sizeof(Counters), "two counter sets hold it");
+
+struct RrSide {
+  const uint64_t *off, *B_off;  // search direction, reverse direction
+  const uint32_t *E, *B_E;
+  uint32_t* vis;
+  uint32_t* q[2];
+  uint32_t* fb[3];
+  uint64_t* heavy;
+  uint64_t nf;
+};
+
+struct RrArgs {
+  RrSide s[2];
+  int ns;
+  uint64_t n, threshold;
+  uint32_t max_rounds;
+  Counters* ctr;
+  RrState* st;
+};
+
+// A vertex claimed by a push round joins the next frontier in both forms.
+template <int K>
+__device__ __forceinline__ void rr_emit(const RrSide& S, uint32_t tm, const uint32_t* v,
+                                        uint32_t* qout, uint32_t* fb_out, Counters* c,
+                                        unsigned long long& next_edges) {
+  warp_append_batch<K>(tm, v, qout, &c->next);
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (tm & (1u << k)) {
+      atomicOr(&fb_out[v[k] >> 5], 1u << (v[k] & 31));
+      next_edges += S.off[v[k] + 1] - S.off[v[k]];
+    }
+}
+
+__global__ void __launch_bounds__(kRrThreads, 1) k_reach_rounds(RrArgs a) {
+  __shared__ WarpExpandSmem ssm[kRrWarps];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5, tid = threadIdx.x;
+  const uint64_t gw = (uint64_t)blockIdx.x * kRrWarps + wid, nw = (uint64_t)gridDim.x * kRrWarps;
+  const uint64_t gt = (uint64_t)blockIdx.x * kRrThreads + tid, nt = (uint64_t)gridDim.x * kRrThreads;
+  const uint64_t nwords = (a.n + 31) >> 5;
+  const bool lead = blockIdx.x == 0 && tid == 0;
+  WarpExpandSmem& sm = ssm[wid];
+  uint32_t target = 0;
+  auto barrier = [&]() { return grid_barrier(&a.st->arrive, &a.st->failed, target); };
+  uint64_t nf0 = a.s[0].nf, nf1 = a.ns > 1 ? a.s[1].nf : 0, ne0 = 0, ne1 = 0, pf0 = 0, pf1 = 0;
+  uint32_t rd0 = 0, rd1 = 0, round = 0;
+  unsigned long long t_e[2] = {0, 0}, t_x[2] = {0, 0}, t_u[2] = {0, 0};  // lead thread
+  for (int k = 0; k < a.ns; k++)
+    for (uint64_t w = gt; w < nwords; w += nt) {
+      a.s[k].fb[1][w] = 0;
+      a.s[k].fb[2][w] = 0;
+    }
+  if (!barrier()) return;
+  for (; (nf0 | nf1) && round < a.max_rounds; round++) {
+    Counters* c0 = a.ctr + kRrCtr + 2 * (round % 3);
+    if (blockIdx.x == 0 && tid < 2 * sizeof(Counters) / 8)  // last read a barrier ago
+      ((unsigned long long*)(a.ctr + kRrCtr + 2 * ((round + 1) % 3)))[tid] = 0;
+    for (int k = 0; k < a.ns; k++) {
+      const RrSide& S = a.s[k];
+      const uint64_t nf = k ? nf1 : nf0, ne = k ? ne1 : ne0;
+      uint32_t* clear = S.fb[(round + 2) % 3];
+      for (uint64_t w = gt; w < nwords; w += nt) clear[w] = 0;
+      if (nf == 0) continue;
+      Counters* c = c0 + k;
+      const uint32_t* qin = S.q[round & 1];
+      uint32_t* qout = S.q[(round + 1) & 1];
+      const uint32_t* fb_in = S.fb[round % 3];
+      uint32_t* fb_out = S.fb[(round + 1) % 3];
+      unsigned long long scanned = 0, next_edges = 0, expanded = 0, unvisited = 0;
+      if (round == 0 || nf + ne < a.threshold) {
+        // --- push: 32 vertices per warp step, fewer when that leaves warps idle
+        const uint64_t per = (nf + nw - 1) / nw;
+        const uint32_t chunk = (uint32_t)(per > 32 ? 32 : per);
+        for (uint64_t b = gw * chunk; b < nf; b += nw * chunk) {
+          uint64_t beg = 0, d = 0;
+          if (lane < chunk && b + lane < nf) {
+            const uint32_t u = ld_cg(&qin[b + lane]);
+            beg = S.off[u];
+            d = S.off[u + 1] - beg;
+            expanded++;
+            if (d > kRrHeavy) {
+              const unsigned long long old =
+                  atomicAdd(&c->heavy, (1ull << kPackShift) + (d + kHeavyChunk - 1) / kHeavyChunk);
+              S.heavy[old >> kPackShift] = ((uint64_t)u << 32) | (old & kPackMask);
+              d = 0;
+            }
+          }
+          scanned += d;
+          expand_claim<kPushK>(sm, beg, (uint32_t)d, S.E, S.vis,
+                               [&](uint32_t tm, const uint32_t* v) {
+                                 rr_emit<kPushK>(S, tm, v, qout, fb_out, c, next_edges);
+                               });
+        }
+      } else {
+        // --- pull: a warp owns 32 consecutive vertices at a time
+        for (uint64_t w = gw; w < nwords; w += nw) {
+          const uint32_t vw = __ldcg(&S.vis[w]);
+          const uint64_t v = w * 32 + lane;
+          const bool t = v < a.n && !((vw >> lane) & 1u);
+          uint64_t j = 0, e = 0;
+          bool found = false;
+          if (t) {
+            const uint64_t b = S.B_off[v];
+            e = S.B_off[v + 1];
+            j = b;
+            found = pull_scan<true>(S.B_E, fb_in, j, e < b + kPullSolo ? e : b + kPullSolo);
+            scanned += j - b;
+            unvisited++;
+          }
+          pull_long<true>(S.B_E, fb_in, __ballot_sync(kFull, t && !found && j < e), j, e, found,
+                          scanned);
+          const uint32_t mk = __ballot_sync(kFull, found);
+          if (mk) {
+            if (lane == 0) {
+              fb_out[w] = mk;
+              S.vis[w] = vw | mk;
+            }
+            const unsigned long long pos = warp_append(&c->next, found);
+            if (found) {
+              qout[pos] = (uint32_t)v;
+              next_edges += S.off[v + 1] - S.off[v];
+            }
+          }
+        }
+      }
+      scanned = warp_sum(scanned);
+      next_edges = warp_sum(next_edges);
+      expanded = warp_sum(expanded);
+      unvisited = warp_sum(unvisited);
+      if (lane == 0) {
+        if (scanned) atomicAdd(&c->edges, scanned);
+        if (next_edges) atomicAdd(&c->next_edges, next_edges);
+        if (expanded) atomicAdd(&c->expanded, expanded);
+        if (unvisited) atomicAdd(&c->unvisited, unvisited);
+      }
+    }
+    if (!barrier()) return;
+    if (__ldcg(&c0->heavy) | (a.ns > 1 ? __ldcg(&c0[1].heavy) : 0)) {
+      // --- heavy vertices: their chunks in one contiguous range per warp
+      for (int k = 0; k < a.ns; k++) {
+        const RrSide& S = a.s[k];
+        Counters* c = c0 + k;
+        const unsigned long long packed = __ldcg(&c->heavy);
+        const uint64_t nh = packed >> kPackShift, total = packed & kPackMask;
+        const uint64_t per = (total + nw - 1) / nw;
+        const uint64_t c_beg = gw * per, c_end = c_beg + per < total ? c_beg + per : total;
+        unsigned long long scanned = 0, next_edges = 0;
+        if (nh && c_beg < c_end) {
+          uint64_t h = 0, hi = nh - 1;  // last entry whose first chunk is <= c_beg
+          while (h < hi) {
+            const uint64_t mid = (h + hi + 1) >> 1;
+            if ((uint32_t)ld_cg(&S.heavy[mid]) <= c_beg)
+              h = mid;
+            else
+              hi = mid - 1;
+          }
+          for (uint64_t x = c_beg; x < c_end;) {
+            const uint64_t ent = ld_cg(&S.heavy[h]);
+            const uint64_t cs = (uint32_t)ent;
+            const uint64_t cn = h + 1 < nh ? (uint32_t)ld_cg(&S.heavy[h + 1]) : total;
+            const uint64_t beg = S.off[ent >> 32], end = S.off[(ent >> 32) + 1];
+            for (; x < c_end && x < cn; x++) {
+              const uint64_t e0 = beg + (x - cs) * kHeavyChunk;
+              uint32_t v[kHeavyK], tm = 0;
+#pragma unroll
+              for (int i = 0; i < kHeavyK; i++) {
+                const uint64_t e = e0 + i * 32 + lane;
+                v[i] = kNone;
+                if (e < end) {
+                  scanned++;
+                  v[i] = __ldg(&S.E[e]);
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < kHeavyK; i++)
+                if (v[i] != kNone && bit_set(S.vis, v[i])) tm |= 1u << i;
+              rr_emit<kHeavyK>(S, tm, v, S.q[(round + 1) & 1], S.fb[(round + 1) % 3], c, next_edges);
+            }
+            h++;
+          }
+        }
+        scanned = warp_sum(scanned);
+        next_edges = warp_sum(next_edges);
+        if (lane == 0) {
+          if (scanned) atomicAdd(&c->edges, scanned);
+          if (next_edges) atomicAdd(&c->next_edges, next_edges);
+        }
+      }
+      if (!barrier()) return;
+    }
+    if (lead)
+      for (int k = 0; k < a.ns; k++) {
+        t_e[k] += __ldcg(&c0[k].edges);
+        t_x[k] += __ldcg(&c0[k].expanded);
+        t_u[k] += __ldcg(&c0[k].unvisited);
+      }
+    if (nf0) {
+      rd0++;
+      pf0 = nf0;
+      nf0 = __ldcg(&c0->next);
+      ne0 = __ldcg(&c0->next_edges);
+    }
+    if (nf1) {
+      rd1++;
+      pf1 = nf1;
+      nf1 = __ldcg(&c0[1].next);
+      ne1 = __ldcg(&c0[1].next_edges);
+    }
+  }
+  if (lead) {
+    RrState& s = *a.st;
+    s.rounds[0] = rd0;
+    s.rounds[1] = rd1;
+    s.nf[0] = nf0;
+    s.nf[1] = nf1;
+    s.nf_edges[0] = ne0;
+    s.nf_edges[1] = ne1;
+    s.prev_nf[0] = pf0;
+    s.prev_nf[1] = pf1;
+    for (int k = 0; k < 2; k++) {
+      s.edges[k] = t_e[k];
+      s.expanded[k] = t_x[k];
+      s.unvisited[k] = t_u[k];
+    }
+    s.odd = round & 1;
+    s.done = 1;
+  }
+}
+
 __global__ void k_queue_to_bitmap(const uint32_t* __restrict__ q, uint64_t nq, uint32_t* fb) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -1631,6 +1887,8 @@ constexpr int async_ctl_set(int k) { return 4 + 2 * k; }
 constexpr int async_ctr_set(int k) { return 8 + k; }
 // Slots prepared for one launch (64 MB to clear per side at most).
 constexpr uint64_t kAsyncSlots = 1ull << 24;
+// Rounds of a search with local searches that k_reach_rounds takes.
+constexpr uint32_t kRrRounds = 16;
 
 enum Mode { M_NONE, M_VGC, M_PUSH, M_PULL };
 
@@ -1669,6 +1927,27 @@ int records_if_low(psc_graph_s* g, bool backward, const VRec** out) {
   PSC_TRY(max_degrees_once(g));
   if (g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg) return PSC_OK;
   return records_once_impl(g, backward, out);
+}
+
+// Whether the device holds k_reach_rounds with a block on every SM.
+static bool rr_ready(int device) {
+  constexpr int kMaxDev = 64;
+  static std::mutex mu;
+  static int state[kMaxDev] = {};
+  if (device < 0 || device >= kMaxDev) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  int& st = state[device];
+  if (st == 0) {
+    int coop = 0, b = 0;
+    st = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_reach_rounds, kRrThreads, 0) ==
+                     cudaSuccess &&
+                 b > 0
+             ? 1
+             : -1;
+    cudaGetLastError();
+  }
+  return st == 1;
 }
 
 // Runs the searches of `ns` sides (1 or 2) to completion.  Side k starts from
@@ -1711,8 +1990,73 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   }
   const bool tr = trace_on();
   bool async = local;
+  // (graphs of low degree have narrow frontiers, so deep ones: not in rounds)
+  bool resident = g->m <= kRrMaxEdges && rr_ready(g->device);
+  if (resident && local) {
+    PSC_TRY(max_degrees_once(g));
+    resident = g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg;
+  }
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
+    // Small graphs: all rounds in one launch, or the first kRrRounds of a search
+    // with local searches (a deep one then goes on below, without rounds).
+    if (resident) {
+      resident = !local;  // local: once
+      RrArgs a = {};
+      a.ns = ns;
+      a.n = n;
+      a.threshold = threshold;
+      a.max_rounds = local ? kRrRounds : 1u << 16;
+      a.ctr = g->ctr;
+      a.st = (RrState*)(g->ctr + kRrState);
+      bool any = false;
+      for (int k = 0; k < ns; k++) {
+        const Side& s = sides[k];
+        RrSide& r = a.s[k];
+        r.off = s.backward ? g->in_off : g->off;
+        r.E = s.backward ? g->in_E : g->E;
+        r.B_off = s.backward ? g->off : g->in_off;
+        r.B_E = s.backward ? g->E : g->in_E;
+        r.vis = s.vis;
+        r.q[0] = (uint32_t*)g->bufs[s.slot_qa].p;
+        r.q[1] = (uint32_t*)g->bufs[s.slot_qb].p;
+        uint32_t* third;
+        PSC_TRY(ensure_t(g, k ? B_FB_C2 : B_FB_C, nwords + 1, &third));
+        r.fb[0] = third;
+        r.fb[1] = (uint32_t*)g->bufs[s.slot_fa].p;
+        r.fb[2] = (uint32_t*)g->bufs[s.slot_fb].p;
+        r.heavy = (uint64_t*)g->bufs[s.slot_heavy].p;
+        r.nf = s.nf;
+        any |= s.nf != 0;
+      }
+      if (any) {
+        PSC_TRY(zero_counters(g));
+        {
+          ProfScope ps(g, F_REACH_PUSH);
+          void* args[] = {&a};
+          PSC_CUDA(cudaLaunchCooperativeKernel((const void*)k_reach_rounds, dim3((unsigned)g->num_sms),
+                                               dim3(kRrThreads), args, 0, g->stream));
+        }
+        PSC_TRY(read_counters(g));
+        const RrState& st = *(const RrState*)(g->hctr + kRrState);
+        if (st.failed || !st.done) return PSC_ERR_ITER_LIMIT;
+        for (int k = 0; k < ns; k++) {
+          Side& s = sides[k];
+          s.rounds += st.rounds[k];
+          s.nf = st.nf[k];
+          s.nf_edges = st.nf_edges[k];
+          s.prev_nf = st.prev_nf[k];
+          if (st.odd) std::swap(g->bufs[s.slot_qa], g->bufs[s.slot_qb]);
+          if (g->profiling)
+            g->prof[F_REACH_PUSH].bytes +=
+                16.0 * (st.expanded[k] + st.unvisited[k]) + 5.0 * st.edges[k];
+          if (tr)
+            std::fprintf(stderr, "reach side %d resident rounds %u left %llu edges %llu\n", k,
+                         st.rounds[k], st.nf[k], st.edges[k]);
+        }
+        continue;
+      }
+    }
     // The sparse part of a search in one launch (k_reach_async): from the
     // start on graphs of low degree (their frontiers grow slowly), else once
     // every active side's frontier is steady, well inside VGC range (at least
