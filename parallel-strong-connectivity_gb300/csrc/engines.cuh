@@ -36,9 +36,13 @@ int build_symmetric(psc_graph_s* g);
 int reach_run(psc_graph_s* g, uint32_t src, bool backward, bool local, uint32_t tau,
               uint32_t pull_div, uint32_t* vis, uint32_t* rounds);
 
-// Forward and backward reachability from one source, run together.
-int reach_pair(psc_graph_s* g, uint32_t src, bool local, uint32_t tau, uint32_t pull_div,
-               uint32_t* vis_f, uint32_t* vis_b, uint32_t* rounds_f, uint32_t* rounds_b);
+// Forward and backward reachability from the first pivot P[0], run together; no
+// search when every vertex was trimmed.  zeros: device count of trimmed vertices
+// (read there when the search starts on the device, so that nothing waits for
+// it before); *n_zeros receives it.
+int reach_first(psc_graph_s* g, const uint32_t* P, const uint64_t* zeros, bool local, uint32_t tau,
+                uint32_t pull_div, uint32_t* vis_f, uint32_t* vis_b, uint32_t* rounds_f,
+                uint32_t* rounds_b, uint64_t* n_zeros);
 
 // Forward and backward reachability from n_srcs device sources at once (the
 // first pivots of a batch of disjoint graphs share one search).  vgc_max:
@@ -69,6 +73,7 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
 struct MsRun {
   const uint32_t* centres = nullptr;
   uint64_t n_remaining = 0;  // plain: centres in all
+  const uint64_t* n_rem_dev = nullptr;  // when set, n_remaining is read here first
   uint64_t cur = 0, step = 1;
   uint64_t label_offset = 0;
   // batch of graphs: the windows of every round (see scc_batch_phases)

@@ -744,6 +744,7 @@ struct MbState {
   // a batch interrupted between two sub-rounds (MB_GROW)
   unsigned long long cap, nf, n0, n1, e0, e1;
   uint32_t set, buf;
+  unsigned long long n_remaining;
 };
 static_assert(sizeof(MbState) <= 2 * sizeof(Counters) && kMbState + 2 <= kCounterSets,
               "the state fits its counter sets");
@@ -819,6 +820,7 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
   if (lane == 0) sh.sm[wid].fail = 0;
   __syncwarp();
 
+  if (a.run.n_rem_dev) a.run.n_remaining = *a.run.n_rem_dev;
   uint64_t cur = a.run.cur, step = a.run.step, label_offset = a.run.label_offset;
   uint64_t round = a.run.round, ne0 = a.run.ne[0], ne1 = a.run.ne[1];
   uint64_t batches = 0, subs = 0, slots = 0;
@@ -1152,6 +1154,7 @@ __global__ void __launch_bounds__(kMbThreads, 1) k_ms_batches(MbArgs a) {
     s.heavy_edges = t_he;
     s.heavy_probes = t_hp;
     s.slots = slots;
+    s.n_remaining = a.run.n_remaining;
     s.cap = cap;
     s.nf = nf;
     s.n0 = n0;
@@ -1466,6 +1469,8 @@ int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, 
     }
     PSC_TRY(read_counters(g));
     if (s.failed || s.why == MB_RUNNING) return PSC_ERR_ITER_LIMIT;
+    run->n_remaining = s.n_remaining;
+    run->n_rem_dev = nullptr;
     run->cur = s.cur;
     run->step = s.step;
     run->label_offset = s.label_offset;

@@ -1417,6 +1417,7 @@ struct RrState {
   unsigned long long nf[2], nf_edges[2], prev_nf[2];
   unsigned long long edges[2], expanded[2], unvisited[2];
   uint32_t done, odd;  // the frontiers lie in q[odd]
+  unsigned long long zeros;
 };
 static_assert(sizeof(RrState) <= 2 * sizeof(Counters), "two counter sets hold it");
 
@@ -1435,6 +1436,10 @@ struct RrArgs {
   int ns;
   uint64_t n, threshold;
   uint32_t max_rounds;
+  // first launch of a search: the sources, and (optional) the count of trimmed
+  // vertices, with which there is one source or none
+  const uint32_t* srcs;
+  const uint64_t* zeros;
   Counters* ctr;
   RrState* st;
 };
@@ -1470,8 +1475,24 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_reach_rounds(RrArgs a) {
     for (uint64_t w = gt; w < nwords; w += nt) {
       a.s[k].fb[1][w] = 0;
       a.s[k].fb[2][w] = 0;
+      if (a.srcs) a.s[k].vis[w] = 0;
     }
+  uint64_t zeros = 0;
+  if (a.zeros) {
+    zeros = *a.zeros;
+    nf0 = nf1 = zeros < a.n ? 1 : 0;
+    if (a.ns < 2) nf1 = 0;
+  }
   if (!barrier()) return;
+  if (a.srcs) {
+    for (int k = 0; k < a.ns; k++)
+      for (uint64_t i = gt; i < (k ? nf1 : nf0); i += nt) {
+        const uint32_t v = __ldg(&a.srcs[i]);
+        atomicOr(&a.s[k].vis[v >> 5], 1u << (v & 31));
+        a.s[k].q[0][i] = v;
+      }
+    if (!barrier()) return;
+  }
   for (; (nf0 | nf1) && round < a.max_rounds; round++) {
     Counters* c0 = a.ctr + kRrCtr + 2 * (round % 3);
     if (blockIdx.x == 0 && tid < 2 * sizeof(Counters) / 8)  // last read a barrier ago
@@ -1644,6 +1665,7 @@ __global__ void __launch_bounds__(kRrThreads, 1) k_reach_rounds(RrArgs a) {
       s.unvisited[k] = t_u[k];
     }
     s.odd = round & 1;
+    s.zeros = zeros;
     s.done = 1;
   }
 }
@@ -1953,9 +1975,12 @@ static bool rr_ready(int device) {
 // Runs the searches of `ns` sides (1 or 2) to completion.  Side k starts from
 // srcs[k], or, when d_srcs is given, every side starts from the n_dsrc device
 // sources d_srcs.
+// zeros (with d_srcs): the device count of trimmed vertices; there is one source
+// if it is below n, else none; *n_zeros receives it.
 static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs, bool local,
                        uint32_t tau, uint32_t pull_div, const uint32_t* d_srcs = nullptr,
-                       uint64_t n_dsrc = 0, uint64_t vgc_max = 0) {
+                       uint64_t n_dsrc = 0, uint64_t vgc_max = 0, const uint64_t* zeros = nullptr,
+                       uint64_t* n_zeros = nullptr) {
   const uint64_t n = g->n, nwords = (n + 31) / 32;
   // heavy-list fields: < 2^24 entries (m / kHeavyDeg), < 2^32 chunks
   if (g->m >> 36) return PSC_ERR_TOO_LARGE;
@@ -1965,6 +1990,19 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   if (pull_div == 0) pull_div = 20;
   const uint64_t threshold = g->m / pull_div;
   const uint64_t slack = !local ? 0 : g->m > kHeavyDeg ? kAsyncSlack : std::min(n, kAsyncSlack);
+  // (graphs of low degree have narrow frontiers, so deep ones: not in rounds)
+  bool resident = g->m <= kRrMaxEdges && rr_ready(g->device);
+  if (resident && local) {
+    PSC_TRY(max_degrees_once(g));
+    resident = g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg;
+  }
+  const bool start_there = resident && d_srcs;  // the launch sets its sources itself
+  if (zeros && !start_there) {
+    PSC_CUDA(cudaMemcpyAsync(&g->hctr->aux0, zeros, 8, cudaMemcpyDeviceToHost, g->stream));
+    PSC_CUDA(cudaStreamSynchronize(g->stream));
+    *n_zeros = g->hctr->aux0;
+    n_dsrc = *n_zeros < n ? 1 : 0;
+  }
   for (int k = 0; k < ns; k++) {
     Side& s = sides[k];
     void* p;
@@ -1973,29 +2011,22 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
     PSC_TRY(ensure(g, s.slot_fa, (nwords + 1) * 4, &p));
     PSC_TRY(ensure(g, s.slot_fb, (nwords + 1) * 4, &p));
     PSC_TRY(ensure(g, s.slot_heavy, (n + 1) * 8, &p));
-    PSC_CUDA(cudaMemsetAsync(s.vis, 0, nwords * 4, g->stream));
-    if (d_srcs) {
-      if (n_dsrc)
-        k_reach_init_multi<<<grid_for(g, n_dsrc, 256), 256, 0, g->stream>>>(
-            s.vis, (uint32_t*)g->bufs[s.slot_qa].p, d_srcs, n_dsrc);
-      s.nf = n_dsrc;
-    } else {
-      k_reach_init<<<1, 1, 0, g->stream>>>(s.vis, (uint32_t*)g->bufs[s.slot_qa].p, srcs[k]);
-      s.nf = 1;
-    }
+    s.nf = d_srcs ? n_dsrc : 1;
     s.nf_edges = 0;
     s.prev_nf = 0;
     s.pull = false;
     s.rounds = 0;
+    if (start_there) continue;
+    PSC_CUDA(cudaMemsetAsync(s.vis, 0, nwords * 4, g->stream));
+    if (!d_srcs)
+      k_reach_init<<<1, 1, 0, g->stream>>>(s.vis, (uint32_t*)g->bufs[s.slot_qa].p, srcs[k]);
+    else if (n_dsrc)
+      k_reach_init_multi<<<grid_for(g, n_dsrc, 256), 256, 0, g->stream>>>(
+          s.vis, (uint32_t*)g->bufs[s.slot_qa].p, d_srcs, n_dsrc);
   }
   const bool tr = trace_on();
   bool async = local;
-  // (graphs of low degree have narrow frontiers, so deep ones: not in rounds)
-  bool resident = g->m <= kRrMaxEdges && rr_ready(g->device);
-  if (resident && local) {
-    PSC_TRY(max_degrees_once(g));
-    resident = g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg;
-  }
+  bool first_launch = start_there;
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
     // Small graphs: all rounds in one launch, or the first kRrRounds of a search
@@ -2029,6 +2060,12 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         r.nf = s.nf;
         any |= s.nf != 0;
       }
+      if (first_launch) {
+        a.srcs = d_srcs;
+        a.zeros = zeros;
+        any = true;
+        first_launch = false;
+      }
       if (any) {
         PSC_TRY(zero_counters(g));
         {
@@ -2040,6 +2077,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         PSC_TRY(read_counters(g));
         const RrState& st = *(const RrState*)(g->hctr + kRrState);
         if (st.failed || !st.done) return PSC_ERR_ITER_LIMIT;
+        if (a.zeros) *n_zeros = st.zeros;
         for (int k = 0; k < ns; k++) {
           Side& s = sides[k];
           s.rounds += st.rounds[k];
@@ -2325,11 +2363,11 @@ int reach_run(psc_graph_s* g, uint32_t src, bool backward, bool local, uint32_t 
   return PSC_OK;
 }
 
-int reach_pair(psc_graph_s* g, uint32_t src, bool local, uint32_t tau, uint32_t pull_div,
-               uint32_t* vis_f, uint32_t* vis_b, uint32_t* rounds_f, uint32_t* rounds_b) {
+int reach_first(psc_graph_s* g, const uint32_t* P, const uint64_t* zeros, bool local, uint32_t tau,
+                uint32_t pull_div, uint32_t* vis_f, uint32_t* vis_b, uint32_t* rounds_f,
+                uint32_t* rounds_b, uint64_t* n_zeros) {
   Side s[2] = {make_side(false, vis_f, 0), make_side(true, vis_b, 1)};
-  const uint32_t srcs[2] = {src, src};
-  PSC_TRY(reach_sides(g, s, 2, srcs, local, tau ? tau : 512, pull_div));
+  PSC_TRY(reach_sides(g, s, 2, nullptr, local, tau ? tau : 512, pull_div, P, 1, 0, zeros, n_zeros));
   if (rounds_f) *rounds_f = s[0].rounds;
   if (rounds_b) *rounds_b = s[1].rounds;
   return PSC_OK;

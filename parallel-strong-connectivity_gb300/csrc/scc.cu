@@ -51,8 +51,12 @@ struct TrimEmit {
 // waits only at the end of its chunk.
 constexpr uint64_t kPermChunk = 32 * 32;
 
-__global__ void k_perm_gather(const uint32_t* __restrict__ nz, uint64_t np, FeistelKey key,
-                              uint32_t* P) {
+// zeros: count of the trimmed vertices (on the device, as the scan left it).
+__global__ void k_perm_gather(const uint32_t* __restrict__ nz, uint64_t n,
+                              const uint64_t* __restrict__ zeros, uint64_t seed, uint32_t* P) {
+  const uint64_t np = n - *zeros;
+  if (np == 0) return;
+  const FeistelKey key = feistel_key(np, seed);
   const unsigned lane = lane_id();
   const uint64_t gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -191,32 +195,30 @@ static int scc_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t* p) {
   uint32_t *P, *nz, *centers, *front, *vf, *vb;
   PSC_TRY(ensure_t(g, B_P, n + 1, &P));
   PSC_TRY(ensure_t(g, B_TMP32, n + 1, &nz));
-  // trim
+  // trim; the count of trimmed vertices stays on the device until the first
+  // pivot's search has run
   uint64_t n_zeros = 0;
+  const uint64_t* zeros = nullptr;
   // algorithmic bytes: two offsets of each direction read, an 8-byte label and
   // (for the live vertices) a 4-byte index written
-  PSC_TRY(scan_emit_flags(g, n, ZeroFlag{g->off, g->in_off}, TrimEmit{labels, nz}, &n_zeros, F_TRIM,
-                          28.0));
-  const uint64_t np = n - n_zeros;
-  if (np > 0) {
-    FeistelKey key = feistel_key(np, p->seed);
+  PSC_TRY(scan_emit_flags(g, n, ZeroFlag{g->off, g->in_off}, TrimEmit{labels, nz}, nullptr, F_TRIM,
+                          28.0, 0, &zeros));
+  {
     ProfScope ps(g, F_TRIM);
-    ps.bytes = 8.0 * np;
-    k_perm_gather<<<grid_for(g, np, tb), tb, 0, g->stream>>>(nz, np, key, P);
+    ps.bytes = 8.0 * n;
+    k_perm_gather<<<grid_for(g, n, tb), tb, 0, g->stream>>>(nz, n, zeros, p->seed, P);
   }
-  uint64_t label_offset = n_zeros + 1;
   PSC_CUDA(cudaEventRecord(g->ph[1], g->stream));
+  // first pivot (scc.hpp:316-350)
+  PSC_TRY(ensure_t(g, B_VIS_F, (n + 31) / 32 + 1, &vf));
+  PSC_TRY(ensure_t(g, B_VIS_B, (n + 31) / 32 + 1, &vb));
+  uint32_t r1 = 0, r2 = 0;
+  PSC_TRY(reach_first(g, P, zeros, p->local_reach != 0, p->tau, p->pull_div, vf, vb, &r1, &r2,
+                      &n_zeros));
+  g->stats.reach_rounds = r1 + r2;
+  const uint64_t np = n - n_zeros;
+  uint64_t label_offset = n_zeros + 1;
   if (np > 0) {
-    // first pivot (scc.hpp:316-350)
-    uint32_t src = 0;
-    PSC_CUDA(cudaMemcpyAsync(&g->hctr->aux1, P, 4, cudaMemcpyDeviceToHost, g->stream));
-    PSC_CUDA(cudaStreamSynchronize(g->stream));
-    std::memcpy(&src, &g->hctr->aux1, 4);
-    PSC_TRY(ensure_t(g, B_VIS_F, (n + 31) / 32 + 1, &vf));
-    PSC_TRY(ensure_t(g, B_VIS_B, (n + 31) / 32 + 1, &vb));
-    uint32_t r1 = 0, r2 = 0;
-    PSC_TRY(reach_pair(g, src, p->local_reach != 0, p->tau, p->pull_div, vf, vb, &r1, &r2));
-    g->stats.reach_rounds = r1 + r2;
     uint32_t* done;  // finished vertices after the first pivot (frontier slot, free by now)
     PSC_TRY(ensure_t(g, B_FB_A, (n + 31) / 32 + 1, &done));
     {
@@ -227,31 +229,37 @@ static int scc_phases(psc_graph_s* g, uint64_t* labels, const psc_params_t* p) {
                                                             done);
     }
     PSC_TRY(ensure_t(g, B_CENTERS, np + 1, &centers));
+    const bool resident = ms_run_ready(g);
     uint64_t nc = 0;
-    PSC_TRY(scan_emit_flags(g, np, NotDoneBitAt{P, done}, CopyAt{P, centers, 0}, &nc, F_COMPACT, 8.0,
-                      4.0));
+    const uint64_t* nc_dev = nullptr;
+    PSC_TRY(scan_emit_flags(g, np, NotDoneBitAt{P, done}, CopyAt{P, centers, 0},
+                            resident ? nullptr : &nc, F_COMPACT, 8.0, 4.0,
+                            resident ? &nc_dev : nullptr));
     label_offset++;
     PSC_CUDA(cudaEventRecord(g->ph[2], g->stream));
 
     // prefix-doubling batches (scc.hpp:365-473)
     PSC_TRY(ensure_t(g, B_FRONT, np + 1, &front));
-    const uint64_t n_remaining = nc;
+    uint64_t n_remaining = nc;
     uint64_t step_size = 1, cur_offset = 0, finished = 0;
     uint64_t in_ne = 1, out_ne = 1;
-    const bool resident = ms_run_ready(g);
-    while (finished != n_remaining) {
+    while (nc_dev || finished != n_remaining) {
       if (resident) {
         // batches back to back in one launch, up to one that it leaves to the
         // steps below
         MsRun run;
         run.centres = centers;
         run.n_remaining = n_remaining;
+        run.n_rem_dev = nc_dev;  // (the first time)
         run.cur = cur_offset;
         run.step = step_size;
         run.label_offset = label_offset;
         run.ne[0] = out_ne;
         run.ne[1] = in_ne;
-        PSC_TRY(ms_run(g, labels, p, &run, std::min(step_size, n_remaining - cur_offset)));
+        PSC_TRY(ms_run(g, labels, p, &run,
+                       nc_dev ? 1 : std::min(step_size, n_remaining - cur_offset)));
+        nc_dev = nullptr;
+        n_remaining = run.n_remaining;
         cur_offset = finished = run.cur;
         step_size = run.step;
         label_offset = run.label_offset;
