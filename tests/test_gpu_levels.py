@@ -52,6 +52,17 @@ def _tree(fan, extra=1_700_000):
     return psc.HostGraph.from_edges(n, np.concatenate(src), np.concatenate(dst))
 
 
+def _band(top, n=20_011):
+    """Vertex u has 0 to top edges into the 60 vertices after it (and u -> u + 1 every 7th)."""
+    rng = np.random.default_rng(top)
+    deg = rng.integers(0, top + 1, n)
+    src = np.repeat(np.arange(n), deg)
+    dst = np.minimum(src + rng.integers(1, 61, len(src)), n - 1)
+    chain = np.arange(0, n - 1, 7)
+    return psc.HostGraph.from_edges(n, np.concatenate([src, chain]),
+                                    np.concatenate([dst, chain + 1]))
+
+
 GRAPHS = {
     "path": lambda: psc.HostGraph.from_edges(3001, np.arange(3000), np.arange(1, 3001)),
     "grid_narrow": lambda: psc.HostGraph.grid(3, 4001, 0.9, seed=5),
@@ -62,6 +73,11 @@ GRAPHS = {
     "edges_65535": lambda: _tree([257, 255]),
     "edges_65537": lambda: _tree([65537, 1]),
     "hub_then_fan": lambda: _tree([33, 9, 70, 3]),
+    # eight lanes per entry up to degree 8, the balanced expansion above it
+    "fan_8": lambda: _tree([8] * 5),
+    "fan_9": lambda: _tree([9] * 4),
+    "degrees_0_to_8": lambda: _band(8),
+    "degrees_0_to_12": lambda: _band(12),
 }
 
 
