@@ -21,13 +21,14 @@ namespace psc {
 // scan per digit.  Tiles are numbered by a ticket, so the tiles that one waits for
 // are running or done; every wait is bounded.
 // R-MAT 2^22, 6.6e7 edges, 3 passes: histogram 0.37, scan 0.03 and scatter 0.60 ms
-// per pass -> one read of 0.08 ms and 0.53 per pass; sources 0.35 -> 0.15, offsets
+// per pass -> one read of 0.08 ms and 0.49 per pass; sources 0.35 -> 0.15, offsets
 // 0.28 -> 0.08.
 // ---------------------------------------------------------------------------
 constexpr int kRsBits = 8;
 constexpr int kRsBins = 1 << kRsBits;
 constexpr int kRsBlock = 256;
-constexpr int kRsTile = 3072;  // pairs per block and pass (12 per thread)
+constexpr int kRsTile = 4608;  // pairs per block and pass (12 per thread)
+constexpr int kEsTile = 3072;  // edges per block of k_edge_sources (4608: 163 instead of 126 us)
 constexpr int kRsMaxPasses = 4;
 constexpr int kRsLook = 4;
 constexpr uint32_t kRsSpin = 1u << 22;  // polls of one wait
@@ -35,7 +36,7 @@ constexpr uint32_t kRsSpin = 1u << 22;  // polls of one wait
 // all tiles up to it.
 constexpr uint64_t kRsCount = 1ull << 62, kRsPrefix = 2ull << 62, kRsValue = kRsCount - 1;
 
-// src[e] = the vertex whose adjacency holds edge e.  A block takes kRsTile
+// src[e] = the vertex whose adjacency holds edge e.  A block takes kEsTile
 // consecutive edges: each vertex whose list begins inside the tile marks its first
 // edge, and a running maximum over the marks gives every edge its owner (instead
 // of a binary search per edge).
@@ -57,11 +58,11 @@ __device__ __forceinline__ uint64_t edge_owner(const uint64_t* __restrict__ off,
 // steps were most of its time).
 __global__ void k_tile_owners(const uint64_t* __restrict__ off, uint64_t n, uint64_t m,
                               uint32_t* owner) {
-  const uint64_t ends = 2 * ((m + kRsTile - 1) / kRsTile);
+  const uint64_t ends = 2 * ((m + kEsTile - 1) / kEsTile);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ends;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t e0 = (i >> 1) * kRsTile;
-    const uint64_t e1 = e0 + kRsTile < m ? e0 + kRsTile : m;
+    const uint64_t e0 = (i >> 1) * kEsTile;
+    const uint64_t e1 = e0 + kEsTile < m ? e0 + kEsTile : m;
     owner[i] = (uint32_t)edge_owner(off, n, (i & 1) ? e1 - 1 : e0);
   }
 }
@@ -69,16 +70,16 @@ __global__ void k_tile_owners(const uint64_t* __restrict__ off, uint64_t n, uint
 __global__ void __launch_bounds__(kRsBlock)
     k_edge_sources(const uint64_t* __restrict__ off, const uint32_t* __restrict__ owner,
                    uint64_t m, uint32_t* src) {
-  constexpr int NW = kRsBlock / 32, PER = kRsTile / NW;
-  __shared__ uint32_t mark[kRsTile];
+  constexpr int NW = kRsBlock / 32, PER = kEsTile / NW;
+  __shared__ uint32_t mark[kEsTile];
   __shared__ uint32_t wmax[NW];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5, tid = threadIdx.x;
-  const uint64_t ntiles = (m + kRsTile - 1) / kRsTile;
+  const uint64_t ntiles = (m + kEsTile - 1) / kEsTile;
   for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint64_t e0 = tile * kRsTile;
-    const uint64_t e1 = e0 + kRsTile < m ? e0 + kRsTile : m;
+    const uint64_t e0 = tile * kEsTile;
+    const uint64_t e1 = e0 + kEsTile < m ? e0 + kEsTile : m;
     const uint64_t v0 = __ldg(&owner[2 * tile]), v1 = __ldg(&owner[2 * tile + 1]);
-    for (int i = tid; i < kRsTile; i += kRsBlock) mark[i] = 0;
+    for (int i = tid; i < kEsTile; i += kRsBlock) mark[i] = 0;
     __syncthreads();
     for (uint64_t v = v0 + 1 + tid; v <= v1; v += kRsBlock)
       atomicMax(&mark[__ldg(&off[v]) - e0], (uint32_t)(v - v0));
@@ -151,23 +152,30 @@ __global__ void __launch_bounds__(kRsBins) k_rs_starts(unsigned long long* hist)
   h[threadIdx.x] = start;
 }
 
-// One stable pass.  Each warp owns kRsTile / 8 consecutive pairs of the tile
+// One stable pass.  Each warp owns a twelfth of the tile, consecutive pairs
 // (chunks of 32 in order, lanes in order), held in registers.  The tile is sorted
 // by digit in shared memory (warp counts, a block scan over digits, ranked
 // placement), then written out so that consecutive threads write consecutive
 // positions of one digit's run: coalesced stores instead of one sector per pair.
-constexpr int kRsPer = kRsTile / kRsBlock;  // keys per thread
+// 384 threads and three blocks an SM: the pass is a chain of ballots, shared-memory
+// round trips and block barriers, so it lives on warps in flight; the values are
+// loaded only behind the ranking, which keeps the registers low enough for it.
+// (load and solve of R-MAT 2^22, 6.7e7 edges: 256 threads x 12 pairs 5.17 ms, 384 x 12
+// 5.02, 384 x 8 and 512 x 8 5.04, 384 x 10 5.12, 512 x 12 5.19.)
+constexpr int kRpBlock = 384;
+constexpr int kRsPer = kRsTile / kRpBlock;  // keys per thread
+static_assert(kRsTile % kRpBlock == 0 && kRsTile % kRsBlock == 0, "whole chunks per warp");
 
 // (Pairs as 64-bit words between passes were measured and dropped: 0.61 ms a pass
-// instead of 0.53, the ranked placement then meets twice the bank conflicts.)
-__global__ void __launch_bounds__(kRsBlock)
+// instead of 0.53 then, the ranked placement then meets twice the bank conflicts.)
+__global__ void __launch_bounds__(kRpBlock, 3)
     k_rs_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint64_t m,
               int shift, const unsigned long long* __restrict__ starts, uint32_t* ticket,
               unsigned long long* status, uint32_t* kout, uint32_t* vout,
               unsigned long long* failed) {
-  constexpr int NW = kRsBlock / 32;
+  constexpr int NW = kRpBlock / 32;
   constexpr int PER_WARP = kRsTile / NW;
-  static_assert(kRsBins == kRsBlock, "one digit per thread in the digit scan");
+  static_assert(kRsBins <= kRpBlock, "one digit per thread in the digit scan");
   __shared__ uint32_t skey[kRsTile];
   __shared__ uint32_t sval[kRsTile];
   __shared__ uint32_t wcnt[NW][kRsBins];
@@ -192,63 +200,65 @@ __global__ void __launch_bounds__(kRsBlock)
     const uint64_t i = base + c * 32 + lane;
     key[c] = i < m ? __ldg(&kin[i]) : 0u;
   }
-#pragma unroll
-  for (int c = 0; c < kRsPer; c++) {
-    const uint64_t i = base + c * 32 + lane;
-    val[c] = i < m ? __ldg(&vin[i]) : 0u;
-  }
-  // lanes of a chunk with the same digit, found by one ballot per digit bit
-  unsigned peers[kRsPer];
+  // rank of each pair among the warp's pairs of its digit: lanes of a chunk with the
+  // same digit are found by one ballot per digit bit (by atomicOr of lane masks in
+  // shared memory: 0.63 ms a pass instead of 0.52)
+  uint32_t rank[kRsPer];
 #pragma unroll
   for (int c = 0; c < kRsPer; c++) {
     const bool in = base + c * 32 + lane < m;
+    const uint32_t d = (key[c] >> shift) & (kRsBins - 1);
     unsigned p = __ballot_sync(kFull, in);
-    const uint32_t d = key[c] >> shift;
 #pragma unroll
     for (int b = 0; b < kRsBits; b++) {
       const bool bit = (d >> b) & 1u;
       const unsigned v = __ballot_sync(kFull, bit);
       p &= bit ? v : ~v;
     }
-    peers[c] = in ? p : 0u;
-    if (in && (p & lt) == 0) wcnt[wid][d & (kRsBins - 1)] += __popc(p);
+    const uint32_t at = wcnt[wid][d];
     __syncwarp();
+    rank[c] = at + __popc(p & lt);
+    if (in && (p & lt) == 0) wcnt[wid][d] = at + __popc(p);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int c = 0; c < kRsPer; c++) {
+    const uint64_t i = base + c * 32 + lane;
+    val[c] = i < m ? __ldg(&vin[i]) : 0u;
   }
   __syncthreads();
   // digit tid: the tile's count is published, then its start in the sorted tile
   // and each warp's base inside it
+  const bool dig = kRpBlock == kRsBins || tid < kRsBins;
   uint32_t total = 0;
 #pragma unroll
-  for (int w = 0; w < NW; w++) total += wcnt[w][tid];
+  for (int w = 0; w < NW; w++) total += dig ? wcnt[w][tid] : 0u;
   volatile unsigned long long* row = status + tile * kRsBins + tid;
-  *row = (tile ? kRsCount : kRsPrefix) | total;
+  if (dig) *row = (tile ? kRsCount : kRsPrefix) | total;
   uint64_t all = 0;
-  const uint32_t start = (uint32_t)block_excl_scan<kRsBlock>(total, scan_sm, &all);
+  const uint32_t start = (uint32_t)block_excl_scan<kRpBlock>(total, scan_sm, &all);
   uint32_t run = start;
 #pragma unroll
   for (int w = 0; w < NW; w++) {
-    const uint32_t c = wcnt[w][tid];
-    wcnt[w][tid] = run;
-    run += c;
+    if (dig) {
+      const uint32_t c = wcnt[w][tid];
+      wcnt[w][tid] = run;
+      run += c;
+    }
   }
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < kRsPer; c++) {
-    const uint32_t d = (key[c] >> shift) & (kRsBins - 1);
-    uint32_t lp = 0;
-    if (peers[c]) lp = wcnt[wid][d] + __popc(peers[c] & lt);
-    __syncwarp();
-    if (peers[c]) {
+    if (base + c * 32 + lane < m) {
+      const uint32_t lp = wcnt[wid][(key[c] >> shift) & (kRsBins - 1)] + rank[c];
       skey[lp] = key[c];
       sval[lp] = val[c];
-      if ((peers[c] & lt) == 0) wcnt[wid][d] += __popc(peers[c]);
     }
-    __syncwarp();
   }
   // look back, kRsLook tiles' words at a time (8 / 16 / 32 at a time: 1 / 2 / 8 %
   // slower; the pass is bound by instructions, not by this wait)
   uint64_t before = 0;
-  bool open = tile > 0;
+  bool open = dig && tile > 0;
   for (uint64_t t = tile; open;) {
     unsigned long long x[kRsLook];
 #pragma unroll
@@ -273,14 +283,14 @@ __global__ void __launch_bounds__(kRsBlock)
     t -= t < (uint64_t)kRsLook ? t : (uint64_t)kRsLook;
     if (t == 0) open = false;
   }
-  if (tile) *row = kRsPrefix | (before + total);
-  gbase[tid] = starts[tid] + before - start;
+  if (dig && tile) *row = kRsPrefix | (before + total);
+  if (dig) gbase[tid] = starts[tid] + before - start;
   __syncthreads();
   if (s_bad) {
     if (tid == 0) *failed = 1;
     return;
   }
-  for (uint32_t j = tid; j < tcount; j += kRsBlock) {
+  for (uint32_t j = tid; j < tcount; j += kRpBlock) {
     const uint32_t k = skey[j];
     const uint64_t pos = gbase[(k >> shift) & (kRsBins - 1)] + j;
     kout[pos] = k;
@@ -383,7 +393,7 @@ static int rs_scratch(psc_graph_s* g, uint64_t cnt, RsScratch* r) {
 
 // The owners use the status words' room (a sort clears those before each pass).
 static void launch_edge_sources(psc_graph_s* g, const RsScratch& r, uint32_t* src) {
-  const uint64_t ntiles = (g->m + kRsTile - 1) / kRsTile;
+  const uint64_t ntiles = (g->m + kEsTile - 1) / kEsTile;
   uint32_t* owner = (uint32_t*)r.status;
   k_tile_owners<<<grid_for(g, 2 * ntiles, 128), 128, 0, g->stream>>>(g->off, g->n, g->m, owner);
   k_edge_sources<<<(unsigned)std::min<uint64_t>(ntiles, g->num_sms * 8), kRsBlock, 0, g->stream>>>(
@@ -423,7 +433,7 @@ static int rs_sort(psc_graph_s* g, uint64_t cnt, int passes, const uint32_t* kin
     const bool first = p == 0, last = p + 1 == passes;
     const uint32_t* ki = first ? kin : (const uint32_t*)pair[(p + 1) & 1];
     uint32_t* ko = last ? kout : (uint32_t*)pair[p & 1];
-    k_rs_pass<<<(unsigned)ntiles, kRsBlock, 0, g->stream>>>(
+    k_rs_pass<<<(unsigned)ntiles, kRpBlock, 0, g->stream>>>(
         ki, first ? vin : ki + cnt, cnt, p * kRsBits, r.hist + (uint64_t)p * kRsBins, r.ticket,
         r.status, ko, last ? vout : ko + cnt, r.failed);
     PSC_CUDA(cudaGetLastError());

@@ -1,5 +1,5 @@
 """Device transpose and symmetrisation (csrc/transpose.cu): exact against the host graph
-library at the edges of tiles (3,072 pairs) and digits (2^8, 2^16 ids), with hubs, long runs of
+library at the edges of tiles (4,608 pairs) and digits (2^8, 2^16 ids), with hubs, long runs of
 vertices without edges, and more tiles than run at once."""
 import numpy as np
 import pytest
@@ -30,7 +30,7 @@ def _random(n, m, seed, skew=1.0):
 
 
 CASES = {
-    **{f"m_{m}": (lambda m=m: _random(300, m, m)) for m in (1, 31, 3071, 3072, 3073, 6145)},
+    **{f"m_{m}": (lambda m=m: _random(300, m, m)) for m in (1, 31, 383, 385, 3073, 4607, 4608, 4609, 9217)},
     **{f"n_{n}": (lambda n=n: _random(n, 20011, n)) for n in (1, 2, 255, 256, 257, 65535, 65536, 65537)},
     "skewed": lambda: _random(1 << 20, 700_017, 5, skew=6.0),
     "many_tiles": lambda: _random((1 << 21) + 3, 4_000_001, 6),
