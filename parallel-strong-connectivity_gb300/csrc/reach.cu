@@ -1052,309 +1052,154 @@ __global__ void __launch_bounds__(BLOCK) k_reach_heavy(ReachSide s0, ReachSide s
   }
 }
 
-// Pull round: B_* is the reverse direction of the search, A_off the search
-// direction's offsets (for the next round's edge count).  A warp owns 32
-// consecutive vertices; each unvisited one scans its in-edges for a frontier
-// vertex, kPullP edges in flight, alone for its first kPullSolo in-edges; the
-// longer in-lists left over are then scanned by the whole warp, one vertex at
-// a time, 32 * kPullP edges per step, until a hit.
-#ifndef PSC_PULL_W
-#define PSC_PULL_W 4
-#endif
-constexpr int kPullW = PSC_PULL_W;  // bitmap words per warp step
-#ifndef PSC_PULL_STAGED
-#define PSC_PULL_STAGED 1
-#endif
-constexpr bool kPullStaged = PSC_PULL_STAGED != 0;  // tiles staged by bulk copies
+// Pull round: B_* is the reverse direction of the search.  A warp takes `wps` words
+// of the visited bitmap (at most 32, one per lane), lists the vertices that are
+// neither visited nor dead in shared memory, and scans the in-lists of the listed
+// ones for a frontier vertex, 32 * kPullB vertices at a time: the ranges of all, the
+// first in-edges of all, their frontier bits (dense rounds often hit at once), then
+// each vertex alone up to kPullSolo in-edges, kPullP in flight, then the long
+// in-lists left over by the whole warp, 32 * kPullP edges per step, until a hit.
+//
+// What bounds it: four dependent trips to memory per step (words, range, first
+// in-edge, frontier bit).  Without the list a lane owned a fixed vertex, two thirds
+// of the lanes of a first pull round on R-MAT 2^26 and 98 % of a second had nothing
+// to do, and the steps were as many as the bitmap has words.
+// R-MAT 2^26 (6.7e7 vertices, 6.1e8 edges), per side: first pull 480 -> 330 us (tiles
+// staged by bulk copies before), second 315 -> 65 us.  SCC 5.02 -> 4.15 ms.
+// dead (optional): bitmap of vertices without in-edges in this direction, which no
+// pull can reach; they keep their visited bit clear, and still count as unvisited
+// (the work of the reference's dense round).  The next round's out-edge count is
+// left to k_pull_out_edges, off this chain.
+// (vertices per lane and blocks an SM, SCC of R-MAT 2^26 / load and SCC of 2^22: 2 and
+// 6 4.12 / 4.90 ms, 4 and 4 4.11 / 4.94, 8 and 4 4.48 / 5.11; scanning a lane's
+// vertices together instead of one after the other 4.26 / 4.97)
+constexpr int kPullB = 2;
 
-// One warp step of a pull round over W adjacent bitmap words (32 W vertices)
-// starting at word w: lane's vertex of word k is unvisited when t[k], with
-// in-list [b[k], e[k]).  The first in-edges of all W vertices are loaded
-// together (dense rounds often hit at once), then each unvisited vertex
-// scans alone, then the long in-lists left over are scanned by the whole
-// warp; the words' new frontier bits are written with one store each.
-template <int W>
-__device__ __forceinline__ void pull_step(uint64_t w, uint64_t nwords, const uint32_t* vw,
-                                          const bool* t, const uint64_t* b, const uint64_t* e,
-                                          const uint32_t* __restrict__ B_E,
-                                          const uint32_t* __restrict__ fb_in, uint32_t* vis,
-                                          uint32_t* fb_out, unsigned long long& cnt,
-                                          unsigned long long& scanned) {
-  const unsigned lane = lane_id();
-  bool f[W];
-  uint64_t j[W], lim[W];
-  uint32_t x[W];
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1536 / BLOCK)
+    k_reach_pull(const uint64_t* __restrict__ B_off, const uint32_t* __restrict__ B_E,
+                 const uint32_t* __restrict__ fb_in, uint32_t* vis, uint32_t* fb_out, uint64_t n,
+                 Counters* ctr, const uint32_t* __restrict__ dead, uint32_t wps) {
+  constexpr int B = kPullB;
+  __shared__ uint16_t lists[BLOCK / 32][1024];
+  __shared__ uint32_t founds[BLOCK / 32][32];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  uint16_t* list = lists[wid];
+  uint32_t* found = founds[wid];
+  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
+  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
+  const uint64_t nwords = (n + 31) >> 5;
+  unsigned long long cnt = 0, scanned = 0, unvisited = 0;
+  for (uint64_t base = gw * wps; base < nwords; base += nw * wps) {
+    const uint64_t w = base + lane;
+    const bool mine = lane < wps && w < nwords;
+    const uint32_t vw = mine ? vis[w] : ~0u;
+    const uint32_t dw = mine && dead ? __ldg(&dead[w]) : 0u;
+    uint32_t un = ~vw;
+    if (mine && w * 32 + 32 > n) un &= (1u << (n & 31)) - 1u;
+    unvisited += __popc(un);
+    uint32_t live = un & ~dw;
+    const uint32_t c = __popc(live);
+    uint32_t incl = c;
 #pragma unroll
-  for (int k = 0; k < W; k++) {
-    lim[k] = e[k] < b[k] + kPullSolo ? e[k] : b[k] + kPullSolo;
-    j[k] = b[k];
-    x[k] = t[k] && j[k] < lim[k] ? __ldg(&B_E[j[k]]) : 0xFFFFFFFFu;
-  }
-#pragma unroll
-  for (int k = 0; k < W; k++) {
-    f[k] = x[k] != 0xFFFFFFFFu && fb_test(fb_in, x[k]);
-    if (t[k] && j[k] < lim[k]) j[k]++;
-  }
-#pragma unroll
-  for (int k = 0; k < W; k++)
-    if (t[k] && !f[k]) f[k] = pull_scan(B_E, fb_in, j[k], lim[k]);
-#pragma unroll
-  for (int k = 0; k < W; k++)
-    if (t[k]) scanned += j[k] - b[k];
-#pragma unroll
-  for (int k = 0; k < W; k++)
-    pull_long(B_E, fb_in, __ballot_sync(kFull, t[k] && !f[k] && j[k] < e[k]), j[k], e[k], f[k],
-              scanned);
-#pragma unroll
-  for (int k = 0; k < W; k++) {
-    const uint32_t mk = __ballot_sync(kFull, f[k]);
-    if (lane == 0 && w + k < nwords) {
-      fb_out[w + k] = mk;
-      if (mk) vis[w + k] = vw[k] | mk;
-      cnt += __popc(mk);
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kFull, incl, o);
+      if ((int)lane >= o) incl += t;
     }
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    if (total == 0) {
+      if (mine) fb_out[w] = 0;
+      continue;
+    }
+    found[lane] = 0;
+    for (uint32_t r = incl - c; live; live &= live - 1)
+      list[r++] = (uint16_t)(lane * 32 + (__ffs(live) - 1));
+    __syncwarp();
+    const uint64_t v0 = base * 32;
+    for (uint32_t i0 = 0; i0 < total; i0 += 32 * B) {
+      uint32_t li[B], x[B];
+      uint64_t j[B], e[B], lim[B];
+      bool f[B];
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        const uint32_t i = i0 + k * 32 + lane;
+        li[k] = i < total ? list[i] : 0u;
+        j[k] = e[k] = 0;
+        if (i < total) {
+          j[k] = __ldg(&B_off[v0 + li[k]]);
+          e[k] = __ldg(&B_off[v0 + li[k] + 1]);
+        }
+        scanned -= j[k];
+      }
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        lim[k] = e[k] < j[k] + kPullSolo ? e[k] : j[k] + kPullSolo;
+        x[k] = j[k] < lim[k] ? __ldg(&B_E[j[k]]) : kNone;
+      }
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        f[k] = x[k] != kNone && fb_test(fb_in, x[k]);
+        if (j[k] < lim[k]) j[k]++;
+      }
+#pragma unroll
+      for (int k = 0; k < B; k++)
+        if (!f[k]) f[k] = pull_scan(B_E, fb_in, j[k], lim[k]);
+#pragma unroll
+      for (int k = 0; k < B; k++) scanned += j[k];
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        pull_long(B_E, fb_in, __ballot_sync(kFull, !f[k] && j[k] < e[k]), j[k], e[k], f[k], scanned);
+        if (f[k]) atomicOr(&found[li[k] >> 5], 1u << (li[k] & 31));
+      }
+    }
+    __syncwarp();
+    if (mine) {
+      const uint32_t fw = found[lane];
+      fb_out[w] = fw;
+      if (fw) vis[w] = vw | fw;
+      cnt += __popc(fw);
+    }
+    __syncwarp();
   }
-}
-
-__device__ __forceinline__ void flush_pull_counters(Counters* ctr, unsigned long long cnt,
-                                                    unsigned long long scanned,
-                                                    unsigned long long unvisited) {
+  cnt = warp_sum(cnt);
   scanned = warp_sum(scanned);
   unvisited = warp_sum(unvisited);
-  if (lane_id() == 0) {
+  if (lane == 0) {
     if (cnt) atomicAdd(&ctr->next, cnt);
     if (scanned) atomicAdd(&ctr->edges, scanned);
     if (unvisited) atomicAdd(&ctr->unvisited, unvisited);
   }
 }
 
-// A warp's W words read from global memory: visited words and in-list ranges.
-// dead (optional): bitmap of vertices without in-edges in this direction,
-// which no pull can reach; they are skipped like visited ones (no in-list
-// range read) but keep their visited bit clear, and still count as
-// unvisited (the work of the reference's dense round).
-template <int W>
-__device__ __forceinline__ void pull_load_global(uint64_t w, uint64_t nwords, uint64_t n,
-                                                 const uint64_t* __restrict__ B_off,
-                                                 const uint32_t* __restrict__ dead,
-                                                 const uint32_t* vis, uint32_t* vw, bool* t,
-                                                 uint64_t* b, uint64_t* e,
-                                                 unsigned long long& unvisited) {
-  const unsigned lane = lane_id();
-  uint32_t dw[W];
-#pragma unroll
-  for (int k = 0; k < W; k++) {
-    vw[k] = w + k < nwords ? vis[w + k] : ~0u;
-    dw[k] = dead && w + k < nwords ? __ldg(&dead[w + k]) : 0u;
-  }
-#pragma unroll
-  for (int k = 0; k < W; k++) {
-    const uint64_t v = (w + k) * 32 + lane;
-    t[k] = v < n && !(((vw[k] | dw[k]) >> lane) & 1u);
-    b[k] = e[k] = 0;
-    if (t[k]) {
-      b[k] = B_off[v];
-      e[k] = B_off[v + 1];
-    }
-    unvisited += v < n && !((vw[k] >> lane) & 1u) ? 1 : 0;  // dead ones included
-  }
-}
-
-// Pull round reading the visited words and in-list offsets from global
-// memory: W words per warp step, so W dependent chains (visited word,
-// in-list range, first in-edge, frontier bit) overlap.  The next round's
-// out-edge count is left to k_pull_out_edges, off this chain.
-template <int BLOCK, int W>
-__global__ void __launch_bounds__(BLOCK)
-    k_reach_pull(const uint64_t* __restrict__ B_off, const uint32_t* __restrict__ B_E,
-                 const uint32_t* __restrict__ fb_in, uint32_t* vis, uint32_t* fb_out, uint64_t n,
-                 Counters* ctr, const uint32_t* __restrict__ dead) {
-  const unsigned wid = threadIdx.x >> 5;
-  const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
-  const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
-  const uint64_t nwords = (n + 31) >> 5;
-  unsigned long long cnt = 0, scanned = 0, unvisited = 0;
-  for (uint64_t w = gw * W; w < nwords; w += nw * W) {
-    uint32_t vw[W];
-    bool t[W];
-    uint64_t b[W], e[W];
-    pull_load_global<W>(w, nwords, n, B_off, dead, vis, vw, t, b, e, unvisited);
-    pull_step<W>(w, nwords, vw, t, b, e, B_E, fb_in, vis, fb_out, cnt, scanned);
-  }
-  flush_pull_counters(ctr, cnt, scanned, unvisited);
-}
-
-// ---------------------------------------------------------------------------
-// Bulk asynchronous copies into shared memory (cp.async.bulk, the 1-D form of
-// the tensor memory accelerator's copies) completing on an mbarrier.  Every
-// wait is bounded: past kStageSpin polls it gives up and the kernel reports
-// the failure through its counters instead of waiting on.
-// ---------------------------------------------------------------------------
-constexpr uint32_t kStageSpin = 1u << 20;
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-// dst, src 16-byte aligned, bytes a multiple of 16
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes,
-                                              uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kStageSpin; i++)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
-// Pull round with staged steps: each warp works through its steps of W words
-// (32 W vertices) in grid-stride order and keeps its own two shared-memory
-// buffers; lane 0 copies the visited words and in-list offsets of the step
-// after next into the buffer just worked on (bulk asynchronous copies on the
-// warp's own mbarrier), so the loads left on the warp's dependent chain are
-// the first in-edge and the frontier bit, and no warp waits for another.  A
-// step is staged when its copy stays inside the arrays (offsets
-// [v0, v0 + 32 W + 2) with v0 + 32 W + 1 <= n); the last steps are read from
-// global memory like k_reach_pull.  A copy that does not arrive within the
-// bounded wait sets ctr->aux1 and the warp stops (the host reports it).
-template <int BLOCK, int W>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK)
-    k_reach_pull_staged(const uint64_t* __restrict__ B_off, const uint32_t* __restrict__ B_E,
-                        const uint32_t* __restrict__ fb_in, uint32_t* vis, uint32_t* fb_out,
-                        uint64_t n, Counters* ctr) {
-  constexpr uint32_t NW = BLOCK / 32;
-  constexpr uint32_t SV = 32 * W;  // vertices per step
-  constexpr uint32_t OFF_BYTES = (SV + 2) * 8;
-  constexpr uint32_t VIS_BYTES = W * 4;
-  static_assert(OFF_BYTES % 16 == 0 && VIS_BYTES % 16 == 0, "bulk copies of 16-byte multiples");
-  __shared__ __align__(128) uint64_t soff[NW][2][SV + 2];
-  __shared__ __align__(16) uint32_t svis[NW][2][W];
-  __shared__ __align__(8) uint64_t bar[NW][2];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  const uint64_t nwords = (n + 31) >> 5;
-  const uint64_t nsteps = (nwords + W - 1) / W;
-  const uint64_t s0 = (uint64_t)blockIdx.x * NW + wid, sstep = (uint64_t)gridDim.x * NW;
-  auto staged = [&](uint64_t st) { return st * SV + SV + 1 <= n; };
-  auto issue = [&](uint64_t st, int b) {  // lane 0
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[wid][b], OFF_BYTES + VIS_BYTES);
-    bulk_copy_g2s(soff[wid][b], B_off + st * SV, OFF_BYTES, &bar[wid][b]);
-    bulk_copy_g2s(svis[wid][b], vis + st * W, VIS_BYTES, &bar[wid][b]);
-  };
-  if (lane == 0) {
-    mbar_init(&bar[wid][0], 1);
-    mbar_init(&bar[wid][1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
-  // bit b: the phase parity to wait for / a copy in flight, of buffer b
-  uint32_t parity = 0, pending = 0;
-  for (int b = 0; b < 2; b++) {
-    const uint64_t st = s0 + b * sstep;
-    if (st < nsteps && staged(st)) {
-      if (lane == 0) issue(st, b);
-      pending |= 1u << b;
-    }
-  }
-  unsigned long long cnt = 0, scanned = 0, unvisited = 0;
-  bool failed = false;
-  int buf = 0;
-  for (uint64_t st = s0; st < nsteps; st += sstep, buf ^= 1) {
-    const uint64_t w = st * W;
-    uint32_t vw[W];
-    bool t[W];
-    uint64_t b[W], e[W];
-    if ((pending >> buf) & 1u) {
-      const bool ok = mbar_wait_bounded(&bar[wid][buf], (parity >> buf) & 1u);
-      if (__any_sync(kFull, !ok)) {  // giving up is decided warp-wide
-        failed = true;
-        break;
-      }
-      parity ^= 1u << buf;
-      pending &= ~(1u << buf);
-#pragma unroll
-      for (int k = 0; k < W; k++) {
-        const uint32_t li = k * 32 + lane;
-        vw[k] = svis[wid][buf][k];
-        t[k] = !((vw[k] >> lane) & 1u);
-        b[k] = e[k] = 0;
-        if (t[k]) {
-          b[k] = soff[wid][buf][li];
-          e[k] = soff[wid][buf][li + 1];
-        }
-        unvisited += t[k] ? 1 : 0;
-      }
-      // every lane has its values: the buffer may take the step after next
-      __syncwarp();
-      const uint64_t nt = st + 2 * sstep;
-      if (nt < nsteps && staged(nt)) {
-        if (lane == 0) issue(nt, buf);
-        pending |= 1u << buf;
-      }
-    } else {
-      pull_load_global<W>(w, nwords, n, B_off, nullptr, vis, vw, t, b, e, unvisited);
-    }
-    pull_step<W>(w, nwords, vw, t, b, e, B_E, fb_in, vis, fb_out, cnt, scanned);
-  }
-  if (failed) {
-    // the copies still in flight land before the block's shared memory goes
-    if (pending & 1u) mbar_wait_bounded(&bar[wid][0], parity & 1u);
-    if (pending & 2u) mbar_wait_bounded(&bar[wid][1], (parity >> 1) & 1u);
-    if (lane == 0) atomicOr(&ctr->aux1, 1ull);
-  }
-  flush_pull_counters(ctr, cnt, scanned, unvisited);
-}
-
-// A pull round's grid: the resident blocks of the kernel (a grid-stride loop
-// covers the rest), fewer when the bitmap has fewer warp steps than that.
-template <int BLOCK, bool STAGED = false>
-static unsigned pull_grid(int num_sms, uint64_t nwords) {
+// A pull round on the resident blocks of the kernel, words per warp step as many
+// as give every warp two steps (4 to 32).
+template <int BLOCK>
+static void launch_pull(int num_sms, cudaStream_t st, const uint64_t* B_off, const uint32_t* B_E,
+                        const uint32_t* fb_in, uint32_t* vis, uint32_t* fb_out, uint64_t n,
+                        Counters* ctr, const uint32_t* dead) {
   static int per_sm = [] {
     int b = 0;
-    cudaError_t e =
-        STAGED ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                     &b, k_reach_pull_staged<BLOCK, kPullW>, BLOCK, 0)
-               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_reach_pull<BLOCK, kPullW>,
-                                                               BLOCK, 0);
-    if (e != cudaSuccess || b < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_reach_pull<BLOCK>, BLOCK, 0) !=
+            cudaSuccess ||
+        b < 1) {
       cudaGetLastError();
       b = 1;
     }
     return b;
   }();
-  const uint64_t steps = (nwords + kPullW - 1) / kPullW;
-  const uint64_t want = (steps + BLOCK / 32 - 1) / (BLOCK / 32);
-  const uint64_t cap = (uint64_t)num_sms * per_sm;
-  return (unsigned)std::max<uint64_t>(1, std::min(want, cap));
+  const uint64_t nwords = (n + 31) / 32, cap = (uint64_t)num_sms * per_sm;
+  uint32_t wps = 32;
+  while (wps > 4 && nwords < 2 * cap * (BLOCK / 32) * wps) wps /= 2;
+  const uint64_t want = (nwords + wps * (BLOCK / 32) - 1) / (wps * (BLOCK / 32));
+  k_reach_pull<BLOCK><<<(unsigned)std::max<uint64_t>(1, std::min(want, cap)), BLOCK, 0, st>>>(
+      B_off, B_E, fb_in, vis, fb_out, n, ctr, dead, wps);
 }
-
-constexpr uint64_t kPullStagedTile = 32ull * kPullW;  // vertices of a staged warp step
 
 constexpr uint64_t kPullExactBelow = 1u << 14;
 constexpr uint32_t kSampleProbes = 32 * 64;
 constexpr uint32_t kSampleHits = 50;
+constexpr int kSampleK = 8;  // probes per lane in flight (70 -> 29 us when 2 % are hits)
+static_assert(kSampleProbes % (32 * kSampleK) == 0, "whole batches");
 
 __global__ void k_pull_out_edges(const uint32_t* __restrict__ fb, const uint64_t* __restrict__ A_off,
                                  uint64_t n, uint32_t seed, Counters* ctr) {
@@ -1379,13 +1224,21 @@ __global__ void k_pull_out_edges(const uint32_t* __restrict__ fb, const uint64_t
   if (blockIdx.x != 0 || threadIdx.x >= 32) return;
   unsigned long long sum = 0;
   uint32_t hits = 0;
-  for (uint32_t base = 1; base <= kSampleProbes && hits < kSampleHits; base += 32) {
-    const uint32_t idx = (uint32_t)(hash32(seed + base + lane) % n);
-    const bool hit = fb_test(fb, idx);
-    const uint32_t m = __ballot_sync(kFull, hit);
-    const uint32_t rank = __popc(m & ((1u << lane) - 1));
-    if (hit && hits + rank < kSampleHits) sum += A_off[idx + 1] - A_off[idx];
-    hits += __popc(m);
+  for (uint32_t base = 1; base <= kSampleProbes && hits < kSampleHits; base += 32 * kSampleK) {
+    uint32_t idx[kSampleK], word[kSampleK];
+#pragma unroll
+    for (int k = 0; k < kSampleK; k++) {
+      idx[k] = (uint32_t)(hash32(seed + base + k * 32 + lane) % n);
+      word[k] = __ldg(&fb[idx[k] >> 5]);
+    }
+#pragma unroll
+    for (int k = 0; k < kSampleK; k++) {
+      const bool hit = (word[k] >> (idx[k] & 31)) & 1u;
+      const uint32_t m = __ballot_sync(kFull, hit);
+      const uint32_t rank = __popc(m & ((1u << lane) - 1));
+      if (hit && hits + rank < kSampleHits) sum += A_off[idx[k] + 1] - A_off[idx[k]];
+      hits += __popc(m);
+    }
   }
   sum = warp_sum(sum);
   if (hits > kSampleHits) hits = kSampleHits;
@@ -1899,9 +1752,6 @@ struct Side {
   uint64_t nf = 0, nf_edges = 0, prev_nf = 0;
   bool pull = false;
   uint32_t rounds = 0;
-  // unvisited vertices that some pull could still reach, after the last
-  // pull round (an upper bound; UINT64_MAX before the first)
-  uint64_t live = UINT64_MAX;
 };
 
 // Counter sets of k_reach_async: the control words of side k, and its counters.
@@ -2254,33 +2104,16 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       const uint32_t* fa = (const uint32_t*)g->bufs[s.slot_fa].p;
       uint32_t* fbo = (uint32_t*)g->bufs[s.slot_fb].p;
       const uint32_t* dead = (const uint32_t*)g->bufs[B_DEAD].p + (s.backward ? nwords + 1 : 0);
-      // Few vertices left that a pull could reach (on R-MAT 2^26 the second
-      // pull round finds 1-2 M of the 41 M unvisited, the rest have no
-      // in-edge): the global-memory kernel with the dead bitmap reads only
-      // their ranges, where the staged one copies every range.
-      const bool sparse = s.live != UINT64_MAX && 8 * s.live < n;
       switch (g->block) {
         case 128:
-          k_reach_pull<128, kPullW><<<pull_grid<128>(g->num_sms, nwords), 128, 0, g->stream>>>(
-              B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset, dead);
+          launch_pull<128>(g->num_sms, g->stream, B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset, dead);
           break;
         case 512:
-          k_reach_pull<512, kPullW><<<pull_grid<512>(g->num_sms, nwords), 512, 0, g->stream>>>(
-              B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset, dead);
+          launch_pull<512>(g->num_sms, g->stream, B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset, dead);
           break;
         default:
-          // staged tiles when at least one tile fits inside the arrays and
-          // they are 16-byte aligned (bulk copies)
-          if (kPullStaged && !sparse && n >= kPullStagedTile + 1 && ((uintptr_t)B_off & 15) == 0 &&
-              ((uintptr_t)s.vis & 15) == 0) {
-            k_reach_pull_staged<kReachBlock, kPullW>
-                <<<pull_grid<kReachBlock, true>(g->num_sms, nwords), kReachBlock, 0, g->stream>>>(
-                    B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset);
-          } else {
-            k_reach_pull<kReachBlock, kPullW>
-                <<<pull_grid<kReachBlock>(g->num_sms, nwords), kReachBlock, 0, g->stream>>>(
-                    B_off, B_E, fa, s.vis, fbo, n, g->ctr + s.cset, dead);
-          }
+          launch_pull<kReachBlock>(g->num_sms, g->stream, B_off, B_E, fa, s.vis, fbo, n,
+                                   g->ctr + s.cset, dead);
       }
       k_pull_out_edges<<<grid_for(g, nwords, 256), 256, 0, g->stream>>>(
           fbo, A_off, n, hash32((uint32_t)s.rounds), g->ctr + s.cset);
@@ -2326,7 +2159,6 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       Side& s = sides[k];
       if (mode[k] == M_NONE) continue;
       const Counters& c = g->hctr[s.cset];
-      if (mode[k] == M_PULL && c.aux1) return PSC_ERR_ITER_LIMIT;  // a staged copy never came
       if (g->profiling) {
         // algorithmic bytes: 16 per adjacency range read, 4 + 1 per edge
         // (target id, visited flag), 5 per new frontier vertex; pull: 16 per
@@ -2336,12 +2168,6 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         g->prof[fam].bytes += mode[k] == M_PULL
                                   ? 16.0 * c.unvisited + 5.0 * c.edges + 0.25 * n + 1.0 * c.next
                                   : 16.0 * c.expanded + 5.0 * c.edges + 5.0 * c.next;
-      }
-      if (mode[k] == M_PULL) {
-        // unvisited minus the dead ones (all unvisited but sources) minus found
-        const uint64_t dead_n = g->dead_count[s.backward ? 1 : 0];
-        const uint64_t u = c.unvisited > dead_n ? c.unvisited - dead_n : 0;
-        s.live = u > c.next ? u - c.next : 0;
       }
       if (mode[k] == M_PULL)
         std::swap(g->bufs[s.slot_fa], g->bufs[s.slot_fb]);
@@ -2567,9 +2393,7 @@ extern "C" int psc_reach_noalloc(const uint64_t* d_off, const uint32_t* d_E,
         continue;
       }
     } else {
-      k_reach_pull<kReachBlock, kPullW>
-          <<<pull_grid<kReachBlock>(nd.num_sms, nwords), kReachBlock, 0, s>>>(
-              B_off, B_E, fa, vis, fb, n, ctr, nullptr);
+      launch_pull<kReachBlock>(nd.num_sms, s, B_off, B_E, fa, vis, fb, n, ctr, nullptr);
       k_pull_out_edges<<<na_grid(nd.num_sms, nwords, 256), 256, 0, s>>>(fb, A_off, n,
                                                                         hash32(r), ctr);
       std::swap(fa, fb);
