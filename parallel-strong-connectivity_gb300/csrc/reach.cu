@@ -335,7 +335,7 @@ __device__ __forceinline__ void vgc_direct(const ReachSide& S, uint64_t ub, uint
 // Other chunk vertices are expanded directly (heavy ones by the whole grid).
 template <int BLOCK, int QCAP, int K, bool SPEC>
 __global__ void __launch_bounds__(BLOCK)
-    k_reach_vgc(ReachSide s0, ReachSide s1, uint32_t tau, uint32_t chunk) {
+    k_reach_vgc(ReachSide s0, ReachSide s1, uint32_t tau, uint32_t chunk, uint32_t hlim) {
   __shared__ WarpExpandSmem sm[BLOCK / 32];
   __shared__ QEnt sq[BLOCK / 32][QCAP];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
@@ -368,9 +368,9 @@ __global__ void __launch_bounds__(BLOCK)
       ub = S.off[u];
       du = S.off[u + 1] - ub;
       (sd ? exp1 : exp0)++;
-      if (du > kHeavyDeg) heavy_push(S, u, du);
+      if (du > hlim) heavy_push(S, u, du);
     }
-    uint32_t big = __ballot_sync(kFull, lane < cnt && du >= tq && du <= kHeavyDeg);
+    uint32_t big = __ballot_sync(kFull, lane < cnt && du >= tq && du <= hlim);
     while (big) {
       const int l = __ffs(big) - 1;
       big &= big - 1;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(BLOCK)
       if (lane == 0) (sd ? scanned1 : scanned0) += bd;
       vgc_direct<K>(S, bb, bd, nedges);
     }
-    const bool seed = lane < cnt && du > 0 && du < tq;
+    const bool seed = lane < cnt && du > 0 && du < tq && du <= hlim;
     const uint32_t smask = __ballot_sync(kFull, seed);
     if (seed) Q[__popc(smask & ((1u << lane) - 1))] = QEnt{ub, u, (uint32_t)du};
     const uint32_t nseed = __popc(smask);
@@ -987,11 +987,20 @@ __global__ void k_async_collect(const uint32_t* __restrict__ slot, const AsyncCt
 
 // Heavy vertices of both sides: the chunks of a side's heavy list are cut
 // into one contiguous range per warp; a warp finds the entry of its first
-// chunk once, then claims kHeavyChunk edges per step (a heavy vertex has
-// more than 64 chunks, so the next entry is at most one step away).
+// chunk once, then claims kHeavyChunk edges per step (every entry has a
+// chunk, so the next entry is at most one step away).  What a warp claims
+// collects in shared memory and goes to the next frontier kHeavyBuf / 2 and more
+// vertices at a time: one reservation per chunk was an atomic on the same word
+// every 3 ns, and the chunks waited for it.
+// R-MAT 2^26, 1.7e7 edges of both sides: 443 -> 225 us (8 instead of 4 edges in flight
+// per lane without the buffer 325; with it, 4 or 8 edges and 512 or 1,024 entries
+// 220 to 229; 16 edges 300).
+constexpr uint32_t kHeavyBuf = 512;
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_reach_heavy(ReachSide s0, ReachSide s1) {
+  __shared__ uint32_t bufs[BLOCK / 32][kHeavyBuf];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  uint32_t* buf = bufs[wid];
   const uint64_t gw = (uint64_t)blockIdx.x * (BLOCK / 32) + wid;
   const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
 #pragma unroll 1
@@ -1015,6 +1024,21 @@ __global__ void __launch_bounds__(BLOCK) k_reach_heavy(ReachSide s0, ReachSide s
     uint64_t cs = (uint32_t)ent, cn = h + 1 < nh ? (uint32_t)__ldg(&S.heavy[h + 1]) : total;
     uint64_t beg = S.off[ent >> 32], end = S.off[(ent >> 32) + 1];
     unsigned long long scanned = 0, next_edges = 0;
+    uint32_t held = 0;  // claimed vertices in buf (warp-uniform)
+    auto flush = [&] {
+      __syncwarp();
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(&S.ctr->next, (unsigned long long)held);
+      base = __shfl_sync(kFull, base, 0);
+#pragma unroll 4
+      for (uint32_t i = lane; i < held; i += 32) {
+        const uint32_t v = buf[i];
+        S.qout[base + i] = v;
+        next_edges += S.off[v + 1] - S.off[v];
+      }
+      __syncwarp();
+      held = 0;
+    };
     for (uint64_t c = c_beg; c < c_end; c++) {
       if (c >= cn) {
         h++;
@@ -1038,11 +1062,15 @@ __global__ void __launch_bounds__(BLOCK) k_reach_heavy(ReachSide s0, ReachSide s
 #pragma unroll
       for (int k = 0; k < kHeavyK; k++)
         if (e0 + k * 32 + lane < end && bit_set(S.vis, v[k])) tm |= 1u << k;
-      warp_append_batch<kHeavyK>(tm, v, S.qout, &S.ctr->next);
 #pragma unroll
-      for (int k = 0; k < kHeavyK; k++)
-        if (tm & (1u << k)) next_edges += S.off[v[k] + 1] - S.off[v[k]];
+      for (int k = 0; k < kHeavyK; k++) {
+        const uint32_t mk = __ballot_sync(kFull, (tm >> k) & 1u);
+        if ((tm >> k) & 1u) buf[held + __popc(mk & ((1u << lane) - 1u))] = v[k];
+        held += __popc(mk);
+      }
+      if (held > kHeavyBuf - kHeavyChunk) flush();
     }
+    if (held) flush();
     scanned = warp_sum(scanned);
     next_edges = warp_sum(next_edges);
     if (lane == 0) {
@@ -1618,19 +1646,24 @@ static int launch_async(psc_graph_s* g, bool rec, const ReachSide& a, const Reac
 #define PSC_VGC_SPEC_CHUNK 8
 #endif
 constexpr uint64_t kVgcSpecChunk = PSC_VGC_SPEC_CHUNK;
+// Out-degree above which a vertex of a sparse VGC round (one vertex per warp) goes to
+// k_reach_heavy: a warp takes some 5 us per 256 edges, so the round waits for its
+// largest vertex, and the extra launch costs about what 2,048 edges do (second round
+// of R-MAT 2^26: 335 + 225 us with 8,192, 183 + 241 with 2,048, 184 + 244 with 1,024).
+constexpr uint32_t kVgcHeavy = 2048;
 static void launch_vgc(psc_graph_s* g, unsigned blocks, const ReachSide& a, const ReachSide& b,
-                       uint32_t tau, uint32_t chunk, bool spec) {
+                       uint32_t tau, uint32_t chunk, bool spec, uint32_t hlim) {
   cudaStream_t st = g->stream;
   if (vgc_narrow(g)) {
     if (spec)
-      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKNarrow, true><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk);
+      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKNarrow, true><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk, hlim);
     else
-      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKNarrow, false><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk);
+      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKNarrow, false><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk, hlim);
   } else {
     if (spec)
-      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKWide, true><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk);
+      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKWide, true><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk, hlim);
     else
-      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKWide, false><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk);
+      k_reach_vgc<kVgcBlock, kVgcQueue, kVgcKWide, false><<<blocks, kVgcBlock, 0, st>>>(a, b, tau, chunk, hlim);
   }
 }
 
@@ -2078,7 +2111,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       const uint64_t chunks = (v_items + chunk - 1) / chunk;
       const uint64_t blocks = std::min(max_blocks, (chunks + kVgcBlock / 32 - 1) / (kVgcBlock / 32));
       launch_vgc(g, (unsigned)std::max<uint64_t>(1, blocks), vg[0], vg[1], tau, (uint32_t)chunk,
-                 chunk <= kVgcSpecChunk);
+                 chunk <= kVgcSpecChunk, chunk == 1 ? kVgcHeavy : (uint32_t)kHeavyDeg);
     }
     if (np) {
       ProfScope ps(g, F_REACH_PUSH);

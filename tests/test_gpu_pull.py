@@ -66,3 +66,26 @@ def test_pull_matches_definition(n, hub):
     finally:
         for p in ptrs:
             lib.psc_device_free(p)
+
+
+def test_sparse_round_hands_large_vertices_to_the_grid():
+    """Past the resident rounds and a stopped resident search (a vertex of 8,193 out-edges), a
+    round of three vertices around the direct limit of 2,048 out-edges, without pulls."""
+    hub, fans, side = 8193, (2048, 2049, 5000), 1500
+    src, dst = [np.arange(24), np.full(hub, 24)], [np.arange(1, 25), 25 + np.arange(hub)]
+    n = 25 + hub
+    top = n + np.arange(3)
+    src.append(np.full(3, 25))
+    dst.append(top)
+    n += 3
+    for t, d in zip(top, fans):
+        src += [np.full(d, t), [n + d - 1]]
+        dst += [n + np.arange(d), [n + d]]
+        n += d + 1
+    e = np.arange(1_500_000)
+    src.append(n + e % side)
+    dst.append(n + e // side)
+    g = psc.HostGraph.from_edges(n + side, np.concatenate(src), np.concatenate(dst))
+    with psc.DeviceGraph(g) as dg:
+        for back, off, E, s in ((False, g.off, g.E, 0), (True, g.in_off, g.in_E, n - 1)):
+            assert np.array_equal(dg.reach(s, backward=back), O.reach_seq(g.n, off, E, s))
