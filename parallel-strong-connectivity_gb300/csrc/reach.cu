@@ -1785,6 +1785,8 @@ struct Side {
   uint64_t nf = 0, nf_edges = 0, prev_nf = 0;
   bool pull = false;
   uint32_t rounds = 0;
+  // unvisited vertices that some pull could still reach, after a pull round
+  uint64_t live = 0;
 };
 
 // Counter sets of k_reach_async: the control words of side k, and its counters.
@@ -2067,7 +2069,12 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       if (s.nf == 0) continue;
       any = true;
       s.rounds++;
-      const bool want_pull = (s.nf + s.nf_edges) >= threshold;
+      // A search that pulls goes on pulling while that looks at less: the live
+      // vertices and the bitmaps' words (fifth round of R-MAT 2^26, 2.5e6 frontier and
+      // 1e5 live vertices: 0.29 ms pushed, with the bitmaps turned into queues,
+      // 0.14 pulled).
+      const bool want_pull = (s.nf + s.nf_edges) >= threshold ||
+                             (s.pull && s.nf >= s.live + nwords / 4);
       uint32_t* qa = (uint32_t*)g->bufs[s.slot_qa].p;
       uint32_t* fa = (uint32_t*)g->bufs[s.slot_fa].p;
       if (want_pull && !s.pull) {
@@ -2182,11 +2189,12 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
       for (int k = 0; k < ns; k++)
         if (mode[k] != M_NONE)
           std::fprintf(stderr, "reach side %d round %u mode %s nf %llu next %llu edges %llu "
-                       "expanded %llu unvisited %llu waves %llu t %.3f ms\n",
+                       "expanded %llu unvisited %llu live %llu waves %llu t %.3f ms\n",
                        k, sides[k].rounds, mode[k] == M_VGC ? "vgc" : mode[k] == M_PUSH ? "push" : "pull",
                        (unsigned long long)sides[k].nf, g->hctr[sides[k].cset].next,
                        g->hctr[sides[k].cset].edges, g->hctr[sides[k].cset].expanded,
-                       g->hctr[sides[k].cset].unvisited, g->hctr[sides[k].cset].waves, us);
+                       g->hctr[sides[k].cset].unvisited, (unsigned long long)sides[k].live,
+                       g->hctr[sides[k].cset].waves, us);
     }
     for (int k = 0; k < ns; k++) {
       Side& s = sides[k];
@@ -2201,6 +2209,10 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         g->prof[fam].bytes += mode[k] == M_PULL
                                   ? 16.0 * c.unvisited + 5.0 * c.edges + 0.25 * n + 1.0 * c.next
                                   : 16.0 * c.expanded + 5.0 * c.edges + 5.0 * c.next;
+      }
+      if (mode[k] == M_PULL) {  // unvisited minus the dead ones (all but sources) minus found
+        const uint64_t gone = g->dead_count[s.backward ? 1 : 0] + c.next;
+        s.live = c.unvisited > gone ? c.unvisited - gone : 0;
       }
       if (mode[k] == M_PULL)
         std::swap(g->bufs[s.slot_fa], g->bufs[s.slot_fb]);
