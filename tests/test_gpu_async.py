@@ -54,11 +54,26 @@ def _ladder(n=20000):
     return _edges(n, (v, v + 1), (v[::7] + 1, v[::7]))
 
 
+def _band(top, n=60011):
+    """Vertex u leads to up to top of the 40 after it (every 5th to the next one too); one vertex
+    of 70 out-edges keeps the graph off the records."""
+    r = np.random.default_rng(top)
+    d = r.integers(0, top + 1, n)
+    s = np.repeat(np.arange(n), d)
+    v = np.arange(0, n, 5)
+    return _edges(n, (s, (s + r.integers(1, 41, len(s))) % n), (v, (v + 1) % n),
+                  (np.full(70, 11), 12 + np.arange(70)))
+
+
 GRAPHS = {
     "ladder": (_ladder, 0),
     "grid": (lambda: psc.HostGraph.grid(301, 217, 0.5, seed=3), 4000),
     "knn": (lambda: psc.HostGraph.knn(30011, 5, seed=4), 17),
     "hub_behind_strip": (_hub_behind_strip, 0),
+    # eight lanes per entry up to degree 8, the balanced expansion above it
+    "band_7": (lambda: _band(7), 3),
+    "band_8": (lambda: _band(8), 3),
+    "band_11": (lambda: _band(11), 3),
     "tree": (lambda: _tree(17), 0),
     **{f"degree_{d}": (lambda d=d: _regular(d), 7) for d in (1, 5, 6, 7, 12, 13, 63, 64, 65)},
 }
