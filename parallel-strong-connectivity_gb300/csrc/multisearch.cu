@@ -348,14 +348,14 @@ struct MsQEnt {
 // Claims of one batch for pivot lab inside subproblem sub: each candidate's
 // label and adjacency range are loaded together, then the first table probes
 // (atomicCAS) of all K candidates are issued before any is resolved.  Returns
-// the mask of new pairs; sets *failed if an insert gave up.
+// the mask of new pairs; failed: the mask of inserts that gave up.
 template <int K, bool ADJ = true>
 __device__ __forceinline__ uint32_t ms_vgc_claim(const uint32_t* w, uint64_t* vb, uint64_t* ve,
                                                  uint64_t sub, uint32_t lab,
                                                  const uint64_t* __restrict__ off,
                                                  const uint64_t* labels,
                                                  unsigned long long* T, uint64_t mask,
-                                                 uint32_t& probes, bool& failed) {
+                                                 uint32_t& probes, uint32_t& failed) {
   uint64_t key[K], old[K], h[K];
 #pragma unroll
   for (int k = 0; k < K; k++) {
@@ -387,47 +387,52 @@ __device__ __forceinline__ uint32_t ms_vgc_claim(const uint32_t* w, uint64_t* vb
       const int r = old[k] == kEmpty ? 1 : old[k] == key[k] ? 0
                     : table_insert_from(T, mask, key[k], h[k], kProbeLimit - 1, &probes);
       if (r == 1) tm |= 1u << k;
-      failed |= r < 0;
+      if (r < 0) failed |= 1u << k;
     }
   return tm;
 }
 
 // Places this lane's new pairs (bit k of tm) into the warp's queue while it
-// has room, then spills (w, lab) pairs: one warp scan, at most one atomic.
+// has room, then spills (w, lab) pairs: a ballot per step, at most one atomic.
+// Returns the warp's new pairs.
 template <int K>
-__device__ __forceinline__ void ms_vgc_place(uint32_t tm, const uint32_t* w, const uint64_t* vb,
-                                             const uint64_t* ve, uint32_t lab, MsQEnt* Q,
-                                             uint32_t& tail, uint32_t tq, uint64_t* Fout,
-                                             unsigned long long* next_ctr) {
+__device__ __forceinline__ uint32_t ms_vgc_place(uint32_t tm, const uint32_t* w, const uint64_t* vb,
+                                                 const uint64_t* ve, uint32_t lab, MsQEnt* Q,
+                                                 uint32_t& tail, uint32_t tq, uint64_t* Fout,
+                                                 unsigned long long* next_ctr) {
   const unsigned lane = lane_id();
-  const uint32_t cnt = __popc(tm);
-  uint32_t incl = cnt;
+  unsigned m[K];
+  uint32_t total = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(kFull, incl, o);
-    if ((int)lane >= o) incl += t;
+  for (int k = 0; k < K; k++) {
+    m[k] = __ballot_sync(kFull, (tm >> k) & 1u);
+    total += __popc(m[k]);
   }
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  if (total == 0) return;
+  if (total == 0) return 0;
   const uint32_t room = tq - tail;
   const uint32_t nloc = total < room ? total : room;
   unsigned long long sbase = 0;
-  if (total > nloc && lane == 0) sbase = atomicAdd(next_ctr, (unsigned long long)(total - nloc));
-  sbase = __shfl_sync(kFull, sbase, 0);
-  uint32_t r = incl - cnt;
+  if (total > nloc) {
+    if (lane == 0) sbase = atomicAdd(next_ctr, (unsigned long long)(total - nloc));
+    sbase = __shfl_sync(kFull, sbase, 0);
+  }
+  uint32_t b = 0;
 #pragma unroll
-  for (int k = 0; k < K; k++)
-    if (tm & (1u << k)) {
+  for (int k = 0; k < K; k++) {
+    if ((m[k] >> lane) & 1u) {
+      const uint32_t r = b + __popc(m[k] & ((1u << lane) - 1u));
       if (r < nloc) {
         const uint64_t vd = ve[k] - vb[k];
         Q[tail + r] = MsQEnt{vb[k], w[k], (uint32_t)(vd < 0xFFFFFFFFull ? vd : 0xFFFFFFFFull)};
       } else {
         Fout[sbase + (r - nloc)] = ((uint64_t)w[k] << 32) | lab;
       }
-      r++;
     }
+    b += __popc(m[k]);
+  }
   tail += nloc;
   __syncwarp();
+  return total;
 }
 
 // VGC sub-round for up to two sides: one frontier pair (u, l) per warp.  If
@@ -483,10 +488,10 @@ __device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,
           const uint64_t e = b + k * 32 + lane;
           w[k] = e < ue ? __ldg(&S.E[e]) : 0xFFFFFFFFu;
         }
-        bool fk = false;
+        uint32_t fm = 0;
         const uint32_t tm = ms_vgc_claim<kMsK, false>(w, vb, ve, sub, lab, S.off, labels, S.T,
-                                                      S.mask, probes, fk);
-        failed |= fk;
+                                                      S.mask, probes, fm);
+        failed |= fm != 0;
         (sd ? in1 : in0) += __popc(tm);
 #pragma unroll
         for (int k = 0; k < kMsK; k++) keys[k] = ((uint64_t)w[k] << 32) | lab;
@@ -504,80 +509,108 @@ __device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,
     // its share of the table's free room (the first wave always runs)
     uint32_t head = 0, tail = 1, ins = 0;
     while (head < tail && tail < tq && (head == 0 || ins < S.vgc_budget)) {
-      const uint32_t wave = min(32u, tail - head);
+      uint32_t wave = min(32u, tail - head);
       uint64_t beg = 0;
       uint32_t deg = 0, x = 0;
-      bool spill_self = false;
       if (lane < wave) {
         const MsQEnt q = Q[head + lane];
         x = q.v;
         beg = q.beg;
         deg = q.deg;
-        if (deg > tq) {
-          spill_self = true;
-          deg = 0;
-        }
-        if (lane > 0 || head > 0) (sd ? ex1 : ex0)++;
       }
-      head += wave;
-      __syncwarp();
-      if (__any_sync(kFull, spill_self)) emit(spill_self, x);
-      (sd ? sc1 : sc0) += deg;
-      bool failed = false;
-      uint32_t incl = deg;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(kFull, incl, o);
-        if ((int)lane >= o) incl += t;
-      }
-      const uint32_t total = __shfl_sync(kFull, incl, 31);
-      sm.excl[lane] = incl - deg;
-      sm.beg[lane] = beg;
-      __syncwarp();
-      for (uint32_t base = 0; base < total; base += 32 * kMsK) {
+      const uint32_t head0 = head;
+      bool fk = false;  // an insert of this lane failed
+      if (!__any_sync(kFull, deg > 8)) {
+        // eight lanes per vertex, lane j takes its target j (no scan, no search)
+        wave = min(wave, 4u * kMsK);
+        head += wave;
+        const unsigned grp = lane >> 3, j = lane & 7;
         uint32_t w[kMsK];
-        int sl[kMsK];
         uint64_t vb[kMsK], ve[kMsK];
 #pragma unroll
         for (int k = 0; k < kMsK; k++) {
-          const uint32_t gi = base + k * 32 + lane;
           w[k] = 0xFFFFFFFFu;
-          sl[k] = 0;
-          if (gi < total) {
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-              int mid = (lo + hi + 1) >> 1;
-              if (sm.excl[mid] <= gi)
-                lo = mid;
-              else
-                hi = mid - 1;
-            }
-            sl[k] = lo;
-            w[k] = __ldg(&S.E[sm.beg[lo] + (gi - sm.excl[lo])]);
+          if (4 * k + grp < wave) {
+            const MsQEnt& q = Q[head0 + 4 * k + grp];
+            if (j < q.deg) w[k] = __ldg(&S.E[q.beg + j]);
           }
         }
-        bool fk = false;
+        if (lane < wave) {
+          (sd ? sc1 : sc0) += deg;
+          if (head0 + lane > 0) (sd ? ex1 : ex0)++;
+        }
+        uint32_t fm = 0;
         const uint32_t tm = ms_vgc_claim<kMsK>(w, vb, ve, sub, lab, S.off, labels, S.T, S.mask,
-                                               probes, fk);
-        // a failure is charged to the source lane of the failed edge
-        if (fk) {
+                                               probes, fm);
+        if (fm) {
+          fk = true;
 #pragma unroll
           for (int k = 0; k < kMsK; k++)
-            if (w[k] != 0xFFFFFFFFu) atomicOr(&sm.fail, 1u << sl[k]);
+            if ((fm >> k) & 1u) atomicOr(&sm.fail, 1u << (4 * k + grp));
         }
         (sd ? in1 : in0) += __popc(tm);
-        ins += __reduce_add_sync(kFull, (unsigned)__popc(tm));
-        ms_vgc_place<kMsK>(tm, w, vb, ve, lab, Q, tail, tq, S.Fout, &S.ctr->next);
+        ins += ms_vgc_place<kMsK>(tm, w, vb, ve, lab, Q, tail, tq, S.Fout, &S.ctr->next);
+      } else {
+        head += wave;
+        const bool spill_self = deg > tq;
+        if (spill_self) deg = 0;
+        if (lane < wave && head0 + lane > 0) (sd ? ex1 : ex0)++;
+        if (__any_sync(kFull, spill_self)) emit(spill_self, x);
+        (sd ? sc1 : sc0) += deg;
+        uint32_t incl = deg;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(kFull, incl, o);
+          if ((int)lane >= o) incl += t;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        sm.excl[lane] = incl - deg;
+        sm.beg[lane] = beg;
+        __syncwarp();
+        for (uint32_t base = 0; base < total; base += 32 * kMsK) {
+          uint32_t w[kMsK];
+          int sl[kMsK];
+          uint64_t vb[kMsK], ve[kMsK];
+#pragma unroll
+          for (int k = 0; k < kMsK; k++) {
+            const uint32_t gi = base + k * 32 + lane;
+            w[k] = 0xFFFFFFFFu;
+            sl[k] = 0;
+            if (gi < total) {
+              int lo = 0, hi = 31;
+              while (lo < hi) {
+                int mid = (lo + hi + 1) >> 1;
+                if (sm.excl[mid] <= gi)
+                  lo = mid;
+                else
+                  hi = mid - 1;
+              }
+              sl[k] = lo;
+              w[k] = __ldg(&S.E[sm.beg[lo] + (gi - sm.excl[lo])]);
+            }
+          }
+          uint32_t fm = 0;
+          const uint32_t tm = ms_vgc_claim<kMsK>(w, vb, ve, sub, lab, S.off, labels, S.T, S.mask,
+                                                 probes, fm);
+          // a failure is charged to the source lane of the failed edge
+          if (fm) {
+            fk = true;
+#pragma unroll
+            for (int k = 0; k < kMsK; k++)
+              if ((fm >> k) & 1u) atomicOr(&sm.fail, 1u << sl[k]);
+          }
+          (sd ? in1 : in0) += __popc(tm);
+          ins += ms_vgc_place<kMsK>(tm, w, vb, ve, lab, Q, tail, tq, S.Fout, &S.ctr->next);
+        }
       }
-      __syncwarp();
-      failed = (sm.fail >> lane) & 1u;
-      __syncwarp();
-      if (lane == 0) sm.fail = 0;
-      __syncwarp();
       (sd ? pr1 : pr0) += probes;
       probes = 0;
-      const bool rq = failed && lane < wave;
-      if (__any_sync(kFull, rq)) {
+      __syncwarp();
+      if (__any_sync(kFull, fk)) {  // a vertex with a failed insert comes back as a pair
+        const bool rq = ((sm.fail >> lane) & 1u) && lane < wave;
+        __syncwarp();
+        if (lane == 0) sm.fail = 0;
+        __syncwarp();
         emit(rq, x);
         if (rq) (sd ? rq1 : rq0)++;
       }
