@@ -16,11 +16,13 @@
 // an atomic in the source's own shared memory, and the segment lengths are
 // written once per level.  A level is then: read the own segments, load targets,
 // claim (the ranges of the candidates are loaded alongside), store, barrier.
-// Sixteen entries whose degrees are at most 8 are expanded by eight lanes each,
-// which needs neither the prefix sum nor the search of the balanced expansion
-// (BFS 7.46 -> 6.49 ms and reachability 5.58 -> 5.17 on the graphs below).
-// BFS of a 1021 x 2043 grid (2,813 levels): 49.8 -> 6.5 ms, 2.0-2.3 us per level;
-// backward push reachability on kNN 1.5e6: 37.6 -> 5.2 ms.
+// Entries of at most kLvFew edges are expanded by eight lanes each, which needs
+// neither the prefix sum nor the search of the balanced expansion (BFS 7.46 -> 6.49
+// ms and reachability 5.58 -> 5.17 on the graphs below), by code for 4, 8, 16 or 32
+// entries, so that a warp with three entries does not step through empty places
+// (6.76 -> 6.08 and 4.69 -> 4.13; with 8 or 32 entries only, 6.2 to 8.1 and 5.1).
+// BFS of a 1021 x 2043 grid (2,813 levels): 49.8 -> 6.1 ms, 2.1 us per level;
+// backward push reachability on kNN 1.5e6: 37.6 -> 4.6 ms.
 //
 // The cluster hands the search back to the host's wide rounds when a level
 // outgrows it (more than kLvMaxEdges edges, a full segment, or the
@@ -43,7 +45,8 @@ constexpr int kLvBlocks = 16;    // blocks of the cluster
 constexpr int kLvThreads = 512;  // one warp per segment
 constexpr int kLvCap = 256;      // entries of one segment
 constexpr int kLvK = 8;          // edges in flight per lane, balanced expansion
-constexpr int kLvStep = 16;      // entries a warp takes at a time
+constexpr int kLvStep = 32;      // entries a warp takes at a time
+constexpr uint32_t kLvFew = 24;  // edges of an entry that eight lanes expand
 // Frontiers that enter the cluster, and the edges of a level that it keeps.
 // 16 SMs claim about 10 edges per ns, so a level of 2^16 edges takes about as
 // long as a host round of the whole GPU costs before it does any work.
@@ -232,26 +235,38 @@ __global__ void __launch_bounds__(kLvThreads) k_levels(LvArgs a, Claim claim) {
       deal(tm, v, r, kk);
     };
     for (uint32_t i0 = 0; i0 < seg; i0 += kLvStep) {
-      // low degrees: eight lanes per entry, lane j takes edge j (no scan, no search)
-      constexpr int N = kLvStep / 4;
+      // low degrees: eight lanes per entry, lane j takes edges j, j + 8, ...
       const unsigned grp = lane >> 3, ej = lane & 7;
-      uint64_t rr[N];
-      bool big = false;
-#pragma unroll
-      for (int k = 0; k < N; k++) {
-        const uint32_t i = i0 + 4 * k + grp;
-        rr[k] = i < seg ? sh.rng[cur][wid][i] : 0ull;
-        big |= (rr[k] & 0xFFFFFFull) > 8;
-      }
-      if (!__any_sync(kFull, big)) {
+      auto few = [&](auto kk) {
+        constexpr int N = decltype(kk)::value;
+        uint64_t rr[N], r[N];
         uint32_t v[N];
-        uint64_t r[N];
+        bool big = false;
 #pragma unroll
-        for (int k = 0; k < N; k++)
-          v[k] = ej < (rr[k] & 0xFFFFFFull) ? __ldg(&a.E[(rr[k] >> 24) + ej]) : kNone;
-        claim_all(v, r, std::integral_constant<int, N>());
+        for (int k = 0; k < N; k++) {
+          const uint32_t i = i0 + 4 * k + grp;
+          rr[k] = i < seg ? sh.rng[cur][wid][i] : 0ull;
+          big |= (rr[k] & 0xFFFFFFull) > kLvFew;
+        }
+        if (__any_sync(kFull, big)) return false;
+        for (uint32_t j = ej;; j += 8) {
+          bool more = false;
+#pragma unroll
+          for (int k = 0; k < N; k++) {
+            const uint32_t d = (uint32_t)(rr[k] & 0xFFFFFFull);
+            v[k] = j < d ? __ldg(&a.E[(rr[k] >> 24) + j]) : kNone;
+            more |= j + 8 < d;
+          }
+          claim_all(v, r, kk);
+          if (!__any_sync(kFull, more)) return true;
+        }
+      };
+      const uint32_t left = seg - i0;
+      if (left <= 4    ? few(std::integral_constant<int, 1>())
+          : left <= 8  ? few(std::integral_constant<int, 2>())
+          : left <= 16 ? few(std::integral_constant<int, 4>())
+                       : few(std::integral_constant<int, kLvStep / 4>()))
         continue;
-      }
       // balanced expansion: the warp walks the concatenated ranges of the step's
       // entries, up to kLvK edges per lane in flight (the steps that nobody needs
       // are skipped as a whole)

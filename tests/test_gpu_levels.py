@@ -73,11 +73,13 @@ GRAPHS = {
     "edges_65535": lambda: _tree([257, 255]),
     "edges_65537": lambda: _tree([65537, 1]),
     "hub_then_fan": lambda: _tree([33, 9, 70, 3]),
-    # eight lanes per entry up to degree 8, the balanced expansion above it
+    # eight lanes per entry up to degree 24, the balanced expansion above it
     "fan_8": lambda: _tree([8] * 5),
     "fan_9": lambda: _tree([9] * 4),
     "degrees_0_to_8": lambda: _band(8),
     "degrees_0_to_12": lambda: _band(12),
+    "degrees_0_to_24": lambda: _band(24),
+    "degrees_0_to_27": lambda: _band(27),
 }
 
 
