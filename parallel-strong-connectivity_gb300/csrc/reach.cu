@@ -814,8 +814,10 @@ __global__ void __launch_bounds__(BLOCK)
 // than kRecEdges targets comes back to the front of the queue with its next
 // ones, which its lanes load during the wave (at most kLowWave such entries,
 // which are never given away: kAsyncKeep stay).
+// A wave holds 6 to 8 entries on average, so there is code for 4, 8 and 12 of them.
 // Reach of the first pivot (both sides): kNN 10^7 (depth about 3,700) in rounds
-// 10.1 ms, k_reach_async 8.6, this 4.5; 4096^2 grid 8.2, 7.8, 4.2.  Waves of 8 / 12 /
+// 10.1 ms, k_reach_async 8.6, this 4.3 (always 12 entries 4.5, 8 or 12 4.8, 4 or 12
+// 4.5); 4096^2 grid 8.2, 7.8, 4.2 (4.2, 4.7, 4.4).  Waves of 8 / 12 /
 // 16 entries: 4.6 / 4.5 / 4.9 ms on kNN; kAsyncKeep 12 / 16 / 20: 4.5 / 4.5 / 4.7;
 // 1 / 2 / 3 / 5 blocks per SM: 5.9 / 5.0 / 4.9 / 5.0 (waves of 16), so three.
 constexpr int kLowWave = 12;
@@ -826,7 +828,6 @@ __global__ void __launch_bounds__(BLOCK)
     k_reach_async_low(ReachSide s0, ReachSide s1, AsyncCtl* c0, AsyncCtl* c1, uint32_t slots,
                       uint32_t backlog_max) {
   static_assert((QCAP & (QCAP - 1)) == 0 && QCAP >= 64, "ring queue");
-  constexpr int K = kLowWave / 4;
   __shared__ uint4 srec[BLOCK / 32][QCAP][2];
   __shared__ uint32_t sv[BLOCK / 32][QCAP];
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
@@ -874,112 +875,121 @@ __global__ void __launch_bounds__(BLOCK)
       uint32_t flags;
       if (look) ht = ld_head_tail(L.C);
       if (check) flags = ld_flags(L.C);
-      // target j of entry 4 k + grp, and the one kRecEdges further on
-      uint32_t w[K], old[K], nx[K], lo[K], more = 0;
-      uint4 ra[K], rb[K];
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t* word = (const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0];
-        lo[k] = word[0];
-        w[k] = word[2 + (j < (unsigned)kRecEdges ? j : 0)];
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t deg = 4 * k + grp < n ? lo[k] & 0xFFFFFFu : 0u;
-        if (j >= (unsigned)kRecEdges || j >= deg) w[k] = kNone;
-        more |= (deg > (uint32_t)kRecEdges ? 1u : 0u) << k;
-      }
-      const bool any_more = __any_sync(kFull, more);
-      if (any_more) {
+      auto step = [&](auto kk) {
+        constexpr int K = decltype(kk)::value;
+        // target j of entry 4 k + grp, and the one kRecEdges further on
+        uint32_t w[K], old[K], nx[K], lo[K], more = 0;
+        uint4 ra[K], rb[K];
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          const uint64_t beg =
-              ((uint64_t)((const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0])[1] << 8) | (lo[k] >> 24);
-          nx[k] = kNone;
-          if (((more >> k) & 1u) && j < (unsigned)kRecEdges && kRecEdges + j < (lo[k] & 0xFFFFFFu))
-            nx[k] = __ldg(&E[beg + kRecEdges + j]);
+          const uint32_t* word = (const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0];
+          lo[k] = word[0];
+          w[k] = word[2 + (j < (unsigned)kRecEdges ? j : 0)];
         }
-      }
-      // the claims, with the candidates' records
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        old[k] = ~0u;
-        ra[k].x = 0;
-        if (w[k] != kNone) {
-          old[k] = atomicOr(&vis[w[k] >> 5], 1u << (w[k] & 31));
-          ld_rec(rec + w[k], ra[k], rb[k]);
-          ed++;
-        }
-      }
-      // place the claimed ones (a vertex without out-edges is done)
-      unsigned m[K];
-      uint32_t tot = 0;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        m[k] = __ballot_sync(kFull, !((old[k] >> (w[k] & 31)) & 1u) && (ra[k].x & 0xFFFFFFu));
-        tot += __popc(m[k]);
-      }
-      const uint32_t room = QCAP - (t - h);
-      const uint32_t nloc = min(tot, room);
-      uint32_t at = t;
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const uint32_t q = at + __popc(m[k] & lt);
-        if (((m[k] >> lane) & 1u) && q - t < nloc) {
-          R[q & (QCAP - 1)][0] = ra[k];
-          R[q & (QCAP - 1)][1] = rb[k];
-          V[q & (QCAP - 1)] = w[k];
-        }
-        at += __popc(m[k]);
-      }
-      if (tot > nloc) {  // a full queue: the rest goes to the slots
-        const uint32_t spill = L.reserve(tot - nloc);
-        at = t;
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          const uint32_t q = at + __popc(m[k] & lt) - t;
-          if (((m[k] >> lane) & 1u) && q >= nloc) L.slot[spill + (q - nloc)] = w[k];
-          at += __popc(m[k]);
+          const uint32_t deg = 4 * k + grp < n ? lo[k] & 0xFFFFFFu : 0u;
+          if (j >= (unsigned)kRecEdges || j >= deg) w[k] = kNone;
+          more |= (deg > (uint32_t)kRecEdges ? 1u : 0u) << k;
         }
-      }
-      t += nloc;
-      if (lane == 0) ex += nloc;
-      // entries with targets left return to the front, in the places just read
-      const uint32_t h0 = h;
-      h += n;
-      if (any_more) {
+        const bool any_more = __any_sync(kFull, more);
+        if (any_more) {
 #pragma unroll
-        for (int k = K - 1; k >= 0; k--) {
-          const unsigned back = __ballot_sync(kFull, j == 0 && ((more >> k) & 1u));
-          if (back) {
-            // the group's own entry moves from place 4 k + grp to place (h - 1 - later ones)
-            const bool mv = (more >> k) & 1u;
-            const uint32_t from = (h0 + 4 * k + grp) & (QCAP - 1);
-            const uint32_t to = (h - 1 - __popc(back >> (8 * grp + 1))) & (QCAP - 1);
-            uint32_t lo = 0, hi = 0, x = 0;
-            if (mv && j == 0) {
-              const uint2 hd = *(const uint2*)&R[from][0];
-              lo = hd.x;
-              hi = hd.y;
-              x = V[from];
-            }
-            __syncwarp();
-            if (mv) {
-              uint32_t* word = (uint32_t*)&R[to][0];
-              if (j < (unsigned)kRecEdges) word[2 + j] = nx[k];
-              if (j == 0) {
-                const uint64_t r = ((((uint64_t)hi << 32) | lo) + ((uint64_t)kRecEdges << 24)) - kRecEdges;
-                word[0] = (uint32_t)r;
-                word[1] = (uint32_t)(r >> 32);
-                V[to] = x;
-              }
-            }
-            __syncwarp();
-            h -= __popc(back);
+          for (int k = 0; k < K; k++) {
+            const uint64_t beg =
+                ((uint64_t)((const uint32_t*)&R[(h + 4 * k + grp) & (QCAP - 1)][0])[1] << 8) | (lo[k] >> 24);
+            nx[k] = kNone;
+            if (((more >> k) & 1u) && j < (unsigned)kRecEdges && kRecEdges + j < (lo[k] & 0xFFFFFFu))
+              nx[k] = __ldg(&E[beg + kRecEdges + j]);
           }
         }
-      }
-      __syncwarp();
+        // the claims, with the candidates' records
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          old[k] = ~0u;
+          ra[k].x = 0;
+          if (w[k] != kNone) {
+            old[k] = atomicOr(&vis[w[k] >> 5], 1u << (w[k] & 31));
+            ld_rec(rec + w[k], ra[k], rb[k]);
+            ed++;
+          }
+        }
+        // place the claimed ones (a vertex without out-edges is done)
+        unsigned m[K];
+        uint32_t tot = 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          m[k] = __ballot_sync(kFull, !((old[k] >> (w[k] & 31)) & 1u) && (ra[k].x & 0xFFFFFFu));
+          tot += __popc(m[k]);
+        }
+        const uint32_t room = QCAP - (t - h);
+        const uint32_t nloc = min(tot, room);
+        uint32_t at = t;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          const uint32_t q = at + __popc(m[k] & lt);
+          if (((m[k] >> lane) & 1u) && q - t < nloc) {
+            R[q & (QCAP - 1)][0] = ra[k];
+            R[q & (QCAP - 1)][1] = rb[k];
+            V[q & (QCAP - 1)] = w[k];
+          }
+          at += __popc(m[k]);
+        }
+        if (tot > nloc) {  // a full queue: the rest goes to the slots
+          const uint32_t spill = L.reserve(tot - nloc);
+          at = t;
+#pragma unroll
+          for (int k = 0; k < K; k++) {
+            const uint32_t q = at + __popc(m[k] & lt) - t;
+            if (((m[k] >> lane) & 1u) && q >= nloc) L.slot[spill + (q - nloc)] = w[k];
+            at += __popc(m[k]);
+          }
+        }
+        t += nloc;
+        if (lane == 0) ex += nloc;
+        // entries with targets left return to the front, in the places just read
+        const uint32_t h0 = h;
+        h += n;
+        if (any_more) {
+#pragma unroll
+          for (int k = K - 1; k >= 0; k--) {
+            const unsigned back = __ballot_sync(kFull, j == 0 && ((more >> k) & 1u));
+            if (back) {
+              // the group's own entry moves from place 4 k + grp to place (h - 1 - later ones)
+              const bool mv = (more >> k) & 1u;
+              const uint32_t from = (h0 + 4 * k + grp) & (QCAP - 1);
+              const uint32_t to = (h - 1 - __popc(back >> (8 * grp + 1))) & (QCAP - 1);
+              uint32_t lo = 0, hi = 0, x = 0;
+              if (mv && j == 0) {
+                const uint2 hd = *(const uint2*)&R[from][0];
+                lo = hd.x;
+                hi = hd.y;
+                x = V[from];
+              }
+              __syncwarp();
+              if (mv) {
+                uint32_t* word = (uint32_t*)&R[to][0];
+                if (j < (unsigned)kRecEdges) word[2 + j] = nx[k];
+                if (j == 0) {
+                  const uint64_t r = ((((uint64_t)hi << 32) | lo) + ((uint64_t)kRecEdges << 24)) - kRecEdges;
+                  word[0] = (uint32_t)r;
+                  word[1] = (uint32_t)(r >> 32);
+                  V[to] = x;
+                }
+              }
+              __syncwarp();
+              h -= __popc(back);
+            }
+          }
+        }
+        __syncwarp();
+      };
+      if (n <= 4)
+        step(std::integral_constant<int, 1>());
+      else if (n <= 8)
+        step(std::integral_constant<int, 2>());
+      else
+        step(std::integral_constant<int, kLowWave / 4>());
       if (look) {
         const uint32_t give = L.share(ht, t - h, backlog_max);
         if (give) L.put(V, QCAP - 1, t, give);
