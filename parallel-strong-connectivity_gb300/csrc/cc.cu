@@ -1084,7 +1084,7 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
   bool pull = false;
   g->ldd_trace.clear();
   const VRec* rec = nullptr;
-  const bool resident = lr_ready(g);
+  const bool resident = !g->shared && lr_ready(g);
   if (resident) PSC_TRY(records_if_low(g, false, &rec));
   bool centres_in = false;  // the round's centres are in place already
   while (nf > 0 || sampled < (uint32_t)kLddSamples) {

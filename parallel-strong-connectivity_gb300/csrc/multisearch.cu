@@ -1424,6 +1424,7 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
 }
 
 bool ms_run_ready(psc_graph_s* g) {
+  if (g->shared) return false;
   constexpr int kMaxDev = 64;
   static std::mutex mu;
   static int state[kMaxDev] = {};

@@ -1915,7 +1915,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   const uint64_t threshold = g->m / pull_div;
   const uint64_t slack = !local ? 0 : g->m > kHeavyDeg ? kAsyncSlack : std::min(n, kAsyncSlack);
   // (graphs of low degree have narrow frontiers, so deep ones: not in rounds)
-  bool resident = g->m <= kRrMaxEdges && rr_ready(g->device);
+  bool resident = g->m <= kRrMaxEdges && !g->shared && rr_ready(g->device);
   if (resident && local) {
     PSC_TRY(max_degrees_once(g));
     resident = g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg;
@@ -1949,7 +1949,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
           s.vis, (uint32_t*)g->bufs[s.slot_qa].p, d_srcs, n_dsrc);
   }
   const bool tr = trace_on();
-  bool async = local;
+  bool async = local && !g->shared;
   bool first_launch = start_there;
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
