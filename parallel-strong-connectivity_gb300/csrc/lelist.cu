@@ -726,6 +726,11 @@ __global__ void __launch_bounds__(BLOCK) k_le_heavy(LeLevel a) {
 // edges per lane: 12 and 8 gave 4.8 / 2.1 / 6.0 / 8.3 / 30.2, 24 and 4 4.4 / 2.3 / 6.8
 // / 9.4 / 24.5.
 // ---------------------------------------------------------------------------
+// Above 2^23 vertices a batch of hub pairs outgrows the table and is done twice, and
+// levels are wide: launch by launch is faster there (symmetrised R-MAT, resident /
+// from the host: n = 2^22, 3.3e7 edges 9.5 / 15.0 ms, 1.3e8 edges 14.6 / 18.1; 2^23,
+// 1.3e8 edges 25.0 / 30.2; 2^24, 6.7e7 edges 50.1 / 41.9, 2.6e8 edges 116 / 74).
+constexpr uint64_t kLbMaxVerts = 1ull << 23;
 constexpr int kLbThreads = 512;
 constexpr int kLbK = 4;  // light pairs: edges in flight per lane
 constexpr int kLbWarps = kLbThreads / 32;
@@ -1231,7 +1236,7 @@ int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* l
   uint64_t prev_ne = n >> 1;
   // inserts per scanned edge at each level of the previous batch
   std::vector<double> ratio, ratio_next;
-  const bool resident = le_batches_ready(g);
+  const bool resident = n <= kLbMaxVerts && le_batches_ready(g);
   while (finished < n) {
     if (resident) {
       bool done = false;
