@@ -759,12 +759,12 @@ def cpu_baseline_batch(g, vb, seeds, sample, budget_s: float = 15.0) -> dict:
 # divided by the family's profiled scopes (the launches counted in the
 # roofline entry).  A workload without a capture of its current dominant
 # kernels reports null.
-#   scc_rmat26 / reach_pull: k_reach_pull_staged, k_reach_pull,
-#     k_pull_out_edges and k_queue_to_bitmap, 6,605 MB over 2 solves x 6 scopes
-#   scc_knn / reach_vgc: k_reach_vgc, 10,912 MB over 185 launches
+#   scc_rmat26 / reach_pull: k_reach_pull, k_pull_out_edges and
+#     k_queue_to_bitmap, 6,575 MB over 2 solves x 8 scopes
+#   scc_knn / reach_vgc: k_reach_async_low, 5,067 MB over 2 launches
 NCU_TRAFFIC: dict = {
-    ("scc_rmat26", "reach_pull"): 550.4e6,
-    ("scc_knn", "reach_vgc"): 59.0e6,
+    ("scc_rmat26", "reach_pull"): 410.9e6,
+    ("scc_knn", "reach_vgc"): 2533.7e6,
 }
 
 
