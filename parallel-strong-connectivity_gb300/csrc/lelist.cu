@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "engines.cuh"
+#include "le_room.h"
 #include "levels.cuh"
 #include "pull.cuh"
 #include "scan.cuh"
@@ -764,6 +765,9 @@ struct LbArgs {
   Counters* ctr;
   LbState* st;
 };
+static_assert(sizeof(*LbArgs::Lk) == kLeKeyBytes && sizeof(*LbArgs::Ld) == kLeDistBytes &&
+                  sizeof(*LbArgs::Ls) == kLeSlotBytes,
+              "le_room counts in the arrays' element sizes");
 
 __global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
   __shared__ LbShared sh;
@@ -1154,11 +1158,11 @@ static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint
     PSC_TRY(ensure_t(g, B_PB, cap, &a.F[1]));
     PSC_TRY(ensure_t(g, B_PA2, cap, &a.lv.Hk));
     PSC_TRY(ensure_t(g, B_PB2, cap, &a.lv.Hs));
-    PSC_TRY(le_list_reserve(g, *L + 2 * cap, *L, lcap));
-    // (an earlier call may have left longer buffers)
-    *lcap = std::max(*lcap, std::min<uint64_t>((g->bufs[B_PH].bytes - 16) / 8,
-                                               (g->bufs[B_AUX3].bytes - 16) / 4));
-    PSC_TRY(ensure_t(g, B_TB, (*lcap + 1) / 2, &a.Ls));
+    PSC_TRY(le_list_reserve(g, le_entries_wanted(*L, cap), *L, lcap));
+    // (keys and distances may be longer than asked for, from an earlier call)
+    PSC_TRY(ensure_t(g, B_TB, le_room(g->bufs[B_PH].bytes, g->bufs[B_AUX3].bytes, SIZE_MAX), &a.Ls));
+    a.lcap = le_room(g->bufs[B_PH].bytes, g->bufs[B_AUX3].bytes, g->bufs[B_TB].bytes);
+    if (a.lcap < le_entries_wanted(*L, cap)) return PSC_ERR_TABLE_FULL;  // (sizes disagree)
     PSC_CUDA(cudaMemsetAsync(a.lv.T, 0xFF, cap * 8, g->stream));
     PSC_TRY(zero_counters(g));
     a.lv.off = g->off;
@@ -1172,7 +1176,6 @@ static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint
     a.finished = *finished;
     a.step = *step;
     a.L = *L;
-    a.lcap = *lcap;
     a.Lk = (uint64_t*)g->bufs[B_PH].p;
     a.Ld = (uint32_t*)g->bufs[B_AUX3].p;
     a.dist = dist;
