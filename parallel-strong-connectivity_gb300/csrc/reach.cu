@@ -35,6 +35,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "async_rules.h"
 #include "common.cuh"
 #include "engines.cuh"
 #include "levels.cuh"
@@ -473,8 +474,9 @@ __global__ void __launch_bounds__(BLOCK)
 // Idle warps hold tickets (consecutive indexes drawn from ctl->head) and poll the
 // slot of their ticket; givers reserve slots from ctl->tail and write vertex ids
 // into them, so a slot has one writer and one reader and needs no lock.  A
-// vertex enters the slots at most once (it is claimed once, and a ticket's
-// vertices are expanded before anything is given away).  ctl->fin counts the
+// vertex enters the slots at most once while the launch runs (it is claimed once, and
+// a ticket's vertices are expanded before any of them could be given away, see
+// async_rules.h).  ctl->fin counts the
 // vertices taken from the slots whose searches have ended; when it equals
 // ctl->tail nothing is queued and nobody works, and whoever sees that marks the
 // side done.  No warp waits for a block that may not be running: all work is
@@ -488,11 +490,7 @@ __global__ void __launch_bounds__(BLOCK)
 constexpr uint32_t kTaken = 0xFFFFFFFEu;  // a slot whose vertex was taken (ids are smaller)
 constexpr uint32_t kAsyncDone = 1, kAsyncHeavy = 2, kAsyncWide = 4, kAsyncFull = 8, kAsyncYield = 16;
 constexpr uint32_t kAsyncStop = kAsyncHeavy | kAsyncWide | kAsyncFull | kAsyncYield;
-constexpr uint32_t kAsyncKeep = 16;
 constexpr uint32_t kAsyncSpin = 1u << 16;  // polls of one wait: some 50 ms
-// Vertices put into the slots a second time when a launch stops: at most 32 per
-// resident warp.
-constexpr uint64_t kAsyncSlack = 1u << 18;
 
 // Two lines: the flags are polled by idle warps, and every access to one line
 // takes its turn in the L2 (with the flags beside head and tail, and polled four
@@ -529,6 +527,7 @@ struct AsyncLink {
   AsyncCtl *c0, *c1;  // both sides: a stop is for both
   volatile uint32_t* slot;
   uint32_t slots, nw;  // prepared slots; warps of the grid
+  uint32_t most;       // vertices that a warp takes at a time
 
   __device__ void stop(uint32_t why) const {
     atomicOr(&c0->flags, why);
@@ -552,9 +551,7 @@ struct AsyncLink {
       const uint2 c = ld_head_tail(C);
       fl = quit ? kAsyncHeavy : ld_flags(C);
       if (!fl && none) {
-        // one ticket, or a warp's share of the backlog
-        const int32_t backlog = (int32_t)(c.y - c.x);
-        take = backlog > (int32_t)nw ? min(32u, (uint32_t)backlog / nw) : 1u;
+        take = async_take((int32_t)(c.y - c.x), nw, most);
         first = atomicAdd(&C->head, take);
       }
     }
@@ -605,7 +602,7 @@ struct AsyncLink {
                                             uint32_t backlog_max) const {
     const int32_t hungry = (int32_t)(ht.x - ht.y);
     if (hungry < 0 && (uint32_t)-hungry > backlog_max && lane_id() == 0) stop(kAsyncWide);
-    return hungry > 0 && held > kAsyncKeep ? min(held - kAsyncKeep, (uint32_t)hungry) : 0u;
+    return async_give(hungry, held);
   }
 
   // Puts the last n of the ring's vertices (places [t - n, t)) into the slots.
@@ -650,7 +647,7 @@ __global__ void __launch_bounds__(BLOCK)
     const uint32_t* __restrict__ E = sd ? s1.E : s0.E;
     uint32_t* vis = sd ? s1.vis : s0.vis;
     const AsyncLink L{sd ? c1 : c0, c0, c1, sd ? s1.qout : s0.qout, slots,
-                      (uint32_t)(gridDim.x * (BLOCK / 32))};
+                      (uint32_t)(gridDim.x * (BLOCK / 32)), kAsyncTake};
     uint32_t tk = kNone;               // this lane's ticket
     uint32_t h = 0, t = 0, items = 0;  // ring queue [h, t); vertices taken for this search
     unsigned long long ed = 0, ex = 0;
@@ -690,7 +687,7 @@ __global__ void __launch_bounds__(BLOCK)
       }
       const uint32_t h0 = h;
       const bool few = !__any_sync(kFull, deg > 8);
-      if (few) wave = min(wave, 16u);
+      if (few) wave = min(wave, kAsyncFewWave);
       h += wave;
       // Claims the lane's candidates w[0 .. N) (steps from lim on have none), their
       // ranges loaded alongside, and queues the new ones.
@@ -757,7 +754,7 @@ __global__ void __launch_bounds__(BLOCK)
         ex += lane < wave;
         const bool big = deg > kHeavyDeg;
         if (__any_sync(kFull, big)) {  // not for this launch: back to the slots
-          quit = true;  // (so a warp puts back at most 32, see kAsyncSlack)
+          quit = true;  // (so a warp puts back at most what it took, see kAsyncSlack)
           if (big) {
             L.slot[atomicAdd(&L.C->tail, 1u)] = x;
             deg = 0;
@@ -820,9 +817,6 @@ __global__ void __launch_bounds__(BLOCK)
 // 4.5); 4096^2 grid 8.2, 7.8, 4.2 (4.2, 4.7, 4.4).  Waves of 8 / 12 /
 // 16 entries: 4.6 / 4.5 / 4.9 ms on kNN; kAsyncKeep 12 / 16 / 20: 4.5 / 4.5 / 4.7;
 // 1 / 2 / 3 / 5 blocks per SM: 5.9 / 5.0 / 4.9 / 5.0 (waves of 16), so three.
-constexpr int kLowWave = 12;
-static_assert(kLowWave <= (int)kAsyncKeep, "entries that came back are kept");
-
 template <int BLOCK, int QCAP>
 __global__ void __launch_bounds__(BLOCK)
     k_reach_async_low(ReachSide s0, ReachSide s1, AsyncCtl* c0, AsyncCtl* c1, uint32_t slots,
@@ -843,7 +837,7 @@ __global__ void __launch_bounds__(BLOCK)
     const uint32_t* __restrict__ E = sd ? s1.E : s0.E;
     uint32_t* vis = sd ? s1.vis : s0.vis;
     const AsyncLink L{sd ? c1 : c0, c0, c1, sd ? s1.qout : s0.qout, slots,
-                      (uint32_t)(gridDim.x * (BLOCK / 32))};
+                      (uint32_t)(gridDim.x * (BLOCK / 32)), kAsyncTakeLow};
     uint32_t tk = kNone;               // this lane's ticket
     uint32_t h = 0, t = 0, items = 0;  // ring queue [h, t); vertices taken for this search
     uint32_t ed = 0;
@@ -1674,7 +1668,9 @@ static int launch_async(psc_graph_s* g, bool rec, const ReachSide& a, const Reac
       if (rec) per_sm = std::min(per_sm, kAsyncRecBlocks);
       if (per_sm < 1) per_sm = 1;
     }
-    kernel<<<(unsigned)(g->num_sms * per_sm), kVgcBlock, 0, g->stream>>>(a, b, ca, cb, slots, backlog);
+    const uint64_t blocks = std::min<uint64_t>((uint64_t)g->num_sms * per_sm,
+                                               kAsyncMaxWarps / (kVgcBlock / 32));
+    kernel<<<(unsigned)blocks, kVgcBlock, 0, g->stream>>>(a, b, ca, cb, slots, backlog);
     return PSC_OK;
   });
 }
