@@ -19,7 +19,9 @@ namespace psc {
 // by looking back over the tiles before it (decoupled look-back: a tile publishes
 // its digit counts, later their prefix sums), so there is no histogram pass and no
 // scan per digit.  Tiles are numbered by a ticket, so the tiles that one waits for
-// are running or done; every wait is bounded.
+// are running or done; every wait is bounded.  A tile that gives up sets *failed: keys
+// that no pass wrote must not be used as places, so every later kernel of the sort,
+// and the offsets made of it, then writes nothing (k_rs_pass, k_bounds).
 // R-MAT 2^22, 6.6e7 edges, 3 passes: histogram 0.37, scan 0.03 and scatter 0.60 ms
 // per pass -> one read of 0.08 ms and 0.49 per pass; sources 0.35 -> 0.15, offsets
 // 0.28 -> 0.08.
@@ -31,7 +33,10 @@ constexpr int kRsTile = 4608;  // pairs per block and pass (12 per thread)
 constexpr int kEsTile = 3072;  // edges per block of k_edge_sources (4608: 163 instead of 126 us)
 constexpr int kRsMaxPasses = 4;
 constexpr int kRsLook = 4;
-constexpr uint32_t kRsSpin = 1u << 22;  // polls of one wait
+#ifndef PSC_RS_SPIN
+#define PSC_RS_SPIN (1u << 22)
+#endif
+constexpr uint32_t kRsSpin = PSC_RS_SPIN;  // polls of one wait
 // Status word of a (tile, digit): nothing yet, the tile's count, or the count of
 // all tiles up to it.
 constexpr uint64_t kRsCount = 1ull << 62, kRsPrefix = 2ull << 62, kRsValue = kRsCount - 1;
@@ -186,10 +191,11 @@ __global__ void __launch_bounds__(kRpBlock, 3)
   const unsigned lt = (1u << lane) - 1;
   if (tid == 0) {
     s_tile = atomicAdd(ticket, 1u);
-    s_bad = 0;
+    s_bad = *(volatile unsigned long long*)failed != 0;
   }
   for (int b = lane; b < kRsBins; b += 32) wcnt[wid][b] = 0;
   __syncthreads();
+  if (s_bad) return;  // an earlier pass gave up (or a tile of this one: its waiters do too)
   const uint64_t tile = s_tile;
   const uint64_t tbase = tile * kRsTile;
   const uint64_t base = tbase + (uint64_t)wid * PER_WARP;
@@ -270,7 +276,8 @@ __global__ void __launch_bounds__(kRpBlock, 3)
       if (!open) break;
       uint32_t spin = 0;
       while (!(x[k] >> 62)) {
-        if (++spin > kRsSpin) {
+        if (++spin > kRsSpin ||
+            ((spin & 1023u) == 0 && *(volatile unsigned long long*)failed)) {
           s_bad = 1;
           open = false;
           break;
@@ -308,8 +315,11 @@ struct GapEnt {
   uint64_t first, last, value;  // off[first .. last] = value
 };
 
+// Nothing is written when the sort that made t gave up (*failed).
 __global__ void k_bounds(const uint32_t* __restrict__ t, uint64_t m, uint64_t n, uint64_t* off,
-                         GapEnt* gaps, unsigned long long* ngaps) {
+                         GapEnt* gaps, unsigned long long* ngaps,
+                         const unsigned long long* __restrict__ failed) {
+  if (*failed) return;
   // ids after the one before place i, up to the one at place i
   auto place = [&](uint64_t i, uint64_t a, uint64_t b) {
     if (b + 1 > a + kGapLong) {
@@ -362,7 +372,8 @@ static int fill_bounds(psc_graph_s* g, const uint32_t* t, uint64_t m, uint64_t* 
   {
     ProfScope ps(g, F_TRANSPOSE);
     ps.bytes = 4.0 * m + 8.0 * n;
-    k_bounds<<<grid_for(g, m + 1, 256), 256, 0, g->stream>>>(t, m, n, off, gaps, ngaps);
+    k_bounds<<<grid_for(g, m + 1, 256), 256, 0, g->stream>>>(t, m, n, off, gaps, ngaps,
+                                                             &g->ctr[3].aux1);
     k_fill_gaps<<<g->num_sms * 4, 256, 0, g->stream>>>(gaps, ngaps, off);
   }
   PSC_CUDA(cudaGetLastError());
@@ -386,7 +397,7 @@ static int rs_scratch(psc_graph_s* g, uint64_t cnt, RsScratch* r) {
   PSC_TRY(ensure_t(g, B_AUX3, ntiles * kRsBins, &r->status));
   PSC_TRY(ensure_t(g, B_SCAN2, kRsMaxPasses * kRsBins + 2, &r->hist));
   r->ticket = (uint32_t*)(r->hist + kRsMaxPasses * kRsBins);
-  r->failed = &g->ctr[3].aux1;  // staging set, read by rs_check
+  r->failed = &g->ctr[3].aux1;  // staging set, read by rs_check and fill_bounds
   PSC_CUDA(cudaMemsetAsync(r->failed, 0, 8, g->stream));
   return PSC_OK;
 }
