@@ -41,6 +41,11 @@ constexpr int kMsVgcBlock = 128;
 constexpr int kMsVgcQueue = 512;
 constexpr int kMsK = 8;        // VGC: edges in flight per lane
 constexpr int kMsExpandK = 4;  // expand: fewer registers, more warps
+// An insert gives up after this many probes: the table is too full.  Every further insert
+// of the sub-round would spend as many, so the work at hand stops there and comes back
+// as pairs, after the table has grown (4 R-MAT and kNN graphs of 2^16 to 2^20 vertices in
+// a batch, a first pivot outside the giant component, so that hubs meet the small tables of
+// a first batch: 129 -> 5.7 ms of multi-search).
 constexpr uint32_t kProbeLimit = 256;
 
 struct MsSide {
@@ -491,14 +496,15 @@ __device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,
         uint32_t fm = 0;
         const uint32_t tm = ms_vgc_claim<kMsK, false>(w, vb, ve, sub, lab, S.off, labels, S.T,
                                                       S.mask, probes, fm);
-        failed |= fm != 0;
         (sd ? in1 : in0) += __popc(tm);
 #pragma unroll
         for (int k = 0; k < kMsK; k++) keys[k] = ((uint64_t)w[k] << 32) | lab;
         warp_append_batch<kMsK>(tm, keys, S.Fout, &S.ctr->next);
+        failed = __any_sync(kFull, fm != 0);
+        if (failed) break;  // (the pair comes back whole: see kProbeLimit)
       }
       (sd ? pr1 : pr0) += probes;
-      const bool rq = __any_sync(kFull, failed) && lane == 0;
+      const bool rq = failed && lane == 0;
       emit(rq, u);
       if (rq) (sd ? rq1 : rq0)++;
       continue;
@@ -613,6 +619,7 @@ __device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,
         __syncwarp();
         emit(rq, x);
         if (rq) (sd ? rq1 : rq0)++;
+        break;
       }
     }
     // spill what is left in the queue with one reservation
@@ -673,8 +680,11 @@ __device__ __forceinline__ void ms_heavy_round(const MsSide& s0, const MsSide& s
     uint64_t sub = ld_cg(&labels[key >> 32]), beg = S.off[key >> 32], end = S.off[(key >> 32) + 1];
     unsigned long long scanned = 0, requeued = 0, ins = 0;
     uint32_t probes = 0;
+    bool over = false;  // this warp has seen an insert of the pair fail
     for (uint64_t c = c_beg; c < c_end; c++) {
+      if (over && c < cn) continue;
       if (c >= cn) {
+        over = false;
         h++;
         key = ld_cg(&S.Fheavy[h]);
         cs = cn;
@@ -711,8 +721,8 @@ __device__ __forceinline__ void ms_heavy_round(const MsSide& s0, const MsSide& s
       ins += __popc(tm);
       warp_append_batch<K>(tm, nk, S.Fout, &S.ctr->next);
       bool rq = false;
-      if (__any_sync(kFull, failed) && lane == 0)
-        rq = !(atomicOr(&S.hflag[h], kRequeued) & kRequeued);
+      over = __any_sync(kFull, failed);
+      if (over && lane == 0) rq = !(atomicOr(&S.hflag[h], kRequeued) & kRequeued);
       const unsigned long long pos = warp_append(&S.ctr->next, rq);
       if (rq) {
         S.Fout[pos] = key;
@@ -1206,6 +1216,14 @@ static uint64_t pow2_at_least(uint64_t x) {
   return c;
 }
 
+// Slots that leave the local searches from nf pairs (up to min(tau, 64) new pairs each)
+// room below half load, at most 2^27; 0 when there are none.
+static uint64_t ms_vgc_room(bool local, uint64_t nf, uint64_t ne, uint32_t tau, uint64_t vgc_limit) {
+  if (!local || nf > vgc_limit) return 0;
+  return std::min<uint64_t>(1ull << 27,
+                            pow2_at_least(2 * (ne + nf * std::min<uint32_t>(tau, 64))));
+}
+
 // Rehash the table in slot tslot into a new table of capacity cap2.
 // (in a buffer of at least `room` slots).
 static int ms_grow(psc_graph_s* g, int tslot, uint64_t cap, uint64_t cap2, uint64_t room = 0) {
@@ -1301,13 +1319,12 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
       g->stats.subrounds++;
       // room for the VGC local searches of this sub-round: up to
       // min(tq, 64) new pairs each, while the table stays below 2^27 slots
-      const uint64_t want = (local && s.nf <= vgc_limit) ? s.nf * std::min<uint32_t>(tau, 64) : 0;
-      const bool vgc_room = want && s.cap < (1ull << 27) && s.ne + want > s.cap / 2;
+      const uint64_t room = ms_vgc_room(local, s.nf, s.ne, tau, vgc_limit);
+      const bool vgc_room = room > s.cap;
       if (s.grow || 2 * s.ne > s.cap || vgc_room) {
         // keep the load at most 1/2 (1/4 right after growing)
         uint64_t cap2 = pow2_at_least(std::max<uint64_t>(4 * s.ne, 2 * s.cap));
-        if (vgc_room)
-          cap2 = std::max(cap2, std::min<uint64_t>(1ull << 27, pow2_at_least(2 * (s.ne + want))));
+        if (vgc_room) cap2 = std::max(cap2, room);
         if (cap2 > (1ull << 40)) return PSC_ERR_TABLE_FULL;
         PSC_TRY(ms_grow(g, s.t_slot, s.cap, cap2));
         s.cap = cap2;
@@ -1529,9 +1546,13 @@ int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, 
       continue;
     }
     if (s.why != MB_GROW) break;
-    // grow both tables of the batch at hand to a quarter load (the other set and
-    // what a sub-round writes anew need not keep their contents)
-    const uint64_t cap2 = pow2_at_least(std::max<uint64_t>(4 * std::max(s.e0, s.e1), 2 * s.cap));
+    // grow both tables of the batch at hand to a quarter load, with room for the local
+    // searches of the next sub-round as ms_pair makes it (the other set and what a
+    // sub-round writes anew need not keep their contents)
+    uint64_t cap2 = std::max<uint64_t>(4 * std::max(s.e0, s.e1), 2 * s.cap);
+    for (int k = 0; k < 2; k++)
+      cap2 = std::max(cap2, ms_vgc_room(a.local, k ? s.n1 : s.n0, k ? s.e1 : s.e0, a.tau, a.vgc_limit));
+    cap2 = pow2_at_least(cap2);
     if (cap2 > (1ull << 40)) return PSC_ERR_TABLE_FULL;
     a.cap = cap2;
     a.nf = s.nf;
