@@ -727,13 +727,20 @@ __global__ void __launch_bounds__(BLOCK) k_le_heavy(LeLevel a) {
 // edges per lane: 12 and 8 gave 4.8 / 2.1 / 6.0 / 8.3 / 30.2, 24 and 4 4.4 / 2.3 / 6.8
 // / 9.4 / 24.5.
 // ---------------------------------------------------------------------------
-// Above 2^23 vertices a batch of hub pairs outgrows the table and is done twice, and
-// levels are wide: launch by launch is faster there (symmetrised R-MAT, resident /
-// from the host: n = 2^22, 3.3e7 edges 9.5 / 15.0 ms, 1.3e8 edges 14.6 / 18.1; 2^23,
-// 1.3e8 edges 25.0 / 30.2; 2^24, 6.7e7 edges 50.1 / 41.9, 2.6e8 edges 116 / 74).
+// Above 2^23 vertices levels are wide and the tables large: launch by launch is faster
+// there (symmetrised R-MAT, resident / from the host: n = 2^22, 1.3e8 edges 14.3 / 18.3 ms;
+// 2^23, 1.3e8 edges 29.6 / 37.8; with tables of 2^24 slots, 2^24, 6.7e7 edges 50.1 / 41.9,
+// 2.6e8 edges 116 / 74).
 constexpr uint64_t kLbMaxVerts = 1ull << 23;
+// Bound on the edges of a level, for the heavy list's fields: they then belong to fewer
+// than 2^24 pairs of more than kLeHeavy edges (a batch's seeds are fewer than 2^24 anyway).
+constexpr uint64_t kLbLevelEdges = (kLeHeavy + 1) << 24;
 constexpr int kLbThreads = 512;
-constexpr int kLbK = 4;  // light pairs: edges in flight per lane
+// Light pairs: edges in flight per lane.  Large graphs have wide levels, which live on
+// loads in flight (random graph of 2^23 vertices and 6.7e7 edges, beta 3: 62.9 ms with 4, 56.7 with
+// 8, 54.5 with 12; from the host 54.4), small ones narrow levels (kNN 2^20 47.4, 47.8, 49.6).
+constexpr int kLbK = 4, kLbKWide = 12;
+constexpr uint64_t kLbWideVerts = 1ull << 21;  // more vertices: kLbKWide
 constexpr int kLbWarps = kLbThreads / 32;
 constexpr int kLbCtr = 4;     // counter sets 4-6: three levels in rotation
 constexpr int kLbState = 10;  // counter sets 10-11
@@ -769,6 +776,7 @@ static_assert(sizeof(*LbArgs::Lk) == kLeKeyBytes && sizeof(*LbArgs::Ld) == kLeDi
                   sizeof(*LbArgs::Ls) == kLeSlotBytes,
               "le_room counts in the arrays' element sizes");
 
+template <int K>
 __global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
   __shared__ LbShared sh;
   const unsigned wid = threadIdx.x >> 5, tid = threadIdx.x;
@@ -831,7 +839,7 @@ __global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
       v.Ld = a.Ld + L + ne;
       v.Ls = a.Ls + L + ne;
       v.ctr = c;
-      le_expand_round<kLbK>(v, le_chunk(nf, nw), sh.sm[wid], sh.sp[wid], gw, nw);
+      le_expand_round<K>(v, le_chunk(nf, nw), sh.sm[wid], sh.sp[wid], gw, nw);
       if (!barrier()) return;
       if (__ldcg(&c->heavy)) {
         le_heavy_round<kLeK>(v, gw, nw);
@@ -846,7 +854,8 @@ __global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
       nf = __ldcg(&c->next);
       ne += nf;
       buf ^= 1;
-      if (__ldcg(&c->fail) || 2 * ne > cap || (__ldcg(&c->next_edges) >> kLeHeavyShift)) {
+      if (__ldcg(&c->fail) || 2 * ne > cap ||
+          __ldcg(&c->next_edges) >= kLbLevelEdges) {
         undo = true;
         break;
       }
@@ -1127,12 +1136,14 @@ static bool le_batches_ready(psc_graph_s* g) {
   std::lock_guard<std::mutex> lock(mu);
   int& st = state[g->device];
   if (st == 0) {
-    int coop = 0, b = 0;
+    int coop = 0, b0 = 0, b1 = 0;
     st = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device) == cudaSuccess &&
                  coop &&
-                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_le_batches, kLbThreads, 0) ==
-                     cudaSuccess &&
-                 b > 0
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_le_batches<kLbK>, kLbThreads,
+                                                               0) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_le_batches<kLbKWide>,
+                                                               kLbThreads, 0) == cudaSuccess &&
+                 b0 > 0 && b1 > 0
              ? 1
              : -1;
     cudaGetLastError();
@@ -1146,10 +1157,11 @@ static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint
                       uint32_t* next_dist, uint64_t* lcap, uint64_t* L, uint64_t* finished,
                       uint64_t* step, uint64_t* prev_ne, bool* done) {
   const uint64_t n = g->n;
-  // room for the pairs of the first batches (a pair for most vertices) at a
-  // quarter load.  Heavy-list fields: a level's pairs are at most cap / 2 = 2^23,
-  // over fewer than 2^40 edges (checked before the level).
-  const uint64_t cap = std::min<uint64_t>(1ull << 24, p2(std::max<uint64_t>(8192, 4 * n)));
+  // room for a batch's pairs at half load: on kNN with beta 3 every batch has 2.25 per
+  // vertex.  (4 n slots, at most 2^24: kNN 6x10^6 302 ms and with beta 3, every batch done
+  // twice, 591; now 206 and 197; from the host 628 and 487.)  The heavy list's fields
+  // are checked before a level (kLbLevelEdges).
+  const uint64_t cap = std::min<uint64_t>(1ull << 26, p2(std::max<uint64_t>(8192, 6 * n)));
   const uint64_t hthr = kLeHeavy;
   for (;;) {
     LbArgs a = {};
@@ -1185,8 +1197,10 @@ static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint
     {
       ProfScope ps(g, F_LE);
       void* args[] = {&a};
-      PSC_CUDA(cudaLaunchCooperativeKernel((const void*)k_le_batches, dim3((unsigned)g->num_sms),
-                                           dim3(kLbThreads), args, 0, g->stream));
+      PSC_CUDA(cudaLaunchCooperativeKernel(n > kLbWideVerts ? (const void*)k_le_batches<kLbKWide>
+                                                            : (const void*)k_le_batches<kLbK>,
+                                           dim3((unsigned)g->num_sms), dim3(kLbThreads), args, 0,
+                                           g->stream));
     }
     PSC_TRY(read_counters(g));
     const LbState& s = *(const LbState*)(g->hctr + kLbState);
