@@ -642,6 +642,7 @@ extern "C" int psc_scc_batch_device(psc_graph_t g, const psc_params_t* p, const 
     p = &def;
   }
   if (!(p->beta > 0)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   PSC_TRY(scc_batch_run(g, p, seeds, d_labels));
   return call_end(g);
@@ -656,6 +657,7 @@ extern "C" int psc_scc_batch(psc_graph_t g, const psc_params_t* p, const uint64_
     p = &def;
   }
   if (!(p->beta > 0)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint64_t* d;
   PSC_TRY(ensure_t(g, B_LABELS, g->n, &d));
@@ -682,6 +684,7 @@ int cc_batch_run(psc_graph_s* g, double beta, uint32_t* d_labels) {
 
 extern "C" int psc_cc_batch(psc_graph_t g, double beta, uint32_t* labels_out) {
   if (!g || !labels_out || !(beta > 0) || g->num_graphs == 0) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t* d;
   PSC_TRY(ensure_t(g, B_AUX0, g->n + 1, &d));

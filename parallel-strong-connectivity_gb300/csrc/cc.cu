@@ -1084,7 +1084,7 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
   bool pull = false;
   g->ldd_trace.clear();
   const VRec* rec = nullptr;
-  const bool resident = !g->shared && lr_ready(g);
+  const bool resident = lr_ready(g);
   if (resident) PSC_TRY(records_if_low(g, false, &rec));
   bool centres_in = false;  // the round's centres are in place already
   while (nf > 0 || sampled < (uint32_t)kLddSamples) {
@@ -1117,7 +1117,7 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
         void* args[] = {&a};
         PSC_CUDA(cudaLaunchCooperativeKernel(
             rec ? (const void*)k_ldd_rounds<true> : (const void*)k_ldd_rounds<false>,
-            dim3((unsigned)g->num_sms), dim3(kLrThreads), args, lr_smem(rec != nullptr), g->stream));
+            dim3(resident_sms(g)), dim3(kLrThreads), args, lr_smem(rec != nullptr), g->stream));
       }
       PSC_TRY(read_counters(g));
       const LrState& st = *(const LrState*)(g->hctr + kLrState);
@@ -1369,6 +1369,7 @@ extern "C" int psc_cc(psc_graph_t g, double beta, uint32_t* labels_out, uint32_t
                       uint64_t* n_forest) {
   if (!g || !labels_out || !(beta > 0)) return PSC_ERR_INVALID;
   if ((forest_out == nullptr) != (n_forest == nullptr)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t *d, *df = nullptr;
   PSC_TRY(ensure_t(g, B_AUX0, g->n + 1, &d));
@@ -1394,6 +1395,7 @@ extern "C" int psc_ldd_rounds(psc_graph_t g, uint32_t* out, uint32_t cap, uint32
 
 extern "C" int psc_ldd(psc_graph_t g, double beta, uint32_t* label_out, uint32_t* parent_out) {
   if (!g || !label_out || !(beta > 0)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t *d, *dp = nullptr;
   PSC_TRY(ensure_t(g, B_AUX0, g->n + 1, &d));

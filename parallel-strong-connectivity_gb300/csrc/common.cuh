@@ -140,9 +140,6 @@ struct psc_graph_s {
   cudaEvent_t ph[4] = {nullptr, nullptr, nullptr, nullptr};  // SCC phase marks
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> grow_events;  // table resizes
   // graph-offset table of a batch of disjoint graphs (psc_batch_set)
-  // Solves of other handles run beside this one's (request server): rounds from the
-  // host instead of launches that hold every SM for a phase (see run_batch in server.cu).
-  bool shared = false;
   uint32_t num_graphs = 0;
   std::vector<uint64_t> vbase;     // host copy, num_graphs + 1 vertex bases
   uint64_t* d_vbase = nullptr;     // device copy

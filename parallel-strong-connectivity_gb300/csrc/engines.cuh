@@ -1,5 +1,6 @@
 // Host entry points of the device engines, shared between translation units.
 #pragma once
+#include "calls.h"
 #include "common.cuh"
 
 namespace psc {
@@ -17,6 +18,11 @@ int alloc_graph_arrays(psc_graph_s* g, bool symmetric);
 int batch_attach(psc_graph_s* g, const uint64_t* vbase, uint32_t num_graphs, bool check);
 int call_begin(psc_graph_s* g);
 int call_end(psc_graph_s* g);
+
+// SMs that a resident launch takes (see calls.h).
+inline unsigned resident_sms(const psc_graph_s* g) {
+  return (unsigned)resident_share(g->num_sms, calls_at_work(g->device));
+}
 
 // The adjacency records of one direction, built once per handle; *out is null for
 // a graph with a vertex above kRecMaxDeg, for a batch of graphs (a server admits

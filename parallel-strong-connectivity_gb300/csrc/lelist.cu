@@ -1199,7 +1199,7 @@ static int le_batches(psc_graph_s* g, const uint32_t* centers, double beta, uint
       void* args[] = {&a};
       PSC_CUDA(cudaLaunchCooperativeKernel(n > kLbWideVerts ? (const void*)k_le_batches<kLbKWide>
                                                             : (const void*)k_le_batches<kLbK>,
-                                           dim3((unsigned)g->num_sms), dim3(kLbThreads), args, 0,
+                                           dim3(resident_sms(g)), dim3(kLbThreads), args, 0,
                                            g->stream));
     }
     PSC_TRY(read_counters(g));
@@ -1467,6 +1467,7 @@ using namespace psc;
 
 extern "C" int psc_bfs(psc_graph_t g, uint32_t src, uint32_t* dist_out, uint32_t* rounds) {
   if (!g || !dist_out || src >= g->n) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t* d;
   PSC_TRY(ensure_t(g, B_TMP32, g->n + 1, &d));
@@ -1481,6 +1482,7 @@ extern "C" int psc_bfs(psc_graph_t g, uint32_t src, uint32_t* dist_out, uint32_t
 extern "C" int psc_lelist(psc_graph_t g, const uint32_t* perm, double beta, uint32_t* out,
                           uint64_t cap, uint64_t* len) {
   if (!g || !perm || !len || !(beta > 0) || (cap && !out)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t* centers;
   // the priority order lives in the pivot slot (u32[n])

@@ -1441,7 +1441,6 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
 }
 
 bool ms_run_ready(psc_graph_s* g) {
-  if (g->shared) return false;
   constexpr int kMaxDev = 64;
   static std::mutex mu;
   static int state[kMaxDev] = {};
@@ -1516,7 +1515,7 @@ int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, 
       void* args[] = {&a};
       PSC_CUDA(cudaLaunchCooperativeKernel(
           run->sched ? (const void*)k_ms_batches<true> : (const void*)k_ms_batches<false>,
-          dim3((unsigned)g->num_sms), dim3(kMbThreads), args, sizeof(MbShared), g->stream));
+          dim3(resident_sms(g)), dim3(kMbThreads), args, sizeof(MbShared), g->stream));
     }
     PSC_TRY(read_counters(g));
     if (s.failed || s.why == MB_RUNNING) return PSC_ERR_ITER_LIMIT;

@@ -1668,7 +1668,7 @@ static int launch_async(psc_graph_s* g, bool rec, const ReachSide& a, const Reac
       if (rec) per_sm = std::min(per_sm, kAsyncRecBlocks);
       if (per_sm < 1) per_sm = 1;
     }
-    const uint64_t blocks = std::min<uint64_t>((uint64_t)g->num_sms * per_sm,
+    const uint64_t blocks = std::min<uint64_t>((uint64_t)resident_sms(g) * per_sm,
                                                kAsyncMaxWarps / (kVgcBlock / 32));
     kernel<<<(unsigned)blocks, kVgcBlock, 0, g->stream>>>(a, b, ca, cb, slots, backlog);
     return PSC_OK;
@@ -1911,7 +1911,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   const uint64_t threshold = g->m / pull_div;
   const uint64_t slack = !local ? 0 : g->m > kHeavyDeg ? kAsyncSlack : std::min(n, kAsyncSlack);
   // (graphs of low degree have narrow frontiers, so deep ones: not in rounds)
-  bool resident = g->m <= kRrMaxEdges && !g->shared && rr_ready(g->device);
+  bool resident = g->m <= kRrMaxEdges && rr_ready(g->device);
   if (resident && local) {
     PSC_TRY(max_degrees_once(g));
     resident = g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg;
@@ -1945,7 +1945,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
           s.vis, (uint32_t*)g->bufs[s.slot_qa].p, d_srcs, n_dsrc);
   }
   const bool tr = trace_on();
-  bool async = local && !g->shared;
+  bool async = local;
   bool first_launch = start_there;
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
@@ -1991,7 +1991,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         {
           ProfScope ps(g, F_REACH_PUSH);
           void* args[] = {&a};
-          PSC_CUDA(cudaLaunchCooperativeKernel((const void*)k_reach_rounds, dim3((unsigned)g->num_sms),
+          PSC_CUDA(cudaLaunchCooperativeKernel((const void*)k_reach_rounds, dim3(resident_sms(g)),
                                                dim3(kRrThreads), args, 0, g->stream));
         }
         PSC_TRY(read_counters(g));
@@ -2296,6 +2296,7 @@ using namespace psc;
 extern "C" int psc_reach(psc_graph_t g, uint32_t src, int dir, int local, uint32_t tau,
                          uint8_t* dst_out, uint32_t* rounds) {
   if (!g || !dst_out || src >= g->n || (dir != 0 && dir != 1)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint32_t* vis;
   uint8_t* bytes;

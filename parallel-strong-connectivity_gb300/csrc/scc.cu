@@ -311,6 +311,7 @@ extern "C" int psc_scc(psc_graph_t g, const psc_params_t* p, uint64_t* labels_ou
     p = &def;
   }
   if (!(p->beta > 0)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   uint64_t* d;
   PSC_TRY(ensure_t(g, B_LABELS, g->n, &d));
@@ -327,6 +328,7 @@ extern "C" int psc_scc_device(psc_graph_t g, const psc_params_t* p, uint64_t* d_
     p = &def;
   }
   if (!(p->beta > 0)) return PSC_ERR_INVALID;
+  CallScope scope(g->device);
   PSC_TRY(call_begin(g));
   PSC_TRY(scc_run(g, p, d_labels));
   return call_end(g);

@@ -236,11 +236,6 @@ int run_batch(psc_server_s* S, std::vector<Request*>& B, int kind, uint64_t tick
   const auto t_begin = Clock::now();
   psc_graph_s* g = nullptr;
   PSC_TRY(make_handle(n, m, &g, m <= kUrgentEdges ? S->urgent_priority : 0));
-  // With several batches at work a launch that holds every SM for a whole phase makes
-  // the others wait, and its idle warps poll beside their kernels: saturated stream of
-  // 240 mixed requests 900 to 1,280 graphs/s with resident launches (k_reach_rounds,
-  // k_reach_async, k_ms_batches, k_ldd_rounds), 1,410 to 1,435 in rounds.
-  g->shared = S->cfg.workers > 1;
   auto stamp = [&](const char* what) -> int {
     if (!tr) return PSC_OK;
     PSC_CUDA(cudaStreamSynchronize(g->stream));
@@ -313,6 +308,7 @@ int run_batch(psc_server_s* S, std::vector<Request*>& B, int kind, uint64_t tick
     PSC_CUDA(cudaGetLastError());
     PSC_TRY(stamp("upload"));
     slot.take();
+    CallScope scope(g->device);
     if (tr)
       marks.emplace_back("slot", std::chrono::duration<double, std::milli>(Clock::now() - t_begin).count());
     // SCC needs the in-edges: built on the device when they did not come along

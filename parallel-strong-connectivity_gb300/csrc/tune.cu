@@ -33,6 +33,7 @@ extern "C" int psc_tune_scc(psc_graph_t g, const uint64_t* seeds, uint32_t reps,
   if (!g || !p || !(p->beta > 0)) return PSC_ERR_INVALID;
   if (reps == 0) reps = 2;
   PSC_CUDA(cudaSetDevice(g->device));
+  CallScope scope(g->device);
   uint64_t* d;
   PSC_TRY(ensure_t(g, B_LABELS, g->n, &d));
   uint32_t trials = 0;
