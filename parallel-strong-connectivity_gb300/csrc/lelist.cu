@@ -50,9 +50,15 @@ __global__ void k_fill_u32(uint32_t* a, uint64_t n, uint32_t v) {
     a[i] = v;
 }
 
-__global__ void k_bfs_init(uint32_t* dist, uint32_t* q, uint32_t src) {
+// The source, queued and (when it has edges) listed for k_bfs_heavy, which expands it
+// without a push kernel before.  The counters are zero.
+__global__ void k_bfs_init(uint32_t* dist, uint32_t* q, uint32_t src,
+                           const uint64_t* __restrict__ off, uint64_t* heavy, Counters* ctr) {
   dist[src] = 0;
   q[0] = src;
+  const uint64_t deg = off[src + 1] - off[src];
+  heavy[0] = (uint64_t)src << 32;
+  if (deg) ctr->heavy = (1ull << kPackShift) + (deg + kBfsChunk - 1) / kBfsChunk;
 }
 
 template <int BLOCK, int K>
@@ -293,16 +299,18 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
   PSC_TRY(ensure_t(g, B_FB_A, nwords + 1, &fa));
   PSC_TRY(ensure_t(g, B_FB_B, nwords + 1, &fb));
   k_fill_u32<<<grid_for(g, n, 256), 256, 0, g->stream>>>(dist, n, kNone);
-  k_bfs_init<<<1, 1, 0, g->stream>>>(dist, qa, src);
+  PSC_TRY(zero_counters(g));
+  k_bfs_init<<<1, 1, 0, g->stream>>>(dist, qa, src, g->off, heavy, g->ctr);
   const uint64_t threshold = g->m / 20;
   uint64_t nf = 1, nf_edges = 0;
+  LvGate gate;
   bool pull = false;
   uint32_t level = 0;
   const bool cluster = !(g->m >> 40) && levels_ready<BfsClaim>(g->device);
   while (nf > 0) {
     const bool want_pull = (nf + nf_edges) >= threshold;
     // narrow push levels run back to back on one cluster (levels.cuh)
-    if (cluster && !want_pull && !pull && nf <= kLvMaxFront && nf_edges <= kLvMaxEdges) {
+    if (cluster && !want_pull && !pull && gate.enter(level, nf, nf_edges)) {
       PSC_TRY(zero_counters(g));
       {
         ProfScope ps(g, F_LE);
@@ -311,6 +319,7 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
       }
       PSC_TRY(read_counters(g));
       const Counters& c = g->hctr[0];
+      gate.ran(c.aux0);
       if (c.aux0) {  // else the first level was too wide: a round of the whole grid
         level += (uint32_t)c.aux0;
         if (level > n + 1) return PSC_ERR_ITER_LIMIT;
@@ -332,14 +341,17 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
       PSC_TRY(zero_counters(g));
       k_bfs_b2q<<<grid_for(g, nwords, 256), 256, 0, g->stream>>>(fa, nwords, qa, g->ctr);
       pull = false;
+      gate.pulled();
     }
-    PSC_TRY(zero_counters(g));
+    if (level > 1 || pull) PSC_TRY(zero_counters(g));
     if (!pull) {
       ProfScope ps(g, F_LE);
-      k_bfs_push<kLeBlock, kLeK><<<grid_for(g, nf, kLeBlock), kLeBlock, 0, g->stream>>>(
-          g->off, g->E, qa, nf, dist, level, qb, heavy, hthr, g->ctr);
-      k_bfs_heavy<kLeBlock, kLeK><<<g->num_sms * 4, kLeBlock, 0, g->stream>>>(
-          g->off, g->E, heavy, dist, level, qb, g->ctr);
+      if (level > 1)
+        k_bfs_push<kLeBlock, kLeK><<<grid_for(g, nf, kLeBlock), kLeBlock, 0, g->stream>>>(
+            g->off, g->E, qa, nf, dist, level, qb, heavy, hthr, g->ctr);
+      if (level == 1 || nf_edges > hthr)
+        k_bfs_heavy<kLeBlock, kLeK><<<g->num_sms * 4, kLeBlock, 0, g->stream>>>(
+            g->off, g->E, heavy, dist, level, qb, g->ctr);
       std::swap(qa, qb);
       swap_bufs(g, B_QA, B_QB);
     } else {

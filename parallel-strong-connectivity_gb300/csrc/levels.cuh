@@ -25,8 +25,8 @@
 // backward push reachability on kNN 1.5e6: 37.6 -> 4.6 ms.
 //
 // The cluster hands the search back to the host's wide rounds when a level
-// outgrows it (more than kLvMaxEdges edges, a full segment, or the
-// push/pull switch): every vertex of the next frontier is then written to the
+// outgrows it (more than kLvMaxEdges edges, a vertex of more than kLvMaxDeg, which one warp
+// would expand alone, a full segment, or the push/pull switch): every vertex of the next frontier is then written to the
 // caller's queue.  No wait depends on anything but the hardware barrier, which
 // all threads of the cluster reach the same number of times (every branch
 // around it is taken on values that all blocks read from the same segment
@@ -52,6 +52,10 @@ constexpr uint32_t kLvFew = 24;  // edges of an entry that eight lanes expand
 // long as a host round of the whole GPU costs before it does any work.
 constexpr uint64_t kLvMaxFront = 8192;
 constexpr uint64_t kLvMaxEdges = 1 << 16;
+// Out-edges of one vertex: four steps of a warp.  (Without this bound a hub of up to 65,536 was
+// expanded by one warp: allocation-free reachability from the hub of R-MAT 2^20 0.29 ms with host
+// rounds alone, 1.76 with the cluster, now 0.30; BFS of R-MAT 2^18 0.92 -> 0.17.)
+constexpr uint32_t kLvMaxDeg = 1024;
 // Edge sums are kept in 32 bits: a vertex, a warp and a block count for at
 // most kLvSat each, far above kLvMaxEdges (16 * kLvSat < 2^32).
 constexpr uint32_t kLvSat = 1u << 20;
@@ -101,6 +105,35 @@ struct ReachClaim {
   __device__ bool won(uint32_t v, uint32_t old) const { return !((old >> (v & 31)) & 1u); }
 };
 
+// Edges that a vertex counts for in the sums (kLvSat ends the launch).
+__device__ __forceinline__ uint32_t lv_edges(uint64_t r) {
+  const uint32_t d = (uint32_t)(r & 0xFFFFFFull);
+  return d > kLvMaxDeg ? kLvSat : d;
+}
+
+// Whether narrow push levels should go to the cluster: from the second level on, and not
+// while they grow so fast that the next one or two will be wide (a launch of the cluster
+// costs some 5 us more than a host round: BFS of R-MAT 2^12 122 us with host rounds alone,
+// 133 with one cluster level among them).  Launches that came back after a level or two
+// (hubs) hold the next ones off, as does a pull round, after which few levels are left.
+struct LvGate {
+  uint64_t prev = 0;  // out-edges of the last level
+  uint32_t rest = 0, penalty = 1;
+  bool enter(uint32_t level, uint64_t nf, uint64_t nf_edges) {
+    const bool slow = nf_edges <= 4 * (prev > 8 ? prev : 8);
+    prev = nf_edges;
+    if (level == 0 || !slow || nf > kLvMaxFront || nf_edges > kLvMaxEdges) return false;
+    if (rest == 0) return true;
+    rest--;
+    return false;
+  }
+  void pulled() { rest = 3; }
+  void ran(uint64_t levels) {
+    rest = levels < 3 ? penalty : 0;
+    penalty = levels < 3 ? (penalty < 64 ? 2 * penalty : 64) : 1;
+  }
+};
+
 __device__ __forceinline__ uint64_t lv_pack(uint64_t beg, uint64_t end) {
   const uint64_t d = end - beg;
   return (beg << 24) | (d < 0xFFFFFFull ? d : 0xFFFFFFull);
@@ -133,7 +166,7 @@ __global__ void __launch_bounds__(kLvThreads) k_levels(LvArgs a, Claim claim) {
     const uint64_t r = lv_pack(a.off[u], a.off[u + 1]);
     sh.rng[0][k % kLvBlocks][k / kLvBlocks] = r;
     sh.vid[0][k % kLvBlocks][k / kLvBlocks] = u;
-    e_in += min((uint32_t)(r & 0xFFFFFFull), kLvSat);
+    e_in = min(e_in + lv_edges(r), kLvSat);
   }
   e_in = __reduce_add_sync(kFull, min(e_in, kLvSat));
   if (lane == 0 && e_in) atomicAdd(&sh.my_edges[1], e_in);
@@ -212,7 +245,7 @@ __global__ void __launch_bounds__(kLvThreads) k_levels(LvArgs a, Claim claim) {
             atomicAdd(&a.ctr->next_edges, (unsigned long long)(a.off[v[k] + 1] - a.off[v[k]]));
             my_e = kLvSat;
           }
-          my_e = min(my_e + min((uint32_t)(r[k] & 0xFFFFFFull), kLvSat), kLvSat);
+          my_e = min(my_e + lv_edges(r[k]), kLvSat);
         }
         j += __popc(m[k]);
       }

@@ -2447,17 +2447,19 @@ extern "C" int psc_reach_noalloc(const uint64_t* d_off, const uint32_t* d_E,
   k_reach_init<<<1, 1, 0, s>>>(vis, qa, src);
   const uint64_t threshold = m / 20;
   uint64_t nf = 1, nf_edges = 0;
+  LvGate gate;
   bool pull = false;
   uint32_t r = 0;
   const bool cluster = levels_ready<ReachClaim>(dev);
   while (nf > 0) {
     const bool want_pull = (nf + nf_edges) >= threshold;
     // narrow push rounds run back to back on one cluster (levels.cuh)
-    if (cluster && !want_pull && !pull && nf <= kLvMaxFront && nf_edges <= kLvMaxEdges) {
+    if (cluster && !want_pull && !pull && gate.enter(r, nf, nf_edges)) {
       PSC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), s));
       PSC_TRY(launch_levels(LvArgs{A_off, A_E, qa, nf, qb, threshold, r, ctr}, ReachClaim{vis}, s));
       PSC_CUDA(cudaMemcpyAsync(&hc, ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s));
       PSC_CUDA(cudaStreamSynchronize(s));
+      gate.ran(hc.aux0);
       if (hc.aux0) {  // else the first round was too wide: one of the whole grid
         r += (uint32_t)hc.aux0;
         if (r > n + 2) return PSC_ERR_ITER_LIMIT;
@@ -2477,6 +2479,7 @@ extern "C" int psc_reach_noalloc(const uint64_t* d_off, const uint32_t* d_E,
       PSC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), s));
       k_bitmap_to_queue<<<na_grid(nd.num_sms, nwords, 256), 256, 0, s>>>(fa, nwords, qa, ctr);
       pull = false;
+      gate.pulled();
     }
     PSC_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), s));
     if (!pull) {
