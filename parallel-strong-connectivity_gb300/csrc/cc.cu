@@ -1092,6 +1092,8 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
     if (resident && !pull && !centres_in && nf + nf_edges < std::max<uint64_t>(threshold, 1) &&
         nf <= kLddWideEdges && nf_edges <= kLddWideEdges) {
       LrArgs a = {};
+      PSC_TRY(ensure_t(g, B_HEAVY, n + 1, &a.big));
+      if (g->rec_refused) rec = nullptr;  // (that may have taken their room)
       a.off = g->off;
       a.E = g->E;
       a.rec = rec;
@@ -1099,7 +1101,6 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
       a.parent = tree;
       a.q[0] = qa;
       a.q[1] = qb;
-      PSC_TRY(ensure_t(g, B_HEAVY, n + 1, &a.big));
       a.perm = perm;
       a.G = G;
       a.work = work_d;

@@ -11,6 +11,7 @@
 
 #include "../../include/psc.h"
 #include "psc_hash.h"
+#include "scratch.h"
 
 namespace psc {
 
@@ -82,11 +83,6 @@ constexpr int kCounterSets = 20;
 // ---------------------------------------------------------------------------
 // Host-side helpers
 // ---------------------------------------------------------------------------
-struct DevBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-};
-
 struct ProfEntry {
   uint64_t launches = 0;
   double ms = 0;
@@ -118,6 +114,7 @@ struct psc_graph_s {
   int le_heavy_blocks = 0; // same for the LE-list heavy-pair kernel
   bool deg_known = false;    // max_deg holds the largest out- / in-degree
   bool rec_known[2] = {false, false};  // B_REC_F / B_REC_B hold the adjacency records
+  bool rec_refused = false;  // they were given back for memory: not built again
   bool dead_known = false;   // B_DEAD holds the unreachable-vertex bitmaps
   uint64_t dead_count[2] = {0, 0};  // vertices with no in-edge / no out-edge
   // per LDD round of the last psc_ldd / psc_cc call: first candidate index,

@@ -6,6 +6,8 @@
 namespace psc {
 
 int ensure_keep(psc_graph_s* g, int b, size_t bytes, size_t keep, void** out);
+// Gives the buffer of slot b back to the pool.
+int release_buf(psc_graph_s* g, int b);
 // A handle with its stream, counters and events for a graph of n vertices
 // and m edges, and its graph arrays from the stream-ordered pool
 // (in_off/in_E alias off/E when symmetric).

@@ -87,41 +87,58 @@ int cuda_status(cudaError_t e) {
   return PSC_ERR_CUDA;
 }
 
-int ensure(psc_graph_s* g, int b, size_t bytes, void** out) {
-  DevBuf& d = g->bufs[b];
-  if (d.bytes < bytes) {
-    if (d.p) PSC_CUDA(cudaFreeAsync(d.p, g->stream));
-    d.p = nullptr;
-    d.bytes = 0;
-    cudaError_t e = cudaMallocAsync(&d.p, bytes, g->stream);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      d.p = nullptr;
-      return cuda_status(e);
-    }
-    d.bytes = bytes;
+namespace {
+struct StreamPool {
+  psc_graph_s* g;
+  int slot;
+  int alloc(void** p, size_t bytes) {
+    const cudaError_t e = cudaMallocAsync(p, bytes, g->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
   }
-  *out = d.p;
+  int free(void* p) { return (int)cudaFreeAsync(p, g->stream); }
+  int copy(void* to, const void* from, size_t bytes) {
+    return (int)cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, g->stream);
+  }
+  // The adjacency records, unless they are what is being allocated.  What is queued on the
+  // stream may still read them; a launch to come takes them from records_if_low again.
+  bool spare(int e) {
+    if (e != (int)cudaErrorMemoryAllocation || slot == B_REC_F || slot == B_REC_B) return false;
+    bool any = false;
+    for (int d = 0; d < 2; d++) {
+      DevBuf& r = g->bufs[d ? B_REC_B : B_REC_F];
+      if (r.p) any = cudaFreeAsync(r.p, g->stream) == cudaSuccess;
+      r = DevBuf{};
+      g->rec_known[d] = false;
+    }
+    if (!any) return false;
+    g->rec_refused = true;
+    cudaMemPool_t pool;
+    return cudaStreamSynchronize(g->stream) == cudaSuccess &&
+           cudaDeviceGetDefaultMemPool(&pool, g->device) == cudaSuccess &&
+           cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+  }
+};
+
+int grow(psc_graph_s* g, int b, size_t bytes, size_t keep, void** out) {
+  StreamPool ops{g, b};
+  const int e = scratch_grow(ops, g->bufs[b], bytes, keep);
+  if (e) return cuda_status((cudaError_t)e);
+  *out = g->bufs[b].p;
   return PSC_OK;
 }
+}  // namespace
+
+int ensure(psc_graph_s* g, int b, size_t bytes, void** out) { return grow(g, b, bytes, 0, out); }
 
 int ensure_keep(psc_graph_s* g, int b, size_t bytes, size_t keep, void** out) {
+  return grow(g, b, bytes, keep, out);
+}
+
+int release_buf(psc_graph_s* g, int b) {
   DevBuf& d = g->bufs[b];
-  if (d.bytes >= bytes) {
-    *out = d.p;
-    return PSC_OK;
-  }
-  void* np = nullptr;
-  cudaError_t e = cudaMallocAsync(&np, bytes, g->stream);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return cuda_status(e);
-  }
-  if (d.p && keep) PSC_CUDA(cudaMemcpyAsync(np, d.p, keep, cudaMemcpyDeviceToDevice, g->stream));
   if (d.p) PSC_CUDA(cudaFreeAsync(d.p, g->stream));
-  d.p = np;
-  d.bytes = bytes;
-  *out = np;
+  d = DevBuf{};
   return PSC_OK;
 }
 

@@ -1265,12 +1265,18 @@ int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* l
   uint64_t prev_ne = n >> 1;
   // inserts per scanned edge at each level of the previous batch
   std::vector<double> ratio, ratio_next;
-  const bool resident = n <= kLbMaxVerts && le_batches_ready(g);
+  bool resident = n <= kLbMaxVerts && le_batches_ready(g);
   while (finished < n) {
     if (resident) {
       bool done = false;
-      PSC_TRY(le_batches(g, centers, beta, dist, next_dist, &lcap, &L, &finished, &step, &prev_ne,
-                         &done));
+      const int st = le_batches(g, centers, beta, dist, next_dist, &lcap, &L, &finished, &step,
+                                &prev_ne, &done);
+      if (st == PSC_ERR_OOM) {  // no room for its tables: the host's grow with the batches
+        resident = false;
+        for (int b : {B_PA2, B_PB2, B_TB}) PSC_TRY(release_buf(g, b));
+      } else {
+        PSC_TRY(st);
+      }
       if (done) break;
       ratio.clear();
     }

@@ -1476,7 +1476,8 @@ static uint64_t mb_cap_max(const psc_graph_s* g) {
   return std::min<uint64_t>(1ull << 20, std::max<uint64_t>(1ull << 13, pow2_at_least(16 * g->n)));
 }
 
-int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, uint64_t window) {
+static int ms_run_resident(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run,
+                           uint64_t window) {
   if (g->m >> 36) return PSC_ERR_TOO_LARGE;  // heavy-list fields, as in ms_pair
   MbArgs a = {};
   a.off = g->off;
@@ -1570,6 +1571,22 @@ int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, 
     }
   }
   run->done = s.why == MB_DONE;
+  return PSC_OK;
+}
+
+// Without room for two sets of tables the batch at hand is left to ms_pair, from its start
+// (an interrupted one has written no label).
+int ms_run(psc_graph_s* g, uint64_t* labels, const psc_params_t* p, MsRun* run, uint64_t window) {
+  const int st = ms_run_resident(g, labels, p, run, window);
+  if (st != PSC_ERR_OOM) return st;
+  for (int b : {B_TF2, B_TB2}) PSC_TRY(release_buf(g, b));
+  if (run->n_rem_dev) {
+    PSC_CUDA(cudaMemcpyAsync(&g->hctr->aux0, run->n_rem_dev, 8, cudaMemcpyDeviceToHost, g->stream));
+    PSC_CUDA(cudaStreamSynchronize(g->stream));
+    run->n_remaining = g->hctr->aux0;
+    run->n_rem_dev = nullptr;
+  }
+  run->done = run->sched ? run->round >= run->rounds : run->cur >= run->n_remaining;
   return PSC_OK;
 }
 

@@ -1884,7 +1884,7 @@ Side make_side(bool backward, uint32_t* vis, int second) {
 
 int records_if_low(psc_graph_s* g, bool backward, const VRec** out) {
   *out = nullptr;
-  if (g->num_graphs || (g->m >> 40)) return PSC_OK;
+  if (g->num_graphs || (g->m >> 40) || g->rec_refused) return PSC_OK;
   PSC_TRY(max_degrees_once(g));
   if (g->max_deg[0] > kRecMaxDeg || g->max_deg[1] > kRecMaxDeg) return PSC_OK;
   return records_once_impl(g, backward, out);

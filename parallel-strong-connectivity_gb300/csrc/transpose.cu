@@ -564,13 +564,6 @@ struct SymEmit {
   }
 };
 
-static void release(psc_graph_s* g, int b) {
-  DevBuf& d = g->bufs[b];
-  if (d.p) cudaFreeAsync(d.p, g->stream);
-  d.p = nullptr;
-  d.bytes = 0;
-}
-
 int build_symmetric(psc_graph_s* g) {
   const uint64_t n = g->n, m = g->m;
   uint64_t* off_s = nullptr;
@@ -605,8 +598,8 @@ int build_symmetric(psc_graph_s* g) {
     PSC_TRY(rs_sort(g, c, passes, v1, k1, pair, r, v, k));
     PSC_TRY(rs_check(g));
     const uint32_t *A = v, *B = k;  // sources, targets
-    release(g, B_AUX3);
-    release(g, B_SCAN2);
+    PSC_TRY(release_buf(g, B_AUX3));
+    PSC_TRY(release_buf(g, B_SCAN2));
     // the kept pairs: sources and targets
     uint32_t *asel = (uint32_t*)pair[0], *bsel = (uint32_t*)pair[1];
     PSC_TRY(scan_emit_flags(g, c, SymKeep{A, B}, SymEmit{A, B, asel, bsel}, &ms, F_TRANSPOSE,
@@ -615,11 +608,11 @@ int build_symmetric(psc_graph_s* g) {
     if (ms) PSC_CUDA(cudaMemcpyAsync(E_s, bsel, ms * 4, cudaMemcpyDeviceToDevice, g->stream));
     PSC_CUDA(cudaMallocAsync((void**)&off_s, (n + 1) * 8, g->stream));
     PSC_TRY(fill_bounds(g, asel, ms, off_s));
-    release(g, B_AUX0);
-    release(g, B_AUX1);
-    release(g, B_AUX2);
-    release(g, B_QA);
-    release(g, B_SCAN3);
+    PSC_TRY(release_buf(g, B_AUX0));
+    PSC_TRY(release_buf(g, B_AUX1));
+    PSC_TRY(release_buf(g, B_AUX2));
+    PSC_TRY(release_buf(g, B_QA));
+    PSC_TRY(release_buf(g, B_SCAN3));
   } else {
     PSC_CUDA(cudaMallocAsync((void**)&E_s, 4, g->stream));
     PSC_CUDA(cudaMallocAsync((void**)&off_s, (n + 1) * 8, g->stream));
