@@ -269,8 +269,15 @@ inline unsigned grid_for(psc_graph_s* g, uint64_t items, unsigned block, unsigne
 // *arrive counts arrivals, *target what it has to reach (one per thread,
 // starting at 0).  The wait is bounded: past kGridSpin polls, or once another
 // block has given up, *failed is set and false is returned to every thread of
-// the block, which then leaves the kernel.
-constexpr uint32_t kGridSpin = 1u << 23;
+// the block, which then leaves the kernel.  A poll takes 0.2 us, so the bound
+// lasts 54 s: work between two barriers is not limited by anything smaller (a level of
+// LE-lists on a dense graph is up to 10^10 offers, and a launch may have a share of the SMs only;
+// 2^23 polls were 1.7 s), and reaching it fails the call.
+constexpr uint32_t kGridSpinDefault = 1u << 28;
+#ifndef PSC_GRID_SPIN
+#define PSC_GRID_SPIN kGridSpinDefault
+#endif
+constexpr uint32_t kGridSpin = PSC_GRID_SPIN;
 
 __device__ __forceinline__ bool grid_barrier(uint32_t* arrive, uint32_t* failed,
                                              uint32_t& target) {
