@@ -383,7 +383,8 @@ __global__ void __launch_bounds__(BLOCK)
 //
 // LOW, for graphs with adjacency records: the expansion of k_reach_async_low with
 // labels (eight lanes per entry, the records in the queue, one trip per hop), its
-// searches cut after kLddWaves waves so that a round lasts as long as its hops.
+// searches cut after kLddWaves waves so that a round lasts as long as its hops (see
+// rec_rules.h for the least number of waves).
 // Device time of connectivity, before -> now: symmetrised kNN 10^6 3.38 -> 0.81
 // ms, kNN 8x10^6 6.96 -> 2.95, grid 2048 x 4000 7.75 -> 2.25, R-MAT 2^24 3.12 ->
 // 1.95.  Cut after 6 / 10 / 16 / 24 waves: kNN 10^6 0.69 / 0.81 / 0.91 / 1.03, the grid
@@ -392,8 +393,6 @@ __global__ void __launch_bounds__(BLOCK)
 constexpr int kLrThreads = 384;
 constexpr int kLrWarps = kLrThreads / 32;
 constexpr int kLrRing = 128;
-constexpr int kLrWave = 12;
-constexpr uint32_t kLddWaves = 10;
 constexpr uint64_t kLddWideEdges = 1 << 18;
 constexpr int kLrCtr = 4;     // counter sets 4-6: three rounds in rotation
 constexpr int kLrState = 10;  // counter sets 10-13
@@ -606,7 +605,7 @@ __global__ void __launch_bounds__(kLrThreads, 1) k_ldd_rounds(LrArgs a) {
       why = LR_DONE;
       break;
     }
-    if (round < a.n_work && round - round0 >= kLrRounds) {
+    if (round - round0 >= (round < a.n_work ? kLrRounds : kLrMaxRounds)) {
       why = LR_PAUSE;
       break;
     }

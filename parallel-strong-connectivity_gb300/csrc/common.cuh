@@ -11,6 +11,7 @@
 
 #include "../../include/psc.h"
 #include "psc_hash.h"
+#include "rec_rules.h"
 #include "scratch.h"
 
 namespace psc {
@@ -462,16 +463,11 @@ __device__ __forceinline__ void warp_expand(WarpExpandSmem& sm, uint64_t beg, ui
 // local search on a graph of low degree loads the record of a candidate
 // alongside its claim, so a hop is one trip to memory instead of two
 // (range, then targets).  Built once per handle and direction.
-constexpr int kRecEdges = 6;
 struct __align__(32) VRec {
   uint64_t hdr;  // beg << 24 | deg
   uint32_t e[kRecEdges];
 };
 static_assert(sizeof(VRec) == 32, "one sector");
-
-// Largest degree of a graph that uses records: nearly all of its vertices have
-// few edges beyond the record.
-constexpr uint64_t kRecMaxDeg = 64;
 
 __device__ __forceinline__ uint64_t adj_hdr(uint64_t beg, uint64_t end) {
   const uint64_t d = end - beg;
