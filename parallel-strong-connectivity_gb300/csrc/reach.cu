@@ -501,22 +501,31 @@ struct __align__(128) AsyncCtl {
   uint32_t fin, flags, marked, pad1[29];
 };
 static_assert(sizeof(AsyncCtl) == 2 * sizeof(Counters), "two counter sets hold it");
+// Counter sets of a launch: the control words of both sides, then their counters.
+constexpr int kAsyncSet = 4, kAsyncSets = 6;
 
-// The slots of up to two sides (kNone behind the starting frontier) and their control
-// words, whose other words are zero.  A side without slots is done from the start.
+// The slots of up to two sides (kNone behind the starting frontier), and the counter sets
+// from kAsyncSet on: zero, with both sides' control words.  A side without a frontier is done
+// from the start.
 __global__ void k_async_prepare(const uint32_t* __restrict__ q0, uint32_t nf0, uint32_t* slot0,
-                                AsyncCtl* c0, const uint32_t* __restrict__ q1, uint32_t nf1,
-                                uint32_t* slot1, AsyncCtl* c1, uint32_t slots) {
+                                const uint32_t* __restrict__ q1, uint32_t nf1, uint32_t* slot1,
+                                uint32_t slots, Counters* ctr) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += stride) {
     slot0[i] = i < nf0 ? __ldg(&q0[i]) : kNone;
     if (slot1) slot1[i] = i < nf1 ? __ldg(&q1[i]) : kNone;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    c0->tail = nf0;
-    c0->flags = nf0 ? 0u : kAsyncDone;
-    c1->tail = nf1;
-    c1->flags = nf1 ? 0u : kAsyncDone;
+  if (blockIdx.x == 0) {
+    unsigned long long* z = (unsigned long long*)(ctr + kAsyncSet);
+    for (uint32_t i = threadIdx.x; i < kAsyncSets * sizeof(Counters) / 8; i += blockDim.x) z[i] = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      AsyncCtl* c = (AsyncCtl*)(ctr + kAsyncSet);
+      c[0].tail = nf0;
+      c[0].flags = nf0 ? 0u : kAsyncDone;
+      c[1].tail = nf1;
+      c[1].flags = nf1 ? 0u : kAsyncDone;
+    }
   }
 }
 
@@ -572,7 +581,8 @@ struct AsyncLink {
     if (lane < take) tk = first + lane;
     v = kNone;
     unsigned got = 0;
-    for (uint32_t spin = 1; !fl; spin++) {
+    // (the tickets' own looks at the flags, 16 polls apart, do not fall together)
+    for (uint32_t spin = 1 + (first & 15u); !fl; spin++) {
       if (tk != kNone && tk < slots) v = slot[tk];
       got = __ballot_sync(kFull, v != kNone);
       if (got) break;
@@ -1844,8 +1854,8 @@ struct Side {
 };
 
 // Counter sets of k_reach_async: the control words of side k, and its counters.
-constexpr int async_ctl_set(int k) { return 4 + 2 * k; }
-constexpr int async_ctr_set(int k) { return 8 + k; }
+constexpr int async_ctl_set(int k) { return kAsyncSet + 2 * k; }
+constexpr int async_ctr_set(int k) { return kAsyncSet + 4 + k; }
 // Slots prepared for one launch (64 MB to clear per side at most).
 constexpr uint64_t kAsyncSlots = 1ull << 24;
 // Rounds of a search with local searches that k_reach_rounds takes.
@@ -2063,7 +2073,6 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         const bool low = g->deg_known && g->max_deg[0] <= kRecMaxDeg && g->max_deg[1] <= kRecMaxDeg;
         if (low) backlog = n;
         if (!vgc_max) backlog = std::min<uint64_t>(backlog, 4 * vgc_limit);
-        PSC_TRY(zero_counters(g));
         ReachSide sd[2] = {};
         bool rec = low;
         AsyncCtl* ctl[2];
@@ -2079,7 +2088,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
           nf[a] = (uint32_t)s.nf;
         }
         k_async_prepare<<<grid_for(g, slots, 256, 4), 256, 0, g->stream>>>(
-            sd[0].qin, nf[0], sd[0].qout, ctl[0], sd[1].qin, nf[1], sd[1].qout, ctl[1], slots);
+            sd[0].qin, nf[0], sd[0].qout, sd[1].qin, nf[1], sd[1].qout, slots, g->ctr);
         if (na == 1) {  // the second side is done from the start
           sd[1] = sd[0];
           sd[1].ctr = g->ctr + async_ctr_set(1);
