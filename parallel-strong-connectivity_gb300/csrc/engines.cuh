@@ -31,6 +31,9 @@ inline unsigned resident_sms(const psc_graph_s* g) {
 // batches by what a solve without records holds), or without memory for them.
 int records_if_low(psc_graph_s* g, bool backward, const VRec** out);
 
+// g->max_deg (largest out- / in-degree), computed once per handle.
+int max_degrees_once(psc_graph_s* g);
+
 // Builds in_off/in_E from off/E on the device (in-lists sorted by source).
 int build_transpose(psc_graph_s* g);
 // Replaces off/E by their symmetrisation on the device (both directions,

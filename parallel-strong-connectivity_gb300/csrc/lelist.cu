@@ -306,6 +306,9 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
   LvGate gate;
   bool pull = false;
   uint32_t level = 0;
+  // whether there are vertices for k_bfs_heavy: asked after four levels that listed none
+  bool hubs = !g->deg_known || g->max_deg[0] > hthr;
+  uint32_t unlisted = 0;
   const bool cluster = !(g->m >> 40) && levels_ready<BfsClaim>(g->device);
   while (nf > 0) {
     const bool want_pull = (nf + nf_edges) >= threshold;
@@ -349,7 +352,7 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
       if (level > 1)
         k_bfs_push<kLeBlock, kLeK><<<grid_for(g, nf, kLeBlock), kLeBlock, 0, g->stream>>>(
             g->off, g->E, qa, nf, dist, level, qb, heavy, hthr, g->ctr);
-      if (level == 1 || nf_edges > hthr)
+      if (level == 1 || (hubs && nf_edges > hthr))
         k_bfs_heavy<kLeBlock, kLeK><<<g->num_sms * 4, kLeBlock, 0, g->stream>>>(
             g->off, g->E, heavy, dist, level, qb, g->ctr);
       std::swap(qa, qb);
@@ -373,6 +376,13 @@ int bfs_run(psc_graph_s* g, uint32_t src, uint32_t* dist, uint32_t* rounds_out) 
     }
     nf = g->hctr[0].next;
     nf_edges = g->hctr[0].next_edges;
+    if (hubs && !pull) {
+      unlisted = g->hctr[0].heavy ? 0 : unlisted + 1;
+      if (unlisted == 4) {
+        PSC_TRY(max_degrees_once(g));
+        hubs = g->max_deg[0] > hthr;
+      }
+    }
   }
   if (rounds_out) *rounds_out = level;
   return PSC_OK;

@@ -1731,43 +1731,6 @@ static void launch_vgc(psc_graph_s* g, unsigned blocks, const ReachSide& a, cons
   }
 }
 
-// Largest out-degree (out[0]) and in-degree (out[1]) of the graph.
-__global__ void k_max_degrees(const uint64_t* __restrict__ off, const uint64_t* __restrict__ in_off,
-                              uint64_t n, unsigned long long* out) {
-  unsigned long long a = 0, b = 0;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
-    const unsigned long long x = off[v + 1] - off[v], y = in_off[v + 1] - in_off[v];
-    a = x > a ? x : a;
-    b = y > b ? y : b;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long x = __shfl_xor_sync(kFull, a, o), y = __shfl_xor_sync(kFull, b, o);
-    a = x > a ? x : a;
-    b = y > b ? y : b;
-  }
-  if (lane_id() == 0) {
-    if (a) atomicMax(&out[0], a);
-    if (b) atomicMax(&out[1], b);
-  }
-}
-
-// Once per handle (the graph does not change): max_deg, for the choice of the
-// search without rounds.
-static int max_degrees_once(psc_graph_s* g) {
-  if (g->deg_known) return PSC_OK;
-  unsigned long long* d = &g->ctr[2].aux0;  // aux0, aux1 of the staging set
-  PSC_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), g->stream));
-  k_max_degrees<<<grid_for(g, g->n, 256), 256, 0, g->stream>>>(g->off, g->in_off, g->n, d);
-  PSC_CUDA(cudaGetLastError());
-  PSC_TRY(read_counters(g));
-  g->max_deg[0] = g->hctr[2].aux0;
-  g->max_deg[1] = g->hctr[2].aux1;
-  g->deg_known = true;
-  return PSC_OK;
-}
-
 // Adjacency records of one direction (see VRec).
 __global__ void k_build_records(const uint64_t* __restrict__ off, const uint32_t* __restrict__ E,
                                 uint64_t n, VRec* rec) {
@@ -1891,6 +1854,43 @@ Side make_side(bool backward, uint32_t* vis, int second) {
 }
 
 }  // namespace
+
+// Largest out-degree (out[0]) and in-degree (out[1]) of the graph.
+__global__ void k_max_degrees(const uint64_t* __restrict__ off, const uint64_t* __restrict__ in_off,
+                              uint64_t n, unsigned long long* out) {
+  unsigned long long a = 0, b = 0;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
+       v += (uint64_t)gridDim.x * blockDim.x) {
+    const unsigned long long x = off[v + 1] - off[v], y = in_off[v + 1] - in_off[v];
+    a = x > a ? x : a;
+    b = y > b ? y : b;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long x = __shfl_xor_sync(kFull, a, o), y = __shfl_xor_sync(kFull, b, o);
+    a = x > a ? x : a;
+    b = y > b ? y : b;
+  }
+  if (lane_id() == 0) {
+    if (a) atomicMax(&out[0], a);
+    if (b) atomicMax(&out[1], b);
+  }
+}
+
+// Once per handle (the graph does not change): max_deg, for the choice of the
+// search without rounds and of the heavy launches of BFS.
+int max_degrees_once(psc_graph_s* g) {
+  if (g->deg_known) return PSC_OK;
+  unsigned long long* d = &g->ctr[2].aux0;  // aux0, aux1 of the staging set
+  PSC_CUDA(cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), g->stream));
+  k_max_degrees<<<grid_for(g, g->n, 256), 256, 0, g->stream>>>(g->off, g->in_off, g->n, d);
+  PSC_CUDA(cudaGetLastError());
+  PSC_TRY(read_counters(g));
+  g->max_deg[0] = g->hctr[2].aux0;
+  g->max_deg[1] = g->hctr[2].aux1;
+  g->deg_known = true;
+  return PSC_OK;
+}
 
 int records_if_low(psc_graph_s* g, bool backward, const VRec** out) {
   *out = nullptr;
