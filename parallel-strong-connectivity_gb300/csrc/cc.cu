@@ -383,8 +383,7 @@ __global__ void __launch_bounds__(BLOCK)
 //
 // LOW, for graphs with adjacency records: the expansion of k_reach_async_low with
 // labels (eight lanes per entry, the records in the queue, one trip per hop), its
-// searches cut after kLddWaves waves so that a round lasts as long as its hops (see
-// rec_rules.h for the least number of waves).
+// searches cut after ldd_waves() waves so that a round lasts as long as its hops.
 // Device time of connectivity, before -> now: symmetrised kNN 10^6 3.38 -> 0.81
 // ms, kNN 8x10^6 6.96 -> 2.95, grid 2048 x 4000 7.75 -> 2.25, R-MAT 2^24 3.12 ->
 // 1.95.  Cut after 6 / 10 / 16 / 24 waves: kNN 10^6 0.69 / 0.81 / 0.91 / 1.03, the grid
@@ -430,6 +429,7 @@ struct LrArgs {
   uint64_t G;
   const uint32_t* work;  // candidate indexes offered in round 1, 2, ... (0 from n_work on)
   uint32_t n_work, round, sampled;
+  uint32_t waves;  // of a search on records (ldd_waves)
   uint64_t nf, nf_edges, threshold;
   Counters* ctr;
   LrState* st;
@@ -457,7 +457,7 @@ __device__ __forceinline__ void ldd_low_round(const LrArgs& a, const uint32_t* q
     }
     uint32_t h = 0, t = cnt;
     __syncwarp();
-    for (uint32_t wave = 0; h != t && wave < kLddWaves; wave++) {
+    for (uint32_t wave = 0; h != t && wave < a.waves; wave++) {
       const uint32_t n = min((uint32_t)kLrWave, t - h);
       // target j of entry 4 k + grp, and the one kRecEdges further on
       uint32_t w[K], old[K], nx[K], lo[K], lab[K], src[K], more = 0;
@@ -1106,6 +1106,7 @@ int ldd_run(psc_graph_s* g, double beta, uint32_t* d_label, uint32_t* tree) {
       a.n_work = (uint32_t)work_of.size();
       a.round = round;
       a.sampled = sampled;
+      a.waves = ldd_waves(std::max(g->max_deg[0], g->max_deg[1]));
       a.nf = nf;
       a.nf_edges = nf_edges;
       a.threshold = threshold;

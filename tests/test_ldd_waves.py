@@ -26,10 +26,12 @@ int main() {
   for (int trial = 0; trial < 50000; trial++) {
     srand(trial);
     const int chunk = 1 + rand() % 32, kind = rand() % 3;
+    const int top = 1 + rand() % (int)kRecMaxDeg;  // the graph's largest degree
+    const uint32_t waves = ldd_waves(top);
     std::deque<std::pair<int, int>> q;
     for (int i = 0; i < chunk; i++)
-      q.push_back({i, kind == 0 ? (int)kRecMaxDeg : kind == 1 ? rand() % (int)(kRecMaxDeg + 1) : rand() % 8});
-    for (uint32_t wave = 0; !q.empty() && wave < kLddWaves; wave++) {
+      q.push_back({i, kind == 0 ? top : kind == 1 ? rand() % (top + 1) : rand() % top % 8});
+    for (uint32_t wave = 0; !q.empty() && wave < waves; wave++) {
       const int n = (int)q.size() < kLrWave ? (int)q.size() : kLrWave;
       std::deque<std::pair<int, int>> back;
       for (int i = 0; i < n; i++) {
@@ -38,7 +40,7 @@ int main() {
         if (e.second > kRecEdges) back.push_back({e.first, e.second - kRecEdges});
       }
       for (int i = rand() % (n * kRecEdges + 1); i > 0 && q.size() < 100; i--)
-        q.push_back({-1, rand() % (int)(kRecMaxDeg + 1)});
+        q.push_back({-1, rand() % (top + 1)});
       q.insert(q.begin(), back.begin(), back.end());
     }
     for (auto& e : q) bad += e.first >= 0 && e.first < kLrWave;
