@@ -76,9 +76,8 @@ struct Counters {
   unsigned long long waves;        // local-search waves of VGC rounds (trace)
   unsigned long long pad[2];
 };
-// sets 0-1: search sides; 2-3: staging; 4-9: the searches without rounds
-// (reach.cu); 4-17: the sub-rounds and the state of the resident multi-search
-// (multisearch.cu)
+// sets 0-1: search sides; 2-3: staging; 4-17: counters and state of the launch at work that
+// runs without the host (searches, multi-search, LDD and LE-list rounds)
 constexpr int kCounterSets = 20;
 
 // ---------------------------------------------------------------------------

@@ -77,10 +77,11 @@ int ms_pair(psc_graph_s* g, const uint32_t* front, uint64_t n_front, uint64_t la
             const uint64_t* labels, const psc_params_t* p, const uint64_t prev_ne[2],
             MsResult out[2], const uint32_t* front_labels = nullptr, uint64_t vgc_max = 0);
 
-// Prefix-doubling batches back to back in one resident launch (k_ms_batches):
-// from the state in *run on, until all centres are done (run->done) or a batch
-// needs more table than the launch has, which is then left to ms_pair
-// untouched (its labels are written only by its partition).
+// Prefix-doubling batches back to back in resident launches (k_ms_batches), with the
+// tables grown between launches: from the state in *run on, until all centres are
+// done (run->done) or a batch is left to ms_pair: a window of more than kMbWindow
+// centres, or no memory for the tables (an interrupted batch has written no label, its
+// partition does that, so it starts again there).
 struct MsRun {
   const uint32_t* centres = nullptr;
   uint64_t n_remaining = 0;  // plain: centres in all

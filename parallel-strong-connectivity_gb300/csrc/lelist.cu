@@ -433,7 +433,9 @@ __global__ void k_le_seed(const uint32_t* __restrict__ centers, uint64_t start, 
 // one 64-bit atomic on ctr->heavy = count << kLeHeavyShift | edge offset, so
 // list order and edge offsets agree: Hs is increasing and entry h owns the
 // virtual edges [Hs[h], Hs[h + 1]).
-constexpr uint64_t kLeHeavy = 128;
+// hthr: kLeHeavy in resident batches, kLeHeavyHost from the host (LE-lists of R-MAT 2^26 290 ms with
+// 128, 279 with 256).
+constexpr uint64_t kLeHeavy = 128, kLeHeavyHost = 256;
 constexpr int kLeHeavyShift = 40;
 constexpr uint32_t kLeProbes = 256;  // probe limit of a sized-by-estimate level
 constexpr uint64_t kLeHeavyMask = (1ull << kLeHeavyShift) - 1;
@@ -469,8 +471,8 @@ __device__ __forceinline__ int le_insert(unsigned long long* T, uint64_t mask, u
 // Once a lane of the warp has failed, the warp stops probing and counts its
 // further offers as failures (the rerun makes them all again).  Called by all
 // 32 lanes.
-// Ls (optional) receives each new pair's table slot.
-template <int K>
+// RES (resident batches): Ls receives each new pair's table slot.
+template <int K, bool RES>
 __device__ __forceinline__ void le_offer(const uint64_t* __restrict__ off, const uint32_t (&w)[K],
                                          const uint64_t (&key)[K], uint32_t level,
                                          unsigned long long* T, uint64_t mask, uint32_t limit,
@@ -487,7 +489,8 @@ __device__ __forceinline__ void le_offer(const uint64_t* __restrict__ off, const
     if (key[k] != kEmpty && full) {
       fails++;
     } else if (key[k] != kEmpty) {
-      const int r = le_insert(T, mask, key[k], limit, &probes, slot[k]);
+      const int r = RES ? le_insert(T, mask, key[k], limit, &probes, slot[k])
+                        : table_insert(T, mask, key[k], limit, &probes);
       if (r == 1) {
         tm |= 1u << k;
         atomicMin(&next_dist[w[k]], level);
@@ -516,7 +519,7 @@ __device__ __forceinline__ void le_offer(const uint64_t* __restrict__ off, const
     if (tm & (1u << k)) {
       Fout[fb++] = key[k];
       Lk[lb] = ((uint64_t)w[k] << 32) | (key[k] >> 32);
-      if (Ls) Ls[lb] = slot[k];
+      if (RES) Ls[lb] = slot[k];
       Ld[lb++] = level;
       next_edges += off[w[k] + 1] - off[w[k]];
     }
@@ -546,7 +549,15 @@ struct LeLevel {
   Counters* ctr;
 };
 
-template <int K>
+// What a level reads beside the graph: written earlier in the same launch when it is a
+// resident one, and then read past L1; else through it (R-MAT 2^26: a fifth of the
+// distance reads hit there).
+template <bool RES, class T>
+__device__ __forceinline__ T le_ld(const T* p) {
+  return RES ? ld_cg(p) : __ldg(p);
+}
+
+template <int K, bool RES>
 __device__ __forceinline__ void le_expand_round(const LeLevel& a, uint32_t chunk,
                                                 WarpExpandSmem& sm, uint32_t* sp, uint64_t gw,
                                                 uint64_t nw) {
@@ -558,11 +569,11 @@ __device__ __forceinline__ void le_expand_round(const LeLevel& a, uint32_t chunk
     uint64_t beg = 0, rem = 0;
     uint32_t p = 0;
     if (lane < chunk && i < a.nf) {
-      const uint64_t key = ld_cg(&a.Fin[i]);
+      const uint64_t key = le_ld<RES>(&a.Fin[i]);
       const uint32_t u = (uint32_t)key;
       p = (uint32_t)(key >> 32);
-      beg = a.off[u];
-      rem = a.off[u + 1] - beg;
+      beg = __ldg(&a.off[u]);
+      rem = __ldg(&a.off[u + 1]) - beg;
       if (rem > a.hthr) {
         const unsigned long long old =
             atomicAdd(&a.ctr->heavy, (1ull << kLeHeavyShift) + (unsigned long long)rem);
@@ -612,10 +623,10 @@ __device__ __forceinline__ void le_expand_round(const LeLevel& a, uint32_t chunk
 #pragma unroll
         for (int k = 0; k < K; k++) {
           key[k] = kEmpty;
-          if (w[k] != kNone && a.level < ld_cg(&a.dist[w[k]]))
+          if (w[k] != kNone && a.level < le_ld<RES>(&a.dist[w[k]]))
             key[k] = ((uint64_t)sp[src[k]] << 32) | w[k];
         }
-        le_offer<K>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld,
+        le_offer<K, RES>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld,
                     a.Ls, a.ctr, probes, fails, next_edges);
       }
       __syncwarp();
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(BLOCK) k_le_expand(LeLevel a) {
   __shared__ uint32_t s_p[BLOCK];
   const unsigned wid = threadIdx.x >> 5;
   const uint64_t nw = (uint64_t)gridDim.x * (BLOCK / 32);
-  le_expand_round<K>(a, le_chunk(a.nf, nw), sm[wid], s_p + wid * 32,
+  le_expand_round<K, false>(a, le_chunk(a.nf, nw), sm[wid], s_p + wid * 32,
                      (uint64_t)blockIdx.x * (BLOCK / 32) + wid, nw);
 }
 
@@ -656,7 +667,7 @@ __global__ void __launch_bounds__(BLOCK) k_le_expand(LeLevel a) {
 // entry's data held warp-uniform; an entry has more than 32 * K edges, so a
 // step spans at most two entries.
 // (warp gw of nw)
-template <int K>
+template <int K, bool RES>
 __device__ __forceinline__ void le_heavy_round(const LeLevel& a, uint64_t gw, uint64_t nw) {
   constexpr uint64_t kStep = 32 * K;
   const unsigned long long packed = __ldcg(&a.ctr->heavy);
@@ -670,23 +681,23 @@ __device__ __forceinline__ void le_heavy_round(const LeLevel& a, uint64_t gw, ui
   uint64_t h = 0, hi = nh - 1;  // last entry with Hs <= x_beg
   while (h < hi) {
     const uint64_t mid = (h + hi + 1) >> 1;
-    if (ld_cg(&a.Hs[mid]) <= x_beg)
+    if (le_ld<RES>(&a.Hs[mid]) <= x_beg)
       h = mid;
     else
       hi = mid - 1;
   }
   // entry h: virtual edges [hs, hn), pair key pk, edge list from eb
-  uint64_t hs = ld_cg(&a.Hs[h]), hn = h + 1 < nh ? ld_cg(&a.Hs[h + 1]) : total;
-  uint64_t pk = ld_cg(&a.Hk[h]), eb = a.off[(uint32_t)pk];
+  uint64_t hs = le_ld<RES>(&a.Hs[h]), hn = h + 1 < nh ? le_ld<RES>(&a.Hs[h + 1]) : total;
+  uint64_t pk = le_ld<RES>(&a.Hk[h]), eb = __ldg(&a.off[(uint32_t)pk]);
   unsigned long long scanned = 0, next_edges = 0;
   uint32_t probes = 0, fails = 0;
   for (uint64_t x0 = x_beg; x0 < x_end; x0 += kStep) {
     const bool nxt = x0 + kStep >= hn && h + 1 < nh;
     uint64_t pk2 = 0, eb2 = 0, hn2 = 0;
     if (nxt) {
-      pk2 = ld_cg(&a.Hk[h + 1]);
-      eb2 = a.off[(uint32_t)pk2];
-      hn2 = h + 2 < nh ? ld_cg(&a.Hs[h + 2]) : total;
+      pk2 = le_ld<RES>(&a.Hk[h + 1]);
+      eb2 = __ldg(&a.off[(uint32_t)pk2]);
+      hn2 = h + 2 < nh ? le_ld<RES>(&a.Hs[h + 2]) : total;
     }
     uint32_t w[K];
     uint64_t key[K];
@@ -699,13 +710,13 @@ __device__ __forceinline__ void le_heavy_round(const LeLevel& a, uint64_t gw, ui
         const bool second = x >= hn;
         const uint32_t v = __ldg(&a.E[second ? eb2 + (x - hn) : eb + (x - hs)]);
         scanned++;
-        if (a.level < ld_cg(&a.dist[v])) {
+        if (a.level < le_ld<RES>(&a.dist[v])) {
           w[k] = v;
           key[k] = ((second ? pk2 : pk) & 0xFFFFFFFF00000000ull) | v;
         }
       }
     }
-    le_offer<K>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld, a.Ls,
+    le_offer<K, RES>(a.off, w, key, a.level, a.T, a.mask, a.limit, a.Fout, a.next_dist, a.Lk, a.Ld, a.Ls,
                 a.ctr, probes, fails, next_edges);
     if (nxt) {
       h++;
@@ -728,8 +739,8 @@ __device__ __forceinline__ void le_heavy_round(const LeLevel& a, uint64_t gw, ui
 }
 
 template <int BLOCK, int K>
-__global__ void __launch_bounds__(BLOCK) k_le_heavy(LeLevel a) {
-  le_heavy_round<K>(a, (uint64_t)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
+__global__ void __launch_bounds__(BLOCK, 1280 / BLOCK) k_le_heavy(LeLevel a) {
+  le_heavy_round<K, false>(a, (uint64_t)blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5),
                     (uint64_t)gridDim.x * (BLOCK / 32));
 }
 
@@ -861,10 +872,10 @@ __global__ void __launch_bounds__(kLbThreads, 1) k_le_batches(LbArgs a) {
       v.Ld = a.Ld + L + ne;
       v.Ls = a.Ls + L + ne;
       v.ctr = c;
-      le_expand_round<K>(v, le_chunk(nf, nw), sh.sm[wid], sh.sp[wid], gw, nw);
+      le_expand_round<K, true>(v, le_chunk(nf, nw), sh.sm[wid], sh.sp[wid], gw, nw);
       if (!barrier()) return;
       if (__ldcg(&c->heavy)) {
-        le_heavy_round<kLeK>(v, gw, nw);
+        le_heavy_round<kLeK, true>(v, gw, nw);
         if (!barrier()) return;
       }
       if (lead) {
@@ -1352,7 +1363,7 @@ int lelist_run(psc_graph_s* g, const uint32_t* centers, double beta, uint64_t* l
       // heavy list: at most bound / (hthr + 1) <= 2^23 entries (count field)
       // over at most bound < 2^40 edges (offset field)
       if (bound >> kLeHeavyShift) return PSC_ERR_CAPACITY;
-      const uint64_t hthr = std::max<uint64_t>(kLeHeavy, bound >> 23);
+      const uint64_t hthr = std::max<uint64_t>(kLeHeavyHost, bound >> 23);
       const bool any_heavy = bound > hthr;
       uint64_t *Hk = nullptr, *Hs = nullptr;
       if (any_heavy) {

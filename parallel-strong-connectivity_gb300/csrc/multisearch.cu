@@ -443,12 +443,13 @@ __device__ __forceinline__ uint32_t ms_vgc_place(uint32_t tm, const uint32_t* w,
 // VGC sub-round for up to two sides: one frontier pair (u, l) per warp.  If
 // 0 < deg(u) < tau the warp runs a local BFS for pivot l inside u's
 // subproblem in a shared-memory queue of tq = min(tau, QCAP) vertices: each
-// wave offers l along the edges of up to 32 queued vertices (one vertex per
-// lane when their degrees are at most K, else the balanced expansion); a new
+// wave offers l along the edges of up to 32 queued vertices (while those have at
+// most 8 out-edges, eight lanes per vertex and up to 4 K vertices, else the
+// balanced expansion over all of them); a new
 // pair stays in the queue while there is room, else spills to the next
 // frontier.  Queued vertices with more than tq out-edges and the queue's
 // remainder spill too.  A queued vertex whose expansion hit a failed insert is
-// re-queued as a pair.
+// re-queued as a pair, and the search ends there.
 // (warp gw of nw, with its own sm and queue Q; kMsK edges in flight per lane)
 template <int kMsK, int QCAP>
 __device__ __forceinline__ void ms_vgc_round(const MsSide& s0, const MsSide& s1,

@@ -13,14 +13,15 @@
 //         spilling the rest to the next frontier — used while the frontier is
 //         small, where rounds, not bandwidth, bound the search.  Steady or
 //         low-degree searches leave the rounds altogether (k_reach_async);
-//   pull: the frontier is a bitmap; each warp owns 32 consecutive unvisited
-//         vertices and scans their in-edges until a frontier bit is found,
-//         then writes the visited / next-frontier words with one store
-//         (the reference's dense_update, no atomics).  Dense rounds stage
-//         each warp's next offsets and visited words in shared memory with
-//         bulk asynchronous copies; once few reachable vertices remain, the
-//         global-memory kernel skips vertices without in-edges (a bitmap per
-//         direction, built once per handle), which no pull can reach.
+//   pull: the frontier is a bitmap; a warp takes 4 to 32 words of the visited
+//         bitmap, lists the vertices that are neither visited nor without
+//         in-edges (a bitmap per direction, built once per handle: no pull can
+//         reach those) in shared memory, and scans the in-edges of the listed
+//         ones until a frontier bit is found; the visited / next-frontier words
+//         are written with one store each (the reference's dense_update).
+// On graphs of up to kRrMaxEdges edges push and pull rounds run in one resident
+// launch instead (k_reach_rounds; its pull rounds take 32 consecutive vertices per
+// warp and know no unreachable ones).
 // The push/pull switch follows the reference's rule (REACH::judge, reach.hpp:86-112):
 // push while frontier vertices + their out-edges < m / pull_div (20).  After a
 // push round the out-edge count is exact (gathered by the kernels); after a

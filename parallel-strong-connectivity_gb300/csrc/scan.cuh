@@ -172,8 +172,9 @@ __global__ void __launch_bounds__(kScanBlock) k_flag_tile_sum(Value value, uint6
 
 // Second pass: every warp takes the tile's 64 flag words, two per lane, and
 // sums them up itself, so an item's place is a word's prefix and a popc: no scan per
-// item and no block barrier, only the writes are left (trim of R-MAT 2^26: 222 -> 94 us; the first pass, with the
-// four offsets of an item loaded together, 250 -> 195).
+// item and no block barrier, only the writes are left.  Trim of R-MAT 2^26: this pass
+// 222 -> 94 us; the first one, with the four offsets of an item loaded together, 250
+// -> 195.
 template <class Emit>
 __global__ void __launch_bounds__(kScanBlock) k_flag_tile_emit(const uint32_t* __restrict__ bits,
                                                                Emit emit, uint64_t n,

@@ -16,9 +16,11 @@ namespace psc {
 // What bounds it is the traffic of the passes (16 bytes per pair and pass), as
 // long as nothing else is read: the histograms of all digits come from one read of
 // the keys, and a pass finds the places of its tiles' digit runs while it runs,
-// by looking back over the tiles before it (decoupled look-back: a tile publishes
-// its digit counts, later their prefix sums), so there is no histogram pass and no
-// scan per digit.  Tiles are numbered by a ticket, so the tiles that one waits for
+// by looking back over the tiles before it (decoupled look-back, after D. Merrill and
+// M. Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016, and
+// its use for radix passes by A. Adinets and D. Merrill, "Onesweep", 2022: a tile
+// publishes its digit counts, later their prefix sums), so there is no histogram pass
+// and no scan per digit.  Tiles are numbered by a ticket, so the tiles that one waits for
 // are running or done; every wait is bounded.  A tile that gives up sets *failed: keys
 // that no pass wrote must not be used as places, so every later kernel of the sort,
 // and the offsets made of it, then writes nothing (k_rs_pass, k_bounds).
