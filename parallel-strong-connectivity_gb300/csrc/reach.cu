@@ -1820,8 +1820,6 @@ struct Side {
 // Counter sets of k_reach_async: the control words of side k, and its counters.
 constexpr int async_ctl_set(int k) { return kAsyncSet + 2 * k; }
 constexpr int async_ctr_set(int k) { return kAsyncSet + 4 + k; }
-// Slots prepared for one launch (64 MB to clear per side at most).
-constexpr uint64_t kAsyncSlots = 1ull << 24;
 // Rounds of a search with local searches that k_reach_rounds takes.
 constexpr uint32_t kRrRounds = 16;
 
@@ -1976,6 +1974,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
   }
   const bool tr = trace_on();
   bool async = local;
+  uint32_t full = 0;  // launches that ended for want of slots
   bool first_launch = start_there;
   for (uint64_t iter = 0;; iter++) {
     if (iter > n + 2) return PSC_ERR_ITER_LIMIT;
@@ -2067,7 +2066,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
         go = g->max_deg[0] <= kRecMaxDeg && g->max_deg[1] <= kRecMaxDeg;
       }
       if (go) {
-        const uint32_t slots = (uint32_t)std::min<uint64_t>(n, kAsyncSlots);
+        const uint32_t slots = async_slots(n, std::max(sides[0].nf, ns > 1 ? sides[1].nf : 0), full);
         // queued vertices whose edges reach the pull threshold, or more than a
         // few rounds' worth of local searches: full-width rounds are faster
         uint64_t backlog = std::max<uint64_t>(threshold * n / std::max<uint64_t>(g->m, 1), 1);
@@ -2123,6 +2122,7 @@ static int reach_sides(psc_graph_s* g, Side* sides, int ns, const uint32_t* srcs
                          c.tail, c.flags);
           if (!(c.flags & kAsyncStop) && c.fin != c.tail) return PSC_ERR_ITER_LIMIT;  // cannot be
           if (c.flags & (kAsyncHeavy | kAsyncWide)) async = false;
+          if (c.flags & kAsyncFull) full++;
           s.rounds++;
           s.prev_nf = s.nf;
           s.nf = k.next;

@@ -60,3 +60,30 @@ def test_taken_vertices_are_not_given_away(replay, low, seed):
     bad, given = map(int, subprocess.run([str(replay), str(low), str(seed)], check=True,
                                          capture_output=True, text=True).stdout.split())
     assert given > 10000 and bad == 0
+
+
+def test_slots(tmp_path):
+    """Room for every frontier that a launch takes, never more than the vertices, and enough
+    after a few launches that ran out."""
+    (tmp_path / "s.cpp").write_text(r'''
+#include <cstdio>
+#include <initializer_list>
+#include "async_rules.h"
+using namespace psc;
+int main() {
+  long bad = 0;
+  for (uint64_t n : {1ull, 7ull, 262144ull, 262145ull, 10000000ull, 1ull << 24, 3000000000ull, 4294967294ull})
+    for (uint64_t f : {0ull, 1ull, 9728ull, 1ull << 20, kAsyncSlots / 4})
+      for (uint32_t full = 0; full < 40; full++) {
+        if (f > n) continue;
+        const uint64_t s = async_slots(n, f, full);
+        bad += s < f || s > n || s > kAsyncSlots;
+        bad += full > 2 && s != (n < kAsyncSlots ? n : kAsyncSlots);
+        bad += full && s < async_slots(n, f, full - 1);
+      }
+  printf("%ld\n", bad);
+}
+''')
+    subprocess.run(["g++", "-std=c++17", f"-I{CSRC}", str(tmp_path / "s.cpp"), "-o",
+                    str(tmp_path / "s")], check=True)
+    assert subprocess.run([str(tmp_path / "s")], check=True, capture_output=True).stdout == b"0\n"
