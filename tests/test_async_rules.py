@@ -67,13 +67,14 @@ def test_slots(tmp_path):
     after a few launches that ran out."""
     (tmp_path / "s.cpp").write_text(r'''
 #include <cstdio>
-#include <initializer_list>
 #include "async_rules.h"
 using namespace psc;
 int main() {
   long bad = 0;
-  for (uint64_t n : {1ull, 7ull, 262144ull, 262145ull, 10000000ull, 1ull << 24, 3000000000ull, 4294967294ull})
-    for (uint64_t f : {0ull, 1ull, 9728ull, 1ull << 20, kAsyncSlots / 4})
+  const uint64_t sizes[] = {1, 7, 262144, 262145, 10000000, 1ull << 24, 3000000000ull, 4294967294ull};
+  const uint64_t fronts[] = {0, 1, 9728, 1ull << 20, kAsyncSlots / 4};
+  for (uint64_t n : sizes)
+    for (uint64_t f : fronts)
       for (uint32_t full = 0; full < 40; full++) {
         if (f > n) continue;
         const uint64_t s = async_slots(n, f, full);
